@@ -15,15 +15,21 @@
 // "L" terms (2^j <= 2^{k-j}) contract x_hi first, "R" terms contract x_lo
 // first.  Every representative is <= its complement, so its top bit is 0 and
 // only the rows x_hi < H1/2 of the iterate and of G exist.  Per iteration:
-//   1. U^T = (AL^T Pw)^T, V = Pw BR      (Pw = |O(x)| p(x) at representatives,
-//                                          0 elsewhere; AL, BR: L / R tables)
-//   2. Q_t = U_t B_m (L), A_j^T V_t (R) -> q parts; fold orbits -> ln q
-//   3. M_t = Lq_t B_m^T (L), N_t = A_j Lq_t (R) -> operands of step 4
+//   1. U = AL^T Pw, V = Pw BR            (Pw = |O(x)| p(x) at representatives,
+//                                          0 elsewhere; AL, BR: tables of the
+//                                          words of length a and b, below)
+//   2. the word transforms of U and V -> shares of acc[y]; fold the orbits -> ln q
+//   3. the word transforms of ln q -> ML, NR
 //   4. G = [AL | NR] [ML ; BR^T] with the BA update as epilogue: D, logW,
 //      exp(logW - shift), the new iterate (in place) and block partials of
 //      max D, sum |O| e, max logW, sum |O| p D
 //   5. one-block finalize: ln Z, mx, upper bound, stop test, next shift.
-// All products run on the FP64 tensor-core path (bdc_mma.cuh).  Counts are
+// The contraction of 1 and 4 runs over the words of one length per half, a =
+// floor(k/2) characters of x_hi and b = k - 1 - a of x_lo (2^a + 2^b of them):
+// occurrences of shorter words are fixed combinations of those of length a
+// (bdc_words.cuh).  With the words of every length up to a and b it had twice
+// the length (190 instead of 96 at n = 24, k = 12).
+// The products run on the FP64 tensor-core path (bdc_mma.cuh).  Counts are
 // exact integers < 2^16 widened to FP64; all sums are FP64.  The tile shape
 // and split of the large products are picked at set-up by timing candidates.
 #include <algorithm>
@@ -40,34 +46,19 @@
 #include "bdc_gemm.cuh"
 #include "bdc_mma.cuh"
 #include "bdc_ozaki.cuh"
+#include "bdc_words.cuh"
 
 namespace bdc {
 
 constexpr int kErrShift = 1;  // DevState::error: exp shift out of range, re-scale
 
-// how the fold reads Q_t: 0 = split slices in qparts, 1 = U^T rows (the
-// identity B of an L term), 2 = V rows (the identity A of an R term); the
-// identity terms of the D side are written by the fold as copies of ln q.
-struct FoldTerm {
-    int kind;
-    int j, m, off;
-    int64_t qoff;   // kind 0: first split slice of Q_t in qparts
-    int qs;         // kind 0: number of split slices
-    int idB_left;   // L term with identity B_m: RB rows [off, off+2^j) = Lq_t
-    int idA_right;  // R term with identity A_j: LA columns [KL+off, +2^m) = Lq_t
-};
-
-struct Term {
-    int j, m;       // split point and the low sub-length k - j
-    int left;       // 1: L term (contract x_hi first), 0: R term
-    int off;        // column offset inside AL (L) or BR (R)
-    int idA, idB;   // A_j / B_m is the identity (j == n1 / m == n2)
-};
-
 // tile configurations of the FP64 tensor-core products (BM x BN, warps WM x WN)
-enum MmaConfig { CFG_128x128 = 0, CFG_128x64, CFG_64x128, CFG_64x64, CFG_128x16, CFG_16x128, CFG_128x32, CFG_COUNT };
-static const int kCfgBM[CFG_COUNT] = {128, 128, 64, 64, 128, 16, 128};
-static const int kCfgBN[CFG_COUNT] = {128, 64, 128, 64, 16, 128, 32};
+enum MmaConfig {
+    CFG_128x128 = 0, CFG_128x64, CFG_64x128, CFG_64x64, CFG_128x16, CFG_16x128, CFG_128x32, CFG_64x32, CFG_32x128,
+    CFG_32x64, CFG_COUNT
+};
+static const int kCfgBM[CFG_COUNT] = {128, 128, 64, 64, 128, 16, 128, 64, 32, 32};
+static const int kCfgBN[CFG_COUNT] = {128, 64, 128, 64, 16, 128, 32, 32, 128, 64};
 
 struct Launch {
     GemmDesc* d = nullptr;   // device descriptors
@@ -77,62 +68,16 @@ struct Launch {
     int grid = 0;            // G only: CTAs launched (0: one per tile; fewer: each loops over tiles)
 };
 
-// q side thin product of one term over a slice [s0, s1) of its contraction:
-//   out[i][w] += sum_s small(s)[i] * wide(s)[w]   (i < SMALL, w < WIDE)
-// with small(s) = small + s * small_stride, wide(s) = wide + s * wide_stride;
-// out element (i, w) at out[i * WIDE + w] (L terms: i = yh, w = yl) or
-// out[w * SMALL + i] (R terms: i = yl, w = yh), i.e. Q_t in flat y order.
-struct ThinQ {
-    const void* small;
-    const void* wide;
-    int64_t small_stride, wide_stride;
-    int small_u16, wide_u16;
-    int SMALL, WIDE;
-    int s0, s1;
-    double* out;
-    int out_trans;
-};
-
-// D side thin product of one term, one output row per table row s:
-//   out[s][i] = sum_w wide(s)[w] * Lq'[w][i]      (i < SMALL, w < WIDE)
-// wide(s) = a half-table row (uint16); Lq'[w][i] = ln q at y = i * WIDE + w
-// (L terms, i = yh) or y = w * SMALL + i (R terms, i = yl); out at
-// out[s * out_s + i * out_i] (RB rows or LA columns).
-struct ThinD {
-    const uint16_t* wide;
-    int64_t wide_stride;
-    int SMALL, WIDE;
-    int rows;
-    int lq_trans;
-    double* out;
-    int64_t out_s, out_i;
-    int cta_begin;
-};
-
-// D side, fused over all terms: one entry per CTA, rows [row0, row0 + the
-// CTA's row count) of one term; IT outputs x RT rows per thread, LPR lanes
-// splitting the contraction
-struct ThinDF {
-    const uint16_t* wide;
-    int64_t wide_stride;
-    int SMALL, WIDE, rows, row0;
-    int lq_trans;
-    double* out;
-    int64_t out_s, out_i;
-    int IT, LPR;
-};
-
 }  // namespace bdc
 
 struct FactoredState {
-    int H1 = 0, H2 = 0, KL = 0, KR = 0, Kp = 0, T = 0;
+    int H1 = 0, H2 = 0, KL = 0, KR = 0, Kp = 0;  // KL = 2^a, KR = 2^b words, Kp = KL + KR padded
     int H1h = 0;              // rows held: x_hi in [row0, row0 + H1h) (all x_hi < H1 / 2 on one GPU)
     int row0 = 0;             // first row held (a shard of the rows over several GPUs; 0 on one GPU)
     int64_t i0 = 0, Rl = 0;   // the representatives in those rows: [i0, i0 + Rl) of the ascending list
     int64_t* d_rowstart = nullptr;  // [H1h + 1]: held row r's representatives are [i0 + rowstart[r], i0 + rowstart[r + 1])
     double* rpart = nullptr;        // [2 H1h]: per-row partials of the load
     int rows_smem = 0;              // dynamic shared memory of the row kernels
-    std::vector<bdc::Term> terms;
     double* Pw = nullptr;     // [2^{n-1}]  |O(x)| e(x) at representatives, 0 elsewhere
     double* Lt = nullptr;     // [2^{n-1}]  ln e(x) (p = e / Z)
     double* hx = nullptr;     // [2^{n-1}]  h(x) at representatives
@@ -143,50 +88,29 @@ struct FactoredState {
     std::vector<int> colmax;  // per dense column: largest x_hi of a representative, -1 if none
     double* LA = nullptr;     // [H1h][Kp]  = [AL | NR]
     double* RB = nullptr;     // [Kp][H2]  = [ML ; BR^T]
-    double* UL = nullptr;     // [H2][KL]  (U^T)
-    double* VR = nullptr;     // [H1h][KR]
-    double* ulpart = nullptr; // [S1][H2][KL]
-    double* vrpart = nullptr; // [S2][H1h][KR]
+    double* ulpart = nullptr; // [S1][KL][H2]   split slices of U
+    double* vrpart = nullptr; // [S2][KR][H1h]  split slices of V, word-major
     int S1 = 1, S2 = 1;
-    double* qparts = nullptr; // split slices of the small q products (FoldTerm::qoff)
-    double* qsum = nullptr;   // [T][2^k]  qparts summed over the splits
-    double* qacc = nullptr;   // [2^k]     sum over the terms
-    // thin per-term products, grouped by the small size (index log2 SMALL)
-    bdc::ThinQ* d_thinq[8] = {};
-    int n_thinq[8] = {};
-    bdc::ThinD* d_thind[8] = {};
-    int n_thind[8] = {}, ctas_thind[8] = {};
-    // the same products on the FP64 tensor-core path, used for the size
-    // classes where the tuner found them faster
-    bdc::Launch mq[8], md[8];
-    bool use_mq[8] = {}, use_md[8] = {};
-    // all per-term products of a side in one launch (used when faster)
-    bdc::ThinQ* d_qf = nullptr;
-    int n_qf = 0, qf_stage = 0;
-    // the fused q side split: terms of fewer than 8 small outputs on k_qthin,
-    // 8 to 64 on the FP64 tensor path (k_qthin_mma), where that times faster
-    bdc::ThinQ *d_ql = nullptr, *d_qm = nullptr;
-    int n_ql = 0, n_qm = 0, ql_stage = 0, qm_stage = 0;
-    bool use_qm = false;
-    bdc::ThinDF* d_df[4] = {};  // by log2 IT
-    int n_df[4] = {};
-    // the terms of 2 to 64 outputs on the FP64 tensor path (k_dthin_mma), in
-    // place of a class of d_df where that times faster
-    bdc::ThinDF* d_dm[4] = {};  // by the class of d_df
-    int n_dm[4] = {}, dm_smem[4] = {};
-    bool use_dm[4] = {};
-    bool use_qf = false, use_df = false;
+    uint8_t* d_ns[2] = {};    // slices of each 16 columns of U, of each 16 rows of V
+    // the word transforms (bdc_words.cuh)
+    bdc::WordPlan plan;
+    bdc::WordPlan* d_plan = nullptr;
+    int words_smem = 0, words_threads = 256;
+    void* d_wtab[2] = {};     // each side's weights, terms and their ranges
+    double* qparts = nullptr; // [plan.ctas][2^k]  shares of acc[y] per transform CTA
+    double* qacc = nullptr;   // [2^k]     a shard's sums
+    int* d_mids = nullptr;    // the fold's middles, one per CTA
+    int n_mids = 0;
     double* lnq_full = nullptr;  // [2^k]
     double* epart = nullptr;  // [ctas][8]
     int ctas_g = 0;
     bdc::OzakiG* oz = nullptr;  // G on the int8 tensor cores (when set up and chosen)
     bool use_oz = false;
     bdc::Launch ul, vr, g;
-    bdc::FoldTerm* d_fold = nullptr;
     int launches_per_iter = 0;
-    // independent thin products run as parallel branches
-    cudaStream_t side[8] = {};
-    cudaEvent_t ev_fork = nullptr, ev_join[8] = {};
+    // V runs on a branch beside U
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // a captured chunk of kGraphIters iterations for the threshold graph_a
     cudaGraphExec_t graph = nullptr;
     double graph_a = 0.0;
@@ -213,7 +137,6 @@ __device__ __forceinline__ bool gated(const DevState* st) { return st && (st->do
 
 enum Stage { ST_QBIG = 0, ST_QSMALL, ST_FOLD, ST_DSMALL, ST_G, ST_FIN, ST_COUNT };
 static cudaError_t enqueue_stage(bdc_handle* H, int stage, double a);
-static cudaError_t enqueue_qthin_split(bdc_handle* H, cudaStream_t s, const DevState* st);
 
 // Dense layout of the iterate: row x_hi, column rev(x_lo) (the low half
 // bit-reversed).  A representative x satisfies x <= rev(x) and x <=
@@ -396,6 +319,9 @@ __global__ void __launch_bounds__(256, (BM * BN <= 4096) ? 3 : 2) k_mma_ba(const
 #define BDC_CFG_ARGS_128x16 128, 16, 8, 1
 #define BDC_CFG_ARGS_16x128 16, 128, 1, 8
 #define BDC_CFG_ARGS_128x32 128, 32, 4, 2
+#define BDC_CFG_ARGS_64x32 64, 32, 4, 2
+#define BDC_CFG_ARGS_32x128 32, 128, 2, 4
+#define BDC_CFG_ARGS_32x64 32, 64, 2, 4
 
 static int cfg_smem(int cfg, int layout = -1) {
 #define CASE_(C, ARGS)                                                                          \
@@ -415,17 +341,18 @@ static int cfg_smem(int cfg, int layout = -1) {
         CASE_(CFG_128x16, BDC_CFG_ARGS_128x16)
         CASE_(CFG_16x128, BDC_CFG_ARGS_16x128)
         CASE_(CFG_128x32, BDC_CFG_ARGS_128x32)
+        CASE_(CFG_64x32, BDC_CFG_ARGS_64x32)
+        CASE_(CFG_32x128, BDC_CFG_ARGS_32x128)
+        CASE_(CFG_32x64, BDC_CFG_ARGS_32x64)
     }
 #undef CASE_
     return 0;
 }
 
 // the cp.async mainloop is instantiated for the layouts the products use:
-// 3 (U: both k-major), 0 (V and the solver's A B^T: both contraction-major)
-static bool cp_instantiated(int cfg, int layout) {
-    const bool big = cfg == CFG_128x128 || cfg == CFG_128x64 || cfg == CFG_64x128 || cfg == CFG_64x64;
-    return big && (layout == 0 || layout == 3);
-}
+// 3 (U: both k-major), 0 (V and the solver's A B^T: both contraction-major);
+// the register-staged one for 64x64 tiles (the solver's odd leading dimensions)
+static bool cp_instantiated(int layout) { return layout == 0 || layout == 3; }
 
 static cudaError_t set_smem_attrs() {
     static bool done = false;
@@ -445,17 +372,17 @@ static cudaError_t set_smem_attrs() {
     SET_K((k_mma_ba<ARGS, true, false>), (mma_smem_bytes<ARGS>()))                               \
     SET_K((k_mma_ba<ARGS, false, true>), (mma_cp_smem_bytes<ARGS, false, true, 3>()))            \
     SET_K((k_mma_ba<ARGS, true, true>), (mma_cp_smem_bytes<ARGS, false, true, 3>()))
-    SET_STORE(BDC_CFG_ARGS_128x128)
-    SET_STORE(BDC_CFG_ARGS_128x64)
-    SET_STORE(BDC_CFG_ARGS_64x128)
     SET_STORE(BDC_CFG_ARGS_64x64)
-    SET_STORE(BDC_CFG_ARGS_128x16)
-    SET_STORE(BDC_CFG_ARGS_16x128)
-    SET_STORE(BDC_CFG_ARGS_128x32)
     SET_STORE_CP(BDC_CFG_ARGS_128x128)
     SET_STORE_CP(BDC_CFG_ARGS_128x64)
     SET_STORE_CP(BDC_CFG_ARGS_64x128)
     SET_STORE_CP(BDC_CFG_ARGS_64x64)
+    SET_STORE_CP(BDC_CFG_ARGS_128x16)
+    SET_STORE_CP(BDC_CFG_ARGS_16x128)
+    SET_STORE_CP(BDC_CFG_ARGS_128x32)
+    SET_STORE_CP(BDC_CFG_ARGS_64x32)
+    SET_STORE_CP(BDC_CFG_ARGS_32x128)
+    SET_STORE_CP(BDC_CFG_ARGS_32x64)
     SET_BA(BDC_CFG_ARGS_128x128)
     SET_BA(BDC_CFG_ARGS_128x64)
     SET_BA(BDC_CFG_ARGS_64x128)
@@ -470,20 +397,29 @@ static cudaError_t set_smem_attrs() {
 
 static cudaError_t launch_store(const Launch& L, cudaStream_t s, const DevState* st) {
     if (L.n == 0 || L.tiles == 0) return cudaSuccess;
-    const int lay = cp_instantiated(L.cfg, L.layout) ? L.layout : -1;
+    const int lay = cp_instantiated(L.layout) ? L.layout : -1;
+    if (lay < 0 && L.cfg != CFG_64x64) return cudaErrorInvalidValue;
     const int sm = cfg_smem(L.cfg, lay);
-#define GO_(ARGS)                                                                                          \
-    if (lay == 0) k_mma_store<ARGS, 0><<<L.tiles, 256, sm, s>>>(L.d, L.map, st);                           \
-    else if (lay == 3) k_mma_store<ARGS, 3><<<L.tiles, 256, sm, s>>>(L.d, L.map, st);                      \
-    else k_mma_store<ARGS, -1><<<L.tiles, 256, sm, s>>>(L.d, L.map, st);
+#define GO_(NAME)                                                                                           \
+    case CFG_##NAME:                                                                                        \
+        if (lay == 0) k_mma_store<BDC_CFG_ARGS_##NAME, 0><<<L.tiles, 256, sm, s>>>(L.d, L.map, st);         \
+        else if (lay == 3) k_mma_store<BDC_CFG_ARGS_##NAME, 3><<<L.tiles, 256, sm, s>>>(L.d, L.map, st);    \
+        break;
+    if (lay < 0) {
+        k_mma_store<BDC_CFG_ARGS_64x64, -1><<<L.tiles, 256, sm, s>>>(L.d, L.map, st);
+        return cudaGetLastError();
+    }
     switch (L.cfg) {
-        case CFG_128x128: GO_(BDC_CFG_ARGS_128x128) break;
-        case CFG_128x64: GO_(BDC_CFG_ARGS_128x64) break;
-        case CFG_64x128: GO_(BDC_CFG_ARGS_64x128) break;
-        case CFG_64x64: GO_(BDC_CFG_ARGS_64x64) break;
-        case CFG_128x16: k_mma_store<BDC_CFG_ARGS_128x16, -1><<<L.tiles, 256, sm, s>>>(L.d, L.map, st); break;
-        case CFG_16x128: k_mma_store<BDC_CFG_ARGS_16x128, -1><<<L.tiles, 256, sm, s>>>(L.d, L.map, st); break;
-        case CFG_128x32: k_mma_store<BDC_CFG_ARGS_128x32, -1><<<L.tiles, 256, sm, s>>>(L.d, L.map, st); break;
+        GO_(128x128)
+        GO_(128x64)
+        GO_(64x128)
+        GO_(64x64)
+        GO_(128x16)
+        GO_(16x128)
+        GO_(128x32)
+        GO_(64x32)
+        GO_(32x128)
+        GO_(32x64)
         default: return cudaErrorInvalidValue;
     }
 #undef GO_
@@ -512,761 +448,7 @@ static cudaError_t launch_ba(const Launch& L, const BaEpilogue& ep, cudaStream_t
     return cudaGetLastError();
 }
 
-// ------------------------------------------------------ thin products
-__device__ __forceinline__ double ld_val(const void* p, int u16, int64_t i) {
-    return u16 ? (double)__ldg((const uint16_t*)p + i) : __ldg((const double*)p + i);
-}
-
-// q side: CTA = (descriptor, block of 256 wide indices); blockDim 256.  The
-// small side of a chunk of 64 rows is staged in shared memory and broadcast;
-// each thread streams its wide column (coalesced across the warp) with 8 row
-// loads in flight.  When WIDE < 256 the spare threads take every
-// (256 / WIDE)-th row and the partial sums are added in shared memory.
-template <int SMALL>
-__global__ void __launch_bounds__(256) k_thin_q(const ThinQ* __restrict__ descs, int nblk, const DevState* st) {
-    if (gated(st)) return;
-    const ThinQ& d = descs[blockIdx.x / nblk];
-    const int wb = blockIdx.x % nblk;
-    const int lanes_w = d.WIDE < 256 ? d.WIDE : 256;  // threads along w
-    const int rows_par = 256 / lanes_w;               // threads along s
-    const int tw = threadIdx.x % lanes_w, ts = threadIdx.x / lanes_w;
-    const int w = wb * 256 + tw;
-    const bool active = (w < d.WIDE) && (ts < rows_par);
-    constexpr int CH = 64, U = 8;
-    __shared__ double sm[CH][SMALL];
-    double acc[SMALL];
-#pragma unroll
-    for (int i = 0; i < SMALL; ++i) acc[i] = 0.0;
-    for (int c0 = d.s0; c0 < d.s1; c0 += CH) {
-        const int nrow = min(CH, d.s1 - c0);
-        __syncthreads();
-        for (int e = threadIdx.x; e < CH * SMALL; e += 256) {
-            const int r = e / SMALL, i = e % SMALL;
-            sm[r][i] = (r < nrow) ? ld_val(d.small, d.small_u16, (int64_t)(c0 + r) * d.small_stride + i) : 0.0;
-        }
-        __syncthreads();
-        if (active) {
-            for (int r0 = ts; r0 < nrow; r0 += rows_par * U) {
-                double wv[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int r = r0 + u * rows_par;
-                    wv[u] = (r < nrow) ? ld_val(d.wide, d.wide_u16, (int64_t)(c0 + r) * d.wide_stride + w) : 0.0;
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int r = min(r0 + u * rows_par, CH - 1);  // rows past nrow carry weight 0
-#pragma unroll
-                    for (int i = 0; i < SMALL; ++i) acc[i] = fma(sm[r][i], wv[u], acc[i]);
-                }
-            }
-        }
-    }
-    if (rows_par > 1) {
-        // add the rows_par partial sums of each w (fixed order)
-        __shared__ double red[256];
-        for (int i = 0; i < SMALL; ++i) {
-            __syncthreads();
-            red[threadIdx.x] = active ? acc[i] : 0.0;
-            __syncthreads();
-            if (ts == 0 && w < d.WIDE) {
-                double a = 0.0;
-                for (int q = 0; q < rows_par; ++q) a += red[q * lanes_w + tw];
-                acc[i] = a;
-            }
-        }
-        if (ts != 0) return;
-    }
-    if (w >= d.WIDE) return;
-#pragma unroll
-    for (int i = 0; i < SMALL; ++i) {
-        if (d.out_trans) d.out[(int64_t)w * SMALL + i] = acc[i];
-        else d.out[(int64_t)i * d.WIDE + w] = acc[i];
-    }
-}
-
-// D side: CTA = 16 table rows of one descriptor (64 threads, 4 lanes per
-// row); ln q of the term is staged in shared memory as Lq'[w][i] and read
-// with broadcasts while each lane walks a quarter of its row in 16-byte
-// pieces, two in flight; the 4 partial sums of a row are added by shuffles.
-constexpr int kThinDRows = 16;
-
-template <int SMALL>
-__global__ void __launch_bounds__(64) k_thin_d(const ThinD* __restrict__ descs, int nd,
-                                               const double* __restrict__ lnq_full, const DevState* st) {
-    if (gated(st)) return;
-    int lo = 0, hi = nd - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (descs[mid].cta_begin <= (int)blockIdx.x) lo = mid;
-        else hi = mid - 1;
-    }
-    const ThinD& d = descs[lo];
-    const int q = threadIdx.x & 3;
-    const int row = (blockIdx.x - d.cta_begin) * kThinDRows + (threadIdx.x >> 2);
-    extern __shared__ double lqs[];  // [WIDE][SMALL]
-    const int ny = SMALL * d.WIDE;
-    for (int e = threadIdx.x; e < ny; e += 64) {
-        const int w = e / SMALL, i = e % SMALL;
-        lqs[e] = d.lq_trans ? lnq_full[w * SMALL + i] : lnq_full[i * d.WIDE + w];
-    }
-    __syncthreads();
-    const bool live = row < d.rows;
-    double acc[SMALL];
-#pragma unroll
-    for (int i = 0; i < SMALL; ++i) acc[i] = 0.0;
-    const uint16_t* v = d.wide + (int64_t)(live ? row : 0) * d.wide_stride;
-    if (live && (d.WIDE & 31) == 0 && ((uintptr_t)v & 15) == 0) {
-        // lane q takes the 8-entry pieces q, q + 4, q + 8, ...
-        for (int w0 = q * 8; w0 < d.WIDE; w0 += 64) {
-            uint4 pc[2];
-            pc[0] = __ldg(reinterpret_cast<const uint4*>(v + w0));
-            pc[1] = (w0 + 32 < d.WIDE) ? __ldg(reinterpret_cast<const uint4*>(v + w0 + 32)) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t pk[4] = {pc[h].x, pc[h].y, pc[h].z, pc[h].w};
-                const int wb = w0 + 32 * h;
-                if (wb >= d.WIDE) break;
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const double wv = (double)((pk[u >> 1] >> (16 * (u & 1))) & 0xFFFFu);
-                    const double* lr = lqs + (wb + u) * SMALL;
-#pragma unroll
-                    for (int i = 0; i < SMALL; ++i) acc[i] = fma(wv, lr[i], acc[i]);
-                }
-            }
-        }
-    } else if (live) {
-        for (int w = q; w < d.WIDE; w += 4) {
-            const double wv = (double)(__ldg(v + w));
-            const double* lr = lqs + w * SMALL;
-#pragma unroll
-            for (int i = 0; i < SMALL; ++i) acc[i] = fma(wv, lr[i], acc[i]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < SMALL; ++i) {
-        acc[i] += __shfl_xor_sync(0xFFFFFFFFu, acc[i], 1);
-        acc[i] += __shfl_xor_sync(0xFFFFFFFFu, acc[i], 2);
-    }
-    if (!live || q != 0) return;
-    double* o = d.out + (int64_t)row * d.out_s;
-#pragma unroll
-    for (int i = 0; i < SMALL; ++i) o[(int64_t)i * d.out_i] = acc[i];
-}
-
-static cudaError_t launch_thin_q(int lg, const ThinQ* d, int n, int ny, cudaStream_t s, const DevState* st) {
-    const int small = 1 << lg, wide = ny / small;
-    const int nblk = (wide + 255) / 256;
-    const int grid = n * nblk;
-    switch (lg) {
-        case 0: k_thin_q<1><<<grid, 256, 0, s>>>(d, nblk, st); break;
-        case 1: k_thin_q<2><<<grid, 256, 0, s>>>(d, nblk, st); break;
-        case 2: k_thin_q<4><<<grid, 256, 0, s>>>(d, nblk, st); break;
-        case 3: k_thin_q<8><<<grid, 256, 0, s>>>(d, nblk, st); break;
-        case 4: k_thin_q<16><<<grid, 256, 0, s>>>(d, nblk, st); break;
-        case 5: k_thin_q<32><<<grid, 256, 0, s>>>(d, nblk, st); break;
-        case 6: k_thin_q<64><<<grid, 256, 0, s>>>(d, nblk, st); break;
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
-}
-
-static cudaError_t launch_thin_d(int lg, const ThinD* d, int n, int ctas, int ny, const double* lnq_full,
-                                 cudaStream_t s, const DevState* st) {
-    const size_t sm = sizeof(double) * ny;
-    switch (lg) {
-        case 0: k_thin_d<1><<<ctas, 64, sm, s>>>(d, n, lnq_full, st); break;
-        case 1: k_thin_d<2><<<ctas, 64, sm, s>>>(d, n, lnq_full, st); break;
-        case 2: k_thin_d<4><<<ctas, 64, sm, s>>>(d, n, lnq_full, st); break;
-        case 3: k_thin_d<8><<<ctas, 64, sm, s>>>(d, n, lnq_full, st); break;
-        case 4: k_thin_d<16><<<ctas, 64, sm, s>>>(d, n, lnq_full, st); break;
-        case 5: k_thin_d<32><<<ctas, 64, sm, s>>>(d, n, lnq_full, st); break;
-        case 6: k_thin_d<64><<<ctas, 64, sm, s>>>(d, n, lnq_full, st); break;
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
-}
-
-// q side, every term and slice in one launch: CTA = one ThinQ entry (a term
-// and a slice [s0, s1) of its contraction), 2^k / 16 threads, each owning IT
-// (1 or 2) small indices x 16 / IT consecutive wide indices, the latter read
-// as 16-byte pieces of the table row; 16 FP64 FMAs per row and thread.
-__device__ __forceinline__ void unpack2(const uint32_t p, double* v) {
-    v[0] = (double)(p & 0xFFFFu);
-    v[1] = (double)(p >> 16);
-}
-
-__device__ __forceinline__ void unpack8(const uint4 p, double* v) {
-    unpack2(p.x, v);
-    unpack2(p.y, v + 2);
-    unpack2(p.z, v + 4);
-    unpack2(p.w, v + 6);
-}
-
-// The slice's rows stream through shared memory with cp.async, kQtRows rows a
-// stage and kQtStages stages in flight (the table rows are 16-byte pieces,
-// the small rows 8-byte ones since their stride is odd), so that the CTA keeps
-// tens of kilobytes of loads outstanding without holding them in registers.
-constexpr int kQtRows = 8;
-constexpr int kQtStages = 3;
-
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem));
-}
-
-// small indices a thread covers: up to 8, so that each table entry it
-// converts feeds up to 8 FMAs; the thread's 16 outputs are IT small x 16 / IT
-// wide indices
-__host__ __device__ constexpr int qthin_it(int SMALL) { return SMALL < 8 ? SMALL : 8; }
-
-// the WT = 16 / IT table entries of a thread in one staged row
-template <int WT>
-__device__ __forceinline__ void qthin_entries(const uint8_t* p, double (&v)[WT]) {
-    if constexpr (WT == 16) {
-        const uint4* q = reinterpret_cast<const uint4*>(p);
-        unpack8(q[0], v);
-        unpack8(q[1], v + 8);
-    } else if constexpr (WT == 8) {
-        unpack8(*reinterpret_cast<const uint4*>(p), v);
-    } else if constexpr (WT == 4) {
-        const uint2 q = *reinterpret_cast<const uint2*>(p);
-        unpack2(q.x, v);
-        unpack2(q.y, v + 2);
-    } else {
-        unpack2(*reinterpret_cast<const uint32_t*>(p), v);
-    }
-}
-
-template <int IT>
-__device__ __forceinline__ void qthin_run(const ThinQ& q, int stage_bytes, uint8_t* qsm) {
-    constexpr int WT = 16 / IT;
-    const int nwb = q.WIDE / WT;
-    const int tid = threadIdx.x;
-    const int wb = tid % nwb, ib = tid / nwb;
-    const int i0 = ib * IT, w0 = wb * WT;
-    const uint16_t* wide = (const uint16_t*)q.wide;
-    const double* small = (const double*)q.small;
-    const int wpieces = q.WIDE / 8;              // 16-byte pieces per table row
-    const int wbytes = q.WIDE * 2, sbytes = q.SMALL * 8;
-    const int rows = q.s1 - q.s0;
-    const int nst = (rows + kQtRows - 1) / kQtRows;
-    auto issue = [&](int stg) {
-        uint8_t* base = qsm + (stg % kQtStages) * stage_bytes;
-        const int r0 = q.s0 + stg * kQtRows;
-        const int nr = min(kQtRows, q.s1 - r0);
-        for (int e = tid; e < nr * wpieces; e += blockDim.x) {
-            const int r = e / wpieces, c = e % wpieces;
-            cp_async16(base + r * wbytes + c * 16, wide + (int64_t)(r0 + r) * q.wide_stride + c * 8, 16);
-        }
-        uint8_t* sb = base + kQtRows * wbytes;
-        for (int e = tid; e < nr * q.SMALL; e += blockDim.x) {
-            const int r = e / q.SMALL, c = e % q.SMALL;
-            cp_async8(sb + r * sbytes + c * 8, small + (int64_t)(r0 + r) * q.small_stride + c);
-        }
-    };
-    double acc[16];
-#pragma unroll
-    for (int e = 0; e < 16; ++e) acc[e] = 0.0;
-#pragma unroll
-    for (int p = 0; p < kQtStages - 1; ++p) {
-        if (p < nst) issue(p);
-        cp_async_commit();
-    }
-    for (int stg = 0; stg < nst; ++stg) {
-        cp_async_wait<kQtStages - 2>();
-        __syncthreads();
-        if (stg + kQtStages - 1 < nst) issue(stg + kQtStages - 1);
-        cp_async_commit();
-        const uint8_t* base = qsm + (stg % kQtStages) * stage_bytes;
-        const double* sb = reinterpret_cast<const double*>(base + kQtRows * wbytes);
-        const int nr = min(kQtRows, q.s1 - (q.s0 + stg * kQtRows));
-        if (i0 < q.SMALL) {
-            for (int r = 0; r < nr; ++r) {
-                double v[WT], av[IT];
-                qthin_entries<WT>(base + r * wbytes + w0 * 2, v);
-                // the IT small values in 16-byte pieces (i0 is a multiple of IT)
-                if constexpr (IT >= 2) {
-#pragma unroll
-                    for (int t = 0; t < IT; t += 2) {
-                        const double2 a2 = *reinterpret_cast<const double2*>(sb + r * q.SMALL + i0 + t);
-                        av[t] = a2.x;
-                        av[t + 1] = a2.y;
-                    }
-                } else {
-                    av[0] = sb[r * q.SMALL + i0];
-                }
-#pragma unroll
-                for (int t = 0; t < IT; ++t)
-#pragma unroll
-                    for (int e = 0; e < WT; ++e) acc[t * WT + e] = fma(av[t], v[e], acc[t * WT + e]);
-            }
-        }
-    }
-    cp_async_wait<0>();
-    if (i0 >= q.SMALL) return;
-#pragma unroll
-    for (int e = 0; e < 16; ++e) {
-        const int i = i0 + e / WT, w = w0 + e % WT;
-        if (q.out_trans) q.out[(int64_t)w * q.SMALL + i] = acc[e];
-        else q.out[(int64_t)i * q.WIDE + w] = acc[e];
-    }
-}
-
-__global__ void __launch_bounds__(256) k_qthin(const ThinQ* __restrict__ descs, int stage_bytes, const DevState* st) {
-    if (gated(st)) return;
-    extern __shared__ __align__(16) uint8_t qsm[];
-    const ThinQ& q = descs[blockIdx.x];
-    switch (qthin_it(q.SMALL)) {
-        case 1: qthin_run<1>(q, stage_bytes, qsm); break;
-        case 2: qthin_run<2>(q, stage_bytes, qsm); break;
-        case 4: qthin_run<4>(q, stage_bytes, qsm); break;
-        default: qthin_run<8>(q, stage_bytes, qsm); break;
-    }
-}
-
-// D side, every term in one launch: CTA = one ThinDF entry.  Lq' of the term
-// is staged in shared memory in chunks of 8 contraction indices padded by
-// one double (so that lanes 8 indices apart fall on different banks); each
-// thread accumulates RT rows x IT outputs over its lane's share of the
-// contraction, reading 8 table entries per row at a time, and the LPR lanes
-// of a row group add their partial sums by shuffles.
-constexpr int kDfRT = 4;
-
-template <int IT>
-__global__ void __launch_bounds__(256) k_dthin(const ThinDF* __restrict__ descs, const double* __restrict__ lnq_full,
-                                               const DevState* st) {
-    if (gated(st)) return;
-    extern __shared__ double lq[];
-    const ThinDF& t = descs[blockIdx.x];
-    const int SMALL = t.SMALL, WIDE = t.WIDE;
-    const int cs = 8 * SMALL + 1;  // padded chunk of 8 contraction indices
-    // eight loads per thread in flight, then their stores
-    for (int e0 = threadIdx.x; e0 < SMALL * WIDE; e0 += 8 * blockDim.x) {
-        double v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int e = e0 + u * (int)blockDim.x, w = e / SMALL, i = e % SMALL;
-            v[u] = (e < SMALL * WIDE) ? (t.lq_trans ? __ldg(lnq_full + w * SMALL + i) : __ldg(lnq_full + i * WIDE + w))
-                                      : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int e = e0 + u * (int)blockDim.x, w = e / SMALL, i = e % SMALL;
-            if (e < SMALL * WIDE) lq[(w >> 3) * cs + (w & 7) * SMALL + i] = v[u];
-        }
-    }
-    __syncthreads();
-    const int LPR = t.LPR;
-    const int lane = threadIdx.x % LPR, rest = threadIdx.x / LPR;
-    const int ng = SMALL / IT;
-    const int ig = rest % ng, rg = rest / ng;
-    const int r0 = t.row0 + rg * kDfRT;
-    const int i0 = ig * IT;
-    double acc[kDfRT][IT];
-#pragma unroll
-    for (int r = 0; r < kDfRT; ++r)
-#pragma unroll
-        for (int i = 0; i < IT; ++i) acc[r][i] = 0.0;
-    const uint16_t* rowp[kDfRT];
-#pragma unroll
-    for (int r = 0; r < kDfRT; ++r) rowp[r] = t.wide + (int64_t)min(r0 + r, t.rows - 1) * t.wide_stride;
-    // two chunks of 8 contraction indices per step: both chunks' table loads
-    // are issued before either is used
-    const int step = LPR * 8;
-    for (int w8 = lane * 8; w8 < WIDE; w8 += 2 * step) {
-        const bool two = w8 + step < WIDE;
-        uint32_t pk[2][kDfRT][4];
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int r = 0; r < kDfRT; ++r) {
-                const uint4 q = (c == 0 || two) ? __ldg(reinterpret_cast<const uint4*>(rowp[r] + w8 + c * step))
-                                                : make_uint4(0u, 0u, 0u, 0u);
-                pk[c][r][0] = q.x;
-                pk[c][r][1] = q.y;
-                pk[c][r][2] = q.z;
-                pk[c][r][3] = q.w;
-            }
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            if (c == 1 && !two) break;
-            const double* lc = lq + ((w8 + c * step) >> 3) * cs + i0;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                double v[kDfRT];
-#pragma unroll
-                for (int r = 0; r < kDfRT; ++r) v[r] = (double)((pk[c][r][u >> 1] >> (16 * (u & 1))) & 0xFFFFu);
-#pragma unroll
-                for (int i = 0; i < IT; ++i) {
-                    const double l = lc[u * SMALL + i];
-#pragma unroll
-                    for (int r = 0; r < kDfRT; ++r) acc[r][i] = fma(v[r], l, acc[r][i]);
-                }
-            }
-        }
-    }
-    for (int o = LPR >> 1; o > 0; o >>= 1)
-#pragma unroll
-        for (int r = 0; r < kDfRT; ++r)
-#pragma unroll
-            for (int i = 0; i < IT; ++i) acc[r][i] += __shfl_xor_sync(0xFFFFFFFFu, acc[r][i], o);
-    if (lane != 0) return;
-#pragma unroll
-    for (int r = 0; r < kDfRT; ++r) {
-        if (r0 + r >= t.rows) break;
-#pragma unroll
-        for (int i = 0; i < IT; ++i) t.out[(int64_t)(r0 + r) * t.out_s + (int64_t)(i0 + i) * t.out_i] = acc[r][i];
-    }
-}
-
-// D side on the FP64 tensor path, for the terms of 2 to 64 outputs: CTA =
-// one ThinDF entry of kDmRows table rows, warp w = rows 8w .. 8w + 7, all
-// SMALL outputs as SMALL / 8 mma.sync m8n8k4 tiles (one tile, zero-padded,
-// below 8).  Lq' of the term sits in
-// shared memory at row pitch SMALL + 2 (the four row groups of a B fragment
-// land 8 doubles apart: two wavefronts, the minimum for 256 bytes); the
-// table rows stream through two buffers of kDmChunk entries with cp.async
-// (row pitch kDmPitch entries: 16-byte aligned, rows 4 banks apart).  Within
-// each 16 contraction indices, k-step j of lane column q takes index 4q + j,
-// so that a lane's four A entries are one 8-byte load (A and B use the same
-// order, and the sum does not depend on it).
-constexpr int kDmRows = 64;
-constexpr int kDmChunk = 64;
-constexpr int kDmPitch = 72;
-
-// Lq' row pitch; terms of 2 or 4 outputs use one 8-wide tile, zero-padded
-__host__ __device__ constexpr int dmma_ld(int SMALL) { return (SMALL < 8 ? 8 : SMALL) + 2; }
-static int dthin_mma_smem(int SMALL, int WIDE) {
-    return (int)sizeof(double) * WIDE * dmma_ld(SMALL) + 2 * kDmRows * kDmPitch * (int)sizeof(uint16_t);
-}
-
-template <int NB>
-__device__ __forceinline__ void dthin_mma_run(const ThinDF& t, const double* __restrict__ lnq_full, double* dsm) {
-    const int SMALL = t.SMALL, WIDE = t.WIDE, ld = dmma_ld(SMALL);
-    double* L = dsm;                                         // [WIDE][ld]
-    uint16_t* T = reinterpret_cast<uint16_t*>(dsm + WIDE * ld);  // [2][kDmRows][kDmPitch]
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int gr = lane >> 2, q = lane & 3;
-    auto issue = [&](int c) {
-        uint16_t* buf = T + (c & 1) * kDmRows * kDmPitch;
-        for (int e = tid; e < kDmRows * (kDmChunk / 8); e += 256) {
-            const int r = e / (kDmChunk / 8), piece = e % (kDmChunk / 8);
-            const int row = min(t.row0 + r, t.rows - 1);
-            cp_async16(buf + r * kDmPitch + piece * 8, t.wide + (int64_t)row * t.wide_stride + c * kDmChunk + piece * 8,
-                       16);
-        }
-    };
-    const int nch = WIDE / kDmChunk;
-    // Lq' by 8-byte asynchronous copies in the first chunk's group (all of a
-    // thread's copies in flight at once), zeros past SMALL by plain stores
-    const int SP = NB * 8;  // outputs of the tiles: SMALL, or 8 with zeros past SMALL
-    for (int e = tid; e < SP * WIDE; e += 256) {
-        const int w = e / SP, i = e % SP;
-        if (i >= SMALL) L[w * ld + i] = 0.0;
-        else cp_async8(L + w * ld + i, t.lq_trans ? lnq_full + w * SMALL + i : lnq_full + i * WIDE + w);
-    }
-    issue(0);
-    cp_async_commit();
-    double acc[NB][2];
-#pragma unroll
-    for (int nb = 0; nb < NB; ++nb) acc[nb][0] = acc[nb][1] = 0.0;
-    for (int c = 0; c < nch; ++c) {
-        if (c + 1 < nch) issue(c + 1);
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        const uint16_t* arow = T + (c & 1) * kDmRows * kDmPitch + (warp * 8 + gr) * kDmPitch;
-#pragma unroll
-        for (int ks = 0; ks < kDmChunk / 16; ++ks) {
-            const uint2 pk = *reinterpret_cast<const uint2*>(arow + ks * 16 + 4 * q);
-            const double av[4] = {(double)(pk.x & 0xFFFFu), (double)(pk.x >> 16), (double)(pk.y & 0xFFFFu),
-                                  (double)(pk.y >> 16)};
-            const double* lrow = L + (c * kDmChunk + ks * 16 + 4 * q) * ld + gr;
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-#pragma unroll
-                for (int nb = 0; nb < NB; ++nb) mma_f64(acc[nb][0], acc[nb][1], av[j], lrow[j * ld + nb * 8]);
-        }
-        __syncthreads();  // the buffer is free for chunk c + 2
-    }
-    const int row = t.row0 + warp * 8 + gr;
-    if (row >= t.rows) return;
-#pragma unroll
-    for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int i = nb * 8 + 2 * q + h;
-            if (i < SMALL) t.out[(int64_t)row * t.out_s + (int64_t)i * t.out_i] = acc[nb][h];
-        }
-}
-
-__global__ void __launch_bounds__(256) k_dthin_mma(const ThinDF* __restrict__ descs, const double* __restrict__ lnq_full,
-                                                   const DevState* st) {
-    if (gated(st)) return;
-    extern __shared__ __align__(16) double dmsm[];
-    const ThinDF& t = descs[blockIdx.x];
-    switch (t.SMALL) {
-        case 2:
-        case 4:
-        case 8: dthin_mma_run<1>(t, lnq_full, dmsm); break;
-        case 16: dthin_mma_run<2>(t, lnq_full, dmsm); break;
-        case 32: dthin_mma_run<4>(t, lnq_full, dmsm); break;
-        default: dthin_mma_run<8>(t, lnq_full, dmsm); break;
-    }
-}
-
-// q side on the FP64 tensor path, for the terms of 8 to 64 small outputs
-// at 2^k = 4096 outputs per term: CTA = one ThinQ slice [s0, s1) of the
-// contraction, producing the term's SMALL x WIDE partial product.  Warp w
-// owns small tile ti (8 outputs i) and 64 wide outputs from c0 as eight
-// mma.sync m8n8k4 tiles; tile u's column n stands for w = c0 + 8n + u, so a
-// lane's B entries of one row (n = lane / 4, all u) are 8 adjacent table
-// entries, one 16-byte load.  Rows stream through two buffers of kQmRows
-// (table rows at pitch WIDE, small rows at pitch SMALL + 8: two wavefronts
-// for the four rows of an A fragment); rows past s1 read zero small values.
-constexpr int kQmRows = 32;
-
-__host__ __device__ constexpr int qmma_ld(int SMALL) { return SMALL >= 16 ? SMALL + 8 : SMALL; }
-__host__ __device__ constexpr int qmma_stage(int SMALL, int WIDE) {
-    return kQmRows * (qmma_ld(SMALL) * 8 + WIDE * 2);
-}
-
-__global__ void __launch_bounds__(256) k_qthin_mma(const ThinQ* __restrict__ descs, int stage_bytes,
-                                                   const DevState* st) {
-    if (gated(st)) return;
-    extern __shared__ __align__(16) uint8_t qmsm[];
-    const ThinQ& q = descs[blockIdx.x];
-    const int SMALL = q.SMALL, WIDE = q.WIDE, lds = qmma_ld(SMALL);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int gr = lane >> 2, qq = lane & 3;
-    const int groups = WIDE / 64;  // 64-column groups
-    const int ti = warp / groups, c0 = (warp % groups) * 64;
-    const uint16_t* wide = (const uint16_t*)q.wide;
-    const double* small = (const double*)q.small;
-    const int rows = q.s1 - q.s0;
-    const int nst = (rows + kQmRows - 1) / kQmRows;
-    auto issue = [&](int stg) {
-        uint8_t* base = qmsm + (stg & 1) * stage_bytes;
-        const int r0 = q.s0 + stg * kQmRows;
-        const int nr = min(kQmRows, q.s1 - r0);
-        const int wpieces = WIDE / 8;
-        for (int e = tid; e < nr * wpieces; e += 256) {
-            const int r = e / wpieces, c = e % wpieces;
-            cp_async16(base + r * WIDE * 2 + c * 16, wide + (int64_t)(r0 + r) * q.wide_stride + c * 8, 16);
-        }
-        double* sb = reinterpret_cast<double*>(base + kQmRows * WIDE * 2);
-        for (int e = tid; e < kQmRows * SMALL; e += 256) {
-            const int r = e / SMALL, c = e % SMALL;
-            if (r < nr) cp_async8(sb + r * lds + c, small + (int64_t)(r0 + r) * q.small_stride + c);
-            else sb[r * lds + c] = 0.0;  // rows past the slice contribute nothing
-        }
-    };
-    double acc[8][2];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) acc[u][0] = acc[u][1] = 0.0;
-    issue(0);
-    cp_async_commit();
-    for (int stg = 0; stg < nst; ++stg) {
-        if (stg + 1 < nst) issue(stg + 1);
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        const uint8_t* base = qmsm + (stg & 1) * stage_bytes;
-        const uint16_t* tb = reinterpret_cast<const uint16_t*>(base);
-        const double* sb = reinterpret_cast<const double*>(base + kQmRows * WIDE * 2);
-#pragma unroll 2
-        for (int ks = 0; ks < kQmRows / 4; ++ks) {
-            const int r = ks * 4 + qq;  // the contraction row of this lane's k index
-            const double a = sb[r * lds + ti * 8 + gr];
-            const uint4 pk = *reinterpret_cast<const uint4*>(tb + r * WIDE + c0 + 8 * gr);
-            const uint32_t pw[4] = {pk.x, pk.y, pk.z, pk.w};
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const double b = (double)((pw[u >> 1] >> (16 * (u & 1))) & 0xFFFFu);
-                mma_f64(acc[u][0], acc[u][1], a, b);
-            }
-        }
-        __syncthreads();  // the buffer is free for stage stg + 2
-    }
-    const int i = ti * 8 + gr;
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int w = c0 + 8 * (2 * qq + h) + u;
-            if (q.out_trans) q.out[(int64_t)w * SMALL + i] = acc[u][h];
-            else q.out[(int64_t)i * WIDE + w] = acc[u][h];
-        }
-}
-
-static cudaError_t launch_qthin_mma(const ThinQ* d, int n, int stage_bytes, cudaStream_t s, const DevState* st) {
-    k_qthin_mma<<<n, 256, 2 * stage_bytes, s>>>(d, stage_bytes, st);
-    return cudaGetLastError();
-}
-
-// shared memory of k_qthin: the largest term's stage (table rows + small rows)
-static int qthin_stage_bytes(const std::vector<ThinQ>& v) {
-    int m = 0;
-    for (const auto& q : v) m = std::max(m, kQtRows * (q.WIDE * 2 + q.SMALL * 8));
-    return (m + 15) & ~15;
-}
-
-static cudaError_t launch_qthin(const ThinQ* d, int n, int stage_bytes, cudaStream_t s, const DevState* st) {
-    k_qthin<<<n, 256, stage_bytes * kQtStages, s>>>(d, stage_bytes, st);
-    return cudaGetLastError();
-}
-
-static int dthin_smem(int k) { return (int)sizeof(double) * ((1 << k) + (1 << k) / 8 + 8); }
-
-static cudaError_t launch_dthin(const ThinDF* d, int n, int it, int k, const double* lnq_full, cudaStream_t s,
-                                const DevState* st) {
-    const int sm = dthin_smem(k);
-    switch (it) {
-        case 1: k_dthin<1><<<n, 256, sm, s>>>(d, lnq_full, st); break;
-        case 2: k_dthin<2><<<n, 256, sm, s>>>(d, lnq_full, st); break;
-        case 4: k_dthin<4><<<n, 256, sm, s>>>(d, lnq_full, st); break;
-        case 8: k_dthin<8><<<n, 256, sm, s>>>(d, lnq_full, st); break;
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
-}
-
-static cudaError_t launch_dthin_mma(const ThinDF* d, int n, int smem, const double* lnq_full, cudaStream_t s,
-                                    const DevState* st) {
-    k_dthin_mma<<<n, 256, smem, s>>>(d, lnq_full, st);
-    return cudaGetLastError();
-}
-
-static cudaError_t set_thin_smem(int ny) {
-    const int sm = (int)sizeof(double) * ny;
-    if (sm <= 48 * 1024) return cudaSuccess;
-    cudaError_t e = cudaSuccess;
-#define SET_(S) if (e == cudaSuccess) e = cudaFuncSetAttribute(k_thin_d<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    SET_(1) SET_(2) SET_(4) SET_(8) SET_(16) SET_(32) SET_(64)
-#undef SET_
-    return e;
-}
-
 // ------------------------------------------------------------ small kernels
-// out[i] = sum_s part[s * stride + i] for the UL and VR split-K partials
-__global__ void k_sum_parts(const double* __restrict__ a, int sa, int64_t na, double* __restrict__ oa,
-                            const double* __restrict__ b, int sb, int64_t nb, double* __restrict__ ob,
-                            const DevState* st) {
-    if (gated(st)) return;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < na + nb;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        if (i < na) {
-            double s = 0.0;
-            for (int p = 0; p < sa; ++p) s += a[(int64_t)p * na + i];
-            oa[i] = s;
-        } else {
-            const int64_t j = i - na;
-            double s = 0.0;
-            for (int p = 0; p < sb; ++p) s += b[(int64_t)p * nb + j];
-            ob[j] = s;
-        }
-    }
-}
-
-// q(rep r) = sum_{y in O(r)} acc[y] / (|O(r)| C Z) with acc[y] = sum over
-// terms of Q_t[y] (split slices, or U^T / V rows for identity terms); ln q
-// with the reference's 0 for q == 0 (backend/BAA.cu:573-580), expanded to
-// every y, and copied into RB / LA where a D-side product is the identity.
-// phase 1: qsum[t][y] = sum over the split slices of Q_t
-__global__ void k_qsum(const FoldTerm* __restrict__ terms, int T, const double* __restrict__ qparts, int k,
-                       double* __restrict__ qsum, const DevState* st) {
-    if (gated(st)) return;
-    const int ny = 1 << k;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < T * ny; e += gridDim.x * blockDim.x) {
-        const int t = e / ny, y = e % ny;
-        const FoldTerm& f = terms[t];
-        if (f.kind != 0) continue;
-        const double* q = qparts + f.qoff + y;
-        double a = 0.0;
-        for (int sp = 0; sp < f.qs; ++sp) a += q[(size_t)sp * ny];
-        qsum[e] = a;
-    }
-}
-
-// Q_t[y] from the split sums, or from U^T / V for identity terms (V holds
-// only the rows x_hi < H1h; the rows above are zero)
-__device__ __forceinline__ double term_value(const FoldTerm& f, const double* qsum, int t, int ny,
-                                             const double* ULt, int KL, const double* VR, int KR, int H1h,
-                                             int row0, uint32_t y) {
-    if (f.kind == 0) return qsum[(size_t)t * ny + y];
-    const uint32_t yh = y >> f.m, yl = y & ((1u << f.m) - 1u);
-    if (f.kind == 1) return ULt[(size_t)reverse_bits(yl, f.m) * KL + f.off + yh];  // Q_t = U_t (rows: rev x_lo)
-    // Q_t = V_t at row x_hi = yh: held rows only (the others are another shard's)
-    const uint32_t r = yh - (uint32_t)row0;
-    return (yh >= (uint32_t)row0 && r < (uint32_t)H1h) ? VR[(size_t)r * KR + f.off + yl] : 0.0;
-}
-
-// phase 2: acc[y] = sum_t Q_t[y]: CTA = 32 consecutive y, warp w reads the
-// terms w, w + 8, ... (coalesced along y), and the 8 partial sums are added
-// in a fixed order
-__global__ void __launch_bounds__(256) k_fold_acc(const FoldTerm* __restrict__ terms, int T,
-                                                  const double* __restrict__ qsum, const double* __restrict__ ULt,
-                                                  int KL, const double* __restrict__ VR, int KR, int H1h, int row0,
-                                                  int k, double* __restrict__ acc, const DevState* st) {
-    if (gated(st)) return;
-    __shared__ double part[8][33];
-    const int ny = 1 << k;
-    const int yy = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int y = blockIdx.x * 32 + yy;
-    double a = 0.0;
-    if (y < ny)
-        for (int t = w; t < T; t += 8) a += term_value(terms[t], qsum, t, ny, ULt, KL, VR, KR, H1h, row0, (uint32_t)y);
-    part[w][yy] = a;
-    __syncthreads();
-    if (w == 0 && y < ny) {
-        double s = part[0][yy];
-        for (int j = 1; j < 8; ++j) s += part[j][yy];
-        acc[y] = s;
-    }
-}
-
-// phase 3: q(rep r) = sum_{y in O(r)} acc[y] / (|O(r)| C Z); ln q with the
-// reference's 0 for q == 0 (backend/BAA.cu:573-580), expanded to every y,
-// and copied into RB / LA where a D-side product is the identity.
-__global__ void k_fold_q(const FoldTerm* __restrict__ terms, int T, const double* __restrict__ accv, int k,
-                         double inv_c, double* __restrict__ lnq_full, double* __restrict__ lnq, double* __restrict__ RB,
-                         int H2, double* __restrict__ LA, int Kp, int KL, int H1h, int row0, const DevState* st) {
-    if (gated(st)) return;
-    const int ny = 1 << k;
-    const int y = blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= ny) return;
-    const double inv_z = exp(-st->log_z);
-    const uint32_t r = orbit_rep((uint32_t)y, k);
-    const uint32_t rv = reverse_bits(r, k), cv = complement_bits(r, k), rcv = reverse_bits(cv, k);
-    double acc = accv[r];
-    int nm = 1;
-    if (rv != r) {
-        acc += accv[rv];
-        ++nm;
-    }
-    if (cv != r && cv != rv) {
-        acc += accv[cv];
-        ++nm;
-    }
-    if (rcv != r && rcv != rv && rcv != cv) {
-        acc += accv[rcv];
-        ++nm;
-    }
-    const double q = acc * inv_c * inv_z / (double)nm;
-    const double lq = (q != 0.0) ? log(q) : 0.0;
-    lnq_full[y] = lq;
-    if ((uint32_t)y == r) lnq[y] = lq;  // representatives are < 2^{k-1}
-    for (int t = 0; t < T; ++t) {
-        const FoldTerm& f = terms[t];
-        const uint32_t yh = (uint32_t)y >> f.m, yl = (uint32_t)y & ((1u << f.m) - 1u);
-        if (f.idB_left) RB[(size_t)(f.off + yh) * H2 + reverse_bits(yl, f.m)] = lq;  // M_t = Lq_t
-        const uint32_t r = yh - (uint32_t)row0;  // the held rows of N_t = Lq_t
-        if (f.idA_right && yh >= (uint32_t)row0 && r < (uint32_t)H1h) LA[(size_t)r * Kp + KL + f.off + yl] = lq;
-    }
-}
-
 __global__ void __launch_bounds__(256)
 k_fac_finalize(const double* __restrict__ part, int nb, double a, double eta, DevState* st) {
     if (gated(st)) return;
@@ -1762,116 +944,89 @@ struct TuneFile {
     }
 };
 
-// chooses tile shape and split of one of the wide q-side products by timing
-// them; gen(cfg, S) lists the descriptors of a candidate (S: the split of
-// the longest contraction, kfull its length)
+// chooses tile shape (from cfgs) and split of U or V by timing them together
+// with the transform that reads their slices; gen(cfg, S) lists the
+// descriptors of a candidate (S: the split of the longest contraction, kfull
+// its length), post(cfg, S) runs the transform
 template <typename Gen, typename Post>
-static bdc_status tune_thin(bdc_handle* H, TuneFile& tf, const char* key, Launch& L, Gen&& gen, Post&& post,
-                            int kfull, int max_split, int kmin, const char* what, int* split_out) {
-    const int cfgs[4] = {CFG_128x128, CFG_128x64, CFG_64x128, CFG_64x64};
+static bdc_status tune_product(bdc_handle* H, TuneFile& tf, const char* key, Launch& L, Gen&& gen, Post&& post,
+                               const std::vector<int>& cfgs, int kfull, int max_split, int kmin, const char* what,
+                               int* split_out) {
     float best = 1e30f;
-    int best_cfg = CFG_64x64, best_s = 1;
-    const bool pinned = tf.get(key, &best_cfg, &best_s);
-    for (int ci = 0; ci < 4 && !pinned; ++ci) {
+    int best_cfg = cfgs[0], best_s = 1;
+    bool pinned = tf.get(key, &best_cfg, &best_s);
+    if (pinned && std::find(cfgs.begin(), cfgs.end(), best_cfg) == cfgs.end()) pinned = false;
+    for (int cfg : cfgs) {
+        if (pinned) break;
         for (int S = 1; S <= max_split; S *= 2) {
-            if (kfull / S < kmin) break;
-            std::vector<GemmDesc> v = gen(cfgs[ci], S);
+            if (S > 1 && kfull / S < kmin) break;
+            std::vector<GemmDesc> v = gen(cfg, S);
             Launch T;
-            BDC_CUDA_TRY(make_launch(T, v, cfgs[ci]));
+            BDC_CUDA_TRY(make_launch(T, v, cfg));
             if (T.tiles > 64 * H->num_sms) {
                 free_launch(T);
                 continue;
             }
-            // the product and the sum of its S split slices
+            BDC_CUDA_TRY(post(cfg, S, false));
+            cudaError_t e = cudaSuccess;
             const float ms = time_ms(H, [&] {
-                const cudaError_t e = launch_store(T, H->stream, nullptr);
-                post(S);
-                return e;
-            });
+                const cudaError_t e1 = launch_store(T, H->stream, nullptr);
+                return e1 != cudaSuccess ? e1 : post(cfg, S, true);
+            }, &e);
             free_launch(T);
+            BDC_CUDA_TRY(e);
             if (ms < best) {
                 best = ms;
-                best_cfg = cfgs[ci];
+                best_cfg = cfg;
                 best_s = S;
             }
         }
     }
     if (!pinned) tf.put(key, best_cfg, best_s);
     BDC_CUDA_TRY(make_launch(L, gen(best_cfg, best_s), best_cfg));
+    BDC_CUDA_TRY(post(best_cfg, best_s, false));
     *split_out = best_s;
     if (H->verbose)
-        printf("bdc: tuned %s: tile %dx%d, split %d, %.1f us\n", what, kCfgBM[best_cfg], kCfgBN[best_cfg], best_s,
-               best * 1e3f);
+        printf("bdc: tuned %s: tile %dx%d, split %d, %.1f us with the transform\n", what, kCfgBM[best_cfg],
+               kCfgBN[best_cfg], best_s, best * 1e3f);
     return BDC_OK;
 }
 
-// A thin q-side product as a matrix product on the tensor-core path, in the
-// orientation whose long side (the wide index w) is M:
-//   C(w, i) = sum_s wide(s)[w] small(s)[i] over s in [s0, s1)
-static GemmDesc thin_q_desc(const ThinQ& q) {
-    Operand A, B;
-    A.ptr = q.wide;
-    A.ld = q.wide_stride;
-    A.kind = q.wide_u16 ? OP_U16 : OP_F64;
-    A.trans = 1;
-    B.ptr = q.small;
-    B.ld = q.small_stride;
-    B.kind = q.small_u16 ? OP_U16 : OP_F64;
-    B.trans = 0;
-    GemmDesc d = make_desc(k_offset(A, true, q.s0), k_offset(B, false, q.s0), q.out, q.out_trans ? q.SMALL : 1,
-                           q.out_trans ? 1 : q.WIDE, q.WIDE, q.SMALL, q.s1 - q.s0);
-    return d;
+// slices of a block whose contraction has length kb, when one of length kfull has S
+static int block_slices(int S, int kb, int kfull) {
+    return std::max(1, (int)(((int64_t)S * kb + kfull - 1) / kfull));
 }
 
-// A thin D-side product: C(s, i) = sum_w wide(s)[w] Lq'[w][i]
-static GemmDesc thin_d_desc(const ThinD& t, const double* lnq_full) {
-    Operand A, B;
-    A.ptr = t.wide;
-    A.ld = t.wide_stride;
-    A.kind = OP_U16;
-    A.trans = 0;
-    B.ptr = lnq_full;
-    B.kind = OP_F64;
-    B.trans = t.lq_trans ? 0 : 1;
-    B.ld = t.lq_trans ? t.SMALL : t.WIDE;
-    return make_desc(A, B, t.out, t.out_s, t.out_i, t.rows, t.SMALL, t.WIDE);
-}
-
-// times the CUDA-core kernel of one size class against the tensor-core
-// launch in a few tile shapes and keeps the fastest
-template <typename Core>
-static bdc_status tune_class(bdc_handle* H, TuneFile& tf, const char* key, const std::vector<GemmDesc>& descs,
-                             Launch& L, bool& use_mma, Core&& core_launch, const char* what, int lg) {
-    const int cfgs[5] = {CFG_128x16, CFG_128x32, CFG_64x64, CFG_128x64, CFG_64x128};
-    int best_cfg = -1, unused = 0;
-    const bool pinned = tf.get(key, &best_cfg, &unused);
-    // the CUDA-core kernels hold one accumulator per small output in
-    // registers, up to 64; wider terms always take a tensor-core tile
-    const bool core_ok = lg <= 6;
-    const float core_ms = (pinned || !core_ok) ? 0.f : time_ms(H, core_launch);
-    float best = core_ok ? core_ms : 1e30f;
-    if (pinned && !core_ok && best_cfg < 0) best_cfg = CFG_64x64;
-    for (int c : cfgs) {
-        if (pinned) break;
-        Launch T;
-        BDC_CUDA_TRY(make_launch(T, descs, c));
-        const float ms = time_ms(H, [&] { return launch_store(T, H->stream, nullptr); });
-        free_launch(T);
-        if (ms < best) {
-            best = ms;
-            best_cfg = c;
-        }
+// the word transforms of both sides; a round has at most 2^{r-3} items, one per thread
+static cudaError_t launch_words(bool q_side, const FactoredState* F, cudaStream_t s, const DevState* st) {
+    const int g = F->plan.ctas, sm = F->words_smem;
+    if (F->words_threads == 256) {
+        if (q_side) k_words_q<256><<<g, 256, sm, s>>>(F->d_plan, F->qparts, st);
+        else k_words_d<256><<<g, 256, sm, s>>>(F->d_plan, F->lnq_full, st);
+    } else {
+        if (q_side) k_words_q<512><<<g, 512, sm, s>>>(F->d_plan, F->qparts, st);
+        else k_words_d<512><<<g, 512, sm, s>>>(F->d_plan, F->lnq_full, st);
     }
-    if (!pinned) tf.put(key, best_cfg, 0);
-    use_mma = best_cfg >= 0;
-    if (use_mma) BDC_CUDA_TRY(make_launch(L, descs, best_cfg));
-    if (H->verbose)
-        printf("bdc: tuned %s, %d outputs per term: %s %.1f us (CUDA cores %.1f us)\n", what, 1 << lg,
-               use_mma ? (best_cfg == CFG_128x16 ? "mma 128x16" : best_cfg == CFG_128x32 ? "mma 128x32"
-                          : best_cfg == CFG_64x64 ? "mma 64x64" : best_cfg == CFG_128x64 ? "mma 128x64" : "mma 64x128")
-                       : "CUDA cores",
-               best * 1e3f, core_ms * 1e3f);
-    return BDC_OK;
+    return cudaGetLastError();
+}
+
+// the largest transform's shared memory (k = 14), for every handle
+static cudaError_t set_words_attrs() {
+    const int smem = std::max(word_smem(12, 11), word_smem(14, 12));
+    cudaError_t e = cudaFuncSetAttribute(k_words_q<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_words_d<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_words_q<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_words_d<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return e;
+}
+
+// N(x, y) for short words on the host
+static int word_occurrences(int x, int nx, int y, int ny) {
+    int d[kWordMaxHalf + 1] = {1};
+    for (int i = 0; i < nx; ++i)
+        for (int j = ny; j > 0; --j)
+            if (((y >> (ny - j)) & 1) == ((x >> (nx - 1 - i)) & 1)) d[j] += d[j - 1];
+    return d[ny];
 }
 
 cudaError_t dgemm_scratch_alloc(DgemmScratch& sc, int max_tiles, cudaStream_t s) {
@@ -1923,8 +1078,7 @@ cudaError_t dgemm_nt(const DgemmScratch& sc, const double* A, int lda, const dou
 bool factored_supports(int n, int k) {
     // needs k < n (W is not the identity), half tables that fit the uint16
     // bundles, a dense 2^{n-1} state that fits comfortably in device memory,
-    // and per-term products of at most 128 small outputs (a term's small side
-    // is 2^min(j, k - j), up to 2^floor(k/2))
+    // and word transforms whose vectors fit in shared memory (k <= 14)
     return k >= 1 && k < n && n >= 2 && n <= 28 && k <= 14;
 }
 
@@ -1988,30 +1142,15 @@ bdc_status factored_init(bdc_handle* H) {
             BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_rows<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, F->rows_smem));
         }
     }
-    const int k = H->k;
-    int KL = 0, KR = 0;
-    for (int j = s.jlo; j <= s.jhi; ++j) {
-        Term t{};
-        t.j = j;
-        t.m = k - j;
-        t.idA = (j == s.n1);
-        t.idB = (t.m == s.n2);
-        if (t.idA && t.idB) return fail(BDC_ERR_UNSUPPORTED, "factored engine: k == n");
-        t.left = t.idB ? 1 : (t.idA ? 0 : (j <= t.m));
-        F->terms.push_back(t);
-    }
-    for (auto& t : F->terms)
-        if (t.left) { t.off = KL; KL += 1 << t.j; }
-    for (auto& t : F->terms)
-        if (!t.left) { t.off = KR; KR += 1 << t.m; }
+    // words of length a of the high half, b of the low half
+    const int k = H->k, wa = k / 2, wb = k - 1 - wa;
+    const int KL = 1 << wa, KR = 1 << wb;
     F->KL = KL;
     F->KR = KR;
     F->Kp = (KL + KR + 7) / 8 * 8;
-    F->T = (int)F->terms.size();
     const int64_t NX = (int64_t)F->H1h * F->H2;  // the dense rows held
     const int ny = 1 << k;
     const int H1 = F->H1h, H2 = F->H2, Kp = F->Kp;  // H1: the rows kept
-    const int KLa = KL > 0 ? KL : 1, KRa = KR > 0 ? KR : 1;
     const int max_split = 16;
 
     auto al = [&](double** p, size_t cnt) -> cudaError_t {
@@ -2023,10 +1162,8 @@ bdc_status factored_init(bdc_handle* H) {
     BDC_CUDA_TRY(al(&F->hx, NX));
     BDC_CUDA_TRY(al(&F->LA, (size_t)H1 * Kp));
     BDC_CUDA_TRY(al(&F->RB, (size_t)Kp * H2));
-    BDC_CUDA_TRY(al(&F->UL, (size_t)H2 * KLa));
-    BDC_CUDA_TRY(al(&F->VR, (size_t)H1 * KRa));
-    BDC_CUDA_TRY(al(&F->ulpart, (size_t)max_split * H2 * KLa));
-    BDC_CUDA_TRY(al(&F->vrpart, (size_t)max_split * H1 * KRa));
+    BDC_CUDA_TRY(al(&F->ulpart, (size_t)max_split * H2 * KL));
+    BDC_CUDA_TRY(al(&F->vrpart, (size_t)max_split * H1 * KR));
     BDC_CUDA_TRY(al(&F->lnq_full, (size_t)ny));
     BDC_CUDA_TRY(cudaMemsetAsync(F->LA, 0, sizeof(double) * H1 * Kp, H->stream));
     BDC_CUDA_TRY(cudaMemsetAsync(F->RB, 0, sizeof(double) * Kp * H2, H->stream));
@@ -2051,14 +1188,11 @@ bdc_status factored_init(bdc_handle* H) {
         }
     }
 
-    // constant table columns of LA (AL) and rows of RB (BR^T); a left term's
-    // A_j or a right term's B_m is never the identity
+    // constant table columns of LA (AL) and rows of RB (BR^T)
     {
-        std::vector<int> colmap(KL + KR + 1);
-        for (auto& t : F->terms) {
-            if (t.left) for (int c = 0; c < (1 << t.j); ++c) colmap[t.off + c] = bundle_offset(t.j) + c;
-            else for (int c = 0; c < (1 << t.m); ++c) colmap[KL + t.off + c] = bundle_offset(t.m) + c;
-        }
+        std::vector<int> colmap(KL + KR);
+        for (int c = 0; c < KL; ++c) colmap[c] = bundle_offset(wa) + c;
+        for (int c = 0; c < KR; ++c) colmap[KL + c] = bundle_offset(wb) + c;
         int* d_cm = nullptr;
         BDC_CUDA_TRY(cudaMalloc(&d_cm, sizeof(int) * colmap.size()));
         BDC_CUDA_TRY(cudaMemcpy(d_cm, colmap.data(), sizeof(int) * colmap.size(), cudaMemcpyHostToDevice));
@@ -2073,436 +1207,174 @@ bdc_status factored_init(bdc_handle* H) {
                                                             nullptr);
     BDC_CUDA_TRY(cudaGetLastError());
 
-    // ---- the two thin products: U^T (H2 x KL) = (AL^T Pw)^T, V (H1h x KR) = Pw BR
+    // ---- the word transforms: one CTA per word and slice of 2^r strings of
+    // the other half.  r = 11 (12 for k > 12, whose words need the larger CTA
+    // anyway): a level's 2^{r+1} coefficients are 32 KB, so that several CTAs
+    // share an SM, and at n = 24 the 2^a * 2 + 2^b CTAs just cover the SMs.
+    {
+        WordPlan& P = F->plan;
+        P.k = k;
+        const int rmax = k <= 12 ? 11 : 12;
+        const int half[2] = {s.n1, s.n2};              // characters of the words' half
+        const int bits[2] = {s.n2, s.n1 - 1};          // free characters of the other half
+        int cta = 0;
+        for (int d = 0; d < 2; ++d) {
+            WordSide& S = P.side[d];
+            S.words_log = d == 0 ? wa : wb;
+            S.last0 = d;  // x_hi read backwards ends in its leading 0
+            S.r = std::min(bits[d], rmax);
+            S.t = bits[d] - S.r;
+            S.leaf0 = d == 0 ? 0 : F->row0;
+            S.leaves = d == 0 ? H2 : H1;
+            S.cta0 = cta;
+            const int W = S.words_log;
+            std::vector<double> wt((size_t)2 << (2 * W), 0.0);
+            std::vector<WordTerm> terms((size_t)kWordTerms << W, WordTerm{0.0, 0, 0});
+            std::vector<int> first((size_t)(kWordMaxHalf + 2) << W, 0);
+            for (int w = 0; w < (1 << W); ++w) {
+                // (the second side's words are consumed from their last character)
+                const int path = d == 0 ? w : (int)reverse_bits((uint32_t)w, W);
+                int cnt = 0;
+                for (int j = 0; j <= W; ++j) {
+                    first[(size_t)w * (kWordMaxHalf + 2) + j] = cnt;
+                    for (int v = 0; v < (1 << j); ++v) {
+                        const int occ = word_occurrences(path, W, v, j);
+                        if (!occ) continue;
+                        const double c = (double)occ / (double)binom(half[d] - j, W - j);
+                        wt[((size_t)w << (W + 1)) + (1 << j) + v] = c;
+                        terms[(size_t)w * kWordTerms + cnt++] = WordTerm{c, v, 0};
+                    }
+                }
+                for (int j = W + 1; j < kWordMaxHalf + 2; ++j) first[(size_t)w * (kWordMaxHalf + 2) + j] = cnt;
+            }
+            const size_t b0 = terms.size() * sizeof(WordTerm), b1 = wt.size() * sizeof(double),
+                         b2 = first.size() * sizeof(int);
+            BDC_CUDA_TRY(cudaMalloc(&F->d_wtab[d], b0 + b1 + b2));
+            uint8_t* tab = (uint8_t*)F->d_wtab[d];
+            BDC_CUDA_TRY(cudaMemcpy(tab, terms.data(), b0, cudaMemcpyHostToDevice));
+            BDC_CUDA_TRY(cudaMemcpy(tab + b0, wt.data(), b1, cudaMemcpyHostToDevice));
+            BDC_CUDA_TRY(cudaMemcpy(tab + b0 + b1, first.data(), b2, cudaMemcpyHostToDevice));
+            S.terms = (const WordTerm*)tab;
+            S.weight = (const double*)(tab + b0);
+            S.first = (const int*)(tab + b0 + b1);
+            S.out = d == 0 ? F->RB : F->LA + KL;
+            S.leaf_stride = d == 0 ? 1 : Kp;
+            S.word_stride = d == 0 ? H2 : 1;
+            S.in = d == 0 ? F->ulpart : F->vrpart;
+            S.slice_stride = (int64_t)S.leaves << S.words_log;
+            BDC_CUDA_TRY(cudaMalloc(&F->d_ns[d], (size_t)(S.leaves + 15) / 16));
+            BDC_CUDA_TRY(cudaMemset(F->d_ns[d], 0, (size_t)(S.leaves + 15) / 16));
+            S.ns = F->d_ns[d];
+            cta += 1 << (S.words_log + S.t);
+            F->words_smem = std::max(F->words_smem, word_smem(k, S.r));
+        }
+        P.ctas = cta;
+        P.parts_l = P.side[1].cta0;
+        F->words_threads = std::max(P.side[0].r, P.side[1].r) <= 11 ? 256 : 512;
+        BDC_CUDA_TRY(set_words_attrs());
+        BDC_CUDA_TRY(cudaMalloc(&F->d_plan, sizeof(WordPlan)));
+        BDC_CUDA_TRY(cudaMemcpy(F->d_plan, &P, sizeof(WordPlan), cudaMemcpyHostToDevice));
+        BDC_CUDA_TRY(al(&F->qparts, (size_t)cta << k));
+        BDC_CUDA_TRY(al(&F->qacc, (size_t)ny));
+        const int mb = k - 2 * fold_edge(k);
+        std::vector<int> mids;
+        for (int m = 0; m < (1 << mb); ++m)
+            if (is_rep((uint32_t)m, mb)) mids.push_back(m);
+        F->n_mids = (int)mids.size();
+        BDC_CUDA_TRY(cudaMalloc(&F->d_mids, sizeof(int) * mids.size()));
+        BDC_CUDA_TRY(cudaMemcpy(F->d_mids, mids.data(), sizeof(int) * mids.size(), cudaMemcpyHostToDevice));
+    }
+    BDC_CUDA_TRY(cudaStreamCreateWithFlags(&F->side, cudaStreamNonBlocking));
+    BDC_CUDA_TRY(cudaEventCreateWithFlags(&F->ev_join, cudaEventDisableTiming));
+    BDC_CUDA_TRY(cudaEventCreateWithFlags(&F->ev_fork, cudaEventDisableTiming));
+
+    // ---- the two thin products: U (KL x H2) = AL^T Pw, V (H1h x KR) = Pw BR
     // Only the rows x_hi <= colmax[c] of a dense column c hold
-    // representatives: U^T contracts each block of columns over those rows
+    // representatives: U contracts each block of columns over those rows
     // only, V each block of rows over the columns that reach it.  The split
-    // of a block is proportional to its contraction; split slices that no
-    // block writes stay zero.
-    if (KL > 0) {
-        // A(m = c, kk = x_hi) = LA[x_hi * Kp + c]; B(kk = x_hi, n = col) = Pw; C(c, col) -> U^T[col][c]
+    // of a block is proportional to its contraction; the transform reads as
+    // many slices as a block has.
+    {
+        // per block of BN columns: the rows it contracts (0: no representative)
+        auto col_rows = [&](int n0, int nb) {
+            int kb = 0;
+            for (int c = n0; c < n0 + nb; ++c) kb = std::max(kb, F->colmax[c] + 1);
+            return kb == 0 ? 0 : std::min(H1, (kb + 15) & ~15);  // rows past the last representative are zero
+        };
+        // A(m = w, kk = x_hi) = LA[x_hi * Kp + w]; B(kk = x_hi, n = col) = Pw; C(w, col) -> U[w][col]
         auto gen = [&](int cfg, int S) {
             std::vector<GemmDesc> v;
             const int BN = kCfgBN[cfg];
             for (int n0 = 0; n0 < H2; n0 += BN) {
-                const int nb = std::min(BN, H2 - n0);
-                int kb = 0;
-                for (int c = n0; c < n0 + nb; ++c) kb = std::max(kb, F->colmax[c] + 1);
+                const int nb = std::min(BN, H2 - n0), kb = col_rows(n0, nb);
                 if (kb == 0) continue;
-                kb = std::min(H1, (kb + 15) & ~15);  // rows past the last representative are zero
-                GemmDesc d = make_desc(op_f64(F->LA, Kp, 1), op_f64(F->Pw + n0, H2, 0), F->ulpart + (int64_t)n0 * KL,
-                                       1, KL, KL, nb, kb);
-                split_k(v, d, std::max(1, (int)(((int64_t)S * kb + H1 - 1) / H1)), (int64_t)H2 * KL);
+                GemmDesc d = make_desc(op_f64(F->LA, Kp, 1), op_f64(F->Pw + n0, H2, 0), F->ulpart + n0, H2, 1, KL, nb, kb);
+                split_k(v, d, block_slices(S, kb, H1), (int64_t)H2 * KL);
             }
             return v;
         };
-        auto post = [&](int S) {
-            k_sum_parts<<<H->num_sms * 4, 256, 0, H->stream>>>(F->ulpart, S, (int64_t)KL * H2, F->UL, F->vrpart, 1, 0,
-                                                               F->VR, nullptr);
+        auto post = [&](int cfg, int S, bool run) -> cudaError_t {
+            if (run) return launch_words(true, F, H->stream, nullptr);
+            std::vector<uint8_t> ns((size_t)(H2 + 15) / 16, 0);
+            const int BN = kCfgBN[cfg];
+            for (int c = 0; c < H2; c += 16) {
+                const int n0 = c / BN * BN, kb = col_rows(n0, std::min(BN, H2 - n0));
+                ns[(size_t)c / 16] = kb == 0 ? 0 : (uint8_t)block_slices(S, kb, H1);
+            }
+            return cudaMemcpy(F->d_ns[0], ns.data(), ns.size(), cudaMemcpyHostToDevice);
         };
-        bdc_status rc = tune_thin(H, tf, "ul", F->ul, gen, post, H1, max_split, 16, "U = AL^T Pw", &F->S1);
+        const std::vector<int> cfgs = KL >= 128  ? std::vector<int>{CFG_128x64, CFG_64x64, CFG_64x128}
+                                      : KL == 64 ? std::vector<int>{CFG_64x64, CFG_64x128}
+                                      : KL == 32 ? std::vector<int>{CFG_32x64, CFG_32x128}
+                                                 : std::vector<int>{CFG_16x128};
+        bdc_status rc = tune_product(H, tf, "u", F->ul, gen, post, cfgs, H1, max_split, 16, "U = AL^T Pw", &F->S1);
         if (rc != BDC_OK) return rc;
     }
-    if (KR > 0) {
-        // A(m = x_hi, kk = col) = Pw; B(kk = col, n = c) = RB[(KL + c) * H2 + col]
+    {
+        // per block of BM rows: the columns [clo, clo + kb) that reach it (kb = 0: none)
+        auto row_cols = [&](int m0, int* clo_out) {
+            int clo = H2, chi = -1;
+            for (int c = 0; c < H2; ++c)
+                if (F->colmax[c] >= m0) {
+                    clo = std::min(clo, c);
+                    chi = c;
+                }
+            if (chi < 0) return 0;
+            clo &= ~15;  // whole k-slices; the columns added at either end are zero in these rows
+            *clo_out = clo;
+            return std::min(H2, (chi + 1 + 15) & ~15) - clo;
+        };
+        // A(m = x_hi, kk = col) = Pw; B(kk = col, n = w) = RB[(KL + w) * H2 + col]; C(x_hi, w) -> V[w][x_hi]
         auto gen = [&](int cfg, int S) {
             std::vector<GemmDesc> v;
             const int BM = kCfgBM[cfg];
             for (int m0 = 0; m0 < H1; m0 += BM) {
-                const int mb = std::min(BM, H1 - m0);
-                int clo = H2, chi = -1;
-                for (int c = 0; c < H2; ++c)
-                    if (F->colmax[c] >= m0) {
-                        clo = std::min(clo, c);
-                        chi = c;
-                    }
-                if (chi < 0) continue;
-                // whole k-slices; the columns added at either end are zero in these rows
-                clo &= ~15;
-                const int kb = std::min(H2, (chi + 1 + 15) & ~15) - clo;
+                int clo = 0;
+                const int mb = std::min(BM, H1 - m0), kb = row_cols(m0, &clo);
+                if (kb == 0) continue;
                 const Operand A = k_offset(op_f64(F->Pw + (int64_t)m0 * H2, H2, 0), true, clo);
                 const Operand B = k_offset(op_f64(F->RB + (int64_t)KL * H2, H2, 1), false, clo);
-                GemmDesc d = make_desc(A, B, F->vrpart + (int64_t)m0 * KR, KR, 1, mb, KR, kb);
-                split_k(v, d, std::max(1, (int)(((int64_t)S * kb + H2 - 1) / H2)), (int64_t)H1 * KR);
+                GemmDesc d = make_desc(A, B, F->vrpart + m0, 1, H1, mb, KR, kb);
+                split_k(v, d, block_slices(S, kb, H2), (int64_t)H1 * KR);
             }
             return v;
         };
-        auto post = [&](int S) {
-            k_sum_parts<<<H->num_sms * 4, 256, 0, H->stream>>>(F->ulpart, 1, 0, F->UL, F->vrpart, S,
-                                                               (int64_t)H1 * KR, F->VR, nullptr);
+        auto post = [&](int cfg, int S, bool run) -> cudaError_t {
+            if (run) return launch_words(true, F, H->stream, nullptr);
+            std::vector<uint8_t> ns((size_t)(H1 + 15) / 16, 0);
+            const int BM = kCfgBM[cfg];
+            for (int r = 0; r < H1; r += 16) {
+                int clo = 0;
+                const int kb = row_cols(r / BM * BM, &clo);
+                ns[(size_t)r / 16] = kb == 0 ? 0 : (uint8_t)block_slices(S, kb, H2);
+            }
+            return cudaMemcpy(F->d_ns[1], ns.data(), ns.size(), cudaMemcpyHostToDevice);
         };
-        bdc_status rc = tune_thin(H, tf, "vr", F->vr, gen, post, H2, max_split, 16, "V = Pw BR", &F->S2);
+        const std::vector<int> cfgs = KR >= 64   ? std::vector<int>{CFG_64x64, CFG_128x64}
+                                      : KR == 32 ? std::vector<int>{CFG_64x32, CFG_128x32}
+                                                 : std::vector<int>{CFG_128x16};
+        bdc_status rc = tune_product(H, tf, "v", F->vr, gen, post, cfgs, H2, max_split, 16, "V = Pw BR", &F->S2);
         if (rc != BDC_OK) return rc;
-    }
-
-    // ---- per-term thin products and the fold plan.  q side: Q_t as a sum of
-    // outer products over the contracted half, split into slices so that the
-    // launch fills the GPU (the fold sums the slices); D side: one row-dot
-    // per half-table row.  Terms whose A_j or B_m is the identity are read or
-    // written directly by the fold.
-    std::vector<ThinQ> tq[8];
-    std::vector<ThinD> td[8];
-    std::vector<FoldTerm> fold;
-    struct QPlan { int term, lg; ThinQ d; int S; };
-    std::vector<QPlan> qplan;
-    int qctas_one = 0;
-    for (int ti = 0; ti < F->T; ++ti) {
-        const Term& t = F->terms[ti];
-        FoldTerm f{};
-        f.j = t.j;
-        f.m = t.m;
-        f.off = t.off;
-        if (t.left && t.idB) {
-            f.kind = 1;       // Q_t = U_t
-            f.idB_left = 1;   // M_t = Lq_t
-        } else if (!t.left && t.idA) {
-            f.kind = 2;        // Q_t = V_t
-            f.idA_right = 1;   // N_t = Lq_t
-        } else {
-            ThinQ q{};
-            ThinD d{};
-            if (t.left) {
-                // Q_t[yh][yl] = sum_{x_lo} U^T[x_lo][off + yh] B_m[x_lo][yl]
-                q.small = F->UL + t.off;
-                q.small_stride = KL;
-                q.small_u16 = 0;
-                q.wide = F->Bp + bundle_offset(t.m);
-                q.wide_stride = H->B.stride;
-                q.wide_u16 = 1;
-                q.SMALL = 1 << t.j;
-                q.WIDE = 1 << t.m;
-                q.s1 = H2;
-                q.out_trans = 0;
-                // M_t[yh][x_lo] = sum_yl B_m[x_lo][yl] Lq[yh][yl] -> RB[off + yh][x_lo]
-                d.wide = F->Bp + bundle_offset(t.m);
-                d.wide_stride = H->B.stride;
-                d.SMALL = 1 << t.j;
-                d.WIDE = 1 << t.m;
-                d.rows = H2;
-                d.lq_trans = 0;
-                d.out = F->RB + (int64_t)t.off * H2;
-                d.out_s = 1;
-                d.out_i = H2;
-            } else {
-                // Q_t[yh][yl] = sum_{x_hi} A_j[x_hi][yh] V[x_hi][off + yl]
-                q.small = F->VR + t.off;
-                q.small_stride = KR;
-                q.small_u16 = 0;
-                q.wide = H->A.rows + (size_t)F->row0 * H->A.stride + bundle_offset(t.j);
-                q.wide_stride = H->A.stride;
-                q.wide_u16 = 1;
-                q.SMALL = 1 << t.m;
-                q.WIDE = 1 << t.j;
-                q.s1 = H1;
-                q.out_trans = 1;
-                // N_t[x_hi][yl] = sum_yh A_j[x_hi][yh] Lq[yh][yl] -> LA[x_hi][KL + off + yl]
-                d.wide = H->A.rows + (size_t)F->row0 * H->A.stride + bundle_offset(t.j);
-                d.wide_stride = H->A.stride;
-                d.SMALL = 1 << t.m;
-                d.WIDE = 1 << t.j;
-                d.rows = H1;
-                d.lq_trans = 1;
-                d.out = F->LA + KL + t.off;
-                d.out_s = Kp;
-                d.out_i = 1;
-            }
-            int lg = 0;
-            while ((1 << lg) < q.SMALL) ++lg;
-            if (lg > 7) return fail(BDC_ERR_UNSUPPORTED, "factored engine: term with more than 128 small outputs");
-            qplan.push_back({ti, lg, q, 1});
-            qctas_one += (q.WIDE + 255) / 256;
-            td[lg].push_back(d);
-        }
-        fold.push_back(f);
-    }
-    // one split count for every q-side product: about 8 CTAs per SM, >= 64 rows a slice
-    int QS = 1;
-    while (qctas_one > 0 && QS < 64 && qctas_one * QS * 2 <= 8 * H->num_sms && std::min(H1, H2) / (QS * 2) >= 64)
-        QS *= 2;
-    int64_t qelems = 0;
-    for (auto& qp : qplan) qelems += (int64_t)QS * ny;
-    BDC_CUDA_TRY(al(&F->qparts, (size_t)std::max<int64_t>(qelems, 1)));
-    BDC_CUDA_TRY(al(&F->qsum, (size_t)F->T * ny));
-    BDC_CUDA_TRY(al(&F->qacc, (size_t)ny));
-    BDC_CUDA_TRY(cudaMemsetAsync(F->qparts, 0, sizeof(double) * std::max<int64_t>(qelems, 1), H->stream));
-    int64_t qo = 0;
-    for (auto& qp : qplan) {
-        fold[qp.term].qoff = qo;
-        fold[qp.term].qs = QS;
-        const int S = qp.d.s1;
-        for (int sp = 0; sp < QS; ++sp) {
-            ThinQ q = qp.d;
-            q.s0 = (int)((int64_t)S * sp / QS);
-            q.s1 = (int)((int64_t)S * (sp + 1) / QS);
-            q.out = F->qparts + qo + (int64_t)sp * ny;
-            tq[qp.lg].push_back(q);
-        }
-        qo += (int64_t)QS * ny;
-    }
-    for (int lg = 0; lg < 8; ++lg) {
-        if (!tq[lg].empty()) {
-            BDC_CUDA_TRY(cudaMalloc(&F->d_thinq[lg], sizeof(ThinQ) * tq[lg].size()));
-            BDC_CUDA_TRY(cudaMemcpy(F->d_thinq[lg], tq[lg].data(), sizeof(ThinQ) * tq[lg].size(), cudaMemcpyHostToDevice));
-            F->n_thinq[lg] = (int)tq[lg].size();
-        }
-        if (!td[lg].empty()) {
-            int cta = 0;
-            for (auto& d : td[lg]) {
-                d.cta_begin = cta;
-                cta += (d.rows + kThinDRows - 1) / kThinDRows;
-            }
-            BDC_CUDA_TRY(cudaMalloc(&F->d_thind[lg], sizeof(ThinD) * td[lg].size()));
-            BDC_CUDA_TRY(cudaMemcpy(F->d_thind[lg], td[lg].data(), sizeof(ThinD) * td[lg].size(), cudaMemcpyHostToDevice));
-            F->n_thind[lg] = (int)td[lg].size();
-            F->ctas_thind[lg] = cta;
-        }
-    }
-    BDC_CUDA_TRY(set_thin_smem(ny));
-    for (int lg = 0; lg < 8; ++lg) {
-        if (F->n_thinq[lg]) {
-            std::vector<GemmDesc> v;
-            for (auto& q : tq[lg]) v.push_back(thin_q_desc(q));
-            char key[16];
-            snprintf(key, sizeof(key), "q%d", lg);
-            bdc_status rc = tune_class(
-                H, tf, key, v, F->mq[lg], F->use_mq[lg],
-                [&] { launch_thin_q(lg, F->d_thinq[lg], F->n_thinq[lg], ny, H->stream, nullptr); },
-                "q-side term products", lg);
-            if (rc != BDC_OK) return rc;
-        }
-        if (F->n_thind[lg]) {
-            std::vector<GemmDesc> v;
-            for (auto& d : td[lg]) v.push_back(thin_d_desc(d, F->lnq_full));
-            char key[16];
-            snprintf(key, sizeof(key), "d%d", lg);
-            bdc_status rc = tune_class(
-                H, tf, key, v, F->md[lg], F->use_md[lg],
-                [&] {
-                    launch_thin_d(lg, F->d_thind[lg], F->n_thind[lg], F->ctas_thind[lg], ny, F->lnq_full, H->stream,
-                                  nullptr);
-                },
-                "D-side term products", lg);
-            if (rc != BDC_OK) return rc;
-        }
-    }
-    for (int lg = 0; lg < 8; ++lg) {
-        BDC_CUDA_TRY(cudaStreamCreateWithFlags(&F->side[lg], cudaStreamNonBlocking));
-        BDC_CUDA_TRY(cudaEventCreateWithFlags(&F->ev_join[lg], cudaEventDisableTiming));
-    }
-    BDC_CUDA_TRY(cudaEventCreateWithFlags(&F->ev_fork, cudaEventDisableTiming));
-    {
-        BDC_CUDA_TRY(cudaMalloc(&F->d_fold, sizeof(FoldTerm) * fold.size()));
-        BDC_CUDA_TRY(cudaMemcpy(F->d_fold, fold.data(), sizeof(FoldTerm) * fold.size(), cudaMemcpyHostToDevice));
-    }
-
-    // ---- the per-term products of each side fused into one launch (per
-    // side, and per output-tile width on the D side), used where the tuner
-    // times them faster than the per-class launches.  They need 16-byte
-    // aligned table rows of >= 16 entries and 2^k / 16 >= 32 threads.
-    {
-        // (the q kernel runs 256 threads, one per 16 outputs at k = 12 and
-        // fewer busy ones below)
-        bool qok = k >= 9 && k <= 12, dok = k >= 9 && k <= 14;
-        std::vector<ThinQ> all_q;
-        for (int lg = 0; lg < 8; ++lg)
-            for (auto& q : tq[lg]) {
-                const int IT = qthin_it(q.SMALL);
-                const int WT = 16 / IT;
-                if ((q.SMALL & (q.SMALL - 1)) != 0 || q.WIDE % WT != 0 || (q.WIDE / WT) * (q.SMALL / IT) != ny / 16 ||
-                    ((uintptr_t)q.wide & 15) != 0 || (q.wide_stride % 8) != 0 || q.wide_u16 != 1 || q.small_u16 != 0)
-                    qok = false;
-                all_q.push_back(q);
-            }
-        std::vector<ThinDF> all_d[4];
-        for (int lg = 0; lg < 8; ++lg)
-            for (auto& d : td[lg]) {
-                if (d.WIDE < 8 || ((uintptr_t)d.wide & 15) != 0 || (d.wide_stride % 8) != 0) dok = false;
-                ThinDF f{};
-                f.wide = d.wide;
-                f.wide_stride = d.wide_stride;
-                f.SMALL = d.SMALL;
-                f.WIDE = d.WIDE;
-                f.rows = d.rows;
-                f.lq_trans = d.lq_trans;
-                f.out = d.out;
-                f.out_s = d.out_s;
-                f.out_i = d.out_i;
-                f.IT = std::min(d.SMALL, 8);
-                f.LPR = std::max(1, std::min(32, d.WIDE / 32));
-                const int ng = d.SMALL / f.IT;
-                if (f.LPR * ng > 256) dok = false;
-                const int rows_per_cta = (256 / (f.LPR * ng)) * kDfRT;
-                int cl = 0;
-                while ((1 << cl) < f.IT) ++cl;
-                for (int r0 = 0; r0 < d.rows; r0 += rows_per_cta) {
-                    f.row0 = r0;
-                    all_d[cl].push_back(f);
-                }
-            }
-        // the classes of 2 to 64 outputs again in 64-row blocks for k_dthin_mma
-        std::vector<ThinDF> all_m[4];
-        bool mok[4] = {false, dok, dok, dok};
-        for (int lg = 0; lg < 8; ++lg)
-            for (auto& d : td[lg]) {
-                int cl = 0;
-                while ((1 << cl) < std::min(d.SMALL, 8)) ++cl;
-                if (cl == 0 || !mok[cl]) continue;
-                if (d.SMALL > 64 || d.WIDE % kDmChunk != 0) {
-                    mok[cl] = false;
-                    continue;
-                }
-                ThinDF f{};
-                f.wide = d.wide;
-                f.wide_stride = d.wide_stride;
-                f.SMALL = d.SMALL;
-                f.WIDE = d.WIDE;
-                f.rows = d.rows;
-                f.lq_trans = d.lq_trans;
-                f.out = d.out;
-                f.out_s = d.out_s;
-                f.out_i = d.out_i;
-                F->dm_smem[cl] = std::max(F->dm_smem[cl], dthin_mma_smem(d.SMALL, d.WIDE));
-                for (int r0 = 0; r0 < d.rows; r0 += kDmRows) {
-                    f.row0 = r0;
-                    all_m[cl].push_back(f);
-                }
-            }
-        int pinned_q = -1, pinned_d = -1, pinned_m = -1, unused = 0;
-        tf.get("qf", &pinned_q, &unused);
-        tf.get("df", &pinned_d, &unused);
-        tf.get("dm", &pinned_m, &unused);  // bit cl: class cl on k_dthin_mma
-        if (const char* dm = getenv("BDC_DTHIN")) pinned_m = !strcmp(dm, "mma") ? 14 : 0;  // forces either form
-        BDC_CUDA_TRY(cudaMemsetAsync(H->d_st, 0, sizeof(DevState), H->stream));
-        if (qok && !all_q.empty()) {
-            F->qf_stage = qthin_stage_bytes(all_q);
-            BDC_CUDA_TRY(cudaFuncSetAttribute(k_qthin, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              F->qf_stage * kQtStages));
-            BDC_CUDA_TRY(cudaMalloc(&F->d_qf, sizeof(ThinQ) * all_q.size()));
-            BDC_CUDA_TRY(cudaMemcpy(F->d_qf, all_q.data(), sizeof(ThinQ) * all_q.size(), cudaMemcpyHostToDevice));
-            F->n_qf = (int)all_q.size();
-            if (pinned_q >= 0) {
-                F->use_qf = pinned_q != 0;
-            } else {
-                const float tc = time_ms(H, [&] { return enqueue_stage(H, ST_QSMALL, -INFINITY); });
-                const float tfu = time_ms(H, [&] { return launch_qthin(F->d_qf, F->n_qf, F->qf_stage, H->stream, nullptr); });
-                F->use_qf = tfu < tc;
-                tf.put("qf", F->use_qf ? 1 : 0, 0);
-                if (H->verbose)
-                    printf("bdc: tuned q-side term products: %s (one launch %.1f us, per class %.1f us)\n",
-                           F->use_qf ? "one launch" : "per class", tfu * 1e3f, tc * 1e3f);
-            }
-            // the terms of 8..64 small outputs on the FP64 tensor path
-            std::vector<ThinQ> q_lo, q_hi;
-            bool qmok = ny == 4096;
-            for (const ThinQ& x : all_q) {
-                if (x.SMALL < 8) {
-                    q_lo.push_back(x);
-                    continue;
-                }
-                if (x.SMALL > 64 || x.SMALL * x.WIDE != 4096 || x.WIDE % 64 != 0) qmok = false;
-                q_hi.push_back(x);
-                F->qm_stage = std::max(F->qm_stage, qmma_stage(x.SMALL, x.WIDE));
-            }
-            F->qm_stage = (F->qm_stage + 15) & ~15;
-            if (F->use_qf && qmok && !q_hi.empty() && 2 * F->qm_stage + 1024 <= 227 * 1024) {
-                BDC_CUDA_TRY(cudaFuncSetAttribute(k_qthin_mma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  2 * F->qm_stage));
-                BDC_CUDA_TRY(cudaMalloc(&F->d_qm, sizeof(ThinQ) * q_hi.size()));
-                BDC_CUDA_TRY(cudaMemcpy(F->d_qm, q_hi.data(), sizeof(ThinQ) * q_hi.size(), cudaMemcpyHostToDevice));
-                F->n_qm = (int)q_hi.size();
-                if (!q_lo.empty()) {
-                    F->ql_stage = qthin_stage_bytes(q_lo);
-                    BDC_CUDA_TRY(cudaMalloc(&F->d_ql, sizeof(ThinQ) * q_lo.size()));
-                    BDC_CUDA_TRY(cudaMemcpy(F->d_ql, q_lo.data(), sizeof(ThinQ) * q_lo.size(), cudaMemcpyHostToDevice));
-                    F->n_ql = (int)q_lo.size();
-                }
-                int pinned_qm = -1;
-                tf.get("qm", &pinned_qm, &unused);
-                if (const char* qm = getenv("BDC_QTHIN")) pinned_qm = !strcmp(qm, "mma") ? 1 : 0;  // forces either form
-                if (pinned_qm >= 0) {
-                    F->use_qm = pinned_qm != 0;
-                } else {
-                    cudaError_t e1 = cudaSuccess, e2 = cudaSuccess;
-                    const float t1 = time_ms(H, [&] {
-                        return launch_qthin(F->d_qf, F->n_qf, F->qf_stage, H->stream, nullptr);
-                    }, &e1);
-                    const float t2 = time_ms(H, [&] { return enqueue_qthin_split(H, H->stream, nullptr); }, &e2);
-                    BDC_CUDA_TRY(e1);
-                    BDC_CUDA_TRY(e2);
-                    F->use_qm = t2 < t1;
-                    tf.put("qm", F->use_qm ? 1 : 0, 0);
-                    if (H->verbose)
-                        printf("bdc: tuned q-side terms of 8..64 outputs: %s (with mma.sync %.1f us, CUDA cores %.1f us)\n",
-                               F->use_qm ? "mma.sync" : "CUDA cores", t2 * 1e3f, t1 * 1e3f);
-                }
-            }
-        }
-        if (dok) {
-            const int sm = dthin_smem(k);
-            if (sm > 48 * 1024) {
-                BDC_CUDA_TRY(cudaFuncSetAttribute(k_dthin<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-                BDC_CUDA_TRY(cudaFuncSetAttribute(k_dthin<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-                BDC_CUDA_TRY(cudaFuncSetAttribute(k_dthin<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-                BDC_CUDA_TRY(cudaFuncSetAttribute(k_dthin<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-            }
-            for (int cl = 0; cl < 4; ++cl) {
-                if (all_d[cl].empty()) continue;
-                BDC_CUDA_TRY(cudaMalloc(&F->d_df[cl], sizeof(ThinDF) * all_d[cl].size()));
-                BDC_CUDA_TRY(cudaMemcpy(F->d_df[cl], all_d[cl].data(), sizeof(ThinDF) * all_d[cl].size(),
-                                        cudaMemcpyHostToDevice));
-                F->n_df[cl] = (int)all_d[cl].size();
-            }
-            if (pinned_d >= 0) {
-                F->use_df = pinned_d != 0;
-            } else {
-                F->use_df = false;
-                const float tc = time_ms(H, [&] { return enqueue_stage(H, ST_DSMALL, -INFINITY); });
-                F->use_df = true;
-                const float tfu = time_ms(H, [&] { return enqueue_stage(H, ST_DSMALL, -INFINITY); });
-                F->use_df = tfu < tc;
-                tf.put("df", F->use_df ? 1 : 0, 0);
-                if (H->verbose)
-                    printf("bdc: tuned D-side term products: %s (fused %.1f us, per class %.1f us)\n",
-                           F->use_df ? "fused" : "per class", tfu * 1e3f, tc * 1e3f);
-            }
-            // classes of the fused launches on the FP64 tensor path
-            int dm_bits = 0, dm_max = 0;
-            auto dm_ok = [&](int cl) {
-                return mok[cl] && !all_m[cl].empty() && F->n_df[cl] > 0 && F->dm_smem[cl] + 1024 <= 227 * 1024;
-            };
-            for (int cl = 1; cl < 4; ++cl)
-                if (dm_ok(cl)) dm_max = std::max(dm_max, F->dm_smem[cl]);
-            if (F->use_df && dm_max > 0)
-                BDC_CUDA_TRY(cudaFuncSetAttribute(k_dthin_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, dm_max));
-            for (int cl = 1; cl < 4 && F->use_df; ++cl) {
-                if (!dm_ok(cl)) continue;
-                BDC_CUDA_TRY(cudaMalloc(&F->d_dm[cl], sizeof(ThinDF) * all_m[cl].size()));
-                BDC_CUDA_TRY(cudaMemcpy(F->d_dm[cl], all_m[cl].data(), sizeof(ThinDF) * all_m[cl].size(),
-                                        cudaMemcpyHostToDevice));
-                F->n_dm[cl] = (int)all_m[cl].size();
-                if (pinned_m >= 0) {
-                    F->use_dm[cl] = (pinned_m >> cl) & 1;
-                } else {
-                    cudaError_t e1 = cudaSuccess, e2 = cudaSuccess;
-                    const float tc = time_ms(H, [&] {
-                        return launch_dthin(F->d_df[cl], F->n_df[cl], 1 << cl, H->k, F->lnq_full, H->stream, nullptr);
-                    }, &e1);
-                    const float tm = time_ms(H, [&] {
-                        return launch_dthin_mma(F->d_dm[cl], F->n_dm[cl], F->dm_smem[cl], F->lnq_full, H->stream,
-                                                nullptr);
-                    }, &e2);
-                    BDC_CUDA_TRY(e1);
-                    BDC_CUDA_TRY(e2);
-                    F->use_dm[cl] = tm < tc;
-                    if (H->verbose)
-                        printf("bdc: tuned D-side terms of class %d (%s outputs): %s (mma.sync %.1f us, CUDA cores %.1f us)\n",
-                               cl, cl == 3 ? "8..64" : (cl == 2 ? "4" : "2"), F->use_dm[cl] ? "mma.sync" : "CUDA cores",
-                               tm * 1e3f, tc * 1e3f);
-                }
-                dm_bits |= (int)F->use_dm[cl] << cl;
-            }
-            if (F->use_df && pinned_m < 0) tf.put("dm", dm_bits, 0);
-        }
     }
 
     // ---- G = LA RB with the BA epilogue; the tile shape is tuned on the
@@ -2562,19 +1434,6 @@ bdc_status factored_init(bdc_handle* H) {
         BDC_CUDA_TRY(cudaMemsetAsync(F->Pw, 0, sizeof(double) * NX, H->stream));
         BDC_CUDA_TRY(cudaMemsetAsync(F->Lt, 0, sizeof(double) * NX, H->stream));
         BDC_CUDA_TRY(cudaMemsetAsync(H->d_st, 0, sizeof(DevState), H->stream));
-        // split slices that the chosen launches never write must read zero
-        BDC_CUDA_TRY(cudaMemsetAsync(F->ulpart, 0, sizeof(double) * max_split * H2 * KLa, H->stream));
-        BDC_CUDA_TRY(cudaMemsetAsync(F->vrpart, 0, sizeof(double) * max_split * H1 * KRa, H->stream));
-    }
-    int nq = 0, nd = 0;
-    for (int lg = 0; lg < 8; ++lg) {
-        nq += F->n_thinq[lg] > 0;
-        nd += F->n_thind[lg] > 0;
-    }
-    if (F->use_qf) nq = (F->use_qm && F->n_ql) ? 2 : 1;
-    if (F->use_df) {
-        nd = 0;
-        for (int cl = 0; cl < 4; ++cl) nd += F->n_df[cl] > 0;
     }
     // G on the int8 tensor cores (bdc_ozaki.cu), with the slicing of its FP64
     // operands, where that times faster than the FP64 product chosen above;
@@ -2589,12 +1448,16 @@ bdc_status factored_init(bdc_handle* H) {
         const bool has_pick = tf.get("oz", &pick, &unused);
         const bool pinned = has_pick && !(force_oz && pick == 0);
         if (!force_fp && !(pinned && pick == 0)) {
-            // an entry of ML (NR) is ln q against a row of B_m (A_j), whose
-            // entries add up to C(n2, m) (C(n1, j)); 1 for an identity table
-            double cmax = 1.0;
-            for (const Term& t : F->terms)
-                if (t.left && !t.idB) cmax = std::max(cmax, (double)binom(s.n2, t.m));
-                else if (!t.left && !t.idA) cmax = std::max(cmax, (double)binom(s.n1, t.j));
+            // an entry of ML is ln q against nonnegative weights that add up to
+            // sum_j C(a, j) C(n2, k - j) / C(n1 - j, a - j); NR the same from
+            // the other side
+            auto weight = [&](int words, int half, int other) {
+                double t = 0.0;
+                for (int j = 0; j <= words; ++j)
+                    t += (double)binom(words, j) * (double)binom(other, k - j) / (double)binom(half - j, words - j);
+                return t;
+            };
+            const double cmax = std::max(1.0, std::max(weight(wa, s.n1, s.n2), weight(wb, s.n2, s.n1)));
             const OzakiInput in{F->LA, F->RB, Kp, KL, KR, H1, H2, F->colmax.data(), F->lnq_full, H->k, cmax};
             const char* why = nullptr;
             bdc_status rc = ozaki_init(H, in, &F->oz, &why);
@@ -2647,9 +1510,9 @@ bdc_status factored_init(bdc_handle* H) {
             }
         }
     }
-    // U, V, the split sums; q-side terms; three fold kernels; D-side terms; G
-    // (plus the slicing kernel on the int8 path); finalize
-    F->launches_per_iter = (F->ul.n > 0) + (F->vr.n > 0) + 1 + nq + 3 + nd + 1 + 1 + (F->use_oz ? 1 : 0);
+    // U, V; the q-side transform; fold; the D-side transform; G (plus the
+    // slicing kernel on the int8 path); finalize
+    F->launches_per_iter = (F->ul.n > 0) + (F->vr.n > 0) + 3 + 1 + 1 + (F->use_oz ? 1 : 0);
     BDC_CUDA_TRY(cudaStreamSynchronize(H->stream));
     return BDC_OK;
 }
@@ -2657,23 +1520,19 @@ bdc_status factored_init(bdc_handle* H) {
 void factored_free(bdc_handle* H) {
     FactoredState* F = H->fac;
     if (!F) return;
-    for (double* p : {F->Pw, F->Lt, F->hx, F->LA, F->RB, F->UL, F->VR, F->ulpart, F->vrpart, F->qparts,
-                      F->qsum, F->qacc, F->lnq_full, F->epart})
+    for (double* p : {F->Pw, F->Lt, F->hx, F->LA, F->RB, F->ulpart, F->vrpart, F->qparts, F->qacc, F->lnq_full,
+                      F->epart})
         cudaFree(p);
     cudaFree(F->Bp);
     cudaFree(F->Ddense);
     cudaFree(F->d_rowstart);
     cudaFree(F->rpart);
-    cudaFree(F->d_qf);
-    cudaFree(F->d_ql);
-    cudaFree(F->d_qm);
-    for (auto* d : F->d_df) cudaFree(d);
-    for (int lg = 0; lg < 8; ++lg) {
-        cudaFree(F->d_thinq[lg]);
-        cudaFree(F->d_thind[lg]);
-        if (F->side[lg]) cudaStreamDestroy(F->side[lg]);
-        if (F->ev_join[lg]) cudaEventDestroy(F->ev_join[lg]);
-    }
+    cudaFree(F->d_plan);
+    cudaFree(F->d_mids);
+    for (auto* d : F->d_wtab) cudaFree(d);
+    for (auto* d : F->d_ns) cudaFree(d);
+    if (F->side) cudaStreamDestroy(F->side);
+    if (F->ev_join) cudaEventDestroy(F->ev_join);
     if (F->ev_fork) cudaEventDestroy(F->ev_fork);
     if (F->graph) cudaGraphExecDestroy(F->graph);
     if (F->cycle) cudaGraphExecDestroy(F->cycle);
@@ -2682,13 +1541,7 @@ void factored_free(bdc_handle* H) {
     cudaFree(F->snap0);
     cudaFree(F->snap1);
     for (Launch* L : {&F->ul, &F->vr, &F->g}) free_launch(*L);
-    for (int lg = 0; lg < 8; ++lg) {
-        free_launch(F->mq[lg]);
-        free_launch(F->md[lg]);
-    }
-    cudaFree(F->d_fold);
     ozaki_free(F->oz);
-    for (auto* d : F->d_dm) cudaFree(d);
     delete F;
     H->fac = nullptr;
 }
@@ -2712,20 +1565,12 @@ static BaEpilogue make_epilogue(bdc_handle* H) {
 
 // the stages of one iteration (enum Stage), each gated by DevState::done / error
 
-// the fused q side split in two: the terms of fewer than 8 small outputs
-// (k_qthin) on a branch beside those of 8 to 64 (k_qthin_mma); neither fills
-// the GPU alone
-static cudaError_t enqueue_qthin_split(bdc_handle* H, cudaStream_t s, const DevState* st) {
-    FactoredState* F = H->fac;
-    cudaError_t e;
-    if (F->n_ql) {
-        if ((e = cudaEventRecord(F->ev_fork, s)) != cudaSuccess) return e;
-        if ((e = cudaStreamWaitEvent(F->side[1], F->ev_fork, 0)) != cudaSuccess) return e;
-        if ((e = launch_qthin(F->d_ql, F->n_ql, F->ql_stage, F->side[1], st)) != cudaSuccess) return e;
-        if ((e = cudaEventRecord(F->ev_join[1], F->side[1])) != cudaSuccess) return e;
-    }
-    if ((e = launch_qthin_mma(F->d_qm, F->n_qm, F->qm_stage, s, st)) != cudaSuccess) return e;
-    return F->n_ql ? cudaStreamWaitEvent(s, F->ev_join[1], 0) : cudaSuccess;
+// acc = the sum of nparts vectors of 2^k -> ln q
+static cudaError_t launch_fold(bdc_handle* H, const double* parts, int nparts, cudaStream_t s) {
+    const FactoredState* F = H->fac;
+    k_words_fold<<<F->n_mids, kFoldThreads, 0, s>>>(parts, nparts, H->k, H->inv_c, F->d_mids, F->lnq_full, H->d_lnq,
+                                                   H->d_st);
+    return cudaGetLastError();
 }
 
 static cudaError_t enqueue_stage(bdc_handle* H, int stage, double a) {
@@ -2736,69 +1581,16 @@ static cudaError_t enqueue_stage(bdc_handle* H, int stage, double a) {
         case ST_QBIG: {
             // U and V are independent: V runs on a branch beside U
             if ((e = cudaEventRecord(F->ev_fork, s)) != cudaSuccess) return e;
-            if ((e = cudaStreamWaitEvent(F->side[0], F->ev_fork, 0)) != cudaSuccess) return e;
-            if ((e = launch_store(F->vr, F->side[0], H->d_st)) != cudaSuccess) return e;
-            if ((e = cudaEventRecord(F->ev_join[0], F->side[0])) != cudaSuccess) return e;
+            if ((e = cudaStreamWaitEvent(F->side, F->ev_fork, 0)) != cudaSuccess) return e;
+            if ((e = launch_store(F->vr, F->side, H->d_st)) != cudaSuccess) return e;
+            if ((e = cudaEventRecord(F->ev_join, F->side)) != cudaSuccess) return e;
             if ((e = launch_store(F->ul, s, H->d_st)) != cudaSuccess) return e;
-            if ((e = cudaStreamWaitEvent(s, F->ev_join[0], 0)) != cudaSuccess) return e;
-            const int64_t na = (int64_t)F->KL * F->H2, nb = (int64_t)F->H1h * F->KR;
-            k_sum_parts<<<H->num_sms * 4, 256, 0, s>>>(F->ulpart, F->S1, F->KL > 0 ? na : 0, F->UL, F->vrpart,
-                                                       F->S2, F->KR > 0 ? nb : 0, F->VR, H->d_st);
-            break;
+            return cudaStreamWaitEvent(s, F->ev_join, 0);
         }
-        case ST_QSMALL:
-            if (F->use_qf && F->use_qm) return enqueue_qthin_split(H, s, H->d_st);
-            if (F->use_qf) return launch_qthin(F->d_qf, F->n_qf, F->qf_stage, s, H->d_st);
-            // fork: each size class on its own branch, joined before the fold
-            if ((e = cudaEventRecord(F->ev_fork, s)) != cudaSuccess) return e;
-            for (int lg = 0; lg < 8; ++lg) {
-                if (!F->n_thinq[lg]) continue;
-                if ((e = cudaStreamWaitEvent(F->side[lg], F->ev_fork, 0)) != cudaSuccess) return e;
-                e = F->use_mq[lg] ? launch_store(F->mq[lg], F->side[lg], H->d_st)
-                                  : launch_thin_q(lg, F->d_thinq[lg], F->n_thinq[lg], 1 << H->k, F->side[lg], H->d_st);
-                if (e != cudaSuccess) return e;
-                if ((e = cudaEventRecord(F->ev_join[lg], F->side[lg])) != cudaSuccess) return e;
-                if ((e = cudaStreamWaitEvent(s, F->ev_join[lg], 0)) != cudaSuccess) return e;
-            }
-            break;
-        case ST_FOLD: {
-            const int ny = 1 << H->k;
-            const int nqs = (F->T * ny + 255) / 256;
-            k_qsum<<<nqs < 4096 ? nqs : 4096, 256, 0, s>>>(F->d_fold, F->T, F->qparts, H->k, F->qsum, H->d_st);
-            k_fold_acc<<<(ny + 31) / 32, 256, 0, s>>>(F->d_fold, F->T, F->qsum, F->UL, F->KL, F->VR, F->KR,
-                                                       F->H1h, F->row0, H->k, F->qacc, H->d_st);
-            k_fold_q<<<(ny + 127) / 128, 128, 0, s>>>(F->d_fold, F->T, F->qacc, H->k, H->inv_c, F->lnq_full,
-                                                       H->d_lnq, F->RB, F->H2, F->LA, F->Kp, F->KL, F->H1h, F->row0,
-                                                       H->d_st);
-            break;
-        }
+        case ST_QSMALL: return launch_words(true, F, s, H->d_st);
+        case ST_FOLD: return launch_fold(H, F->qparts, F->plan.ctas, s);
         case ST_DSMALL:
-            if ((e = cudaEventRecord(F->ev_fork, s)) != cudaSuccess) return e;
-            if (F->use_df) {
-                // one launch per output-tile width, each on its own branch
-                for (int cl = 0; cl < 4; ++cl) {
-                    if (!F->n_df[cl]) continue;
-                    if ((e = cudaStreamWaitEvent(F->side[cl], F->ev_fork, 0)) != cudaSuccess) return e;
-                    e = F->use_dm[cl]
-                            ? launch_dthin_mma(F->d_dm[cl], F->n_dm[cl], F->dm_smem[cl], F->lnq_full, F->side[cl], H->d_st)
-                            : launch_dthin(F->d_df[cl], F->n_df[cl], 1 << cl, H->k, F->lnq_full, F->side[cl], H->d_st);
-                    if (e != cudaSuccess) return e;
-                    if ((e = cudaEventRecord(F->ev_join[cl], F->side[cl])) != cudaSuccess) return e;
-                    if ((e = cudaStreamWaitEvent(s, F->ev_join[cl], 0)) != cudaSuccess) return e;
-                }
-                if (F->use_oz) return ozaki_prepare(F->oz, H->d_st, s);
-                break;
-            }
-            for (int lg = 0; lg < 8; ++lg) {
-                if (!F->n_thind[lg]) continue;
-                if ((e = cudaStreamWaitEvent(F->side[lg], F->ev_fork, 0)) != cudaSuccess) return e;
-                e = F->use_md[lg] ? launch_store(F->md[lg], F->side[lg], H->d_st)
-                                  : launch_thin_d(lg, F->d_thind[lg], F->n_thind[lg], F->ctas_thind[lg], 1 << H->k,
-                                                  F->lnq_full, F->side[lg], H->d_st);
-                if (e != cudaSuccess) return e;
-                if ((e = cudaEventRecord(F->ev_join[lg], F->side[lg])) != cudaSuccess) return e;
-                if ((e = cudaStreamWaitEvent(s, F->ev_join[lg], 0)) != cudaSuccess) return e;
-            }
+            if ((e = launch_words(false, F, s, H->d_st)) != cudaSuccess) return e;
             if (F->use_oz) return ozaki_prepare(F->oz, H->d_st, s);
             break;
         case ST_G:
@@ -2891,10 +1683,7 @@ bdc_status factored_shard_q(bdc_handle* H, double* acc) {
     BDC_CUDA_TRY(enqueue_stage(H, ST_QBIG, -INFINITY));
     BDC_CUDA_TRY(enqueue_stage(H, ST_QSMALL, -INFINITY));
     const int ny = 1 << H->k;
-    const int nqs = (F->T * ny + 255) / 256;
-    k_qsum<<<nqs < 4096 ? nqs : 4096, 256, 0, s>>>(F->d_fold, F->T, F->qparts, H->k, F->qsum, H->d_st);
-    k_fold_acc<<<(ny + 31) / 32, 256, 0, s>>>(F->d_fold, F->T, F->qsum, F->UL, F->KL, F->VR, F->KR, F->H1h, F->row0,
-                                               H->k, F->qacc, H->d_st);
+    k_words_acc<<<(ny + 255) / 256, 256, 0, s>>>(F->qparts, F->plan.parts_l, F->plan.ctas, H->k, F->qacc);
     BDC_CUDA_TRY(cudaGetLastError());
     BDC_CUDA_TRY(cudaMemcpyAsync(acc, F->qacc, sizeof(double) * ny, cudaMemcpyDeviceToHost, s));
     BDC_CUDA_TRY(cudaStreamSynchronize(s));
@@ -2908,9 +1697,7 @@ bdc_status factored_shard_d(bdc_handle* H, const double* acc, double* part5) {
     cudaStream_t s = H->stream;
     const int ny = 1 << H->k;
     BDC_CUDA_TRY(cudaMemcpyAsync(F->qacc, acc, sizeof(double) * ny, cudaMemcpyHostToDevice, s));
-    k_fold_q<<<(ny + 127) / 128, 128, 0, s>>>(F->d_fold, F->T, F->qacc, H->k, H->inv_c, F->lnq_full, H->d_lnq, F->RB,
-                                              F->H2, F->LA, F->Kp, F->KL, F->H1h, F->row0, H->d_st);
-    BDC_CUDA_TRY(cudaGetLastError());
+    BDC_CUDA_TRY(launch_fold(H, F->qacc, 1, s));
     BDC_CUDA_TRY(enqueue_stage(H, ST_DSMALL, -INFINITY));
     BDC_CUDA_TRY(enqueue_stage(H, ST_G, -INFINITY));
     const int nb = F->use_oz ? ozaki_partials(F->oz) : F->ctas_g;
