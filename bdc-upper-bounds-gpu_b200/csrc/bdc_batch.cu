@@ -58,7 +58,7 @@ static bdc_status batch_capture(bdc_batch* B, double a) {
         e = cudaStreamWaitEvent(B->lanes[i], B->fork, 0);
         cudaStream_t keep = H->stream;
         H->stream = B->lanes[i];
-        for (int it = 0; it < kBatchIters && e == cudaSuccess; ++it) e = engine_enqueue_iteration(H, a);
+        if (e == cudaSuccess) e = engine_enqueue_iterations(H, a, kBatchIters);
         H->stream = keep;
         if (e == cudaSuccess) e = cudaEventRecord(B->joins[i], B->lanes[i]);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(B->origin, B->joins[i], 0);
@@ -225,7 +225,7 @@ bdc_status bdc_batch_iterate(bdc_batch_t B, int64_t max_iters, double a, bdc_sta
                 if (H->h_st->done) continue;
                 cudaStream_t keep = H->stream;
                 H->stream = B->launch;
-                cudaError_t e = engine_enqueue_iteration(H, a);
+                cudaError_t e = engine_enqueue_iterations(H, a, 1);
                 H->stream = keep;
                 BDC_CUDA_TRY(e);
             }

@@ -535,9 +535,11 @@ bdc_status engine_bound_error(bdc_handle* H, double* ub_err_bits, double* rate_e
     return BDC_OK;
 }
 
-cudaError_t engine_enqueue_iteration(bdc_handle* H, double a) {
-    if (H->engine == BDC_ENGINE_FACTORED) return factored_enqueue_iteration(H, a);
-    return enqueue_count_iteration(H, a);
+cudaError_t engine_enqueue_iterations(bdc_handle* H, double a, int iters) {
+    if (H->engine == BDC_ENGINE_FACTORED) return factored_enqueue_iterations(H, a, iters);
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < iters && e == cudaSuccess; ++i) e = enqueue_count_iteration(H, a);
+    return e;
 }
 
 bdc_status engine_iterate(bdc_handle* H, int64_t max_iters, double a, bdc_stats* stats) {

@@ -82,7 +82,7 @@ bdc_status engine_bound_error(bdc_handle* H, double* ub_err_bits, double* rate_e
 CountLaunch count_launch(const bdc_handle* H);
 UpdateLaunch update_launch(const bdc_handle* H, double a);
 bdc_status engine_profile(bdc_handle* H, int iters, bdc_profile_t* out);
-cudaError_t engine_enqueue_iteration(bdc_handle* H, double a);  // one iteration, gated by done
+cudaError_t engine_enqueue_iterations(bdc_handle* H, double a, int iters);  // gated by done
 int count_group_size(int k);
 
 // factored engine (bdc_factored.cu)
@@ -119,7 +119,7 @@ double factored_acc_eta();
 bdc_status factored_acc_start(bdc_handle* H, double gap_bits);
 bdc_status factored_acc_buffers(bdc_handle* H);  // the loop's snapshot vectors (before any capture)
 cudaError_t factored_enqueue_acc_steps(bdc_handle* H, int steps, double eta);
-cudaError_t factored_enqueue_iteration(bdc_handle* H, double a);
+cudaError_t factored_enqueue_iterations(bdc_handle* H, double a, int iters);
 // finishes an iteration that stopped on an exp-shift overflow (on H->stream);
 // any other device error is returned as BDC_ERR_NUMERIC
 bdc_status factored_recover(bdc_handle* H, double a);

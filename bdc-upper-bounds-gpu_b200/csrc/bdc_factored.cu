@@ -42,6 +42,7 @@
 
 #include <cstring>
 
+#include "bdc_direct.cuh"
 #include "bdc_engine.cuh"
 #include "bdc_gemm.cuh"
 #include "bdc_mma.cuh"
@@ -102,6 +103,11 @@ struct FactoredState {
     int* d_mids = nullptr;    // the fold's middles, one per CTA
     int n_mids = 0;
     double* lnq_full = nullptr;  // [2^k]
+    // small problems: the iteration straight from the folded matrix (bdc_direct.cuh)
+    bool direct = false;
+    bdc::DirectPlan dp{};
+    int d_lpx = 0, d_m = 1, d_grid = 0;
+    double* d_members = nullptr;
     double* epart = nullptr;  // [ctas][8]
     int ctas_g = 0;
     bdc::OzakiG* oz = nullptr;  // G on the int8 tensor cores (when set up and chosen)
@@ -478,35 +484,7 @@ k_fac_finalize(const double* __restrict__ part, int nb, double a, double eta, De
         __syncthreads();
     }
     if (threadIdx.x != 0) return;
-    mD = red[0][0];
-    sE = red[1][0];
-    mL = red[2][0];
-    sR = red[3][0];
-    st->zero_p = (red[4][0] != 0.0);
-    if (!(sE > 0.0) || !isfinite(sE) || mL > 600.0 || mL < -600.0) {
-        st->error = kErrShift;  // e over/underflowed: re-scale from Lt, then finish
-        st->max_logw = mL;      // relative to shift; k_fac_rescale subtracts it
-        st->max_d = mD;
-        st->rate = sR;
-        return;
-    }
-    // Lt holds ln p + eta D - shift, so ln p' - ln p = eta D - shift - ln Z
-    const double lnz = log(sE);
-    const double ln2 = 0.69314718055994530942;
-    const double mx = st->zero_p ? INFINITY : (eta * mD - st->shift - lnz) / ln2;
-    st->max_d = mD;
-    st->rate = sR;
-    st->best_ub = fmin(st->best_ub, mD);
-    st->best_rate = fmax(st->best_rate, sR);
-    st->lse = st->shift + lnz;
-    st->mx = mx;
-    st->max_logw = mL + st->shift;
-    st->log_z = lnz;
-    // next shift: the largest new ln p plus eta times the current bound on D
-    st->shift = (mL - lnz) + eta * mD;
-    st->zero_p = 0;
-    st->iter += 1;
-    st->done = !(mx >= a);
+    fac_finish(red[0][0], red[1][0], red[2][0], red[3][0], red[4][0], a, eta, st);
 }
 
 // re-scale after an exp over/underflow: Lt -= s, Pw = |O| exp(Lt), sum
@@ -1084,6 +1062,128 @@ bool factored_supports(int n, int k) {
 
 static BaEpilogue make_epilogue(bdc_handle* H);
 
+// ------------------------------------------------------- small problems
+// The direct iteration (bdc_direct.cuh) where the folded matrix has 16-bit
+// entries, at most 512 output representatives and kDirectBytes in all.
+constexpr int64_t kDirectBytes = 40ll << 20;
+constexpr int64_t kDirectReps = 600000;
+// one CTA runs a problem of up to this many passes over its rows (more
+// iterations per launch), more CTAs share a larger one
+constexpr int kDirectSoloPasses = 6;
+
+static int64_t orbit_count(int len) {  // orbits of {id, rev, comp, rev comp} on `len`-bit words
+    if (len == 0) return 1;
+    return ((1ll << len) + (1ll << ((len + 1) / 2)) + ((len % 2 == 0) ? (1ll << (len / 2)) : 0)) / 4;
+}
+
+static bool direct_supports(const bdc_handle* H) {
+    const int64_t ny = (orbit_count(H->k) + 7) / 8 * 8;
+    return H->shard_world == 1 && H->k <= 10 && H->C < 65536.0 && H->R <= kDirectReps && H->R * ny * 2 <= kDirectBytes;
+}
+
+template <bool SOLO, typename F>
+static cudaError_t direct_kernel(int lpx, int m, F&& f) {
+    switch (m * 32 + lpx) {
+        case 32 + 1: return f(k_direct<1, 1, SOLO>, direct_smem(1, 1));
+        case 32 + 2: return f(k_direct<2, 1, SOLO>, direct_smem(2, 1));
+        case 96 + 1: return f(k_direct<1, 3, SOLO>, direct_smem(1, 3));
+        case 96 + 2: return f(k_direct<2, 3, SOLO>, direct_smem(2, 3));
+        case 96 + 4: return f(k_direct<4, 3, SOLO>, direct_smem(4, 3));
+        case 96 + 8: return f(k_direct<8, 3, SOLO>, direct_smem(8, 3));
+        case 96 + 16: return f(k_direct<16, 3, SOLO>, direct_smem(16, 3));
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+static cudaError_t launch_direct(bdc_handle* H, int what, int slot, int iters, double a) {
+    FactoredState* F = H->fac;
+    auto go = [&](auto* k, int smem) {
+        k<<<F->d_grid, kDirectThreads, smem, H->stream>>>(F->dp, what, slot, iters, a, F->eta, F->dout, H->d_st);
+        return cudaGetLastError();
+    };
+    return F->d_grid == 1 ? direct_kernel<true>(F->d_lpx, F->d_m, go) : direct_kernel<false>(F->d_lpx, F->d_m, go);
+}
+
+// `iters` iterations from the current state: one launch with one CTA; else
+// one for the first q, one per iteration and one for the last state
+static cudaError_t enqueue_direct(bdc_handle* H, double a, int iters) {
+    FactoredState* F = H->fac;
+    if (iters < 1) return cudaSuccess;
+    if (F->d_grid == 1) return launch_direct(H, kDirectQ | kDirectD, 0, iters, a);
+    cudaError_t e = launch_direct(H, kDirectQ, 0, 0, a);
+    // (iters > 0 in the kernel: the slot holds an update's statistics)
+    for (int i = 0; i < iters && e == cudaSuccess; ++i)
+        e = launch_direct(H, i + 1 < iters ? kDirectQ | kDirectD : kDirectD, i & 1, i, a);
+    if (e != cudaSuccess) return e;
+    k_direct_finish<<<1, 160, 0, H->stream>>>(F->dp.slot[iters & 1], F->d_grid, a, F->eta, H->d_st);
+    return cudaGetLastError();
+}
+
+static bdc_status direct_init(bdc_handle* H) {
+    FactoredState* F = H->fac;
+    DirectPlan& P = F->dp;
+    std::vector<uint32_t> yreps;
+    std::vector<double> members;
+    for (uint32_t y = 0; y < (1u << H->k); ++y) {
+        if (!is_rep(y, H->k)) continue;
+        uint32_t img[4] = {y, reverse_bits(y, H->k), complement_bits(y, H->k), 0};
+        img[3] = reverse_bits(img[2], H->k);
+        std::sort(img, img + 4);
+        members.push_back((double)(std::unique(img, img + 4) - img));
+        yreps.push_back(y);
+    }
+    P.NY = (int)yreps.size();
+    P.NYp = (P.NY + 7) / 8 * 8;
+    members.resize(P.NYp, 1.0);
+    const int pieces = P.NYp / 8;
+    // lanes and pieces a lane with the fewest idle slots: k <= 4 has 1 piece,
+    // k = 5 .. 10 have 2, 3, 5, 9, 17, 34
+    F->d_m = pieces <= 2 ? 1 : 3;
+    F->d_lpx = 1;
+    while (F->d_lpx * F->d_m < pieces) F->d_lpx *= 2;
+    const int per_pass = kDirectWarps * (32 / F->d_lpx) * (F->d_m == 1 ? std::min(F->d_lpx, 4) : std::min(F->d_lpx, 2));
+    const int64_t passes = (H->R + per_pass - 1) / per_pass;
+    F->d_grid = passes <= kDirectSoloPasses ? 1 : (int)std::min<int64_t>(passes, H->num_sms);
+    P.R = H->R;
+    P.reps = H->d_reps;
+    P.Lt = F->Lt;
+    P.Pw = F->Pw;
+    P.hx = F->hx;
+    P.inv_c = H->inv_c;
+    P.n = H->n;
+    P.n2 = H->s.n2;
+    uint16_t* T = nullptr;
+    uint32_t* d_y = nullptr;
+    const size_t tb = (size_t)H->R * P.NYp * sizeof(uint16_t), vb = sizeof(double) * P.NYp;
+    BDC_CUDA_TRY(cudaMalloc(&T, tb));
+    P.T = T;
+    BDC_CUDA_TRY(cudaMalloc(&F->d_members, vb));
+    P.members = F->d_members;
+    for (DirectSlot& S : P.slot) {
+        BDC_CUDA_TRY(cudaMalloc(&S.part, vb * F->d_grid));
+        BDC_CUDA_TRY(cudaMalloc(&S.stat, sizeof(double) * 8 * F->d_grid));
+        BDC_CUDA_TRY(cudaMalloc(&S.state, sizeof(DevState)));
+    }
+    H->bytes += tb + vb * (2 * F->d_grid + 1);
+    BDC_CUDA_TRY(cudaMemcpy(F->d_members, members.data(), vb, cudaMemcpyHostToDevice));
+    BDC_CUDA_TRY(cudaMalloc(&d_y, sizeof(uint32_t) * yreps.size()));
+    BDC_CUDA_TRY(cudaMemcpy(d_y, yreps.data(), sizeof(uint32_t) * yreps.size(), cudaMemcpyHostToDevice));
+    k_direct_table<<<H->num_sms * 8, 256, 0, H->stream>>>(H->s, H->A, H->B, H->d_reps, H->R, d_y, P.NY, P.NYp, T);
+    BDC_CUDA_TRY(cudaGetLastError());
+    auto attr = [&](auto* k, int smem) {
+        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    };
+    BDC_CUDA_TRY(direct_kernel<true>(F->d_lpx, F->d_m, attr));
+    BDC_CUDA_TRY(direct_kernel<false>(F->d_lpx, F->d_m, attr));
+    BDC_CUDA_TRY(cudaStreamSynchronize(H->stream));
+    cudaFree(d_y);
+    F->launches_per_iter = 1;
+    if (H->verbose)
+        printf("bdc: direct iteration: %d output representatives, %.1f MB, %d lanes a row, %d CTAs\n", P.NY,
+               tb / 1048576.0, F->d_lpx, F->d_grid);
+    return BDC_OK;
+}
+
 bdc_status factored_init(bdc_handle* H) {
     BDC_CUDA_TRY(set_smem_attrs());
     FactoredState* F = new FactoredState();
@@ -1160,6 +1260,17 @@ bdc_status factored_init(bdc_handle* H) {
     BDC_CUDA_TRY(al(&F->Pw, NX));
     BDC_CUDA_TRY(al(&F->Lt, NX));
     BDC_CUDA_TRY(al(&F->hx, NX));
+    if (direct_supports(H)) {
+        F->direct = true;
+        BDC_CUDA_TRY(cudaMemsetAsync(F->hx, 0, sizeof(double) * NX, H->stream));
+        BDC_CUDA_TRY(cudaMemsetAsync(F->Pw, 0, sizeof(double) * NX, H->stream));
+        BDC_CUDA_TRY(cudaMemsetAsync(F->Lt, 0, sizeof(double) * NX, H->stream));
+        BDC_CUDA_TRY(al(&F->epart, (size_t)H->nb_upd * 8));
+        k_fac_rows<2><<<F->H1h, 256, F->rows_smem, H->stream>>>(F->d_rowstart, H->n, F->row0, H->d_h + F->i0, F->hx,
+                                                                nullptr);
+        BDC_CUDA_TRY(cudaGetLastError());
+        return direct_init(H);
+    }
     BDC_CUDA_TRY(al(&F->LA, (size_t)H1 * Kp));
     BDC_CUDA_TRY(al(&F->RB, (size_t)Kp * H2));
     BDC_CUDA_TRY(al(&F->ulpart, (size_t)max_split * H2 * KL));
@@ -1528,6 +1639,13 @@ void factored_free(bdc_handle* H) {
     cudaFree(F->d_rowstart);
     cudaFree(F->rpart);
     cudaFree(F->d_plan);
+    cudaFree(F->d_members);
+    cudaFree((void*)F->dp.T);
+    for (DirectSlot& S : F->dp.slot) {
+        cudaFree(S.part);
+        cudaFree(S.stat);
+        cudaFree(S.state);
+    }
     cudaFree(F->d_mids);
     for (auto* d : F->d_wtab) cudaFree(d);
     for (auto* d : F->d_ns) cudaFree(d);
@@ -1577,6 +1695,8 @@ static cudaError_t enqueue_stage(bdc_handle* H, int stage, double a) {
     FactoredState* F = H->fac;
     cudaStream_t s = H->stream;
     cudaError_t e = cudaSuccess;
+    // (a direct iteration is timed as a whole)
+    if (F->direct) return stage == ST_G ? enqueue_direct(H, a, 1) : cudaSuccess;
     switch (stage) {
         case ST_QBIG: {
             // U and V are independent: V runs on a branch beside U
@@ -1603,15 +1723,21 @@ static cudaError_t enqueue_stage(bdc_handle* H, int stage, double a) {
     return cudaGetLastError();
 }
 
-static cudaError_t enqueue_iteration(bdc_handle* H, double a) {
-    for (int st = 0; st < ST_COUNT; ++st) {
-        cudaError_t e = enqueue_stage(H, st, a);
-        if (e != cudaSuccess) return e;
+static cudaError_t enqueue_iterations(bdc_handle* H, double a, int iters) {
+    if (H->fac->direct) return enqueue_direct(H, a, iters);
+    for (int i = 0; i < iters; ++i) {
+        for (int st = 0; st < ST_COUNT; ++st) {
+            cudaError_t e = enqueue_stage(H, st, a);
+            if (e != cudaSuccess) return e;
+        }
     }
     return cudaSuccess;
 }
 
-cudaError_t factored_enqueue_iteration(bdc_handle* H, double a) { return enqueue_iteration(H, a); }
+static cudaError_t enqueue_iteration(bdc_handle* H, double a) { return enqueue_iterations(H, a, 1); }
+
+cudaError_t factored_enqueue_iterations(bdc_handle* H, double a, int iters) { return enqueue_iterations(H, a, iters); }
+
 
 // the first shift's inputs over every representative (as k_fac_load writes
 // them for its own): a shard sets the same p on every rank, so each one
@@ -1874,7 +2000,7 @@ static bdc_status ensure_graph(bdc_handle* H, double a) {
     BDC_CUDA_TRY(cudaStreamSynchronize(keep));
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(H->own_stream, cudaStreamCaptureModeThreadLocal);
-    for (int i = 0; i < kGraphIters && e == cudaSuccess; ++i) e = enqueue_iteration(H, a);
+    e = e == cudaSuccess ? enqueue_iterations(H, a, kGraphIters) : e;
     cudaError_t e2 = cudaStreamEndCapture(H->own_stream, &g);
     H->stream = keep;
     if (e == cudaSuccess) e = e2;
@@ -1890,20 +2016,24 @@ bdc_status factored_iterate(bdc_handle* H, int64_t max_iters, double a, bdc_stat
     BDC_CUDA_TRY(cudaMemsetAsync(&H->d_st->done, 0, sizeof(int), H->stream));
     const long long it0 = H->h_st->iter;
     long long target = it0 + max_iters;
-    int64_t chunk = 1;
+    // the host reads the state after a chunk: chunks grow from 8 (iterations
+    // past convergence cost their launches only), or start at the largest
+    // when no threshold can end the loop
+    int64_t chunk = a == -INFINITY ? 256 : 8;
     for (int guard = 0; guard < 1000000; ++guard) {
         const long long done_iters = H->h_st->iter;
         const int64_t remaining = target - done_iters;
         if (remaining <= 0) break;
         const int64_t c = chunk < remaining ? chunk : remaining;
         // whole graphs for the bulk of the chunk, single iterations for the rest
-        const int64_t ng = (c >= kGraphIters) ? c / kGraphIters : 0;
+        const bool solo = F->direct && F->d_grid == 1;  // one launch runs them all
+        const int64_t ng = (c >= kGraphIters && !solo) ? c / kGraphIters : 0;
         if (ng > 0) {
             bdc_status rc = ensure_graph(H, a);
             if (rc != BDC_OK) return rc;
         }
         for (int64_t i = 0; i < ng; ++i) BDC_CUDA_TRY(cudaGraphLaunch(F->graph, H->stream));
-        for (int64_t i = ng * kGraphIters; i < c; ++i) BDC_CUDA_TRY(enqueue_iteration(H, a));
+        if (c > ng * kGraphIters) BDC_CUDA_TRY(enqueue_iterations(H, a, (int)(c - ng * kGraphIters)));
         BDC_CUDA_TRY(cudaMemcpyAsync(H->h_st, H->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, H->stream));
         BDC_CUDA_TRY(cudaStreamSynchronize(H->stream));
         if (H->h_st->error == kErrShift) {
@@ -2255,10 +2385,10 @@ bdc_status factored_profile(bdc_handle* H, int iters, bdc_profile_t* out) {
     out->ms_iter = tot / iters;
     out->ms_main = acc[ST_G] / iters;
     // algorithmic work of G: one K-long dot product per representative
-    out->work_main = 2.0 * (double)H->R * (double)(F->KL + F->KR);
+    out->work_main = 2.0 * (double)H->R * (double)(F->direct ? F->dp.NY : F->KL + F->KR);
     out->launches = F->launches_per_iter;
     out->iters = iters;
-    out->main_kind = F->use_oz ? 2 : 1;
+    out->main_kind = F->direct ? 3 : F->use_oz ? 2 : 1;
     out->bytes_main = 40.0 * (double)F->Rl;
     return BDC_OK;
 }

@@ -451,7 +451,7 @@ def ours_arm(args) -> None:
         "data": "synthetic (uniform start; the reference publishes no throughput)",
         "config": workload_config(args.n, args.k, R) | {"parallelism": f"replicas x{world}"},
         "engine": E.engine,
-        "g_product": {0: None, 1: "FP64 mma.sync", 2: "int8 tcgen05 (exact split)"}[prof["main_kind"]],
+        "g_product": {0: None, 1: "FP64 mma.sync", 2: "int8 tcgen05 (exact split)"}.get(prof["main_kind"]),
         "gpu_launches": launches_per_iter * args.steps,
         "profile_ms": {k2: prof[k2] for k2 in ("ms_q", "ms_fold", "ms_d", "ms_update", "ms_iter", "ms_main")},
         "roofline": roofline, "roofline_update": roofline_update,
