@@ -238,17 +238,31 @@ bdc_status bdc_accelerate(bdc_handle_t H, int64_t max_evals, double gap_bits, bd
     return factored_accelerate(H, max_evals, gap_bits, stats);
 }
 
-// The factored engine evaluates I(p;W) and D(x) with one BA map (the G
-// product's epilogue yields both); the map advances the dense iterate, which
-// is then reloaded from p so that the handle still holds p.
+// The factored engine evaluates I(p;W) and D(x) by the products of one
+// iteration, without its update.  The iterate afterwards is p as a fresh
+// load holds it: already so right after a load, else p is written out and
+// loaded again.  (A direct handle runs one BA map, which advances the
+// iterate, and reloads p.)
 static bdc_status factored_eval(bdc_handle_t H, bool with_d) {
     const double* cur = nullptr;
-    bdc_status rc = engine_current_p(H, &cur);  // p in d_p[0]
-    if (rc != BDC_OK) return rc;
-    rc = factored_map(H, H->d_p[0], H->d_p[1], with_d ? H->d_d : nullptr);
-    if (rc != BDC_OK) return rc;
-    const double rate = H->h_st->rate;
-    rc = engine_after_set_p(H);
+    double rate = 0.0;
+    bdc_status rc;
+    if (factored_has_passes(H)) {
+        const bool fresh = H->h_st->iter == 0 && !H->strict_load;
+        rc = factored_evaluate(H, with_d ? H->d_d : nullptr, &rate);
+        if (rc != BDC_OK) return rc;
+        if (!fresh) {
+            rc = engine_current_p(H, &cur);
+            if (rc == BDC_OK) rc = engine_after_set_p(H);
+        }
+    } else {
+        rc = engine_current_p(H, &cur);  // p in d_p[0]
+        if (rc != BDC_OK) return rc;
+        rc = factored_map(H, H->d_p[0], H->d_p[1], with_d ? H->d_d : nullptr);
+        if (rc != BDC_OK) return rc;
+        rate = H->h_st->rate;
+        rc = engine_after_set_p(H);
+    }
     H->h_st->rate = rate;
     return rc;
 }

@@ -392,6 +392,7 @@ bdc_status engine_after_set_p(bdc_handle* H, int strict_zero) {
     bdc_status rc = reset_state(H);
     if (rc != BDC_OK) return rc;
     H->p_set = true;
+    H->strict_load = strict_zero != 0;
     if (H->engine == BDC_ENGINE_FACTORED) {
         rc = factored_load_p(H, strict_zero);
         if (rc != BDC_OK) return rc;
@@ -412,6 +413,8 @@ bdc_status engine_current_p(bdc_handle* H, const double** p) {
 }
 
 bdc_status engine_log_q(bdc_handle* H) {
+    // the factored products where there are any (24/12: 36 ms on the count path, 0.1 ms here)
+    if (factored_has_passes(H)) return factored_log_q(H);
     const double* p = nullptr;
     bdc_status rc = engine_current_p(H, &p);
     if (rc != BDC_OK) return rc;
@@ -422,6 +425,7 @@ bdc_status engine_log_q(bdc_handle* H) {
 }
 
 bdc_status engine_divergence(bdc_handle* H) {
+    if (factored_has_passes(H)) return factored_divergence(H);
     const CountLaunch L = count_launch(H);
     BDC_CUDA_TRY(launch_dpass(L, H->d_lnq, H->d_h, H->inv_c, H->log_c, H->d_d, H->d_st, 0));
     return BDC_OK;

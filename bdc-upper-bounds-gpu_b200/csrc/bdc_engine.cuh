@@ -56,6 +56,7 @@ struct bdc_handle {
     int grid_count = 0;
     int nb_upd = 0;
     bool p_set = false;
+    bool strict_load = false;  // the last load kept exact zeros at ln p = -inf (engine_after_set_p)
     int64_t nonzero_pairs = 0;  // sum over reps of distinct length-k subsequences
     // factored engine
     FactoredState* fac = nullptr;
@@ -124,6 +125,11 @@ cudaError_t factored_enqueue_iterations(bdc_handle* H, double a, int iters);
 // any other device error is returned as BDC_ERR_NUMERIC
 bdc_status factored_recover(bdc_handle* H, double a);
 bdc_status factored_map(bdc_handle* H, const double* p_in, double* p_out, double* D_out);
+// passes at the current iterate (handles with products), the state untouched
+bool factored_has_passes(const bdc_handle* H);
+bdc_status factored_log_q(bdc_handle* H);
+bdc_status factored_divergence(bdc_handle* H);
+bdc_status factored_evaluate(bdc_handle* H, double* D_out, double* rate);
 // Device buffers for dgemm_nt: one product descriptor and a tile map (every
 // tile on descriptor 0) of up to `tiles` 64x64 tiles, allocated once by the
 // caller and reused by every call on one stream.

@@ -262,7 +262,14 @@ __global__ void __launch_bounds__(256, (BM * BN <= 4096) ? 3 : 2) k_mma_ba(const
                 if (!is_rep(x, ep.n)) continue;
                 const double o = (double)orbit_size(x, ep.n);
                 const double D = __ldg(ep.hx + xd) - acc[i][j][h] * ep.inv_c;
-                if (WITH_D) ep.Dout[xd] = D;
+                if (WITH_D) {
+                    if (ep.Dout) ep.Dout[xd] = D;
+                    if (!ep.Lt) {  // an evaluation: no update
+                        mD = fmax(mD, D);
+                        sR = fma(ep.Pw[xd] * inv_z, D, sR);
+                        continue;
+                    }
+                }
                 // an entry that is exactly 0 in the caller's distribution (Lt
                 // holds NaN) takes ln p = 0, as the reference's apply_log_kernel
                 // leaves ln 0 at 0 (backend/BAA.cu:573-580); later iterates keep
@@ -435,7 +442,7 @@ static cudaError_t launch_store(const Launch& L, cudaStream_t s, const DevState*
 // G: A = [A_L | N_R] contiguous along the contraction, B = [M_L ; B_R^T]
 // contiguous along the output columns: the cp.async mainloop with layout 2
 static cudaError_t launch_ba(const Launch& L, const BaEpilogue& ep, cudaStream_t s, const DevState* st) {
-    const bool wd = ep.Dout != nullptr, cp = L.layout == 2;
+    const bool wd = ep.Dout != nullptr || !ep.Lt, cp = L.layout == 2;
     const int sm = cfg_smem(L.cfg, cp ? 2 : -1);
     const int grid = (L.grid > 0 && L.grid < L.tiles) ? L.grid : L.tiles;
 #define GO_(ARGS)                                                                                        \
@@ -1775,8 +1782,8 @@ __global__ void __launch_bounds__(256) k_lnp_all(const double* __restrict__ p, i
 
 bdc_status factored_load_p(bdc_handle* H, int strict_zero) {
     FactoredState* F = H->fac;
-    const int64_t NX = (int64_t)F->H1h * F->H2;  // the dense rows held
-    BDC_CUDA_TRY(cudaMemsetAsync(F->Pw, 0, sizeof(double) * NX, H->stream));
+    // (Pw is zero away from the representatives from set-up on: every kernel
+    // writes it only there, and the load rewrites all of them)
     const int nb = H->nb_upd;
     k_fac_load_rows<<<F->H1h, 256, F->rows_smem, H->stream>>>(F->d_rowstart, H->n, F->row0, H->d_p[0] + F->i0, F->Pw,
                                                               F->Lt, F->rpart, strict_zero);
@@ -1788,6 +1795,89 @@ bdc_status factored_load_p(bdc_handle* H, int strict_zero) {
         k_fac_load_finish<<<1, 32, 0, H->stream>>>(F->rpart, F->H1h, H->k, H->d_st);
     }
     BDC_CUDA_TRY(cudaGetLastError());
+    return BDC_OK;
+}
+
+// ------------------------------------------------ passes at the current p
+// ln q over every y from the representatives' slots
+__global__ void k_lnq_expand(int k, const double* __restrict__ lnq, double* __restrict__ lnq_full) {
+    const int y = blockIdx.x * blockDim.x + threadIdx.x;
+    if (y < (1 << k)) lnq_full[y] = lnq[orbit_rep((uint32_t)y, k)];
+}
+
+// sum over the block partials of sum |O| p D (the evaluation's rate)
+__global__ void __launch_bounds__(256) k_eval_rate(const double* __restrict__ part, int nb, double* __restrict__ out) {
+    __shared__ double red[8];
+    double s = 0.0;
+    for (int b = threadIdx.x; b < nb; b += 256) s += part[(size_t)b * 8 + 3];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 8; ++w) s += red[w];
+    *out = s;
+}
+
+// whether the passes below run on this handle; a direct one has no products
+// (its passes take the count path)
+bool factored_has_passes(const bdc_handle* H) {
+    return H->engine == BDC_ENGINE_FACTORED && !H->fac->direct && H->shard_world == 1;
+}
+
+// ln q of the current iterate into H->d_lnq (0 in the slots that are no
+// representative's): the q side of an iteration, the state untouched
+bdc_status factored_log_q(bdc_handle* H) {
+    const size_t slots = (size_t)1 << (H->k >= 1 ? H->k - 1 : 0);
+    BDC_CUDA_TRY(cudaMemsetAsync(&H->d_st->done, 0, sizeof(int), H->stream));
+    BDC_CUDA_TRY(cudaMemsetAsync(H->d_lnq, 0, sizeof(double) * slots, H->stream));
+    for (int st : {ST_QBIG, ST_QSMALL, ST_FOLD}) BDC_CUDA_TRY(enqueue_stage(H, st, -INFINITY));
+    return BDC_OK;
+}
+
+// the D side from lnq_full: G with an epilogue that leaves the state alone;
+// D per representative into D_out, or nowhere (nullptr)
+static bdc_status eval_d(bdc_handle* H, double* D_out) {
+    FactoredState* F = H->fac;
+    if (D_out && !F->Ddense) {
+        const size_t bytes = sizeof(double) * (size_t)F->H1h * F->H2;
+        BDC_CUDA_TRY(cudaMalloc(&F->Ddense, bytes));
+        H->bytes += bytes;
+    }
+    BDC_CUDA_TRY(launch_words(false, F, H->stream, H->d_st));
+    BaEpilogue ep = make_epilogue(H);
+    ep.Lt = nullptr;
+    ep.Dout = D_out ? F->Ddense : nullptr;
+    BDC_CUDA_TRY(launch_ba(F->g, ep, H->stream, H->d_st));
+    if (!D_out) return BDC_OK;
+    k_fac_rows<1><<<F->H1h, 256, F->rows_smem, H->stream>>>(F->d_rowstart, H->n, F->row0, F->Ddense, D_out + F->i0,
+                                                            H->d_st);
+    BDC_CUDA_TRY(cudaGetLastError());
+    return BDC_OK;
+}
+
+// D per representative for the ln q in H->d_lnq, into H->d_d
+bdc_status factored_divergence(bdc_handle* H) {
+    FactoredState* F = H->fac;
+    const int ny = 1 << H->k;
+    BDC_CUDA_TRY(cudaMemsetAsync(&H->d_st->done, 0, sizeof(int), H->stream));
+    k_lnq_expand<<<(ny + 255) / 256, 256, 0, H->stream>>>(H->k, H->d_lnq, F->lnq_full);
+    BDC_CUDA_TRY(cudaGetLastError());
+    return eval_d(H, H->d_d);
+}
+
+// I(p;W) of the current iterate (nats) and, with D_out, D per representative:
+// one forward evaluation, the state untouched
+bdc_status factored_evaluate(bdc_handle* H, double* D_out, double* rate) {
+    FactoredState* F = H->fac;
+    bdc_status rc = factored_log_q(H);
+    if (rc == BDC_OK) rc = eval_d(H, D_out);
+    if (rc != BDC_OK) return rc;
+    k_eval_rate<<<1, 256, 0, H->stream>>>(F->epart, F->g.grid > 0 ? std::min(F->g.grid, F->g.tiles) : F->g.tiles,
+                                          H->d_scalar + 5);
+    BDC_CUDA_TRY(cudaGetLastError());
+    BDC_CUDA_TRY(cudaMemcpyAsync(rate, H->d_scalar + 5, sizeof(double), cudaMemcpyDeviceToHost, H->stream));
+    BDC_CUDA_TRY(cudaStreamSynchronize(H->stream));
     return BDC_OK;
 }
 
