@@ -67,6 +67,22 @@ __host__ __device__ __forceinline__ bool is_rep(uint32_t x, int len) {
     return orbit_rep(x, len) == x;
 }
 
+// The same at a dense position (bdc_factored.cu): row r = x_hi (its top bit
+// 0), column c = x_lo reversed, mask = 2^{n2} - 1, odd = n & 1.  The reverse
+// of x starts with c and its complement's with ~c, so comparing x with them
+// compares r (for odd n without its last bit) with c and ~c; where those are
+// equal the rest of the two strings is equal too, but for the middle bit of
+// an odd n, which the complement flips.
+__host__ __device__ __forceinline__ bool dense_is_rep(uint32_t r, uint32_t c, uint32_t mask, uint32_t odd) {
+    const uint32_t rr = r >> odd, cn = c ^ mask;
+    return rr <= c && (rr < cn || (rr == cn && !(odd & r)));
+}
+// orbit size of the representative there
+__host__ __device__ __forceinline__ double dense_orbit(uint32_t r, uint32_t c, uint32_t mask, uint32_t odd) {
+    const uint32_t rr = r >> odd;
+    return (rr == c || (!odd && rr == (c ^ mask))) ? 2.0 : 4.0;
+}
+
 __host__ __device__ inline uint32_t binom(uint32_t n, uint32_t k) {
     if (k > n) return 0;
     if (k > n - k) k = n - k;

@@ -66,7 +66,6 @@ struct Launch {
     int* map = nullptr;      // CTA -> descriptor index
     int n = 0, tiles = 0, cfg = CFG_64x64;
     int layout = -1;         // -1: register-staged mainloop; else the cp.async one (see k_mma_store)
-    int grid = 0;            // G only: CTAs launched (0: one per tile; fewer: each loops over tiles)
 };
 
 }  // namespace bdc
@@ -160,14 +159,9 @@ __host__ __device__ __forceinline__ uint32_t fac_loc(uint32_t x, int n, int row0
     return fac_pos(x, n >> 1) - ((uint32_t)row0 << (n >> 1));
 }
 
-// the string at dense position xd of the held rows (fac_pos is an
-// involution), and whether it is a representative: kernels that touch every
-// representative walk the dense arrays in memory order this way, coalesced,
-// instead of the ascending list (whose positions are bit-reversed in a row)
-__device__ __forceinline__ uint32_t fac_str(uint32_t xd, int n, int row0) {
-    return fac_pos(xd + ((uint32_t)row0 << (n >> 1)), n >> 1);
-}
-
+// Kernels that touch every representative walk the dense arrays in memory
+// order and test the position (dense_is_rep), coalesced, instead of the
+// ascending list (whose positions are bit-reversed in a row).
 
 // ------------------------------------------------ products: plain store
 // LAYOUT < 0: register-staged mainloop (any operand kind); otherwise the
@@ -209,87 +203,105 @@ __global__ void __launch_bounds__(256) k_mma_store(const GemmDesc* __restrict__ 
 // rows are x_hi, columns x_lo, x = (x_hi << n2) | x_lo; only representatives
 // are updated; block partials [max D, sum |O| e, max (logW - shift),
 // sum |O| p D, input-zero flag] go to ep.part[blockIdx.x * 8 + 0..4].
-// CTA b takes the tiles b, b + gridDim.x, ... of the ntiles that hold
-// representatives (one each when the grid covers them all); with the cp.async
-// mainloop the next tile's first stages are in flight during this tile's
-// epilogue.
-template <int BM, int BN, int WM, int WN, bool WITH_D, bool CP>
+// CTA b takes tile tiles[b] of those that hold representatives.  The sums
+// leave the fragments through shared memory (the mainloop's, at a pitch of 8
+// extra doubles: 16-byte stores of a fragment's pair without conflicts), so
+// that the update runs a row at a time with 16-byte loads and stores of two
+// adjacent columns: on the fragments themselves every access touched twice
+// the sectors and the orbit tests and addresses were 2/3 of 210 instructions
+// an element.  84 -> 47 us at 24/12 (135 MB of device memory: 21 us).
+template <int BM, int BN, int WM, int WN, bool WITH_D>
 __global__ void __launch_bounds__(256, (BM * BN <= 4096) ? 3 : 2) k_mma_ba(const GemmDesc* __restrict__ descs, const int* __restrict__ tiles,
-                                                   int ntiles, BaEpilogue ep, const DevState* st) {
+                                                   BaEpilogue ep, const DevState* st) {
     using C = MmaCfg<BM, BN, WM, WN>;
+    constexpr int LD = BN + 8;
     if (gated(st)) return;
     extern __shared__ __align__(16) double smem[];
     const GemmDesc& d = descs[0];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, tq = lane & 3;
     const int wm0 = (warp / WN) * (8 * C::MT), wn0 = (warp % WN) * (8 * C::NT);
-    const double shift = st->shift;
-    const double lnz = st->log_z;
-    const double inv_z = exp(-lnz);
-    double mD = -DBL_MAX, sE = 0.0, mL = -DBL_MAX, sR = 0.0, zero = 0.0;
-    int ti = blockIdx.x;
-    if constexpr (CP) {
-        if (ti < ntiles) {
-            const int t = tiles[ti];
-            mma_cp_prologue<BM, BN, false, true, 3>(d, (t / d.tiles_n) * BM, (t % d.tiles_n) * BN, smem);
-        }
-    }
-    for (; ti < ntiles; ti += gridDim.x) {
-    const int t = tiles[ti];
+    const int t = tiles[blockIdx.x];
     const int m0 = (t / d.tiles_n) * BM, n0 = (t % d.tiles_n) * BN;
-    double acc[C::MT][C::NT][2];
-    if constexpr (CP) {
-        mma_cp_body<BM, BN, WM, WN, false, true, 3>(d, m0, n0, smem, acc);
-        if (ti + (int)gridDim.x < ntiles) {
-            const int tn = tiles[ti + gridDim.x];
-            mma_cp_prologue<BM, BN, false, true, 3>(d, (tn / d.tiles_n) * BM, (tn % d.tiles_n) * BN, smem);
+    const int M = d.M, N = d.N;
+    // the state of the tile on its way to L2 while the products run
+    constexpr int LINES = BM * BN / 16;  // 128-byte lines of one array
+    for (int q = threadIdx.x; q < LINES; q += 256) {
+        const int m = m0 + q / (BN / 16), n = n0 + (q % (BN / 16)) * 16;
+        if (m < M && n < N && dense_is_rep((uint32_t)m + (uint32_t)ep.row0, (uint32_t)n + 8, low_mask(ep.n2), 0u)) {
+            const size_t at = ((size_t)m << ep.n2) + n;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(ep.hx + at));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(ep.Pw + at));
+            if (!WITH_D || ep.Lt) asm volatile("prefetch.global.L2 [%0];" ::"l"(ep.Lt + at));
         }
-    } else {
-        mma_mainloop<BM, BN, WM, WN>(d, m0, n0, smem, acc);
     }
+    {
+        double acc[C::MT][C::NT][2];
+        mma_mainloop_cp<BM, BN, WM, WN, false, true, 3>(d, m0, n0, smem, acc);
+        static_assert(BM * LD * (int)sizeof(double) <= mma_cp_smem_bytes<BM, BN, WM, WN, false, true, 3>(), "tile");
 #pragma unroll
-    for (int i = 0; i < C::MT; ++i) {
-        const int m = m0 + wm0 + i * 8 + g;
-        if (m >= d.M) continue;
+        for (int i = 0; i < C::MT; ++i)
 #pragma unroll
-        for (int j = 0; j < C::NT; ++j)
+            for (int j = 0; j < C::NT; ++j)
+                *reinterpret_cast<double2*>(smem + (wm0 + i * 8 + g) * LD + wn0 + j * 8 + 2 * tq) =
+                    make_double2(acc[i][j][0], acc[i][j][1]);
+    }
+    const BaConst kc = ba_const(ep, st);
+    BaStats bs;
+    __syncthreads();
+    constexpr int SEG = BN / 64, ROWS = BM * SEG;  // 64-column segments of rows, one per warp at a time
+#pragma unroll 1
+    for (int q0 = warp; q0 < ROWS; q0 += 16) {
+        double2 hv[2], lv[2], pv[2];
+        bool r0[2], r1[2];
+        uint32_t xd[2];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int n = n0 + wn0 + j * 8 + 2 * tq + h;
-                if (n >= d.N) continue;
-                const uint32_t xd = ((uint32_t)m << ep.n2) | (uint32_t)n;
-                const uint32_t x = fac_pos(xd + ((uint32_t)ep.row0 << ep.n2), ep.n2);
-                if (!is_rep(x, ep.n)) continue;
-                const double o = (double)orbit_size(x, ep.n);
-                const double D = __ldg(ep.hx + xd) - acc[i][j][h] * ep.inv_c;
-                if (WITH_D) {
-                    if (ep.Dout) ep.Dout[xd] = D;
-                    if (!ep.Lt) {  // an evaluation: no update
-                        mD = fmax(mD, D);
-                        sR = fma(ep.Pw[xd] * inv_z, D, sR);
-                        continue;
-                    }
-                }
-                // an entry that is exactly 0 in the caller's distribution (Lt
-                // holds NaN) takes ln p = 0, as the reference's apply_log_kernel
-                // leaves ln 0 at 0 (backend/BAA.cu:573-580); later iterates keep
-                // exact logarithms
-                const double pw = ep.Pw[xd];
-                const double lt = ep.Lt[xd];
-                const bool zero_in = (lt != lt);
-                const double lnp = zero_in ? 0.0 : lt - lnz;
-                const double lw = lnp + ep.eta * D - shift;
-                const double e = exp(lw);
-                ep.Lt[xd] = lw;
-                ep.Pw[xd] = o * e;
-                mD = fmax(mD, D);
-                mL = fmax(mL, lw);
-                sE = fma(o, e, sE);
-                sR = fma(pw * inv_z, D, sR);
-                if (zero_in) zero = 1.0;
+        for (int u = 0; u < 2; ++u) {
+            const int q = q0 + 8 * u, m = m0 + q / SEG, n = n0 + (q % SEG) * 64 + 2 * lane;
+            const bool in = q < ROWS && m < M && n < N;
+            const uint32_t r = (uint32_t)m + kc.row0;
+            r0[u] = in && dense_is_rep(r, (uint32_t)n, kc.mask, kc.odd);
+            r1[u] = in && dense_is_rep(r, (uint32_t)n + 1, kc.mask, kc.odd);
+            xd[u] = ((uint32_t)m << ep.n2) | (uint32_t)n;
+            if (r0[u] || r1[u]) {
+                hv[u] = __ldg(reinterpret_cast<const double2*>(ep.hx + xd[u]));
+                pv[u] = *reinterpret_cast<const double2*>(ep.Pw + xd[u]);
+                if (!WITH_D || ep.Lt) lv[u] = *reinterpret_cast<const double2*>(ep.Lt + xd[u]);
             }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            if (!(r0[u] || r1[u])) continue;
+            const int q = q0 + 8 * u;
+            const uint32_t r = (uint32_t)(m0 + q / SEG) + kc.row0, n = xd[u] & kc.mask;
+            const double2 gv = *reinterpret_cast<const double2*>(smem + (q / SEG) * LD + (q % SEG) * 64 + 2 * lane);
+            if (WITH_D && !ep.Lt) {  // an evaluation: no update
+                const double d0 = hv[u].x - gv.x * kc.inv_c, d1 = hv[u].y - gv.y * kc.inv_c;
+                if (r0[u]) {
+                    bs.mD = fmax(bs.mD, d0);
+                    bs.sR = fma(pv[u].x * kc.inv_z, d0, bs.sR);
+                    if (ep.Dout) ep.Dout[xd[u]] = d0;
+                }
+                if (r1[u]) {
+                    bs.mD = fmax(bs.mD, d1);
+                    bs.sR = fma(pv[u].y * kc.inv_z, d1, bs.sR);
+                    if (ep.Dout) ep.Dout[xd[u] + 1] = d1;
+                }
+                continue;
+            }
+            if (r0[u]) {
+                const double D = ba_update(gv.x, hv[u].x, dense_orbit(r, n, kc.mask, kc.odd), lv[u].x, pv[u].x, kc, bs);
+                if (WITH_D) ep.Dout[xd[u]] = D;
+            }
+            if (r1[u]) {
+                const double D = ba_update(gv.y, hv[u].y, dense_orbit(r, n + 1, kc.mask, kc.odd), lv[u].y, pv[u].y, kc, bs);
+                if (WITH_D) ep.Dout[xd[u] + 1] = D;
+            }
+            *reinterpret_cast<double2*>(ep.Lt + xd[u]) = lv[u];
+            *reinterpret_cast<double2*>(ep.Pw + xd[u]) = pv[u];
+        }
     }
-    }
+    double mD = bs.mD, sE = bs.sE, mL = bs.mL, sR = bs.sR, zero = bs.zero;
     __shared__ double red[5][8];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -381,10 +393,8 @@ static cudaError_t set_smem_attrs() {
     SET_K((k_mma_store<ARGS, 0>), (mma_cp_smem_bytes<ARGS, false, false, 3>()))                 \
     SET_K((k_mma_store<ARGS, 3>), (mma_cp_smem_bytes<ARGS, true, true, 3>()))
 #define SET_BA(ARGS)                                                                             \
-    SET_K((k_mma_ba<ARGS, false, false>), (mma_smem_bytes<ARGS>()))                              \
-    SET_K((k_mma_ba<ARGS, true, false>), (mma_smem_bytes<ARGS>()))                               \
-    SET_K((k_mma_ba<ARGS, false, true>), (mma_cp_smem_bytes<ARGS, false, true, 3>()))            \
-    SET_K((k_mma_ba<ARGS, true, true>), (mma_cp_smem_bytes<ARGS, false, true, 3>()))
+    SET_K((k_mma_ba<ARGS, false>), (mma_cp_smem_bytes<ARGS, false, true, 3>()))                  \
+    SET_K((k_mma_ba<ARGS, true>), (mma_cp_smem_bytes<ARGS, false, true, 3>()))
     SET_STORE(BDC_CFG_ARGS_64x64)
     SET_STORE_CP(BDC_CFG_ARGS_128x128)
     SET_STORE_CP(BDC_CFG_ARGS_128x64)
@@ -396,7 +406,6 @@ static cudaError_t set_smem_attrs() {
     SET_STORE_CP(BDC_CFG_ARGS_64x32)
     SET_STORE_CP(BDC_CFG_ARGS_32x128)
     SET_STORE_CP(BDC_CFG_ARGS_32x64)
-    SET_BA(BDC_CFG_ARGS_128x128)
     SET_BA(BDC_CFG_ARGS_128x64)
     SET_BA(BDC_CFG_ARGS_64x128)
     SET_BA(BDC_CFG_ARGS_64x64)
@@ -442,19 +451,18 @@ static cudaError_t launch_store(const Launch& L, cudaStream_t s, const DevState*
 // G: A = [A_L | N_R] contiguous along the contraction, B = [M_L ; B_R^T]
 // contiguous along the output columns: the cp.async mainloop with layout 2
 static cudaError_t launch_ba(const Launch& L, const BaEpilogue& ep, cudaStream_t s, const DevState* st) {
-    const bool wd = ep.Dout != nullptr || !ep.Lt, cp = L.layout == 2;
-    const int sm = cfg_smem(L.cfg, cp ? 2 : -1);
-    const int grid = (L.grid > 0 && L.grid < L.tiles) ? L.grid : L.tiles;
-#define GO_(ARGS)                                                                                        \
-    if (wd && cp) k_mma_ba<ARGS, true, true><<<grid, 256, sm, s>>>(L.d, L.map, L.tiles, ep, st);         \
-    else if (wd) k_mma_ba<ARGS, true, false><<<grid, 256, sm, s>>>(L.d, L.map, L.tiles, ep, st);         \
-    else if (cp) k_mma_ba<ARGS, false, true><<<grid, 256, sm, s>>>(L.d, L.map, L.tiles, ep, st);         \
-    else k_mma_ba<ARGS, false, false><<<grid, 256, sm, s>>>(L.d, L.map, L.tiles, ep, st);
+    if (L.layout != 2) return cudaErrorInvalidValue;
+    const bool wd = ep.Dout != nullptr || !ep.Lt;
+    const int sm = cfg_smem(L.cfg, 2);
+#define GO_(NAME)                                                                                \
+    case CFG_##NAME:                                                                             \
+        if (wd) k_mma_ba<BDC_CFG_ARGS_##NAME, true><<<L.tiles, 256, sm, s>>>(L.d, L.map, ep, st); \
+        else k_mma_ba<BDC_CFG_ARGS_##NAME, false><<<L.tiles, 256, sm, s>>>(L.d, L.map, ep, st);   \
+        break;
     switch (L.cfg) {
-        case CFG_128x128: GO_(BDC_CFG_ARGS_128x128) break;
-        case CFG_128x64: GO_(BDC_CFG_ARGS_128x64) break;
-        case CFG_64x128: GO_(BDC_CFG_ARGS_64x128) break;
-        case CFG_64x64: GO_(BDC_CFG_ARGS_64x64) break;
+        GO_(128x64)
+        GO_(64x128)
+        GO_(64x64)
         default: return cudaErrorInvalidValue;
     }
 #undef GO_
@@ -1517,33 +1525,23 @@ bdc_status factored_init(bdc_handle* H) {
         ep.part = F->epart;
         ep.eta = 1.0;
         ep.row0 = F->row0;
-        // each shape one CTA per tile, or (when the tiles outnumber them) as
-        // many CTAs as fit on the SMs at once, each looping over tiles with
-        // the next tile's loads in flight during the epilogue
-        auto resident = [&](int c) { return H->num_sms * ((kCfgBM[c] * kCfgBN[c] <= 4096) ? 3 : 2); };
-        int best_persist = 0;
-        const bool pinned = tf.get("g", &best_cfg, &best_persist);
+        int unused = 0;
+        const bool pinned = tf.get("g", &best_cfg, &unused);
         for (int c : cfgs) {
             if (pinned) break;
             Launch T;
             BDC_CUDA_TRY(make_tile_launch(T, d, c, F->colmax));
-            for (int persist = 0; persist < 2; ++persist) {
-                if (persist && T.tiles <= resident(c)) break;
-                T.grid = persist ? resident(c) : 0;
-                const float ms = time_ms(H, [&] { return launch_ba(T, ep, H->stream, H->d_st); });
-                if (ms < best) {
-                    best = ms;
-                    best_cfg = c;
-                    best_persist = persist;
-                }
+            const float ms = time_ms(H, [&] { return launch_ba(T, ep, H->stream, H->d_st); });
+            if (ms < best) {
+                best = ms;
+                best_cfg = c;
             }
             free_launch(T);
         }
-        if (!pinned) tf.put("g", best_cfg, best_persist);
+        if (!pinned) tf.put("g", best_cfg, 0);
         tf.save();
         BDC_CUDA_TRY(make_tile_launch(F->g, d, best_cfg, F->colmax));
-        F->g.grid = best_persist ? std::min(F->g.tiles, resident(best_cfg)) : 0;
-        F->ctas_g = F->g.grid > 0 ? F->g.grid : F->g.tiles;
+        F->ctas_g = F->g.tiles;
         if (H->verbose)
             printf("bdc: tuned G: tile %dx%d, %d of %d tiles hold representatives, %d CTAs, %.1f us%s\n",
                    kCfgBM[best_cfg], kCfgBN[best_cfg], F->g.tiles,
@@ -1873,8 +1871,7 @@ bdc_status factored_evaluate(bdc_handle* H, double* D_out, double* rate) {
     bdc_status rc = factored_log_q(H);
     if (rc == BDC_OK) rc = eval_d(H, D_out);
     if (rc != BDC_OK) return rc;
-    k_eval_rate<<<1, 256, 0, H->stream>>>(F->epart, F->g.grid > 0 ? std::min(F->g.grid, F->g.tiles) : F->g.tiles,
-                                          H->d_scalar + 5);
+    k_eval_rate<<<1, 256, 0, H->stream>>>(F->epart, F->ctas_g, H->d_scalar + 5);
     BDC_CUDA_TRY(cudaGetLastError());
     BDC_CUDA_TRY(cudaMemcpyAsync(rate, H->d_scalar + 5, sizeof(double), cudaMemcpyDeviceToHost, H->stream));
     BDC_CUDA_TRY(cudaStreamSynchronize(H->stream));
@@ -2216,10 +2213,12 @@ __global__ void __launch_bounds__(256) k_acc_extrap(int64_t nx, int n, int row0,
     const int mode = st->ng_mode;
     const double lnz = st->log_z;
     const double beta = (double)st->ng_t / ((double)st->ng_t + 3.0);
+    const int n2 = n >> 1;
+    const uint32_t mask = low_mask(n2);
     double mx = -DBL_MAX;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nx; i += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t xd = (uint32_t)i;
-        if (!is_rep(fac_str(xd, n, row0), n)) continue;
+        if (!dense_is_rep((xd >> n2) + (uint32_t)row0, xd & mask, mask, (uint32_t)n & 1u)) continue;
         double y;
         if (mode == 1) {
             const double a_old = xa[xd], a_new = Lt[xd] - lnz;
@@ -2250,12 +2249,14 @@ __global__ void __launch_bounds__(256) k_acc_pw(int64_t nx, int n, int row0, dou
                                                 double* __restrict__ Pw, double* __restrict__ part, const DevState* st) {
     if (acc_gated(st)) return;
     const double m = st->ng_max;
+    const int n2 = n >> 1;
+    const uint32_t mask = low_mask(n2);
     double sum = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nx; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t xd = (uint32_t)i, x = fac_str(xd, n, row0);
-        if (!is_rep(x, n)) continue;
+        const uint32_t xd = (uint32_t)i, r = (xd >> n2) + (uint32_t)row0, c = xd & mask, odd = (uint32_t)n & 1u;
+        if (!dense_is_rep(r, c, mask, odd)) continue;
         const double l = Lt[xd] - m;
-        const double o = (double)orbit_size(x, n);
+        const double o = dense_orbit(r, c, mask, odd);
         const double e = exp(l);
         Lt[xd] = l;
         Pw[xd] = o * e;
@@ -2328,9 +2329,11 @@ __global__ void __launch_bounds__(256) k_acc_init(int64_t nx, int n, int row0, c
                                                   double* __restrict__ xa, double* __restrict__ xb, DevState* st,
                                                   double gap_nats) {
     const double lnz = st->log_z;
+    const int n2 = n >> 1;
+    const uint32_t mask = low_mask(n2);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nx; i += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t xd = (uint32_t)i;
-        if (!is_rep(fac_str(xd, n, row0), n)) continue;
+        if (!dense_is_rep((xd >> n2) + (uint32_t)row0, xd & mask, mask, (uint32_t)n & 1u)) continue;
         const double l = Lt[xd] - lnz;
         xa[xd] = l;
         xb[xd] = l;

@@ -56,4 +56,48 @@ struct BaEpilogue {
     int row0;                    // global x_hi of the product's row 0 (a shard of the rows; 0 on one GPU)
 };
 
+// what the epilogue's update needs beside the element itself
+struct BaConst {
+    double shift, lnz, inv_z, inv_c, eta;
+    uint32_t mask, odd, row0;
+};
+__device__ __forceinline__ BaConst ba_const(const BaEpilogue& ep, const DevState* st) {
+    BaConst k;
+    k.shift = st->shift;
+    k.lnz = st->log_z;
+    k.inv_z = exp(-k.lnz);
+    k.inv_c = ep.inv_c;
+    k.eta = ep.eta;
+    k.mask = low_mask(ep.n2);
+    k.odd = (uint32_t)ep.n & 1u;
+    k.row0 = (uint32_t)ep.row0;
+    return k;
+}
+
+// a thread's share of the update's statistics
+struct BaStats {
+    double mD = -1.7976931348623157e308, sE = 0.0, mL = -1.7976931348623157e308, sR = 0.0, zero = 0.0;
+};
+
+// the update of one representative (orbit o) whose G value is g: lt, pw are
+// replaced, D is returned.  An entry that is exactly 0 in the caller's
+// distribution (lt is NaN) takes ln p = 0, as the reference's
+// apply_log_kernel leaves ln 0 at 0 (backend/BAA.cu:573-580); later iterates
+// keep exact logarithms.
+__device__ __forceinline__ double ba_update(double g, double h, double o, double& lt, double& pw, const BaConst& k,
+                                            BaStats& s) {
+    const double D = h - g * k.inv_c;
+    const bool zero_in = (lt != lt);
+    const double lw = (zero_in ? 0.0 : lt - k.lnz) + k.eta * D - k.shift;
+    const double e = exp(lw);
+    s.sR = fma(pw * k.inv_z, D, s.sR);
+    lt = lw;
+    pw = o * e;
+    s.mD = D > s.mD ? D : s.mD;  // (a comparison and a select: fmax costs twice that)
+    s.mL = lw > s.mL ? lw : s.mL;
+    s.sE = fma(o, e, s.sE);
+    if (zero_in) s.zero = 1.0;
+    return D;
+}
+
 }  // namespace bdc

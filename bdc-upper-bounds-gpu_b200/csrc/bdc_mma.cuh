@@ -182,68 +182,81 @@ constexpr int mma_cp_smem_bytes() {
     return (int)sizeof(double) * STAGES * CpCfg<BM, BN, AK, BKM>::STAGE;
 }
 
-// one k-slice [k0, k0 + 16) of A and B into one stage
-template <int BM, int BN, bool AK, bool BKM>
-__device__ __forceinline__ void cp_stage(const GemmDesc& d, int m0, int n0, int k0, double* As, double* Bs) {
-    using C = CpCfg<BM, BN, AK, BKM>;
-    const double* A = (const double*)d.A.ptr;
-    const double* B = (const double*)d.B.ptr;
-    const int64_t lda = d.A.ld, ldb = d.B.ld;
-    const int M = d.M, N = d.N, K = d.K;
-    if (AK) {  // BK rows of BM doubles, pieces of two along m
-        constexpr int PIECES = C::BK * BM / 2;
-        for (int e = threadIdx.x; e < PIECES; e += 256) {
-            const int kk = e / (BM / 2), mm = (e % (BM / 2)) * 2;
-            const int k = k0 + kk, m = m0 + mm;
-            const int bytes = (k < K) ? (m + 1 < M ? 16 : (m < M ? 8 : 0)) : 0;
-            cp_async16(As + kk * (BM + 4) + mm, bytes ? A + (int64_t)k * lda + m : A, bytes);
-        }
-    } else {  // BM rows of BK doubles, pieces of two along k
-        constexpr int PIECES = BM * C::BK / 2;
-        for (int e = threadIdx.x; e < PIECES; e += 256) {
-            const int mm = e / (C::BK / 2), kk = (e % (C::BK / 2)) * 2;
-            const int k = k0 + kk, m = m0 + mm;
-            const int bytes = (m < M) ? (k + 1 < K ? 16 : (k < K ? 8 : 0)) : 0;
-            cp_async16(As + mm * C::PK + kk, bytes ? A + (int64_t)m * lda + k : A, bytes);
-        }
-    }
-    if (BKM) {
-        constexpr int PIECES = C::BK * BN / 2;
-        for (int e = threadIdx.x; e < PIECES; e += 256) {
-            const int kk = e / (BN / 2), nn = (e % (BN / 2)) * 2;
-            const int k = k0 + kk, n = n0 + nn;
-            const int bytes = (k < K) ? (n + 1 < N ? 16 : (n < N ? 8 : 0)) : 0;
-            cp_async16(Bs + kk * (BN + 4) + nn, bytes ? B + (int64_t)k * ldb + n : B, bytes);
-        }
-    } else {
-        constexpr int PIECES = BN * C::BK / 2;
-        for (int e = threadIdx.x; e < PIECES; e += 256) {
-            const int nn = e / (C::BK / 2), kk = (e % (C::BK / 2)) * 2;
-            const int k = k0 + kk, n = n0 + nn;
-            const int bytes = (n < N) ? (k + 1 < K ? 16 : (k < K ? 8 : 0)) : 0;
-            cp_async16(Bs + nn * C::PK + kk, bytes ? B + (int64_t)n * ldb + k : B, bytes);
+// One operand's copies of a thread.  KROW: the tile's rows run along the
+// contraction (16 of them, DIM contiguous entries each), else along the
+// operand's own dimension (DIM rows of 16).  A thread's pieces of 16 bytes lie
+// a fixed number of rows apart, so that a slice costs an addition and a copy
+// per piece; the addresses and bounds are worked out once per tile (recomputed
+// for every piece, they were a third of the products' instructions).
+template <int DIM, bool KROW>
+struct CpOperand {
+    static constexpr int PITCH = KROW ? DIM + 4 : 20;
+    static constexpr int PER_ROW = KROW ? DIM / 2 : 8;   // pieces of a row
+    static constexpr int ROWS = KROW ? 16 : DIM;
+    static constexpr int STEP = 256 / PER_ROW;            // rows between a thread's pieces
+    static constexpr int N = (ROWS * PER_ROW + 255) / 256;
+    static constexpr bool GUARD = ROWS * PER_ROW < 256;   // not every thread has a piece
+    const char* base;  // any valid address, for copies of no bytes
+    const char* g;     // the first piece in the next slice
+    int64_t row_step, k_step;
+    int row, col, s, edge;  // edge: bytes (KROW) or rows (else) inside the operand's dimension
+    __device__ __forceinline__ void init(const Operand& o, int at, int lim) {
+        const double* p = (const double*)o.ptr;
+        base = (const char*)p;
+        row = threadIdx.x / PER_ROW;
+        col = (threadIdx.x % PER_ROW) * 2;
+        s = row * PITCH + col;
+        row_step = (int64_t)STEP * o.ld * 8;
+        if (KROW) {
+            const int c = at + col;
+            edge = c + 1 < lim ? 16 : (c < lim ? 8 : 0);
+            g = (const char*)(p + (int64_t)row * o.ld + c);
+            k_step = 16 * o.ld * 8;
+        } else {
+            edge = lim - at;
+            g = (const char*)(p + (int64_t)(at + row) * o.ld + col);
+            k_step = 16 * 8;
         }
     }
-}
-
-// The first STAGES-1 stages of a tile's operands, in flight on return.  Issued
-// by every thread; the shared memory of those stages must be free (after the
-// previous tile's body, which ends with all copies landed and a barrier).
-template <int BM, int BN, bool AK, bool BKM, int STAGES>
-__device__ __forceinline__ void mma_cp_prologue(const GemmDesc& d, int m0, int n0, double* smem) {
-    using C = CpCfg<BM, BN, AK, BKM>;
-    const int nk = (d.K + C::BK - 1) / C::BK;
+    // the slice [k0, k0 + 16) of K into one stage; slices come in order
+    __device__ __forceinline__ void load(int k0, int K, double* stage) {
+        if (!GUARD || row < ROWS) {
 #pragma unroll
-    for (int st = 0; st < STAGES - 1; ++st) {
-        if (st < nk) cp_stage<BM, BN, AK, BKM>(d, m0, n0, st * C::BK, smem + st * C::STAGE, smem + st * C::STAGE + C::A_ELEMS);
-        cp_async_commit();
+            for (int i = 0; i < N; ++i) {
+                int bytes;
+                if (KROW) {
+                    bytes = k0 + row + i * STEP < K ? edge : 0;
+                } else {
+                    const int left = K - k0 - col;
+                    bytes = row + i * STEP < edge ? (left >= 2 ? 16 : (left == 1 ? 8 : 0)) : 0;
+                }
+                cp_async16(stage + s + i * STEP * PITCH, bytes ? g + i * row_step : base, bytes);
+            }
+        }
+        g += k_step;
     }
-}
+};
 
-// The k loop of one tile whose prologue is in flight; returns with every copy
-// landed and the shared memory free.
+template <int BM, int BN, bool AK, bool BKM>
+struct CpLoader {
+    CpOperand<BM, AK> a;
+    CpOperand<BN, BKM> b;
+    int K;
+    __device__ __forceinline__ void init(const GemmDesc& d, int m0, int n0) {
+        a.init(d.A, m0, d.M);
+        b.init(d.B, n0, d.N);
+        K = d.K;
+    }
+    __device__ __forceinline__ void load(int k0, double* stage) {
+        a.load(k0, K, stage);
+        b.load(k0, K, stage + CpCfg<BM, BN, AK, BKM>::A_ELEMS);
+    }
+};
+
+// The k loop of one tile; returns with every copy landed and the shared memory
+// free.
 template <int BM, int BN, int WM, int WN, bool AK, bool BKM, int STAGES>
-__device__ __forceinline__ void mma_cp_body(const GemmDesc& d, int m0, int n0, double* smem,
+__device__ __forceinline__ void mma_mainloop_cp(const GemmDesc& d, int m0, int n0, double* smem,
                                             double (&acc)[MmaCfg<BM, BN, WM, WN>::MT][MmaCfg<BM, BN, WM, WN>::NT][2]) {
     using M_ = MmaCfg<BM, BN, WM, WN>;
     using C = CpCfg<BM, BN, AK, BKM>;
@@ -254,19 +267,26 @@ __device__ __forceinline__ void mma_cp_body(const GemmDesc& d, int m0, int n0, d
     for (int i = 0; i < M_::MT; ++i)
 #pragma unroll
         for (int j = 0; j < M_::NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    CpLoader<BM, BN, AK, BKM> ld;
+    ld.init(d, m0, n0);
     const int nk = (d.K + C::BK - 1) / C::BK;
+#pragma unroll
+    for (int st = 0; st < STAGES - 1; ++st) {
+        if (st < nk) ld.load(st * C::BK, smem + st * C::STAGE);
+        cp_async_commit();
+    }
+    int cur = 0, nxt = STAGES - 1;  // stages of this slice and of the one to fetch
     for (int kt = 0; kt < nk; ++kt) {
         cp_async_wait<STAGES - 2>();
         __syncthreads();
         {
             const int nx = kt + STAGES - 1;
-            if (nx < nk) {
-                double* s = smem + (nx % STAGES) * C::STAGE;
-                cp_stage<BM, BN, AK, BKM>(d, m0, n0, nx * C::BK, s, s + C::A_ELEMS);
-            }
+            if (nx < nk) ld.load(nx * C::BK, smem + nxt * C::STAGE);
             cp_async_commit();
+            nxt = nxt + 1 == STAGES ? 0 : nxt + 1;
         }
-        const double* as = smem + (kt % STAGES) * C::STAGE;
+        const double* as = smem + cur * C::STAGE;
+        cur = cur + 1 == STAGES ? 0 : cur + 1;
         const double* bs = as + C::A_ELEMS;
 #pragma unroll
         for (int kq = 0; kq < C::BK / 4; ++kq) {
@@ -290,13 +310,6 @@ __device__ __forceinline__ void mma_cp_body(const GemmDesc& d, int m0, int n0, d
     }
     cp_async_wait<0>();
     __syncthreads();
-}
-
-template <int BM, int BN, int WM, int WN, bool AK, bool BKM, int STAGES>
-__device__ __forceinline__ void mma_mainloop_cp(const GemmDesc& d, int m0, int n0, double* smem,
-                                                double (&acc)[MmaCfg<BM, BN, WM, WN>::MT][MmaCfg<BM, BN, WM, WN>::NT][2]) {
-    mma_cp_prologue<BM, BN, AK, BKM, STAGES>(d, m0, n0, smem);
-    mma_cp_body<BM, BN, WM, WN, AK, BKM, STAGES>(d, m0, n0, smem, acc);
 }
 
 }  // namespace bdc

@@ -147,7 +147,7 @@ static_assert(kOzW % 2 == 0, "the drain reads accumulator pairs");
 // threads of the product with EPI epilogue warps (beside one TMA producer
 // warp and one MMA warp)
 __host__ __device__ constexpr int oz_threads(int EPI) { return 64 + 32 * EPI; }
-constexpr int kOzTileLd = kOzTN + 1;                  // row pitch of an FP64 tile in shared memory
+constexpr int kOzTileLd = kOzTN + 2;                  // row pitch of an FP64 tile in shared memory (16-byte pairs)
 constexpr int kOzTileBytes = kOzBM * kOzTileLd * 8;  // one FP64 tile
 
 // named barrier 1 among the EPI epilogue warps only
@@ -218,7 +218,7 @@ k_oz_ba(const __grid_constant__ CUtensorMap tmAs, const __grid_constant__ CUtens
     auto aborted = [&]() { return *(volatile int*)&abort_sh != 0; };
     auto give_up = [&]() { atomicExch(&abort_sh, 1); };
 
-    double mD = -DBL_MAX, sE = 0.0, mL = -DBL_MAX, sR = 0.0, zero = 0.0;
+    BaStats bs;
     // producer bookkeeping for the bounded drain on an abort
     int last_use[kOzStages], last_static[2];
     for (int i = 0; i < kOzStages; ++i) last_use[i] = -1;
@@ -323,35 +323,36 @@ k_oz_ba(const __grid_constant__ CUtensorMap tmAs, const __grid_constant__ CUtens
         // the drain of tile it writes buffer it & 1, which the pass of tile
         // it - 2 was the last to read; with one tile a second barrier before
         // the drain.
-        constexpr int PER = kOzBM * kOzTN / (32 * EPI);  // elements per thread in the pass
+        constexpr int PER = kOzBM * kOzTN / (64 * EPI);  // pairs of columns per thread in the pass
         const int q = warp & 3;
         const int part = (warp - 2) >> 2;
         const int r = q * 32 + lane;      // the tile row this thread drains
-        const int et = threadIdx.x - 64;  // 0 .. 32 EPI - 1 in the pass
-        const double shift = st->shift;
-        const double lnz = st->log_z;
-        const double inv_z = exp(-lnz);
+        // in the pass: rows prow + 2 EPI u, columns pcol and pcol + 1
+        const int prow = (int)(threadIdx.x - 64) >> 4, pcol = 2 * (lane & 15);
+        const BaConst kc = ba_const(ep, st);
         const int e = *d_e;
         // the entropy, log iterate and weighted iterate of a tile's pass
-        // elements, loaded before its accumulators are drained; bit u of reps:
-        // element u is a representative
-        double hv[PER], lv[PER], pv[PER];
+        // elements, loaded before its accumulators are drained; bits 2u, 2u + 1
+        // of reps: the pair's columns are representatives
+        double2 hv[PER], lv[PER], pv[PER];
         uint32_t reps = 0;
         auto preload = [&](int it) {
             const int t = tiles[blockIdx.x + it * gridDim.x];
-            const int m0 = (t / g.tiles_n) * kOzBM, n = (t % g.tiles_n) * kOzTN + lane;
+            const int m0 = (t / g.tiles_n) * kOzBM, n = (t % g.tiles_n) * kOzTN + pcol;
             reps = 0;
 #pragma unroll
             for (int u = 0; u < PER; ++u) {
-                const int m = m0 + (et >> 5) + u * EPI;
-                const uint32_t xd = ((uint32_t)m << ep.n2) | (uint32_t)n;
-                const uint32_t xg = xd + ((uint32_t)ep.row0 << ep.n2);
-                const uint32_t x = (xg & ~low_mask(ep.n2)) | reverse_bits(xg & low_mask(ep.n2), ep.n2);
-                const bool rep = (m < g.M) && (n < g.N) && is_rep(x, ep.n);
-                reps |= (uint32_t)rep << u;
-                hv[u] = rep ? __ldg(ep.hx + xd) : 0.0;
-                lv[u] = rep ? ep.Lt[xd] : 0.0;
-                pv[u] = rep ? ep.Pw[xd] : 0.0;
+                const int m = m0 + prow + u * 2 * EPI;
+                const uint32_t xd = ((uint32_t)m << ep.n2) | (uint32_t)n, row = (uint32_t)m + kc.row0;
+                const bool in = (m < g.M) && (n < g.N);
+                const bool r0 = in && dense_is_rep(row, (uint32_t)n, kc.mask, kc.odd);
+                const bool r1 = in && dense_is_rep(row, (uint32_t)n + 1, kc.mask, kc.odd);
+                reps |= ((uint32_t)r0 | ((uint32_t)r1 << 1)) << (2 * u);
+                if (r0 || r1) {
+                    hv[u] = __ldg(reinterpret_cast<const double2*>(ep.hx + xd));
+                    lv[u] = *reinterpret_cast<const double2*>(ep.Lt + xd);
+                    pv[u] = *reinterpret_cast<const double2*>(ep.Pw + xd);
+                }
             }
         };
         if (nmine > 0) preload(0);
@@ -382,8 +383,9 @@ k_oz_ba(const __grid_constant__ CUtensorMap tmAs, const __grid_constant__ CUtens
                         for (int j = 0; j < 4; ++j)
                             gsum[j] = fma((double)((int32_t)v0[j] * 128 + (int32_t)v1[j]), w, gsum[j]);
                     }
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) gtb[r * kOzTileLd + part * kOzCols + c0 + j] = gsum[j];
+                    double2* o = reinterpret_cast<double2*>(gtb + r * kOzTileLd + part * kOzCols + c0);
+                    o[0] = make_double2(gsum[0], gsum[1]);
+                    o[1] = make_double2(gsum[2], gsum[3]);
                 }
             }
             // this warp's part of the TMEM buffer is free for the tile after next
@@ -393,31 +395,26 @@ k_oz_ba(const __grid_constant__ CUtensorMap tmAs, const __grid_constant__ CUtens
             epi_sync(EPI);
             if (aborted()) break;  // uniform: read after the barrier
             const int t = tiles[blockIdx.x + it * gridDim.x];
-            const int m0 = (t / g.tiles_n) * kOzBM, n = (t % g.tiles_n) * kOzTN + lane;
+            const int m0 = (t / g.tiles_n) * kOzBM, n = (t % g.tiles_n) * kOzTN + pcol;
 #pragma unroll
             for (int u = 0; u < PER; ++u) {
-                if (!((reps >> u) & 1u)) continue;
-                const int row = (et >> 5) + u * EPI;
-                const uint32_t xd = ((uint32_t)(m0 + row) << ep.n2) | (uint32_t)n;
-                const uint32_t xg = xd + ((uint32_t)ep.row0 << ep.n2);
-                const uint32_t x = (xg & ~low_mask(ep.n2)) | reverse_bits(xg & low_mask(ep.n2), ep.n2);
-                const double o = (double)orbit_size(x, ep.n);
-                const double pw = pv[u];
-                const double D = hv[u] - gtb[row * kOzTileLd + lane] * ep.inv_c;
-                if (ep.Dout) ep.Dout[xd] = D;
-                // exact zeros of the caller's distribution (Lt = NaN) take ln p = 0
-                // (backend/BAA.cu:573-580)
-                const bool zero_in = (lv[u] != lv[u]);
-                const double lnp = zero_in ? 0.0 : lv[u] - lnz;
-                const double lw = lnp + ep.eta * D - shift;
-                const double ex = exp(lw);
-                ep.Lt[xd] = lw;
-                ep.Pw[xd] = o * ex;
-                mD = fmax(mD, D);
-                mL = fmax(mL, lw);
-                sE = fma(o, ex, sE);
-                sR = fma(pw * inv_z, D, sR);
-                if (zero_in) zero = 1.0;
+                const uint32_t rr = (reps >> (2 * u)) & 3u;
+                if (rr == 0) continue;
+                const int row = prow + u * 2 * EPI;
+                const uint32_t xd = ((uint32_t)(m0 + row) << ep.n2) | (uint32_t)n, rg = (uint32_t)(m0 + row) + kc.row0;
+                const double2 gv = *reinterpret_cast<const double2*>(gtb + row * kOzTileLd + pcol);
+                if (rr & 1u) {
+                    const double D = ba_update(gv.x, hv[u].x, dense_orbit(rg, (uint32_t)n, kc.mask, kc.odd), lv[u].x,
+                                               pv[u].x, kc, bs);
+                    if (ep.Dout) ep.Dout[xd] = D;
+                }
+                if (rr & 2u) {
+                    const double D = ba_update(gv.y, hv[u].y, dense_orbit(rg, (uint32_t)n + 1, kc.mask, kc.odd),
+                                               lv[u].y, pv[u].y, kc, bs);
+                    if (ep.Dout) ep.Dout[xd + 1] = D;
+                }
+                *reinterpret_cast<double2*>(ep.Lt + xd) = lv[u];
+                *reinterpret_cast<double2*>(ep.Pw + xd) = pv[u];
             }
             if (it + 1 < nmine) preload(it + 1);
         }
@@ -429,6 +426,7 @@ k_oz_ba(const __grid_constant__ CUtensorMap tmAs, const __grid_constant__ CUtens
     if (!mma_done) give_up();
     __syncthreads();
     const bool ran = !aborted();
+    double mD = bs.mD, sE = bs.sE, mL = bs.mL, sR = bs.sR, zero = bs.zero;
     if (!ran && threadIdx.x == 0) st->error = kErrOzakiWait;
     __shared__ double red[5][oz_threads(EPI) / 32];
 #pragma unroll

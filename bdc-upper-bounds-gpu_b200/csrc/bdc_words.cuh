@@ -161,12 +161,11 @@ __device__ __forceinline__ int word_round(int rem) { return rem < 4 ? rem : 4; }
 // heap index h; Lp, Lc: longest word of a parent / child node.  LN: the root
 // round, whose words of length k are ln q itself.
 template <int Q>
-__device__ __forceinline__ void word_expand_item(const double* __restrict__ src, double* __restrict__ dst, int u,
-                                                 int h, int i, int Lp, int Lc, int k, const double* __restrict__ lnq,
+__device__ __forceinline__ void word_expand_item(double* wsm, int src, int dst, int u, int h, int i, int Lp, int Lc, int k, const double* __restrict__ lnq,
                                                  double s0, bool root, bool leaf, double* __restrict__ out,
                                                  int64_t leaf_stride, int first, int leaf0, int leaves) {
     const int l = word_len(h), val = h - (1 << l);
-    const double* p = src + (root ? 0 : ((int64_t)u << (Lp + 1)));
+    const int p = src + (root ? 0 : (u << (Lp + 1)));
     double X[2 << Q], Y[1 << Q];
 #pragma unroll
     for (int d = 0; d <= Q; ++d)
@@ -174,7 +173,7 @@ __device__ __forceinline__ void word_expand_item(const double* __restrict__ src,
         for (int v = 0; v < (1 << d); ++v) {
             const int idx = (((1 << d) + v) << l) | val;
             double x = 0.0;
-            if (l + d <= Lp) x = (root && l + d == k) ? s0 * __ldg(lnq + idx - (1 << k)) : p[idx];
+            if (l + d <= Lp) x = (root && l + d == k) ? s0 * __ldg(lnq + idx - (1 << k)) : wsm[p + idx];
             X[(1 << d) + v] = x;
         }
     WordExpand<Q>::run(X, Y, 1);
@@ -185,7 +184,7 @@ __device__ __forceinline__ void word_expand_item(const double* __restrict__ src,
             const int at = first + node - leaf0;
             if (at >= 0 && at < leaves) out[(int64_t)at * leaf_stride] = Y[v];
         } else {
-            dst[((int64_t)node << (Lc + 1)) + h] = Y[v];
+            wsm[dst + (node << (Lc + 1)) + h] = Y[v];
         }
     }
 }
@@ -238,8 +237,9 @@ __global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan
         }
     }
     __syncthreads();
-    double* src = c;
-    double* dst = other;
+    // (buffers as offsets: pointers that change roles would be generic ones)
+    const int second = word_buf(k, r);
+    int src = 0, dst = second;
     if (fixed > 0) {
         // consume the fixed last characters: c[z] <- sum_u N(p, u) c[z u] over
         // their subsequences u
@@ -257,14 +257,14 @@ __global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan
             other[h] = x;
         }
         __syncthreads();
-        src = other;
-        dst = c;
+        src = second;
+        dst = 0;
     }
     // the tree over the r free characters
     double* out = S.out + (int64_t)w * S.word_stride;
     if (r == 0) {
         if (tid == 0 && first >= S.leaf0 && first < S.leaf0 + S.leaves)
-            out[(int64_t)(first - S.leaf0) * S.leaf_stride] = src[1];
+            out[(int64_t)(first - S.leaf0) * S.leaf_stride] = wsm[src + 1];
         return;
     }
     for (int i = 0; i < r;) {
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan
             const int u = e >> (Lc + 1), h = e & (tails - 1);
             if (h == 0) continue;
 #define BDC_ITEM_(Q_)                                                                                               \
-    word_expand_item<Q_>(src, dst, u, h, i, Lp, Lc, k, lnq, s0, root, leaf, out, S.leaf_stride, first, S.leaf0, \
+    word_expand_item<Q_>(wsm, src, dst, u, h, i, Lp, Lc, k, lnq, s0, root, leaf, out, S.leaf_stride, first, S.leaf0, \
                          S.leaves)
             switch (q) {
                 case 4: BDC_ITEM_(4); break;
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan
 #undef BDC_ITEM_
         }
         __syncthreads();
-        double* x = src;
+        const int x = src;
         src = dst;
         dst = x;
         i += q;
@@ -297,12 +297,11 @@ __global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan
 // one round of the q side for the item (u, h): the 2^Q children's values at
 // the tail -> X[v], |v| <= Q (read by every thread before any of them writes)
 template <int Q>
-__device__ __forceinline__ void word_contract_load(double (&X)[32], const double* __restrict__ src, int u, int h,
-                                                   int i, int Lc, bool leaf, const WordSide& S, int w, int first) {
+__device__ __forceinline__ void word_contract_load(double (&X)[32], const double* wsm, int src, int u, int h, int i, int Lc, bool leaf, const WordSide& S, int w, int first) {
     double in[1 << Q];
     if (!leaf) {
 #pragma unroll
-        for (int v = 0; v < (1 << Q); ++v) in[v] = src[((int64_t)(u + (v << i)) << (Lc + 1)) + h];
+        for (int v = 0; v < (1 << Q); ++v) in[v] = wsm[src + ((u + (v << i)) << (Lc + 1)) + h];
     } else {
         // the split slices, one after another with every leaf's load in flight
         const double* p = S.in + (int64_t)w * S.leaves + (first + u - S.leaf0);
@@ -330,18 +329,17 @@ __device__ __forceinline__ void word_contract_load(double (&X)[32], const double
 // fixed length the words v z of different tails are distinct); a word whose
 // tail is as long as a child's longest, or with |v| = 0, is written first here
 template <int Q>
-__device__ __forceinline__ void word_contract_add(const double (&X)[32], double* __restrict__ dst, int u, int h,
-                                                  int Lp, int Lc, bool live) {
+__device__ __forceinline__ void word_contract_add(const double (&X)[32], double* wsm, int dst, int u, int h, int Lp, int Lc, bool live) {
     const int l = word_len(h), val = h - (1 << l);
-    double* p = dst + ((int64_t)u << (Lp + 1));
+    const int p = dst + (u << (Lp + 1));
 #pragma unroll
     for (int d = 0; d <= Q; ++d) {
         if (live && l + d <= Lp) {
 #pragma unroll
             for (int v = 0; v < (1 << d); ++v) {
                 const int idx = (((1 << d) + v) << l) | val;
-                if (d == 0 || l == Lc) p[idx] = X[(1 << d) + v];
-                else p[idx] += X[(1 << d) + v];
+                if (d == 0 || l == Lc) wsm[p + idx] = X[(1 << d) + v];
+                else wsm[p + idx] += X[(1 << d) + v];
             }
         }
         __syncthreads();
@@ -371,8 +369,8 @@ __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan
     // the tree, deepest characters first; the rounds alternate between the
     // buffers so that the root ends in the second
     const int rounds = (r + 3) / 4;
-    double* dst = (rounds & 1) ? wsm + word_buf(k, r) : wsm;
-    double* src = (rounds & 1) ? wsm : wsm + word_buf(k, r);
+    const int second = word_buf(k, r);
+    int dst = (rounds & 1) ? second : 0, src = (rounds & 1) ? 0 : second;
     for (int g = rounds - 1; g >= 0; --g) {
         const int i = 4 * g, rem = r - i, q = word_round(rem);
         const int Lp = min(k, rem), Lc = min(k, rem - q);
@@ -383,8 +381,8 @@ __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan
         const bool live = u < (1 << i);
         double X[32];
 #define BDC_ROUND_(Q_)                                                                  \
-    if (live) word_contract_load<Q_>(X, src, u, h, i, Lc, leaf, S, w, first);           \
-    word_contract_add<Q_>(X, dst, u, h, Lp, Lc, live);
+    if (live) word_contract_load<Q_>(X, wsm, src, u, h, i, Lc, leaf, S, w, first);           \
+    word_contract_add<Q_>(X, wsm, dst, u, h, Lp, Lc, live);
         switch (q) {
             case 4: BDC_ROUND_(4) break;
             case 3: BDC_ROUND_(3) break;
@@ -392,10 +390,13 @@ __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan
             default: BDC_ROUND_(1) break;
         }
 #undef BDC_ROUND_
-        double* x = src;
+        const int x = src;
         src = dst;
         dst = x;
     }
+    // the root is in the second buffer
+    const double* root = wsm + second;
+    double* c = wsm;
     if (r == 0) {
         if (tid == 0) {
             double x = 0.0;
@@ -404,11 +405,11 @@ __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan
                 const int n = S.ns[(first - S.leaf0) >> 4];
                 for (int s = 0; s < n; ++s) x += p[s * S.slice_stride];
             }
-            src[1] = x;
+            wsm[second + 1] = x;
         }
         __syncthreads();
     }
-    // src: the root's words up to length min(k, r).  The fixed last characters
+    // the root's words up to length min(k, r).  The fixed last characters
     // p: a word z u takes N(p, u) t[z], up to `fixed` characters u
     const int fixed = S.last0 + t, tailc = (int)reverse_bits((uint32_t)beta, t) << S.last0;
     const int top = 2 << min(k, r);  // end of the root's heap
@@ -418,14 +419,13 @@ __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan
     __syncthreads();
     const double* wt = aux.weight;
     auto after = [&](int h) {
-        double x = h < top ? src[h] : 0.0;
+        double x = h < top ? root[h] : 0.0;
         for (int d = 1; d <= fixed; ++d) {
             const int g = h >> d;
-            if (g > 0 && g < top) x = fma(aux.occ[(1 << d) + (h & ((1 << d) - 1))], src[g], x);
+            if (g > 0 && g < top) x = fma(aux.occ[(1 << d) + (h & ((1 << d) - 1))], root[g], x);
         }
         return x;
     };
-    double* c = dst;
     for (int h = (1 << (k - a)) + tid; h < nk; h += T) c[h] = after(h);
     __syncthreads();
     // acc[v z] = sum over the splits of y into |v| <= a characters and the rest
