@@ -108,6 +108,7 @@ struct FactoredState {
     int d_lpx = 0, d_m = 1, d_grid = 0;
     double* d_members = nullptr;
     double* epart = nullptr;  // [ctas][8]
+    double* spart = nullptr;  // [kStatRows][8]
     int ctas_g = 0;
     bdc::OzakiG* oz = nullptr;  // G on the int8 tensor cores (when set up and chosen)
     bool use_oz = false;
@@ -210,8 +211,9 @@ __global__ void __launch_bounds__(256) k_mma_store(const GemmDesc* __restrict__ 
 // adjacent columns: on the fragments themselves every access touched twice
 // the sectors and the orbit tests and addresses were 2/3 of 210 instructions
 // an element.  84 -> 47 us at 24/12 (135 MB of device memory: 21 us).
+constexpr int g_stages(int bm, int bn, int, int) { return bm * bn <= 4096 ? 2 : 3; }
 template <int BM, int BN, int WM, int WN, bool WITH_D>
-__global__ void __launch_bounds__(256, (BM * BN <= 4096) ? 3 : 2) k_mma_ba(const GemmDesc* __restrict__ descs, const int* __restrict__ tiles,
+__global__ void __launch_bounds__(256, (BM * BN <= 4096) ? 4 : 2) k_mma_ba(const GemmDesc* __restrict__ descs, const int* __restrict__ tiles,
                                                    BaEpilogue ep, const DevState* st) {
     using C = MmaCfg<BM, BN, WM, WN>;
     constexpr int LD = BN + 8;
@@ -237,8 +239,8 @@ __global__ void __launch_bounds__(256, (BM * BN <= 4096) ? 3 : 2) k_mma_ba(const
     }
     {
         double acc[C::MT][C::NT][2];
-        mma_mainloop_cp<BM, BN, WM, WN, false, true, 3>(d, m0, n0, smem, acc);
-        static_assert(BM * LD * (int)sizeof(double) <= mma_cp_smem_bytes<BM, BN, WM, WN, false, true, 3>(), "tile");
+        mma_mainloop_cp<BM, BN, WM, WN, false, true, g_stages(BM, BN, 0, 0)>(d, m0, n0, smem, acc);
+        static_assert(BM * LD * (int)sizeof(double) <= mma_cp_smem_bytes<BM, BN, WM, WN, false, true, g_stages(BM, BN, 0, 0)>(), "tile");
 #pragma unroll
         for (int i = 0; i < C::MT; ++i)
 #pragma unroll
@@ -354,7 +356,7 @@ static int cfg_smem(int cfg, int layout = -1) {
         switch (layout) {                                                                       \
             case 0: return mma_cp_smem_bytes<ARGS, false, false, 3>();                          \
             case 1: return mma_cp_smem_bytes<ARGS, true, false, 3>();                           \
-            case 2: return mma_cp_smem_bytes<ARGS, false, true, 3>();                           \
+            case 2: return mma_cp_smem_bytes<ARGS, false, true, g_stages(ARGS)>();                           \
             case 3: return mma_cp_smem_bytes<ARGS, true, true, 3>();                            \
             default: return mma_smem_bytes<ARGS>();                                             \
         }
@@ -393,8 +395,8 @@ static cudaError_t set_smem_attrs() {
     SET_K((k_mma_store<ARGS, 0>), (mma_cp_smem_bytes<ARGS, false, false, 3>()))                 \
     SET_K((k_mma_store<ARGS, 3>), (mma_cp_smem_bytes<ARGS, true, true, 3>()))
 #define SET_BA(ARGS)                                                                             \
-    SET_K((k_mma_ba<ARGS, false>), (mma_cp_smem_bytes<ARGS, false, true, 3>()))                  \
-    SET_K((k_mma_ba<ARGS, true>), (mma_cp_smem_bytes<ARGS, false, true, 3>()))
+    SET_K((k_mma_ba<ARGS, false>), (mma_cp_smem_bytes<ARGS, false, true, g_stages(ARGS)>()))                  \
+    SET_K((k_mma_ba<ARGS, true>), (mma_cp_smem_bytes<ARGS, false, true, g_stages(ARGS)>()))
     SET_STORE(BDC_CFG_ARGS_64x64)
     SET_STORE_CP(BDC_CFG_ARGS_128x128)
     SET_STORE_CP(BDC_CFG_ARGS_128x64)
@@ -470,36 +472,57 @@ static cudaError_t launch_ba(const Launch& L, const BaEpilogue& ep, cudaStream_t
 }
 
 // ------------------------------------------------------------ small kernels
+// the statistics of rows part[b * 8 ..] added up by 256 threads, valid in thread 0
+__device__ __forceinline__ void stat_reduce(const double* __restrict__ part, int b0, int b1, double (&v)[5]) {
+    __shared__ double red[5][8];
+    v[0] = v[2] = -DBL_MAX;
+    v[1] = v[3] = v[4] = 0.0;
+#pragma unroll 4
+    for (int b = b0 + (int)threadIdx.x; b < b1; b += 256) {
+        const double* p = part + (size_t)b * 8;
+        v[0] = fmax(v[0], p[0]);
+        v[1] += p[1];
+        v[2] = fmax(v[2], p[2]);
+        v[3] += p[3];
+        v[4] = fmax(v[4], p[4]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int w = 0; w < 5; ++w) {
+            const double t = __shfl_xor_sync(0xFFFFFFFFu, v[w], o);
+            v[w] = (w == 1 || w == 3) ? v[w] + t : fmax(v[w], t);
+        }
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int w = 0; w < 5; ++w) red[w][threadIdx.x >> 5] = v[w];
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int u = 1; u < 8; ++u)
+#pragma unroll
+        for (int w = 0; w < 5; ++w) v[w] = (w == 1 || w == 3) ? v[w] + red[w][u] : fmax(v[w], red[w][u]);
+}
+
+// many partials (large n) first come down to kStatRows rows: one CTA alone
+// took 36 us for the 16,512 of 28/13
+constexpr int kStatRows = 128, kStatMany = 4096;
+__global__ void __launch_bounds__(256) k_fac_stats(const double* __restrict__ part, int nb, double* __restrict__ out,
+                                                   const DevState* st) {
+    if (gated(st)) return;
+    double v[5];
+    const int n = (nb + kStatRows - 1) / kStatRows;
+    stat_reduce(part, blockIdx.x * n, min(nb, (int)(blockIdx.x + 1) * n), v);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int w = 0; w < 5; ++w) out[blockIdx.x * 8 + w] = v[w];
+}
+
 __global__ void __launch_bounds__(256)
 k_fac_finalize(const double* __restrict__ part, int nb, double a, double eta, DevState* st) {
     if (gated(st)) return;
-    __shared__ double red[5][256];
-    double mD = -DBL_MAX, sE = 0.0, mL = -DBL_MAX, sR = 0.0, zero = 0.0;
-    for (int b = threadIdx.x; b < nb; b += 256) {
-        mD = fmax(mD, part[(size_t)b * 8 + 0]);
-        sE += part[(size_t)b * 8 + 1];
-        mL = fmax(mL, part[(size_t)b * 8 + 2]);
-        sR += part[(size_t)b * 8 + 3];
-        zero = fmax(zero, part[(size_t)b * 8 + 4]);
-    }
-    red[0][threadIdx.x] = mD;
-    red[1][threadIdx.x] = sE;
-    red[2][threadIdx.x] = mL;
-    red[3][threadIdx.x] = sR;
-    red[4][threadIdx.x] = zero;
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-            red[0][threadIdx.x] = fmax(red[0][threadIdx.x], red[0][threadIdx.x + s]);
-            red[1][threadIdx.x] += red[1][threadIdx.x + s];
-            red[2][threadIdx.x] = fmax(red[2][threadIdx.x], red[2][threadIdx.x + s]);
-            red[3][threadIdx.x] += red[3][threadIdx.x + s];
-            red[4][threadIdx.x] = fmax(red[4][threadIdx.x], red[4][threadIdx.x + s]);
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x != 0) return;
-    fac_finish(red[0][0], red[1][0], red[2][0], red[3][0], red[4][0], a, eta, st);
+    double v[5];
+    stat_reduce(part, 0, nb, v);
+    if (threadIdx.x == 0) fac_finish(v[0], v[1], v[2], v[3], v[4], a, eta, st);
 }
 
 // re-scale after an exp over/underflow: Lt -= s, Pw = |O| exp(Lt), sum
@@ -1512,6 +1535,7 @@ bdc_status factored_init(bdc_handle* H) {
         int ctas_max = 0;
         for (int c : cfgs) ctas_max = std::max(ctas_max, ((H1 + kCfgBM[c] - 1) / kCfgBM[c]) * ((H2 + kCfgBN[c] - 1) / kCfgBN[c]));
         BDC_CUDA_TRY(al(&F->epart, (size_t)std::max(ctas_max, H->nb_upd) * 8));
+        BDC_CUDA_TRY(al(&F->spart, (size_t)kStatRows * 8));
         float best = 1e30f;
         int best_cfg = CFG_128x64;
         GemmDesc d = make_desc(op_f64(F->LA, Kp, 0), op_f64(F->RB, H2, 0), nullptr, 0, 0, H1, H2, Kp);
@@ -1628,7 +1652,7 @@ bdc_status factored_init(bdc_handle* H) {
     }
     // U, V; the q-side transform; fold; the D-side transform; G (plus the
     // slicing kernel on the int8 path); finalize
-    F->launches_per_iter = (F->ul.n > 0) + (F->vr.n > 0) + 3 + 1 + 1 + (F->use_oz ? 1 : 0);
+    F->launches_per_iter = (F->ul.n > 0) + (F->vr.n > 0) + 3 + 1 + 1 + (F->use_oz ? 1 : F->ctas_g > kStatMany ? 1 : 0);
     BDC_CUDA_TRY(cudaStreamSynchronize(H->stream));
     return BDC_OK;
 }
@@ -1637,7 +1661,7 @@ void factored_free(bdc_handle* H) {
     FactoredState* F = H->fac;
     if (!F) return;
     for (double* p : {F->Pw, F->Lt, F->hx, F->LA, F->RB, F->ulpart, F->vrpart, F->qparts, F->qacc, F->lnq_full,
-                      F->epart})
+                      F->epart, F->spart})
         cudaFree(p);
     cudaFree(F->Bp);
     cudaFree(F->Ddense);
@@ -1722,8 +1746,16 @@ static cudaError_t enqueue_stage(bdc_handle* H, int stage, double a) {
             if (F->use_oz) return ozaki_product(F->oz, make_epilogue(H), H->d_st, s);
             return launch_ba(F->g, make_epilogue(H), s, H->d_st);
         case ST_FIN:
-            k_fac_finalize<<<1, 256, 0, s>>>(F->epart, F->use_oz ? ozaki_partials(F->oz) : F->ctas_g, a, F->eta, H->d_st);
+        {
+            const int nb = F->use_oz ? ozaki_partials(F->oz) : F->ctas_g;
+            if (nb > kStatMany) {
+                k_fac_stats<<<kStatRows, 256, 0, s>>>(F->epart, nb, F->spart, H->d_st);
+                k_fac_finalize<<<1, 256, 0, s>>>(F->spart, kStatRows, a, F->eta, H->d_st);
+            } else {
+                k_fac_finalize<<<1, 256, 0, s>>>(F->epart, nb, a, F->eta, H->d_st);
+            }
             break;
+        }
     }
     return cudaGetLastError();
 }

@@ -94,7 +94,7 @@ __device__ __forceinline__ double word_occ(int p, int c, int u) {
 struct WordAux {
     WordTerm terms[kWordTerms];
     double weight[2 << kWordMaxHalf];
-    double occ[16];
+    __align__(16) double occ[16];
     int first[kWordMaxHalf + 2];
 };
 
@@ -246,14 +246,18 @@ __global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan
         const int capr = min(k - 1, r);
         for (int h = 1 + tid; h < (2 << capr); h += T) {
             double x = c[h];
-            for (int d = 1; d <= fixed; ++d)
-                for (int v = 0; v < (1 << d); ++v) {
-                    const double o = aux.occ[(1 << d) + v];
-                    const int g = (h << d) | v;
-                    if (o == 0.0) continue;
-                    if (g < (2 << cap)) x = fma(o, c[g], x);
-                    else if (g >= nk && g < 2 * nk) x = fma(o * s0, __ldg(lnq + g - nk), x);
+            for (int d = 1; d <= fixed; ++d) {
+                const int g = h << d;  // the 2^d words z u, two at a time
+                const double* p = g < (2 << cap) ? c + g : lnq + (g - nk);
+                if (g >= (2 << cap) && (g < nk || g >= 2 * nk)) break;  // none that long
+                const double f = g < (2 << cap) ? 1.0 : s0;
+                for (int v = 0; v < (1 << d); v += 2) {
+                    const double2 o = *reinterpret_cast<const double2*>(aux.occ + (1 << d) + v);
+                    const double2 q = *reinterpret_cast<const double2*>(p + v);
+                    x = fma(o.x * f, q.x, x);
+                    x = fma(o.y * f, q.y, x);
                 }
+            }
             other[h] = x;
         }
         __syncthreads();
@@ -418,24 +422,39 @@ __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan
     for (int h = tid; h < (2 << a); h += T) aux.weight[h] = __ldg(S.weight + ((size_t)w << (a + 1)) + h);
     __syncthreads();
     const double* wt = aux.weight;
+    // two adjacent words at even heap index h
     auto after = [&](int h) {
-        double x = h < top ? root[h] : 0.0;
+        double2 x = make_double2(0.0, 0.0);
+        if (h < top) x = *reinterpret_cast<const double2*>(root + h);
         for (int d = 1; d <= fixed; ++d) {
             const int g = h >> d;
-            if (g > 0 && g < top) x = fma(aux.occ[(1 << d) + (h & ((1 << d) - 1))], root[g], x);
+            if (g > 0 && g < top) {
+                const double2 o = *reinterpret_cast<const double2*>(aux.occ + (1 << d) + (h & ((1 << d) - 1)));
+                const double t = root[g];
+                x.x = fma(o.x, t, x.x);
+                x.y = fma(o.y, t, x.y);
+            }
         }
         return x;
     };
-    for (int h = (1 << (k - a)) + tid; h < nk; h += T) c[h] = after(h);
+    // (k - a >= 1, so the shortest words read begin at an even index)
+    for (int h = (1 << (k - a)) + 2 * tid; h < nk; h += 2 * T) *reinterpret_cast<double2*>(c + h) = after(h);
     __syncthreads();
-    // acc[v z] = sum over the splits of y into |v| <= a characters and the rest
-    for (int y = tid; y < nk; y += T) {
-        double x = wt[1] * after(nk + y);
-        for (int j = 1; j <= a; ++j) {
+    // acc[v z] = sum over the splits of y into |v| <= a characters and the
+    // rest; two adjacent y share v and their z are adjacent
+    for (int y = 2 * tid; y < nk; y += 2 * T) {
+        const double2 z0 = after(nk + y);
+        double2 x = make_double2(wt[1] * z0.x, wt[1] * z0.y);
+#pragma unroll
+        for (int j = 1; j <= kWordMaxHalf; ++j) {
+            if (j > a) break;
             const int d = k - j;
-            x = fma(wt[(1 << j) + (y >> d)], c[(1 << d) + (y & ((1 << d) - 1))], x);
+            const double w = wt[(1 << j) + (y >> d)];
+            const double2 z = *reinterpret_cast<const double2*>(c + (1 << d) + (y & ((1 << d) - 1)));
+            x.x = fma(w, z.x, x.x);
+            x.y = fma(w, z.y, x.y);
         }
-        part[y] = x;
+        *reinterpret_cast<double2*>(part + y) = x;
     }
 }
 
