@@ -1028,7 +1028,7 @@ static cudaError_t launch_words(bool q_side, const FactoredState* F, cudaStream_
 
 // the largest transform's shared memory (k = 14), for every handle
 static cudaError_t set_words_attrs() {
-    const int smem = std::max(word_smem(12, 11), word_smem(14, 12));
+    const int smem = word_smem(14, 12);
     cudaError_t e = cudaFuncSetAttribute(k_words_q<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_words_d<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_words_q<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -1357,15 +1357,23 @@ bdc_status factored_init(bdc_handle* H) {
     BDC_CUDA_TRY(cudaGetLastError());
 
     // ---- the word transforms: one CTA per word and slice of 2^r strings of
-    // the other half.  r = 11 (12 for k > 12, whose words need the larger CTA
-    // anyway): a level's 2^{r+1} coefficients are 32 KB, so that several CTAs
-    // share an SM, and at n = 24 the 2^a * 2 + 2^b CTAs just cover the SMs.
+    // the other half.  The largest r <= 12 (64 KB a tree level) that still
+    // gives kWordCtas CTAs: a CTA's first and last steps do not shrink with its
+    // slice, but with far fewer CTAs than SMs the rounds' latency is all there
+    // is (22/11: 67 us an iteration with 96 CTAs at r = 10, 80 with 64 at 11;
+    // 24/12: 165 with 96 at r = 12, 168 with 160 at 11, 190 with 320 at 10).
+    // A slice fixes at most 3 characters (WordAux::occ).
+    constexpr int kWordCtas = 80;
     {
         WordPlan& P = F->plan;
         P.k = k;
-        const int rmax = k <= 12 ? 11 : 12;
         const int half[2] = {s.n1, s.n2};              // characters of the words' half
         const int bits[2] = {s.n2, s.n1 - 1};          // free characters of the other half
+        int rmax = 12;
+        auto ctas = [&](int r) {
+            return (KL << (bits[0] - std::min(bits[0], r))) + (KR << (bits[1] - std::min(bits[1], r)));
+        };
+        while (ctas(rmax) < kWordCtas && rmax > std::max({4, bits[0] - 3, bits[1] - 2})) --rmax;
         int cta = 0;
         for (int d = 0; d < 2; ++d) {
             WordSide& S = P.side[d];
@@ -1436,6 +1444,26 @@ bdc_status factored_init(bdc_handle* H) {
     BDC_CUDA_TRY(cudaStreamCreateWithFlags(&F->side, cudaStreamNonBlocking));
     BDC_CUDA_TRY(cudaEventCreateWithFlags(&F->ev_join, cudaEventDisableTiming));
     BDC_CUDA_TRY(cudaEventCreateWithFlags(&F->ev_fork, cudaEventDisableTiming));
+
+    // the candidates below are compared by their times: on an idle GPU the
+    // first ones would run at a lower clock and from cold instruction caches
+    // (the choices at 22/11 and 23/11 then differed by 15 to 30 us a run)
+    if (tf.m.empty()) {
+        cudaEvent_t e0, e1;
+        BDC_CUDA_TRY(cudaEventCreate(&e0));
+        BDC_CUDA_TRY(cudaEventCreate(&e1));
+        cudaError_t e = cudaEventRecord(e0, H->stream);
+        float ms = 0.f;
+        for (int i = 0; i < 100 && ms < 4.f && e == cudaSuccess; ++i) {
+            for (int j = 0; j < 16 && e == cudaSuccess; ++j) e = launch_words(true, F, H->stream, nullptr);
+            if (e == cudaSuccess) e = cudaEventRecord(e1, H->stream);
+            if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+        }
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        BDC_CUDA_TRY(e);
+    }
 
     // ---- the two thin products: U (KL x H2) = AL^T Pw, V (H1h x KR) = Pw BR
     // Only the rows x_hi <= colmax[c] of a dense column c hold
