@@ -62,7 +62,7 @@ static bdc_status make_bundle(bdc_handle* H, int hlen, int mmax, uint16_t** rows
     std::vector<uint32_t> host;
     int* d_over = nullptr;
     bdc_status rc = BDC_OK;
-    if (cudaMalloc(&d_over, sizeof(int)) != cudaSuccess || cudaMemset(d_over, 0, sizeof(int)) != cudaSuccess)
+    if (cudaMalloc(&d_over, sizeof(int)) != cudaSuccess || cudaMemsetAsync(d_over, 0, sizeof(int), H->stream) != cudaSuccess)
         return fail(BDC_ERR_CUDA, "cudaMalloc of the overflow flag failed");
     for (int m = 0; m <= mmax && rc == BDC_OK; ++m) {
         const size_t cnt = (size_t)1 << (hlen + m);
@@ -71,7 +71,7 @@ static bdc_status make_bundle(bdc_handle* H, int hlen, int mmax, uint16_t** rows
         rc = bdc_read_cache_file(path.c_str(), hlen, m, host.data());
         if (rc != BDC_OK) break;
         if (cudaMalloc(&dev[m], cnt * sizeof(uint32_t)) != cudaSuccess ||
-            cudaMemcpy(dev[m], host.data(), cnt * sizeof(uint32_t), cudaMemcpyHostToDevice) != cudaSuccess)
+            upload(dev[m], host.data(), cnt * sizeof(uint32_t)) != cudaSuccess)
             rc = fail(BDC_ERR_CUDA, "uploading %s failed", path.c_str());
     }
     if (rc == BDC_OK) {
@@ -358,6 +358,7 @@ bdc_status engine_init(bdc_handle* H) {
 void engine_free(bdc_handle* H) {
     if (H->stream) cudaStreamSynchronize(H->stream);
     solve_pool_release(H);
+    host_copy_free(H);
     if (H->fac) factored_free(H);
     if (H->stream) cudaStreamSynchronize(H->stream);
     release_tables(H);

@@ -58,6 +58,7 @@ struct bdc_handle {
     bool p_set = false;
     bool strict_load = false;  // the last load kept exact zeros at ln p = -inf (engine_after_set_p)
     int64_t nonzero_pairs = 0;  // sum over reps of distinct length-k subsequences
+    void* staging = nullptr;  // pinned buffers of large pageable copies (bdc_hostcopy.cu), on first use
     // factored engine
     FactoredState* fac = nullptr;
     // scratch blocks of the certified solver, reused across its calls (bdc_solve.cu)
@@ -67,6 +68,22 @@ struct bdc_handle {
 namespace bdc {
 
 bdc_status fail(bdc_status st, const char* fmt, ...) __attribute__((format(printf, 2, 3)));
+
+// Host memory to the device, complete on return.  cudaMemcpy from pageable
+// memory returns once the data is staged, and the handles' streams do not
+// wait for the default stream, so a kernel launched next could read the old
+// contents (large tile maps and descriptor lists did).
+inline cudaError_t upload(void* dst, const void* src, size_t bytes) {
+    const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(cudaStreamLegacy);
+}
+
+// `bytes` between host memory and the device, ordered with the work queued on
+// H->stream; a copy to the host is complete on return.  Large copies from or
+// to pageable memory go through pinned buffers of the handle, several at a
+// time.
+cudaError_t host_copy(bdc_handle* H, void* dst, const void* src, size_t bytes, cudaMemcpyKind kind);
+void host_copy_free(bdc_handle* H);
 
 int select_engine(int requested, int n, int k);
 bdc_status engine_init(bdc_handle* H);

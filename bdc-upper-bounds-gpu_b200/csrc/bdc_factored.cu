@@ -844,9 +844,9 @@ static cudaError_t make_launch(Launch& L, std::vector<GemmDesc> v, int cfg) {
     for (int i = 0; i < (int)v.size(); ++i)
         for (int t = 0; t < v[i].tiles_m * v[i].tiles_n; ++t) map[v[i].tile_begin + t] = i;
     cudaError_t e = cudaMalloc(&L.d, sizeof(GemmDesc) * v.size());
-    if (e == cudaSuccess) e = cudaMemcpy(L.d, v.data(), sizeof(GemmDesc) * v.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload(L.d, v.data(), sizeof(GemmDesc) * v.size());
     if (e == cudaSuccess) e = cudaMalloc(&L.map, sizeof(int) * map.size());
-    if (e == cudaSuccess) e = cudaMemcpy(L.map, map.data(), sizeof(int) * map.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload(L.map, map.data(), sizeof(int) * map.size());
     return e;
 }
 
@@ -907,9 +907,9 @@ static cudaError_t make_tile_launch(Launch& L, GemmDesc d, int cfg, const std::v
     L.tiles = (int)ids.size();
     if (ids.empty()) return cudaSuccess;
     cudaError_t e = cudaMalloc(&L.d, sizeof(GemmDesc));
-    if (e == cudaSuccess) e = cudaMemcpy(L.d, &d, sizeof(GemmDesc), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload(L.d, &d, sizeof(GemmDesc));
     if (e == cudaSuccess) e = cudaMalloc(&L.map, sizeof(int) * ids.size());
-    if (e == cudaSuccess) e = cudaMemcpy(L.map, ids.data(), sizeof(int) * ids.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload(L.map, ids.data(), sizeof(int) * ids.size());
     return e;
 }
 
@@ -960,12 +960,12 @@ struct TuneFile {
     }
 };
 
-// chooses tile shape (from cfgs) and split of U or V by timing them together
-// with the transform that reads their slices; gen(cfg, S) lists the
-// descriptors of a candidate (S: the split of the longest contraction, kfull
-// its length), post(cfg, S) runs the transform
-template <typename Gen, typename Post>
-static bdc_status tune_product(bdc_handle* H, TuneFile& tf, const char* key, Launch& L, Gen&& gen, Post&& post,
+// chooses tile shape (from cfgs) and split of U or V by timing run(candidate),
+// the product together with the transform that reads its slices; gen(cfg, S)
+// lists the descriptors of a candidate (S: the split of the longest
+// contraction, kfull its length), post(cfg, S) tells the transform its slices
+template <typename Gen, typename Post, typename Run>
+static bdc_status tune_product(bdc_handle* H, TuneFile& tf, const char* key, Launch& L, Gen&& gen, Post&& post, Run&& run,
                                const std::vector<int>& cfgs, int kfull, int max_split, int kmin, const char* what,
                                int* split_out) {
     float best = 1e30f;
@@ -983,12 +983,9 @@ static bdc_status tune_product(bdc_handle* H, TuneFile& tf, const char* key, Lau
                 free_launch(T);
                 continue;
             }
-            BDC_CUDA_TRY(post(cfg, S, false));
+            BDC_CUDA_TRY(post(cfg, S));
             cudaError_t e = cudaSuccess;
-            const float ms = time_ms(H, [&] {
-                const cudaError_t e1 = launch_store(T, H->stream, nullptr);
-                return e1 != cudaSuccess ? e1 : post(cfg, S, true);
-            }, &e);
+            const float ms = time_ms(H, [&] { return run(T); }, &e);
             free_launch(T);
             BDC_CUDA_TRY(e);
             if (ms < best) {
@@ -1000,7 +997,7 @@ static bdc_status tune_product(bdc_handle* H, TuneFile& tf, const char* key, Lau
     }
     if (!pinned) tf.put(key, best_cfg, best_s);
     BDC_CUDA_TRY(make_launch(L, gen(best_cfg, best_s), best_cfg));
-    BDC_CUDA_TRY(post(best_cfg, best_s, false));
+    BDC_CUDA_TRY(post(best_cfg, best_s));
     *split_out = best_s;
     if (H->verbose)
         printf("bdc: tuned %s: tile %dx%d, split %d, %.1f us with the transform\n", what, kCfgBM[best_cfg],
@@ -1203,9 +1200,9 @@ static bdc_status direct_init(bdc_handle* H) {
         BDC_CUDA_TRY(cudaMalloc(&S.state, sizeof(DevState)));
     }
     H->bytes += tb + vb * (2 * F->d_grid + 1);
-    BDC_CUDA_TRY(cudaMemcpy(F->d_members, members.data(), vb, cudaMemcpyHostToDevice));
+    BDC_CUDA_TRY(upload(F->d_members, members.data(), vb));
     BDC_CUDA_TRY(cudaMalloc(&d_y, sizeof(uint32_t) * yreps.size()));
-    BDC_CUDA_TRY(cudaMemcpy(d_y, yreps.data(), sizeof(uint32_t) * yreps.size(), cudaMemcpyHostToDevice));
+    BDC_CUDA_TRY(upload(d_y, yreps.data(), sizeof(uint32_t) * yreps.size()));
     k_direct_table<<<H->num_sms * 8, 256, 0, H->stream>>>(H->s, H->A, H->B, H->d_reps, H->R, d_y, P.NY, P.NYp, T);
     BDC_CUDA_TRY(cudaGetLastError());
     auto attr = [&](auto* k, int smem) {
@@ -1270,7 +1267,7 @@ bdc_status factored_init(bdc_handle* H) {
         std::vector<int64_t> rs((size_t)F->H1h + 1);
         for (int q = 0; q <= F->H1h; ++q) rs[(size_t)q] = below(c0 + q) - F->i0;
         BDC_CUDA_TRY(cudaMalloc(&F->d_rowstart, sizeof(int64_t) * rs.size()));
-        BDC_CUDA_TRY(cudaMemcpy(F->d_rowstart, rs.data(), sizeof(int64_t) * rs.size(), cudaMemcpyHostToDevice));
+        BDC_CUDA_TRY(upload(F->d_rowstart, rs.data(), sizeof(int64_t) * rs.size()));
         BDC_CUDA_TRY(cudaMalloc(&F->rpart, sizeof(double) * 2 * (size_t)F->H1h));
         F->rows_smem = rows_smem_bytes(s.n2);
         if (F->rows_smem > 48 * 1024) {
@@ -1344,7 +1341,7 @@ bdc_status factored_init(bdc_handle* H) {
         for (int c = 0; c < KR; ++c) colmap[KL + c] = bundle_offset(wb) + c;
         int* d_cm = nullptr;
         BDC_CUDA_TRY(cudaMalloc(&d_cm, sizeof(int) * colmap.size()));
-        BDC_CUDA_TRY(cudaMemcpy(d_cm, colmap.data(), sizeof(int) * colmap.size(), cudaMemcpyHostToDevice));
+        BDC_CUDA_TRY(upload(d_cm, colmap.data(), sizeof(int) * colmap.size()));
         k_fill_tables<<<H->num_sms * 8, 256, 0, H->stream>>>(H1, H2, Kp, H->A.rows + (size_t)F->row0 * H->A.stride,
                                                             H->A.stride, F->Bp,
                                                             H->B.stride, d_cm, KL, KR, F->LA, F->RB);
@@ -1408,9 +1405,9 @@ bdc_status factored_init(bdc_handle* H) {
                          b2 = first.size() * sizeof(int);
             BDC_CUDA_TRY(cudaMalloc(&F->d_wtab[d], b0 + b1 + b2));
             uint8_t* tab = (uint8_t*)F->d_wtab[d];
-            BDC_CUDA_TRY(cudaMemcpy(tab, terms.data(), b0, cudaMemcpyHostToDevice));
-            BDC_CUDA_TRY(cudaMemcpy(tab + b0, wt.data(), b1, cudaMemcpyHostToDevice));
-            BDC_CUDA_TRY(cudaMemcpy(tab + b0 + b1, first.data(), b2, cudaMemcpyHostToDevice));
+            BDC_CUDA_TRY(upload(tab, terms.data(), b0));
+            BDC_CUDA_TRY(upload(tab + b0, wt.data(), b1));
+            BDC_CUDA_TRY(upload(tab + b0 + b1, first.data(), b2));
             S.terms = (const WordTerm*)tab;
             S.weight = (const double*)(tab + b0);
             S.first = (const int*)(tab + b0 + b1);
@@ -1420,7 +1417,7 @@ bdc_status factored_init(bdc_handle* H) {
             S.in = d == 0 ? F->ulpart : F->vrpart;
             S.slice_stride = (int64_t)S.leaves << S.words_log;
             BDC_CUDA_TRY(cudaMalloc(&F->d_ns[d], (size_t)(S.leaves + 15) / 16));
-            BDC_CUDA_TRY(cudaMemset(F->d_ns[d], 0, (size_t)(S.leaves + 15) / 16));
+            BDC_CUDA_TRY(cudaMemsetAsync(F->d_ns[d], 0, (size_t)(S.leaves + 15) / 16, H->stream));
             S.ns = F->d_ns[d];
             cta += 1 << (S.words_log + S.t);
             F->words_smem = std::max(F->words_smem, word_smem(k, S.r));
@@ -1430,7 +1427,7 @@ bdc_status factored_init(bdc_handle* H) {
         F->words_threads = std::max(P.side[0].r, P.side[1].r) <= 11 ? 256 : 512;
         BDC_CUDA_TRY(set_words_attrs());
         BDC_CUDA_TRY(cudaMalloc(&F->d_plan, sizeof(WordPlan)));
-        BDC_CUDA_TRY(cudaMemcpy(F->d_plan, &P, sizeof(WordPlan), cudaMemcpyHostToDevice));
+        BDC_CUDA_TRY(upload(F->d_plan, &P, sizeof(WordPlan)));
         BDC_CUDA_TRY(al(&F->qparts, (size_t)cta << k));
         BDC_CUDA_TRY(al(&F->qacc, (size_t)ny));
         const int mb = k - 2 * fold_edge(k);
@@ -1439,7 +1436,7 @@ bdc_status factored_init(bdc_handle* H) {
             if (is_rep((uint32_t)m, mb)) mids.push_back(m);
         F->n_mids = (int)mids.size();
         BDC_CUDA_TRY(cudaMalloc(&F->d_mids, sizeof(int) * mids.size()));
-        BDC_CUDA_TRY(cudaMemcpy(F->d_mids, mids.data(), sizeof(int) * mids.size(), cudaMemcpyHostToDevice));
+        BDC_CUDA_TRY(upload(F->d_mids, mids.data(), sizeof(int) * mids.size()));
     }
     BDC_CUDA_TRY(cudaStreamCreateWithFlags(&F->side, cudaStreamNonBlocking));
     BDC_CUDA_TRY(cudaEventCreateWithFlags(&F->ev_join, cudaEventDisableTiming));
@@ -1490,21 +1487,23 @@ bdc_status factored_init(bdc_handle* H) {
             }
             return v;
         };
-        auto post = [&](int cfg, int S, bool run) -> cudaError_t {
-            if (run) return launch_words(true, F, H->stream, nullptr);
+        auto post = [&](int cfg, int S) -> cudaError_t {
             std::vector<uint8_t> ns((size_t)(H2 + 15) / 16, 0);
             const int BN = kCfgBN[cfg];
             for (int c = 0; c < H2; c += 16) {
                 const int n0 = c / BN * BN, kb = col_rows(n0, std::min(BN, H2 - n0));
                 ns[(size_t)c / 16] = kb == 0 ? 0 : (uint8_t)block_slices(S, kb, H1);
             }
-            return cudaMemcpy(F->d_ns[0], ns.data(), ns.size(), cudaMemcpyHostToDevice);
+            return upload(F->d_ns[0], ns.data(), ns.size());
         };
         const std::vector<int> cfgs = KL >= 128  ? std::vector<int>{CFG_128x64, CFG_64x64, CFG_64x128}
                                       : KL == 64 ? std::vector<int>{CFG_64x64, CFG_64x128}
                                       : KL == 32 ? std::vector<int>{CFG_32x64, CFG_32x128}
                                                  : std::vector<int>{CFG_16x128};
-        bdc_status rc = tune_product(H, tf, "u", F->ul, gen, post, cfgs, H1, max_split, 16, "U = AL^T Pw", &F->S1);
+        bdc_status rc = tune_product(H, tf, "u", F->ul, gen, post, [&](const Launch& T) {
+            const cudaError_t e = launch_store(T, H->stream, nullptr);
+            return e != cudaSuccess ? e : launch_words(true, F, H->stream, nullptr);
+        }, cfgs, H1, max_split, 16, "U = AL^T Pw", &F->S1);
         if (rc != BDC_OK) return rc;
     }
     {
@@ -1536,8 +1535,7 @@ bdc_status factored_init(bdc_handle* H) {
             }
             return v;
         };
-        auto post = [&](int cfg, int S, bool run) -> cudaError_t {
-            if (run) return launch_words(true, F, H->stream, nullptr);
+        auto post = [&](int cfg, int S) -> cudaError_t {
             std::vector<uint8_t> ns((size_t)(H1 + 15) / 16, 0);
             const int BM = kCfgBM[cfg];
             for (int r = 0; r < H1; r += 16) {
@@ -1545,12 +1543,19 @@ bdc_status factored_init(bdc_handle* H) {
                 const int kb = row_cols(r / BM * BM, &clo);
                 ns[(size_t)r / 16] = kb == 0 ? 0 : (uint8_t)block_slices(S, kb, H2);
             }
-            return cudaMemcpy(F->d_ns[1], ns.data(), ns.size(), cudaMemcpyHostToDevice);
+            return upload(F->d_ns[1], ns.data(), ns.size());
         };
         const std::vector<int> cfgs = KR >= 64   ? std::vector<int>{CFG_64x64, CFG_128x64}
                                       : KR == 32 ? std::vector<int>{CFG_64x32, CFG_128x32}
                                                  : std::vector<int>{CFG_128x16};
-        bdc_status rc = tune_product(H, tf, "v", F->vr, gen, post, cfgs, H2, max_split, 16, "V = Pw BR", &F->S2);
+        bdc_status rc = tune_product(H, tf, "v", F->vr, gen, post, [&](const Launch& T) {
+            // beside U, as it runs in an iteration
+            const Launch keep = F->vr;
+            F->vr = T;
+            cudaError_t e = enqueue_stage(H, ST_QBIG, -INFINITY);
+            F->vr = keep;
+            return e != cudaSuccess ? e : launch_words(true, F, H->stream, nullptr);
+        }, cfgs, H2, max_split, 16, "V = Pw BR", &F->S2);
         if (rc != BDC_OK) return rc;
     }
 
@@ -1583,7 +1588,9 @@ bdc_status factored_init(bdc_handle* H) {
             if (pinned) break;
             Launch T;
             BDC_CUDA_TRY(make_tile_launch(T, d, c, F->colmax));
-            const float ms = time_ms(H, [&] { return launch_ba(T, ep, H->stream, H->d_st); });
+            cudaError_t e = cudaSuccess;
+            const float ms = time_ms(H, [&] { return launch_ba(T, ep, H->stream, H->d_st); }, &e);
+            BDC_CUDA_TRY(e);
             if (ms < best) {
                 best = ms;
                 best_cfg = c;

@@ -756,7 +756,7 @@ bdc_status ozaki_init(bdc_handle* H, const OzakiInput& in, OzakiG** out, const c
         oz->grid = std::min(oz->tiles, H->num_sms);
         if (oz->tiles > 0) {
             BDC_CUDA_TRY(cudaMalloc(&oz->d_tiles, sizeof(int) * idsP.size()));
-            BDC_CUDA_TRY(cudaMemcpy(oz->d_tiles, idsP.data(), sizeof(int) * idsP.size(), cudaMemcpyHostToDevice));
+            BDC_CUDA_TRY(upload(oz->d_tiles, idsP.data(), sizeof(int) * idsP.size()));
         }
     }
     const bool ok = make_map(&oz->tmAs, oz->As, 2 * KLp, rows, kOzBM) &&

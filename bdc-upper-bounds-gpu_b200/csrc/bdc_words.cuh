@@ -212,6 +212,20 @@ __global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan
     for (int e = tid; e < kWordTerms; e += T) aux.terms[e] = S.terms[w * kWordTerms + e];
     if (tid < kWordMaxHalf + 2) aux.first[tid] = S.first[w * (kWordMaxHalf + 2) + tid];
     if (tid >= 32 && tid < 48) aux.occ[tid - 32] = tid > 32 ? word_occ(tailc, fixed, tid - 32) : 0.0;
+    // ln q to the second buffer where it fits: from global memory each of the
+    // dozen or so term steps below would wait for L2
+    const bool staged = (2 << r) >= nk;
+    if (staged) {
+        for (int y = 2 * tid; y < nk; y += 8 * T) {
+            double2 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (y + 2 * u * T < nk) v[u] = __ldg(reinterpret_cast<const double2*>(lnq + y + 2 * u * T));
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (y + 2 * u * T < nk) *reinterpret_cast<double2*>(other + y + 2 * u * T) = v[u];
+        }
+    }
     // c_w: zero below k - a characters ...
     for (int h = tid; h < (1 << (k - a)); h += T) c[h] = 0.0;
     __syncthreads();
@@ -226,10 +240,16 @@ __global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan
 #pragma unroll 2
             for (int e = e0; e < e1; ++e) {
                 const double wt = aux.terms[e].weight;
-                const double* q = lnq + ((size_t)aux.terms[e].v << d) + z;
+                const int at = (aux.terms[e].v << d) + z;
+                if (staged) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (z + i * T < n) x[i] = fma(wt, __ldg(q + i * T), x[i]);
+                    for (int i = 0; i < 4; ++i)
+                        if (z + i * T < n) x[i] = fma(wt, other[at + i * T], x[i]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (z + i * T < n) x[i] = fma(wt, __ldg(lnq + at + i * T), x[i]);
+                }
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i)
@@ -301,28 +321,13 @@ __global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan
 // one round of the q side for the item (u, h): the 2^Q children's values at
 // the tail -> X[v], |v| <= Q (read by every thread before any of them writes)
 template <int Q>
-__device__ __forceinline__ void word_contract_load(double (&X)[32], const double* wsm, int src, int u, int h, int i, int Lc, bool leaf, const WordSide& S, int w, int first) {
+__device__ __forceinline__ void word_contract_load(double (&X)[32], const double* wsm, int src, int u, int h, int i,
+                                                   int Lc, bool leaf) {
     double in[1 << Q];
-    if (!leaf) {
+    // (a leaf node is its one value)
 #pragma unroll
-        for (int v = 0; v < (1 << Q); ++v) in[v] = wsm[src + ((u + (v << i)) << (Lc + 1)) + h];
-    } else {
-        // the split slices, one after another with every leaf's load in flight
-        const double* p = S.in + (int64_t)w * S.leaves + (first + u - S.leaf0);
-        int n[1 << Q], most = 0;
-#pragma unroll
-        for (int v = 0; v < (1 << Q); ++v) {
-            const int at = first + u + (v << i) - S.leaf0;
-            n[v] = (at >= 0 && at < S.leaves) ? S.ns[at >> 4] : 0;
-            most = max(most, n[v]);
-            in[v] = 0.0;
-        }
-        for (int s = 0; s < most; ++s) {
-#pragma unroll
-            for (int v = 0; v < (1 << Q); ++v)
-                if (s < n[v]) in[v] += __ldg(p + s * S.slice_stride + ((int64_t)v << i));
-        }
-    }
+    for (int v = 0; v < (1 << Q); ++v)
+        in[v] = leaf ? wsm[src + u + (v << i)] : wsm[src + ((u + (v << i)) << (Lc + 1)) + h];
     double Z[2 << Q];
     WordContract<Q>::run(Z, in, 1);
 #pragma unroll
@@ -375,6 +380,35 @@ __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan
     const int rounds = (r + 3) / 4;
     const int second = word_buf(k, r);
     int dst = (rounds & 1) ? second : 0, src = (rounds & 1) ? 0 : second;
+    // the leaves first: the split slices added up, 4 leaves x 4 slices of a
+    // thread in flight (a slice at a time, each added slice waited for L2)
+    for (int i = tid; i < (1 << r); i += 4 * T) {
+        double x[4] = {0.0, 0.0, 0.0, 0.0};
+        int n[4], most = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int at = first + i + q * T - S.leaf0;
+            n[q] = (i + q * T < (1 << r) && at >= 0 && at < S.leaves) ? (int)S.ns[at >> 4] : 0;
+            most = max(most, n[q]);
+        }
+        const double* p = S.in + (int64_t)w * S.leaves + (first + i - S.leaf0);
+        for (int s = 0; s < most; s += 4) {
+            double v[4][4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    v[e][q] = s + e < n[q] ? __ldg(p + (s + e) * S.slice_stride + q * T) : 0.0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) x[q] += v[e][q];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (i + q * T < (1 << r)) wsm[src + i + q * T] = x[q];
+    }
+    __syncthreads();
     for (int g = rounds - 1; g >= 0; --g) {
         const int i = 4 * g, rem = r - i, q = word_round(rem);
         const int Lp = min(k, rem), Lc = min(k, rem - q);
@@ -385,7 +419,7 @@ __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan
         const bool live = u < (1 << i);
         double X[32];
 #define BDC_ROUND_(Q_)                                                                  \
-    if (live) word_contract_load<Q_>(X, wsm, src, u, h, i, Lc, leaf, S, w, first);           \
+    if (live) word_contract_load<Q_>(X, wsm, src, u, h, i, Lc, leaf);         \
     word_contract_add<Q_>(X, wsm, dst, u, h, Lp, Lc, live);
         switch (q) {
             case 4: BDC_ROUND_(4) break;
@@ -401,16 +435,8 @@ __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan
     // the root is in the second buffer
     const double* root = wsm + second;
     double* c = wsm;
-    if (r == 0) {
-        if (tid == 0) {
-            double x = 0.0;
-            if (first >= S.leaf0 && first < S.leaf0 + S.leaves) {
-                const double* p = S.in + (int64_t)w * S.leaves + (first - S.leaf0);
-                const int n = S.ns[(first - S.leaf0) >> 4];
-                for (int s = 0; s < n; ++s) x += p[s * S.slice_stride];
-            }
-            wsm[second + 1] = x;
-        }
+    if (r == 0) {  // no round: the leaf is the root (src is the second buffer)
+        if (tid == 0) wsm[second + 1] = wsm[second];
         __syncthreads();
     }
     // the root's words up to length min(k, r).  The fixed last characters
