@@ -31,6 +31,8 @@
 #include <map>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "bdc_engine.cuh"
 
 namespace bdc {
@@ -1109,6 +1111,338 @@ __global__ void __launch_bounds__(kRsBlock) k_rs_step_mixed(int L, int m, const 
     rs_accept_body(L, m, x, g, ga, st);
 }
 
+// ---- the same loop in one thread-block cluster.  The six launches of a step
+// take about 40 us whatever the size (the chain of their latencies); where the
+// rows of S, folded over the output orbits (a quarter of the entries; a folded
+// entry is at most C(n,k) < 2^24, exact in FP32), fit the
+// shared memory of up to 16 CTAs, the loop stays there: a CTA holds its share of the members' rows
+// and vectors, the q shares and the scalars cross the cluster's shared memory,
+// and a step is six hardware cluster barriers.  Every CTA adds the shares in
+// the same order and takes the same decisions from them, so the control flow
+// is uniform across the cluster.  Measured, an evaluation: 20/10 (205 members,
+// 8 CTAs) 21 us by the launches, 8.2 us here; 16 CTAs take 8.8 us there (the
+// barriers of the wider cluster), so a member's CTA count stops at 8 unless
+// the rows need more.  24/12's 765 members (3.3 MB folded) stay with the launches.
+constexpr int kRcThreads = 512;
+constexpr int kRcSteps = 16;  // steps a launch, as in the other form's graph
+constexpr int kRcStatic = 8192;  // room left for the static shared memory
+
+struct RcPlan {
+    int S, Sc, NY, NYp, m, ctas;
+    const float* rows;      // [S][NYp] folded rows
+    const double* members;  // [NYp] |O(r)|, 1 past NY
+    const uint8_t* w;
+    const double* h;
+    double inv_c;
+};
+
+__host__ __device__ inline size_t rc_smem(int Sc, int NYp) {
+    return sizeof(float) * (size_t)Sc * NYp + sizeof(double) * ((size_t)3 * NYp + (size_t)Sc * (10 + 2 * kAAMax));
+}
+
+__global__ void k_rc_fold(int S, int k, int NY, int NYp, const uint32_t* __restrict__ yreps,
+                          const float* __restrict__ rows, float* __restrict__ out) {
+    const int64_t tot = (int64_t)S * NYp;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
+        const int s = (int)(e / NYp), j = (int)(e % NYp);
+        float v = 0.0f;
+        if (j < NY) {
+            const uint32_t y = yreps[j], r = reverse_bits(y, k), c = complement_bits(y, k), rc = reverse_bits(c, k);
+            const float* row = rows + ((int64_t)s << k);
+            v = row[y];
+            if (r != y) v += row[r];
+            if (c != y && c != r) v += row[c];
+            if (rc != y && rc != r && rc != c) v += row[rc];
+        }
+        out[e] = v;
+    }
+}
+
+__global__ void __launch_bounds__(kRcThreads, 1)
+k_rc_loop(RcPlan P, double* __restrict__ xg, double* __restrict__ flg, double* __restrict__ glg, RsSlots V,
+          RsAAState* __restrict__ stg, int steps) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const int C = P.ctas, rank = (int)cl.block_rank(), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int NYp = P.NYp, Sc = P.Sc, m = P.m, s0 = rank * Sc, n = max(0, min(Sc, P.S - s0));
+    extern __shared__ __align__(16) double rcs[];
+    double* qp = rcs;             // [NYp] this CTA's share of q
+    double* lnq = qp + NYp;       // [NYp]
+    double* mem = lnq + NYp;      // [NYp] 1 / (|O| C)
+    double* x = mem + NYp;        // members' vectors, Sc each
+    double *g = x + Sc, *xa = g + Sc, *ga = xa + Sc, *h = ga + Sc, *w = h + Sc, *D = w + Sc, *wp = D + Sc,
+           *fl = wp + Sc, *gl = fl + Sc, *dF = gl + Sc, *dG = dF + kAAMax * Sc;
+    float* rows = reinterpret_cast<float*>(dG + kAAMax * Sc);  // [Sc][NYp]
+    __shared__ RsAAState S;
+    __shared__ double xch[2][2 * kAAMax], got[2 * kAAMax], M[kAAMax][kAAMax + 1], yv[kAAMax];
+    __shared__ int solved;
+    int buf = 0;
+    if (tid == 0) S = *stg;
+    for (int i = tid; i < n * NYp; i += kRcThreads) rows[i] = P.rows[(int64_t)s0 * NYp + i];
+    for (int y = tid; y < NYp; y += kRcThreads) mem[y] = P.inv_c / P.members[y];
+    for (int i = tid; i < n; i += kRcThreads) {
+        x[i] = xg[s0 + i];
+        fl[i] = flg[s0 + i];
+        gl[i] = glg[s0 + i];
+        h[i] = P.h[s0 + i];
+        w[i] = (double)P.w[s0 + i];
+        for (int a = 0; a < m; ++a) {
+            dF[a * Sc + i] = V.dF[a][s0 + i];
+            dG[a * Sc + i] = V.dG[a][s0 + i];
+        }
+    }
+    __syncthreads();
+    // the sum over the cluster of xch[buf][0 .. cnt)
+    auto exchange = [&](int cnt) {
+        cl.sync();
+        if (tid < cnt) {
+            double v = *cl.map_shared_rank(&xch[buf][tid], 0);
+            for (int c = 1; c < C; ++c) v += *cl.map_shared_rank(&xch[buf][tid], c);
+            got[tid] = v;
+        }
+        buf ^= 1;
+        __syncthreads();
+    };
+    auto wsum = [](double v) {
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+        return v;
+    };
+    auto wmax = [](double v) {
+        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
+        return v;
+    };
+    // the BA map px -> po, recorded as evaluation rec (1 plain, 2 mixed)
+    auto map = [&](const double* px, double* po, int rec) {
+        for (int i = tid; i < n; i += kRcThreads) wp[i] = w[i] * px[i];
+        __syncthreads();
+        for (int y = tid; y < NYp; y += kRcThreads) {
+            double a[4] = {0.0, 0.0, 0.0, 0.0};
+            int i = 0;
+            for (; i + 4 <= n; i += 4)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) a[u] = fma(wp[i + u], (double)rows[(i + u) * NYp + y], a[u]);
+            for (; i < n; ++i) a[0] = fma(wp[i], (double)rows[i * NYp + y], a[0]);
+            qp[y] = (a[0] + a[1]) + (a[2] + a[3]);
+        }
+        cl.sync();
+        for (int y = tid; y < NYp; y += kRcThreads) {
+            double q = 0.0;
+#pragma unroll 8
+            for (int c = 0; c < C; ++c) q += *cl.map_shared_rank(qp + y, c);
+            q *= mem[y];
+            lnq[y] = q > 0.0 ? log(q) : 0.0;
+        }
+        __syncthreads();
+        for (int i = warp; i < n; i += kRcThreads / 32) {
+            double a = 0.0, b = 0.0;
+            int y = lane;
+            for (; y + 32 < NYp; y += 64) {
+                a = fma((double)rows[i * NYp + y], lnq[y], a);
+                b = fma((double)rows[i * NYp + y + 32], lnq[y + 32], b);
+            }
+            if (y < NYp) a = fma((double)rows[i * NYp + y], lnq[y], a);
+            a = wsum(a + b);
+            if (lane == 0) D[i] = h[i] - a * P.inv_c;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            // the exponentials relative to this CTA's largest D; the shares of
+            // the normaliser meet at the cluster's
+            double mx = -DBL_MAX, r = 0.0, z = 0.0;
+            for (int i = lane; i < n; i += 32) {
+                mx = fmax(mx, D[i]);
+                r = fma(wp[i], D[i], r);
+            }
+            mx = wmax(mx);
+            for (int i = lane; i < n; i += 32) {
+                po[i] = px[i] * exp(D[i] - mx);
+                z = fma(w[i], po[i], z);
+            }
+            r = wsum(r);
+            z = wsum(z);
+            if (lane == 0) {
+                xch[buf][0] = mx;
+                xch[buf][1] = r;
+                xch[buf][2] = z;
+            }
+        }
+        __syncthreads();
+        cl.sync();
+        if (warp == 0) {
+            const double* o = lane < C ? cl.map_shared_rank(&xch[buf][0], lane) : nullptr;
+            const double mc = o ? o[0] : -DBL_MAX, mx = wmax(mc);
+            const double f = exp(mc - mx), r = wsum(o ? o[1] : 0.0), z = wsum(o ? f * o[2] : 0.0);
+            if (lane == rank) got[2] = f / z;
+            if (lane == 0) {
+                got[0] = mx;
+                got[1] = r;
+            }
+        }
+        buf ^= 1;
+        __syncthreads();
+        const double inv = got[2];
+        for (int i = tid; i < n; i += kRcThreads) po[i] *= inv;
+        if (tid == 0) {
+            const double u = got[0], r = got[1];
+            if (rec == 1) S.u = u, S.r = r;
+            else S.ua = u, S.ra = r;
+            if (isfinite(u)) S.ub = fmin(S.ub, u);
+            if (isfinite(r)) S.rate = fmax(S.rate, r);
+            S.evals += 1;
+            if (S.ub - S.rate < S.target) {
+                if (rec == 1) S.stop_plain = 1;
+                else S.stop_mixed = 1;
+            }
+        }
+        __syncthreads();
+    };
+    for (int it = 0; it < steps && !S.fin; ++it) {
+        map(x, g, 1);
+        if (!S.stop_plain) {
+            // the pair (x, g): its differences, their Gram row, the weights
+            const bool diff = S.have_last != 0;
+            const int sl = S.npush % m, act = min(S.npush + 1, m);
+            for (int i = tid; i < n; i += kRcThreads) {
+                const double gi = g[i], fi = gi - x[i];
+                if (diff) {
+                    dF[sl * Sc + i] = fi - fl[i];
+                    dG[sl * Sc + i] = gi - gl[i];
+                }
+                fl[i] = fi;
+                gl[i] = gi;
+            }
+            __syncthreads();
+            if (diff) {
+                if (warp < act) {
+                    double a = 0.0, b = 0.0;
+                    for (int i = lane; i < n; i += 32) {
+                        const double d = w[i] * dF[warp * Sc + i];
+                        a = fma(d, dF[sl * Sc + i], a);
+                        b = fma(d, fl[i], b);
+                    }
+                    a = wsum(a);
+                    b = wsum(b);
+                    if (lane == 0) {
+                        xch[buf][warp] = a;
+                        xch[buf][kAAMax + warp] = b;
+                    }
+                }
+                __syncthreads();
+                exchange(2 * kAAMax);
+                if (tid < act) {
+                    S.A[sl][tid] = got[tid];
+                    S.A[tid][sl] = got[tid];
+                    S.b[tid] = got[kAAMax + tid];
+                }
+            }
+            if (tid == 0) solved = 0;
+            __syncthreads();
+            if (diff && warp == 0) {
+                // (A + lambda I) gamma = b in ring order, oldest difference
+                // first (position j: slot (npush - c + j) % m), by Cholesky
+                const int c = act, np = S.npush + 1;
+                auto slot = [&](int j) { return (np - c + j) % m; };
+                double tr = 0.0;
+                for (int j = 0; j < c; ++j) tr += S.A[slot(j)][slot(j)];
+                bool ok = tr > 0.0 && isfinite(tr);
+                const double lam = 1e-12 * tr / c;
+                for (int e = lane; e < c * c; e += 32) {
+                    const int i = e / c, j = e % c;
+                    M[i][j] = S.A[slot(i)][slot(j)] + (i == j ? lam : 0.0);
+                }
+                if (lane < c) yv[lane] = S.b[slot(lane)];
+                __syncwarp();
+                for (int j = 0; j < c && ok; ++j) {
+                    const double d = M[j][j];
+                    ok = d > 0.0;
+                    const double ri = rsqrt(d);
+                    __syncwarp();
+                    if (lane > j && lane < c) M[lane][j] *= ri;
+                    if (lane == j) M[j][j] = ri;  // the inverse of the pivot
+                    __syncwarp();
+                    const int q = c - j - 1;
+                    for (int e = lane; e < q * q; e += 32) {
+                        const int i = j + 1 + e / q, t = j + 1 + e % q;
+                        if (t <= i) M[i][t] = fma(-M[i][j], M[t][j], M[i][t]);
+                    }
+                    __syncwarp();
+                }
+                for (int j = 0; j < c && ok; ++j) {
+                    const double y = yv[j] * M[j][j];
+                    __syncwarp();
+                    if (lane == j) yv[j] = y;
+                    if (lane > j && lane < c) yv[lane] = fma(-M[lane][j], y, yv[lane]);
+                    __syncwarp();
+                }
+                for (int j = c - 1; j >= 0 && ok; --j) {
+                    const double y = yv[j] * M[j][j];
+                    __syncwarp();
+                    if (lane == j) yv[j] = y;
+                    if (lane < j) yv[lane] = fma(-M[j][lane], y, yv[lane]);
+                    __syncwarp();
+                }
+                for (int j = 0; j < c && ok; ++j) ok = isfinite(yv[j]);
+                if (lane == 0) solved = ok ? 1 : 0;
+                if (ok && lane < c) S.gamma[lane] = yv[lane];
+            }
+            __syncthreads();
+            if (tid == 0) {
+                S.solve_ok = solved;
+                if (diff) S.npush += 1;
+                else S.have_last = 1;
+            }
+            __syncthreads();
+            if (S.solve_ok) {
+                // the mixed point, clipped at 0 and normalised, and its map
+                const int c = min(S.npush, m);
+                for (int i = tid; i < n; i += kRcThreads) {
+                    double v = gl[i];
+                    for (int j = 0; j < c; ++j) v -= S.gamma[j] * dG[((S.npush - c + j) % m) * Sc + i];
+                    xa[i] = v > 0.0 ? v : 0.0;
+                }
+                __syncthreads();
+                if (warp == 0) {
+                    double z = 0.0;
+                    for (int i = lane; i < n; i += 32) z = fma(w[i], xa[i], z);
+                    z = wsum(z);
+                    if (lane == 0) xch[buf][0] = z;
+                }
+                __syncthreads();
+                exchange(1);
+                const double inv = got[0] > 0.0 ? 1.0 / got[0] : 0.0;
+                for (int i = tid; i < n; i += kRcThreads) xa[i] *= inv;
+                __syncthreads();
+                map(xa, ga, 2);
+            }
+        }
+        // the next iterate
+        const bool kept = !S.stop_plain && rs_mixed_kept(&S);
+        for (int i = tid; i < n; i += kRcThreads) x[i] = kept ? ga[i] : g[i];
+        __syncthreads();
+        if (tid == 0) {
+            if (S.stop_plain) {
+                S.fin = 1;
+            } else {
+                if (!kept && min(S.npush, m) >= 1) S.npush = 0, S.have_last = 0;
+                if (S.stop_mixed) S.fin = 1;
+                S.solve_ok = 0;
+            }
+        }
+        __syncthreads();
+    }
+    for (int i = tid; i < n; i += kRcThreads) {
+        xg[s0 + i] = x[i];
+        flg[s0 + i] = fl[i];
+        glg[s0 + i] = gl[i];
+        for (int a = 0; a < m; ++a) {
+            V.dF[a][s0 + i] = dF[a * Sc + i];
+            V.dG[a][s0 + i] = dG[a * Sc + i];
+        }
+    }
+    if (rank == 0 && tid == 0) *stg = S;
+    cl.sync();  // no CTA leaves while another may still read its shared memory
+}
+
 struct RsAA {
     int L = 0, m = 0;
     DevBuf f_last, g_last, st;
@@ -1167,12 +1501,96 @@ static cudaError_t rs_enqueue_step(bdc_handle* H, Restricted& rs, RsAA& aa, doub
     return cudaGetLastError();
 }
 
+// The cluster loop's buffers for a restricted problem; ctas = 0 when the rows
+// do not fit 16 CTAs or the device cannot place the cluster
+struct RcLoop {
+    DevBuf rows, members, yreps;
+    RcPlan plan{};
+    size_t smem = 0;
+
+    cudaLaunchConfig_t config(cudaLaunchAttribute* at, cudaStream_t s) const {
+        at->id = cudaLaunchAttributeClusterDimension;
+        at->val.clusterDim.x = (unsigned)plan.ctas;
+        at->val.clusterDim.y = at->val.clusterDim.z = 1;
+        cudaLaunchConfig_t c{};
+        c.gridDim = dim3((unsigned)plan.ctas);
+        c.blockDim = dim3(kRcThreads);
+        c.dynamicSmemBytes = smem;
+        c.stream = s;
+        c.attrs = at;
+        c.numAttrs = 1;
+        return c;
+    }
+    bdc_status init(bdc_handle* H, const Restricted& rs) {
+        std::vector<uint32_t> yr;
+        std::vector<double> mem;
+        for (uint32_t y = 0; y < (1u << H->k); ++y) {
+            if (!is_rep(y, H->k)) continue;
+            uint32_t img[4] = {y, reverse_bits(y, H->k), complement_bits(y, H->k), 0};
+            img[3] = reverse_bits(img[2], H->k);
+            std::sort(img, img + 4);
+            mem.push_back((double)(std::unique(img, img + 4) - img));
+            yr.push_back(y);
+        }
+        RcPlan& P = plan;
+        P.S = rs.S;
+        P.NY = (int)yr.size();
+        P.NYp = (P.NY + 3) / 4 * 4;
+        P.m = kAAMax;
+        mem.resize(P.NYp, 1.0);
+        int optin = 0;
+        BDC_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, H->device));
+        for (P.ctas = 1; P.ctas <= 16; P.ctas *= 2) {
+            P.Sc = (P.S + P.ctas - 1) / P.ctas;
+            smem = rc_smem(P.Sc, P.NYp);
+            if (smem + kRcStatic <= (size_t)optin && (P.Sc <= 32 || P.ctas >= 8)) break;
+        }
+        if (P.ctas > 16) {
+            P.ctas = 0;
+            return BDC_OK;
+        }
+        cudaError_t e = cudaFuncSetAttribute(k_rc_loop, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - kRcStatic);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rc_loop, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        int fit = 0;
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = config(&at, H->stream);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fit, k_rc_loop, &cfg);
+        if (e != cudaSuccess || fit < 1) {
+            (void)cudaGetLastError();
+            P.ctas = 0;
+            return BDC_OK;
+        }
+        BDC_CUDA_TRY(dalloc(rows, sizeof(float) * (size_t)P.S * P.NYp));
+        BDC_CUDA_TRY(dalloc(members, sizeof(double) * P.NYp));
+        BDC_CUDA_TRY(dalloc(yreps, sizeof(uint32_t) * P.NY));
+        BDC_CUDA_TRY(cudaStreamSynchronize(H->stream));  // (a pool block may still be read by queued work)
+        BDC_CUDA_TRY(upload(members.p, mem.data(), sizeof(double) * P.NYp));
+        BDC_CUDA_TRY(upload(yreps.p, yr.data(), sizeof(uint32_t) * P.NY));
+        const int gr = (int)std::min<int64_t>(H->num_sms * 8, ((int64_t)P.S * P.NYp + 255) / 256);
+        k_rc_fold<<<gr, 256, 0, H->stream>>>(P.S, H->k, P.NY, P.NYp, yreps.get<uint32_t>(), rs.rows.get<float>(),
+                                             rows.get<float>());
+        BDC_CUDA_TRY(cudaGetLastError());
+        P.rows = rows.get<float>();
+        P.members = members.get<double>();
+        P.w = rs.w.get<uint8_t>();
+        P.h = rs.h.get<double>();
+        P.inv_c = H->inv_c;
+        return BDC_OK;
+    }
+    cudaError_t launch(cudaStream_t s, const RsAA& aa, double* x) const {
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = config(&at, s);
+        return cudaLaunchKernelEx(&cfg, k_rc_loop, plan, x, aa.f_last.get<double>(), aa.g_last.get<double>(), aa.slots(),
+                                  aa.st.get<RsAAState>(), kRcSteps);
+    }
+};
+
 // accelerated_ba on the restricted problem, resident on the device: runs
 // until the bracket (started from br) is below gap_bits or about max_evals
 // evaluations (checked once per graph of kRsGraphSteps steps); x holds the
 // start and receives the last accepted point
-static bdc_status rs_accelerated(bdc_handle* H, Restricted& rs, RsAA& aa, double* x, double* g, double* xa,
-                                 double* ga, double gap_bits, int64_t max_evals, Bracket& br, int64_t* evals) {
+static bdc_status rs_accelerated(bdc_handle* H, Restricted& rs, RsAA& aa, const RcLoop& rc, double* x, double* g,
+                                 double* xa, double* ga, double gap_bits, int64_t max_evals, Bracket& br, int64_t* evals) {
     cudaStream_t s = H->stream;
     RsAAState hs;
     memset(&hs, 0, sizeof(hs));
@@ -1185,20 +1603,22 @@ static bdc_status rs_accelerated(bdc_handle* H, Restricted& rs, RsAA& aa, double
     // default stream, which cannot be captured), launched on the caller's
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    H->stream = H->own_stream;
-    cudaError_t e = cudaStreamBeginCapture(H->own_stream, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
+    const bool cluster = rc.plan.ctas > 0;
+    if (!cluster) H->stream = H->own_stream;
+    cudaError_t e = cluster ? cudaSuccess : cudaStreamBeginCapture(H->own_stream, cudaStreamCaptureModeThreadLocal);
+    if (!cluster && e == cudaSuccess) {
         for (int k = 0; k < kRsGraphSteps && e == cudaSuccess; ++k) e = rs_enqueue_step(H, rs, aa, x, g, xa, ga);
         const cudaError_t e2 = cudaStreamEndCapture(H->own_stream, &graph);
         if (e == cudaSuccess) e = e2;
     }
     H->stream = s;
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-    // two graphs in flight: while the host reads the state after one, the
-    // next already runs (after the loop finishes every kernel returns at
-    // once, so a graph queued past the end changes nothing)
+    if (!cluster && e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
+    // two graphs (or launches of the cluster loop) in flight: while the host
+    // reads the state after one, the next already runs (after the loop
+    // finishes every kernel returns at once, so a graph queued past the end
+    // changes nothing)
     auto queue = [&](int i) -> cudaError_t {
-        cudaError_t r = cudaGraphLaunch(exec, s);
+        cudaError_t r = cluster ? rc.launch(s, aa, x) : cudaGraphLaunch(exec, s);
         if (r == cudaSuccess) r = cudaMemcpyAsync(aa.host[i], aa.st.p, sizeof(RsAAState), cudaMemcpyDeviceToHost, s);
         if (r == cudaSuccess) r = cudaEventRecord(aa.copied[i], s);
         return r;
@@ -1607,6 +2027,12 @@ bdc_status solve_impl(bdc_handle_t H, double gap_bits, int64_t max_evals, bdc_st
         }
         RsAA aa;
         BDC_CUDA_TRY(aa.init(Sn, kAAMax));
+        RcLoop rcl;
+        rc = rcl.init(H, rs);
+        if (rc != BDC_OK) return rc;
+        if (H->verbose && rcl.plan.ctas > 0)
+            printf("bdc: solve round %d: restricted loop in a cluster of %d CTAs, %zu KB each\n", round, rcl.plan.ctas,
+                   rcl.smem >> 10);
         DevBuf pbak;
         BDC_CUDA_TRY(dalloc(pbak, sizeof(double) * Sn));
         Bracket rb;
@@ -1617,7 +2043,7 @@ bdc_status solve_impl(bdc_handle_t H, double gap_bits, int64_t max_evals, bdc_st
         // target, the copy comes back (its steps set members to zero for
         // good, which BA could not undo) and BA alone runs to the target.
         const double target = std::min(gap_bits * 1e-2, 1e-11);
-        rc = rs_accelerated(H, rs, aa, ps.get<double>(), pg.get<double>(), psa.get<double>(), pga.get<double>(),
+        rc = rs_accelerated(H, rs, aa, rcl, ps.get<double>(), pg.get<double>(), psa.get<double>(), pga.get<double>(),
                             std::max(target, kRestrictedSwitchBits), 400000, rb, &revals);
         if (rc != BDC_OK) return rc;
         if (H->verbose)
@@ -1638,7 +2064,7 @@ bdc_status solve_impl(bdc_handle_t H, double gap_bits, int64_t max_evals, bdc_st
                 rb.add(nb.ub, nb.rate);
             } else {
                 BDC_CUDA_TRY(cudaMemcpyAsync(ps.p, pbak.p, sizeof(double) * Sn, cudaMemcpyDeviceToDevice, s));
-                rc = rs_accelerated(H, rs, aa, ps.get<double>(), pg.get<double>(), psa.get<double>(),
+                rc = rs_accelerated(H, rs, aa, rcl, ps.get<double>(), pg.get<double>(), psa.get<double>(),
                                     pga.get<double>(), target, 400000, rb, &revals);
                 if (rc != BDC_OK) return rc;
             }
