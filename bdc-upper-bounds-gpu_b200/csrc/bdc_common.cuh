@@ -186,7 +186,6 @@ struct DevState {
     double best_rate;    // max over evaluated iterates of I(p;W) (nats): a lower bound
     double ng_prev_rate; // accelerated loop: I(p;W) at the last accepted extrapolated point
     double ng_gap;       // accelerated loop: stop when best_ub - best_rate < this (nats)
-    double ng_max;       // accelerated loop: max of the extrapolated log iterate
     long long ng_t;      // accelerated loop: steps since the last restart (momentum t / (t + 3))
     long long iter;      // iterations done since the last reset
     int cur;             // which of the two p buffers holds the current iterate

@@ -120,10 +120,9 @@ struct FactoredState {
     // a captured chunk of kGraphIters iterations for the threshold graph_a
     cudaGraphExec_t graph = nullptr;
     double graph_a = 0.0;
-    // accelerated loop: the normalised log iterates x_t and x_{t-1}, and the
-    // graph of kAccSteps steps
+    // accelerated loop: the normalised log iterate x_t and the graph of
+    // kAccSteps steps
     double* snap0 = nullptr;
-    double* snap1 = nullptr;
     cudaGraphExec_t cycle = nullptr;
     double cycle_eta = 0.0;
     // captured single BA maps (factored_map), by their vectors
@@ -1721,7 +1720,6 @@ void factored_free(bdc_handle* H) {
     for (auto& m : F->maps)
         if (m.exec) cudaGraphExecDestroy(m.exec);
     cudaFree(F->snap0);
-    cudaFree(F->snap1);
     for (Launch* L : {&F->ul, &F->vr, &F->g}) free_launch(*L);
     ozaki_free(F->oz);
     delete F;
@@ -2250,8 +2248,20 @@ __device__ __forceinline__ double block_max256(double v) {
 
 __device__ __forceinline__ bool acc_gated(const DevState* st) { return st->error != 0 || st->done; }
 
-// decides what the last evaluation means for the iterate: accept (mode 1),
-// restart (mode 2) or nothing yet (mode 0, the fresh start)
+// the device-side stop (the bracket of the evaluated points is below the gap)
+__device__ __forceinline__ bool acc_stop(DevState* st) {
+    if (st->best_ub - st->best_rate < st->ng_gap) st->done = 1;
+    return st->done != 0;
+}
+
+// after the last evaluation of a launch sequence: the host reads done next
+__global__ void k_acc_stop(DevState* st) {
+    if (acc_gated(st) || threadIdx.x != 0) return;
+    acc_stop(st);
+}
+
+// decides what the last evaluation means for the iterate: stop, accept
+// (mode 1), restart (mode 2) or nothing yet (mode 0, the fresh start)
 __global__ void k_acc_decide(DevState* st) {
     if (acc_gated(st) || threadIdx.x != 0) return;
     if (st->ng_mode < 0) {  // set by the host: nothing evaluated since the start
@@ -2260,6 +2270,7 @@ __global__ void k_acc_decide(DevState* st) {
         st->ng_prev_rate = -DBL_MAX;
         return;
     }
+    if (acc_stop(st)) return;
     if (st->rate >= st->ng_prev_rate) {
         st->ng_mode = 1;
         st->ng_prev_rate = st->rate;
@@ -2271,105 +2282,137 @@ __global__ void k_acc_decide(DevState* st) {
     }
 }
 
-// x_{t-1}, x_t (dense, at representatives) and the extrapolated ln y into Lt;
-// block max of ln y
-__global__ void __launch_bounds__(256) k_acc_extrap(int64_t nx, int n, int row0, double* __restrict__ xa,
-                                                    double* __restrict__ xb, double* __restrict__ Lt,
+// x_t (dense, at representatives), the extrapolated ln y into Lt and its
+// |O| y into Pw in one pass, two columns a thread with 16-byte accesses; block
+// max of ln y and block sums of |O| y.  ln y is near-normalised (y = x times a
+// power of the last step), so exp needs no shift; k_acc_setz redoes the pass
+// where it would.  Bound by memory: two reads and three writes of a double a
+// representative.  Measured at 24/12, a whole step: 251 us with a pass for ln y,
+// a pass for its exponentials and four single-block launches, 219 us now
+// (155 us of it the iteration).
+__global__ void __launch_bounds__(256) k_acc_extrap(int64_t pairs, int n, int row0, double* __restrict__ xa,
+                                                    double* __restrict__ Lt, double* __restrict__ Pw,
                                                     double* __restrict__ part, const DevState* st) {
     if (acc_gated(st)) return;
     const int mode = st->ng_mode;
     const double lnz = st->log_z;
     const double beta = (double)st->ng_t / ((double)st->ng_t + 3.0);
     const int n2 = n >> 1;
-    const uint32_t mask = low_mask(n2);
-    double mx = -DBL_MAX;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nx; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t xd = (uint32_t)i;
-        if (!dense_is_rep((xd >> n2) + (uint32_t)row0, xd & mask, mask, (uint32_t)n & 1u)) continue;
-        double y;
-        if (mode == 1) {
-            const double a_old = xa[xd], a_new = Lt[xd] - lnz;
-            xb[xd] = a_old;
-            xa[xd] = a_new;
-            // an input at exact zero (ln p = -inf) stays there
-            y = (a_new == -INFINITY) ? a_new : a_new + beta * (a_new - a_old);
-        } else {
-            y = xa[xd];
-            xb[xd] = y;
+    const uint32_t mask = low_mask(n2), odd = (uint32_t)n & 1u;
+    double mx = -DBL_MAX, sum = 0.0;
+    constexpr int U = 2;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t j0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j0 < pairs; j0 += U * step) {
+        double2 old[U], lt[U];
+        bool in[U][2];
+        uint32_t r[U], c[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t j = j0 + u * step;
+            const uint32_t xd = 2u * (uint32_t)j;
+            r[u] = (xd >> n2) + (uint32_t)row0;
+            c[u] = xd & mask;
+            in[u][0] = j < pairs && dense_is_rep(r[u], c[u], mask, odd);
+            in[u][1] = j < pairs && dense_is_rep(r[u], c[u] + 1u, mask, odd);
+            if (in[u][0] || in[u][1]) {
+                old[u] = reinterpret_cast<const double2*>(xa)[j];
+                if (mode == 1) lt[u] = reinterpret_cast<const double2*>(Lt)[j];
+            }
         }
-        Lt[xd] = y;
-        mx = fmax(mx, y);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (!in[u][0] && !in[u][1]) continue;
+            const int64_t j = j0 + u * step;
+            double nx[2], y[2], pw[2];
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const double ao = v ? old[u].y : old[u].x;
+                if (mode == 1) {
+                    nx[v] = (v ? lt[u].y : lt[u].x) - lnz;
+                    // an input at exact zero (ln p = -inf) stays there
+                    y[v] = (nx[v] == -INFINITY) ? nx[v] : nx[v] + beta * (nx[v] - ao);
+                } else {
+                    nx[v] = y[v] = ao;
+                }
+                if (in[u][v]) {
+                    pw[v] = dense_orbit(r[u], c[u] + v, mask, odd) * exp(y[v]);
+                    mx = fmax(mx, y[v]);
+                    sum += pw[v];
+                }
+            }
+            if (in[u][0] && in[u][1]) {
+                if (mode == 1) reinterpret_cast<double2*>(xa)[j] = make_double2(nx[0], nx[1]);
+                reinterpret_cast<double2*>(Lt)[j] = make_double2(y[0], y[1]);
+                reinterpret_cast<double2*>(Pw)[j] = make_double2(pw[0], pw[1]);
+            } else {
+                const int v = in[u][0] ? 0 : 1;
+                if (mode == 1) xa[2 * j + v] = nx[v];
+                Lt[2 * j + v] = y[v];
+                Pw[2 * j + v] = pw[v];
+            }
+        }
     }
     mx = block_max256(mx);
-    if (threadIdx.x == 0) part[blockIdx.x] = mx;
-}
-
-// one warp
-__global__ void k_acc_max(const double* __restrict__ part, int nb, DevState* st) {
-    if (acc_gated(st)) return;
-    const double m = warp_parts<true>(part, nb, 1);
-    if (threadIdx.x == 0) st->ng_max = m;
-}
-
-// Lt -= max, Pw = |O| exp(Lt); block sums of |O| exp(Lt)
-__global__ void __launch_bounds__(256) k_acc_pw(int64_t nx, int n, int row0, double* __restrict__ Lt,
-                                                double* __restrict__ Pw, double* __restrict__ part, const DevState* st) {
-    if (acc_gated(st)) return;
-    const double m = st->ng_max;
-    const int n2 = n >> 1;
-    const uint32_t mask = low_mask(n2);
-    double sum = 0.0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nx; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t xd = (uint32_t)i, r = (xd >> n2) + (uint32_t)row0, c = xd & mask, odd = (uint32_t)n & 1u;
-        if (!dense_is_rep(r, c, mask, odd)) continue;
-        const double l = Lt[xd] - m;
-        const double o = dense_orbit(r, c, mask, odd);
-        const double e = exp(l);
-        Lt[xd] = l;
-        Pw[xd] = o * e;
-        sum = fma(o, e, sum);
-    }
     sum = block_sum256(sum);
-    if (threadIdx.x == 0) part[blockIdx.x] = sum;
+    if (threadIdx.x == 0) {
+        part[2 * blockIdx.x] = mx;
+        part[2 * blockIdx.x + 1] = sum;
+    }
 }
 
-// ln Z of y and the exp shift of the next update (max ln y + eta * last bound)
-// one warp
-__global__ void k_acc_setz(const double* __restrict__ part, int nb, double eta, DevState* st) {
+// ln Z of y and the exp shift of the next update (max ln y - ln Z + eta * last
+// bound).  One block; where max ln y is so far from 0 that exp lost range, it
+// takes |O| exp(ln y - max) for all of y itself, which is slow and does not
+// happen to a step that the rate accepts.
+constexpr double kAccRange = 40.0;  // (a uniform start over 2^28 inputs has -19.4)
+__global__ void __launch_bounds__(256) k_acc_setz(const double* __restrict__ part, int nb, double eta, int64_t nx, int n,
+                                                  int row0, double* __restrict__ Lt, double* __restrict__ Pw,
+                                                  DevState* st) {
     if (acc_gated(st)) return;
-    const double s = warp_parts<false>(part, nb, 1);
+    double mx = -DBL_MAX, sum = 0.0;
+    for (int b = threadIdx.x; b < nb; b += 256) {
+        mx = fmax(mx, part[2 * b]);
+        sum += part[2 * b + 1];
+    }
+    mx = block_max256(mx);
+    sum = block_sum256(sum);
+    if (!(fabs(mx) <= kAccRange)) {
+        const int n2 = n >> 1;
+        const uint32_t mask = low_mask(n2), odd = (uint32_t)n & 1u;
+        sum = 0.0;
+        for (int64_t i = threadIdx.x; i < nx; i += 256) {
+            const uint32_t xd = (uint32_t)i, r = (xd >> n2) + (uint32_t)row0, c = xd & mask;
+            if (!dense_is_rep(r, c, mask, odd)) continue;
+            const double l = Lt[xd] - mx, v = dense_orbit(r, c, mask, odd) * exp(l);
+            Lt[xd] = l;
+            Pw[xd] = v;
+            sum += v;
+        }
+        sum = block_sum256(sum);
+        mx = 0.0;
+    }
     if (threadIdx.x != 0) return;
-    const double lnz = log(s);
+    const double lnz = log(sum);
     st->log_z = lnz;
-    st->shift = -lnz + eta * st->max_d;
-}
-
-// the device-side stop: the bracket of the evaluated points is below the gap
-__global__ void k_acc_stop(DevState* st) {
-    if (acc_gated(st) || threadIdx.x != 0) return;
-    if (st->best_ub - st->best_rate < st->ng_gap) st->done = 1;
+    st->shift = mx - lnz + eta * st->max_d;
 }
 
 static cudaError_t enqueue_acc_step(bdc_handle* H, double eta) {
     FactoredState* F = H->fac;
-    if (!F->snap0 || !F->snap1) return cudaErrorInvalidValue;  // factored_acc_buffers first
+    if (!F->snap0) return cudaErrorInvalidValue;  // factored_acc_buffers first
     cudaStream_t s = H->stream;
     const int nb = H->nb_upd;
     k_acc_decide<<<1, 32, 0, s>>>(H->d_st);
     const int64_t nx = (int64_t)F->H1h << H->s.n2;  // the dense positions of the held rows
-    k_acc_extrap<<<nb, 256, 0, s>>>(nx, H->n, F->row0, F->snap0, F->snap1, F->Lt, F->epart, H->d_st);
-    k_acc_max<<<1, 32, 0, s>>>(F->epart, nb, H->d_st);
-    k_acc_pw<<<nb, 256, 0, s>>>(nx, H->n, F->row0, F->Lt, F->Pw, F->epart, H->d_st);
-    k_acc_setz<<<1, 32, 0, s>>>(F->epart, nb, eta, H->d_st);
+    k_acc_extrap<<<nb, 256, 0, s>>>(nx / 2, H->n, F->row0, F->snap0, F->Lt, F->Pw, F->epart, H->d_st);
+    k_acc_setz<<<1, 256, 0, s>>>(F->epart, nb, eta, nx, H->n, F->row0, F->Lt, F->Pw, H->d_st);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const double keep = F->eta;
     F->eta = eta;
     e = enqueue_iteration(H, -INFINITY);
     F->eta = keep;
-    if (e != cudaSuccess) return e;
-    k_acc_stop<<<1, 32, 0, s>>>(H->d_st);
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t factored_enqueue_acc_steps(bdc_handle* H, int steps, double eta) {
@@ -2377,23 +2420,23 @@ cudaError_t factored_enqueue_acc_steps(bdc_handle* H, int steps, double eta) {
         cudaError_t e = enqueue_acc_step(H, eta);
         if (e != cudaSuccess) return e;
     }
-    return cudaSuccess;
+    k_acc_stop<<<1, 32, 0, H->stream>>>(H->d_st);
+    return cudaGetLastError();
 }
 
-// the loop's two snapshot vectors (dense, allocated on first use)
+// the loop's snapshot x_t (dense, allocated on first use)
 bdc_status factored_acc_buffers(bdc_handle* H) {
     FactoredState* F = H->fac;
     if (F->snap0) return BDC_OK;
     const size_t NX = (size_t)F->H1h * F->H2;
     BDC_CUDA_TRY(cudaMalloc(&F->snap0, sizeof(double) * NX));
-    BDC_CUDA_TRY(cudaMalloc(&F->snap1, sizeof(double) * NX));
-    H->bytes += 2 * sizeof(double) * NX;
+    H->bytes += sizeof(double) * NX;
     return BDC_OK;
 }
 
-// x_t = x_{t-1} = the current normalised log iterate; nothing evaluated yet
+// x_t = the current normalised log iterate; nothing evaluated yet
 __global__ void __launch_bounds__(256) k_acc_init(int64_t nx, int n, int row0, const double* __restrict__ Lt,
-                                                  double* __restrict__ xa, double* __restrict__ xb, DevState* st,
+                                                  double* __restrict__ xa, DevState* st,
                                                   double gap_nats) {
     const double lnz = st->log_z;
     const int n2 = n >> 1;
@@ -2401,9 +2444,7 @@ __global__ void __launch_bounds__(256) k_acc_init(int64_t nx, int n, int row0, c
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nx; i += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t xd = (uint32_t)i;
         if (!dense_is_rep((xd >> n2) + (uint32_t)row0, xd & mask, mask, (uint32_t)n & 1u)) continue;
-        const double l = Lt[xd] - lnz;
-        xa[xd] = l;
-        xb[xd] = l;
+        xa[xd] = Lt[xd] - lnz;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         st->ng_mode = -1;
@@ -2416,7 +2457,7 @@ bdc_status factored_acc_start(bdc_handle* H, double gap_bits) {
     bdc_status rc = factored_acc_buffers(H);
     if (rc != BDC_OK) return rc;
     FactoredState* F = H->fac;
-    k_acc_init<<<H->nb_upd, 256, 0, H->stream>>>((int64_t)F->H1h << H->s.n2, H->n, F->row0, F->Lt, F->snap0, F->snap1, H->d_st,
+    k_acc_init<<<H->nb_upd, 256, 0, H->stream>>>((int64_t)F->H1h << H->s.n2, H->n, F->row0, F->Lt, F->snap0, H->d_st,
                                                  gap_bits * 0.69314718055994530942);
     BDC_CUDA_TRY(cudaGetLastError());
     return BDC_OK;
