@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(256) k_mma_store(const GemmDesc* __restrict__ 
 // that the update runs a row at a time with 16-byte loads and stores of two
 // adjacent columns: on the fragments themselves every access touched twice
 // the sectors and the orbit tests and addresses were 2/3 of 210 instructions
-// an element.  84 -> 47 us at 24/12 (135 MB of device memory: 21 us).
+// an element.  84 -> 67 us at 24/12 (135 MB of device memory: 21 us).
 constexpr int g_stages(int bm, int bn, int, int) { return bm * bn <= 4096 ? 2 : 3; }
 template <int BM, int BN, int WM, int WN, bool WITH_D>
 __global__ void __launch_bounds__(256, (BM * BN <= 4096) ? 4 : 2) k_mma_ba(const GemmDesc* __restrict__ descs, const int* __restrict__ tiles,
@@ -754,7 +754,6 @@ static Operand op_f64(const double* p, int64_t ld, int trans) {
     Operand o;
     o.ptr = p;
     o.ld = ld;
-    o.kind = OP_F64;
     o.trans = trans;
     return o;
 }
@@ -776,10 +775,9 @@ static GemmDesc make_desc(Operand A, Operand B, double* C, int64_t ldc_m, int64_
 
 // the operand restricted to contraction indices >= k0
 static Operand k_offset(Operand o, bool is_a, int64_t k0) {
-    if (o.kind == OP_EYE || k0 == 0) return o;
+    if (k0 == 0) return o;
     const int64_t step = is_a ? (o.trans ? k0 * o.ld : k0) : (o.trans ? k0 : k0 * o.ld);
-    if (o.kind == OP_U16) o.ptr = (const uint16_t*)o.ptr + step;
-    else o.ptr = (const double*)o.ptr + step;
+    o.ptr = (const double*)o.ptr + step;
     return o;
 }
 
@@ -817,12 +815,11 @@ static void free_launch(Launch& L) {
 }
 
 // the cp.async layout of a list of products, or -1 when a product does not
-// qualify (an operand that is not FP64, an odd leading dimension or a base
-// that is not 16-byte aligned) or the layouts differ
+// qualify (an odd leading dimension or a base that is not 16-byte aligned) or
+// the layouts differ
 static int cp_layout(const std::vector<GemmDesc>& v) {
     int lay = -2;
     for (const auto& d : v) {
-        if (d.A.kind != OP_F64 || d.B.kind != OP_F64) return -1;
         if ((d.A.ld & 1) || (d.B.ld & 1)) return -1;
         if (((uintptr_t)d.A.ptr & 15) || ((uintptr_t)d.B.ptr & 15)) return -1;
         const int l = (d.A.trans ? 1 : 0) | (d.B.trans ? 0 : 2);
@@ -1098,11 +1095,15 @@ static BaEpilogue make_epilogue(bdc_handle* H);
 
 // ------------------------------------------------------- small problems
 // The direct iteration (bdc_direct.cuh) where the folded matrix has 16-bit
-// entries, at most 512 output representatives and kDirectBytes in all.
+// entries, at most 512 output representatives and kDirectBytes in all.  Its
+// time grows with the matrix, that of the products hardly: 18/10 (37 MB) 30 us
+// an iteration against 52, 22/5 (1,049,600 representatives) 76 against 61.5;
+// 21/5 (526,848) takes 23, 16/8 13, 17/9 17.
 constexpr int64_t kDirectBytes = 40ll << 20;
 constexpr int64_t kDirectReps = 600000;
-// one CTA runs a problem of up to this many passes over its rows (more
-// iterations per launch), more CTAs share a larger one
+// one CTA runs a problem of up to this many passes over its rows, many
+// iterations a launch (10/5: 3.8 us each); more CTAs share a larger one, one
+// iteration a launch
 constexpr int kDirectSoloPasses = 6;
 
 static int64_t orbit_count(int len) {  // orbits of {id, rev, comp, rev comp} on `len`-bit words
@@ -1461,7 +1462,7 @@ bdc_status factored_init(bdc_handle* H) {
         BDC_CUDA_TRY(e);
     }
 
-    // ---- the two thin products: U (KL x H2) = AL^T Pw, V (H1h x KR) = Pw BR
+    // ---- the two products of the q side: U (KL x H2) = AL^T Pw, V (H1h x KR) = Pw BR
     // Only the rows x_hi <= colmax[c] of a dense column c hold
     // representatives: U contracts each block of columns over those rows
     // only, V each block of rows over the columns that reach it.  The split

@@ -1,30 +1,19 @@
 // bdc_gemm.cuh -- FP64 tiled matrix products for the factored engine.
 //
-// C(m, n) = alpha * sum_k A(m, k) B(k, n) (+ C) on the CUDA cores in FP64
-// FMA (the tensor cores have no FP64 path on sm_100).  Operands are logical
-// matrices over device memory of three kinds: FP64, uint16 half-table
-// entries (exact small integers, widened on load) and the identity.  Element
-// (r, c) of an operand lives at ptr[r * ld + c] or, transposed, ptr[c * ld + r].
-//
-// Kernels:
-//   k_gemm_tile<128,128>  8x8 outputs per thread, used for the big products
-//   k_gemm_tile<64,64>    4x4 outputs per thread
-//   k_gemm_rows           few output rows (<= 8): one output column per
-//                         thread, B staged in shared memory
-// All launches are "grouped": one launch runs a list of products (GemmDesc)
-// and CTA i finds its product through a prefix table of tile counts.
+// C(m, n) = alpha * sum_k A(m, k) B(k, n) (+ C).  Element (r, c) of an operand
+// lives at ptr[r * ld + c] or, transposed, ptr[c * ld + r].  The kernels are in
+// bdc_mma.cuh (FP64 mma.sync tiles).  All launches are "grouped": one launch
+// runs a list of products (GemmDesc) and CTA i finds its product through a
+// prefix table of tile counts.
 #pragma once
 
 #include "bdc_common.cuh"
 
 namespace bdc {
 
-enum OpKind : int { OP_F64 = 0, OP_U16 = 1, OP_EYE = 2 };
-
 struct Operand {
     const void* ptr = nullptr;
     int64_t ld = 0;
-    int kind = OP_F64;
     int trans = 0;  // 0: (r,c) at ptr[r*ld+c]; 1: at ptr[c*ld+r]
 };
 

@@ -29,9 +29,7 @@ __device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double
 }
 
 __device__ __forceinline__ double opnd_load(const Operand& o, int64_t r, int64_t c) {
-    if (o.kind == OP_EYE) return r == c ? 1.0 : 0.0;
     const int64_t idx = o.trans ? c * o.ld + r : r * o.ld + c;
-    if (o.kind == OP_U16) return (double)__ldg((const uint16_t*)o.ptr + idx);
     return __ldg((const double*)o.ptr + idx);
 }
 
