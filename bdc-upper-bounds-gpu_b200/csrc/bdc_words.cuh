@@ -33,7 +33,7 @@
 // memory accesses per output instead of 12.
 //
 // Bound by the latency of the rounds (2-4 warps a scheduler, a block barrier
-// between rounds), not by a pipe.  At 24/12 q 29 us, fold 8.6, D 26 us; the
+// between rounds), not by a pipe.  At 24/12 q 25 us, fold 8.2, D 22 us; the
 // products per word length that this replaces took 46 + 19 + 50 us and let the
 // large products contract 190 words instead of 96: an iteration 312 -> 155 us
 // with the rest.  512 threads a CTA (22/11: 67 -> 77 us an iteration) and
