@@ -4,7 +4,7 @@
 // The driver copies pageable memory through one pinned buffer on the calling
 // thread: 33.6 MB (24/12) took 1.8 ms in and 6.8 ms out, the latter mostly the
 // first touch of the caller's fresh pages.  Here a few threads each take every
-// kThreads-th piece of 1 MB through two pinned buffers of their own, one being
+// kThreads-th piece of 128 KB through two pinned buffers of their own, one being
 // filled by the DMA engine while the other is copied, so that the copies and
 // the page faults run in parallel.  Small and pinned copies go as before.
 #include <algorithm>
@@ -17,7 +17,11 @@
 
 namespace bdc {
 
-constexpr size_t kPiece = 1 << 20;
+// A host-vector iteration at 24/12 (two copies of 33.6 MB), a handle's first,
+// which pins the buffers, and later ones: 10.7-11.1 ms through the driver; pieces
+// of 1 MB 10-17 and 3.1, 512 KB 8-14 and 3.8, 256 KB 8.4-11.4 and 4.6, 128 KB 6-9 and 5.5.
+// (the largest that leaves the first call no slower than the driver's copies)
+constexpr size_t kPiece = 128 << 10;
 constexpr size_t kStagedFrom = 4 << 20;  // below this the threads cost what they give (0.46 against 0.41 ms a step at 2.1 MB)
 constexpr int kThreads = 6;
 
@@ -29,6 +33,7 @@ struct Lane {
 };
 struct Staging {
     Lane lanes[kThreads];
+    char* pinned = nullptr;  // the lanes' buffers, one allocation
     bool ok = false;
 };
 
@@ -38,26 +43,27 @@ void host_copy_free(bdc_handle* H) {
     if (!S) return;
     for (Lane& l : S->lanes) {
         for (int i = 0; i < 2; ++i) {
-            if (l.buf[i]) cudaFreeHost(l.buf[i]);
             if (l.landed[i]) cudaEventDestroy(l.landed[i]);
         }
         if (l.stream) cudaStreamDestroy(l.stream);
     }
+    if (S->pinned) cudaFreeHost(S->pinned);
     delete S;
 }
 
-// the handle's buffers (12 MB pinned), or null when they cannot be had
+// the handle's buffers (1.5 MB pinned), or null when they cannot be had
 static Staging* staging(bdc_handle* H) {
     Staging* S = (Staging*)H->staging;
     if (S) return S->ok ? S : nullptr;
     S = new (std::nothrow) Staging();
     if (!S) return nullptr;
     H->staging = S;
-    cudaError_t e = cudaSuccess;
+    cudaError_t e = cudaMallocHost(&S->pinned, 2 * kThreads * kPiece);
+    char* at = S->pinned;
     for (Lane& l : S->lanes) {
-        for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
-            e = cudaMallocHost(&l.buf[i], kPiece);
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&l.landed[i], cudaEventDisableTiming);
+        for (int i = 0; i < 2 && e == cudaSuccess; ++i, at += kPiece) {
+            l.buf[i] = at;
+            e = cudaEventCreateWithFlags(&l.landed[i], cudaEventDisableTiming);
         }
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking);
     }
