@@ -1416,8 +1416,11 @@ bdc_status factored_init(bdc_handle* H) {
             S.word_stride = d == 0 ? H2 : 1;
             S.in = d == 0 ? F->ulpart : F->vrpart;
             S.slice_stride = (int64_t)S.leaves << S.words_log;
-            BDC_CUDA_TRY(cudaMalloc(&F->d_ns[d], (size_t)(S.leaves + 15) / 16));
-            BDC_CUDA_TRY(cudaMemsetAsync(F->d_ns[d], 0, (size_t)(S.leaves + 15) / 16, H->stream));
+            // (cleared by an upload like the ones that follow: a memset queued on
+            // the handle's stream could land after them)
+            const std::vector<uint8_t> none((size_t)(S.leaves + 15) / 16, 0);
+            BDC_CUDA_TRY(cudaMalloc(&F->d_ns[d], none.size()));
+            BDC_CUDA_TRY(upload(F->d_ns[d], none.data(), none.size()));
             S.ns = F->d_ns[d];
             cta += 1 << (S.words_log + S.t);
             F->words_smem = std::max(F->words_smem, word_smem(k, S.r));

@@ -1,0 +1,63 @@
+"""The host code of the library over a CUDA runtime without a device
+(fake_cudart.cpp): what a handle's set-up queues and copies, in which order,
+and what its calls do when an allocation or a kernel fails.  Each script runs
+in a process of its own with that runtime preloaded."""
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+from conftest import PKG, REPO
+
+HEAD = """
+import ctypes, os, sys
+sys.path.insert(0, {pkg!r})
+import numpy as np
+import bdc_b200 as bdc
+fake = ctypes.CDLL(None)
+fake.fake_faults.restype = ctypes.c_char_p
+fake.fake_fail_malloc.argtypes = [ctypes.c_size_t]
+fake.fake_copies.argtypes = [ctypes.c_int, ctypes.c_size_t]
+fake.fake_copies.restype = fake.fake_launches.restype = ctypes.c_long
+NO_LIMIT = 2 ** 64 - 1
+faults = lambda: fake.fake_faults().decode()
+"""
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fake") / "libfake.so")
+    inc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-w", f"-I{inc}", "-o", so,
+                    os.path.join(REPO, "tests", "fake_cudart.cpp")], check=True)
+
+    def run(script, **env):
+        e = {k: v for k, v in os.environ.items() if not k.startswith("BDC_")}
+        r = subprocess.run([sys.executable, "-c", HEAD.format(pkg=PKG) + textwrap.dedent(script)],
+                           env=dict(e, LD_PRELOAD=so, **env), capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stdout + r.stderr
+        return r.stdout
+
+    return run
+
+
+@pytest.mark.parametrize("n,k", [(12, 11), (14, 12), (20, 10), (21, 13)])
+@pytest.mark.parametrize("pinned", [False, True])
+def test_set_up_copies_are_ordered(fake, tmp_path, n, k, pinned):
+    """No set-up copy may land on a range that the handle's stream has still
+    to clear, with every tuning choice measured and with all of them pinned
+    (no measurement waits for the stream then)."""
+    tune = tmp_path / "tune.txt"
+    make = f"""
+        E = bdc.Engine({n}, {k}, engine="factored")
+        assert faults() == "", faults()
+        E.close()
+    """
+    fake(make, BDC_TUNE_FILE=str(tune))
+    if pinned:
+        lines = tune.read_text().splitlines()
+        assert {ln.split()[2] for ln in lines} >= {"u", "v", "g"}
+        fake(make, BDC_TUNE_FILE=str(tune))
+        assert tune.read_text().splitlines() == lines  # everything came from the file
