@@ -1892,9 +1892,21 @@ bool factored_has_passes(const bdc_handle* H) {
     return H->engine == BDC_ENGINE_FACTORED && !H->fac->direct && H->shard_world == 1;
 }
 
+// A device error that an earlier call returned stays with the handle until the
+// next load, and the passes' kernels leave at once while it is set, so a pass
+// would hand out what was there before.  Every call that can meet one copies
+// the state back, so the host's copy tells.
+static bdc_status refuse_after_error(const bdc_handle* H) {
+    if (H->h_st->error)
+        return fail(BDC_ERR_NUMERIC, "factored engine: device error %d of an earlier call", H->h_st->error);
+    return BDC_OK;
+}
+
 // ln q of the current iterate into H->d_lnq (0 in the slots that are no
-// representative's): the q side of an iteration, the state untouched
+// representative's): the q side of an iteration.  Of the state only `done` is
+// written (cleared, as the kernels skip their work while it is set).
 bdc_status factored_log_q(bdc_handle* H) {
+    if (bdc_status rs = refuse_after_error(H)) return rs;
     const size_t slots = (size_t)1 << (H->k >= 1 ? H->k - 1 : 0);
     BDC_CUDA_TRY(cudaMemsetAsync(&H->d_st->done, 0, sizeof(int), H->stream));
     BDC_CUDA_TRY(cudaMemsetAsync(H->d_lnq, 0, sizeof(double) * slots, H->stream));
@@ -1925,6 +1937,7 @@ static bdc_status eval_d(bdc_handle* H, double* D_out) {
 
 // D per representative for the ln q in H->d_lnq, into H->d_d
 bdc_status factored_divergence(bdc_handle* H) {
+    if (bdc_status rs = refuse_after_error(H)) return rs;
     FactoredState* F = H->fac;
     const int ny = 1 << H->k;
     BDC_CUDA_TRY(cudaMemsetAsync(&H->d_st->done, 0, sizeof(int), H->stream));

@@ -61,3 +61,32 @@ def test_set_up_copies_are_ordered(fake, tmp_path, n, k, pinned):
         assert {ln.split()[2] for ln in lines} >= {"u", "v", "g"}
         fake(make, BDC_TUNE_FILE=str(tune))
         assert tune.read_text().splitlines() == lines  # everything came from the file
+
+
+def test_passes_refuse_after_a_device_error(fake):
+    """An iteration that ends in a device error leaves no usable iterate: the
+    passes return that error too, until a distribution is loaded."""
+    fake("""
+        E = bdc.Engine(20, 10, engine="factored")
+        p = np.full(E.R, 0.5 ** 20)
+        lnq = np.zeros(bdc.num_q_slots(10))
+        passes = [E.log_q, E.log_w, lambda: E.log_w(lnq), E.divergence, lambda: E.divergence(lnq), E.rate,
+                  E.mi_forward, E.mi_backward]
+
+        def status(call):
+            try:
+                call()
+                return 0
+            except bdc.BDCError as e:
+                return e.status
+
+        for call in passes:
+            E.set_p(p)
+            fake.fake_fault_in(b"k_fac_finalize", 7)
+            numeric = status(lambda: E.iterate(1))
+            fake.fake_fault_in(b"", 0)
+            assert numeric != 0
+            assert status(call) == numeric
+        E.set_p(p)
+        assert [status(c) for c in passes] == [0] * len(passes)
+    """)
