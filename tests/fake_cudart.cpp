@@ -1,7 +1,7 @@
 // A CUDA runtime without a device, preloaded over libcudart so that the host
 // code of libbdc_b200.so runs where there is no GPU: device memory is host
 // memory, copies happen at once, kernels do nothing (the list of
-// representatives is written for them).  What the runtime or the device would
+// representatives is written for them, and an iteration's last kernel counts).  What the runtime or the device would
 // only show now and then is checked on each call instead: copies out of an
 // allocation's range, a copy on the legacy stream over work that a
 // non-blocking stream still has queued, launches without blocks or with more
@@ -45,7 +45,9 @@ struct World {
     std::map<const void*, std::string> kernels;
     std::map<const void*, int> smem_limit;
     std::map<const void*, std::pair<char*, size_t>> vars;
-    std::map<std::string, long> launches;
+    std::map<std::string, long> launches, grids;
+    std::map<void*, int> graphs;  // iterations that a captured graph holds
+    int iterations = 0;           // of the capture that is open or was last
     std::vector<Copy> copies;
     std::string faults;
     cudaStream_t capturing = nullptr;
@@ -108,6 +110,14 @@ bool named(const std::string& mangled, const char* name) {
     return mangled.find(std::to_string(strlen(name)) + name) != std::string::npos;
 }
 
+void advance(int iterations) {
+    for (auto& b : W().blocks)
+        if (b.second.device && b.second.bytes == sizeof(bdc::DevState)) {
+            ((bdc::DevState*)b.first)->iter += iterations;
+            b.second.written = true;
+        }
+}
+
 cudaError_t launch(const void* f, dim3 grid, void** args, size_t smem) {
     World& w = W();
     Lock l(w.mu);
@@ -118,7 +128,13 @@ cudaError_t launch(const void* f, dim3 grid, void** args, size_t smem) {
         return w.last = cudaErrorInvalidValue;
     }
     w.launches[name] += 1;
-    if (w.capturing) return cudaSuccess;
+    w.grids[name] = grid.x;
+    const bool last_of_iteration = named(name, "k_fac_finalize");
+    if (w.capturing) {
+        w.iterations += last_of_iteration;
+        return cudaSuccess;
+    }
+    if (last_of_iteration) advance(1);
     if (named(name, "k_rep_count")) {
         const int n = *(int*)args[0];
         w.reps.clear();
@@ -172,6 +188,12 @@ long fake_launches(const char* part) {
     for (auto& kv : W().launches)
         if (kv.first.find(part) != std::string::npos) t += kv.second;
     return t;
+}
+long fake_grid(const char* kernel) {  // blocks of the kernel's last launch
+    Lock l(W().mu);
+    for (auto& kv : W().grids)
+        if (named(kv.first, kernel)) return kv.second;
+    return 0;
 }
 long fake_copies(int kind, size_t from_bytes) {
     Lock l(W().mu);
@@ -273,20 +295,27 @@ cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
 }
 cudaError_t cudaStreamBeginCapture(cudaStream_t s, cudaStreamCaptureMode) {
     W().capturing = s;
+    W().iterations = 0;
     return cudaSuccess;
 }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
     W().capturing = nullptr;
     *g = (cudaGraph_t)handle();
+    W().graphs[*g] = W().iterations;
     return cudaSuccess;
 }
-cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) {
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t g, unsigned long long) {
     *e = (cudaGraphExec_t)handle();
+    W().graphs[*e] = W().graphs[g];
     return cudaSuccess;
 }
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t) {
+    Lock l(W().mu);
+    advance(W().graphs[e]);
+    return cudaSuccess;
+}
 
 // ---- device
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }

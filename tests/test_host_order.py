@@ -20,7 +20,7 @@ fake = ctypes.CDLL(None)
 fake.fake_faults.restype = ctypes.c_char_p
 fake.fake_fail_malloc.argtypes = [ctypes.c_size_t]
 fake.fake_copies.argtypes = [ctypes.c_int, ctypes.c_size_t]
-fake.fake_copies.restype = fake.fake_launches.restype = ctypes.c_long
+fake.fake_copies.restype = fake.fake_launches.restype = fake.fake_grid.restype = ctypes.c_long
 NO_LIMIT = 2 ** 64 - 1
 faults = lambda: fake.fake_faults().decode()
 """
@@ -89,4 +89,16 @@ def test_passes_refuse_after_a_device_error(fake):
             assert status(call) == numeric
         E.set_p(p)
         assert [status(c) for c in passes] == [0] * len(passes)
+    """)
+
+
+def test_every_pass_of_a_momentum_step_runs_over_the_grid(fake):
+    """A step whose extrapolated point leaves the exponential's range takes all
+    of it again: by as many blocks as the step's own pass."""
+    fake("""
+        E = bdc.Engine(20, 11, engine="factored")
+        E.set_p(np.full(E.R, 0.5 ** 20))
+        E.accelerate(12, 0.0)
+        assert fake.fake_grid(b"k_acc_extrap") > 100
+        assert fake.fake_grid(b"k_acc_setz") == fake.fake_grid(b"k_acc_extrap")
     """)
