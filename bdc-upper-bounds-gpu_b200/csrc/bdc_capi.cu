@@ -156,7 +156,7 @@ bdc_status bdc_set_p(bdc_handle_t H, const double* p, int64_t R) {
         return fail(BDC_ERR_ARG, "bdc_set_p: distribution has %lld entries, (n=%d) has %lld representatives",
                     (long long)R, H->n, (long long)H->R);
     BDC_CUDA_TRY(cudaSetDevice(H->device));
-    BDC_CUDA_TRY(host_copy(H, H->d_p[0], p, sizeof(double) * R, cudaMemcpyHostToDevice));
+    BDC_CUDA_TRY(cudaMemcpyAsync(H->d_p[0], p, sizeof(double) * R, cudaMemcpyHostToDevice, H->stream));
     return engine_after_set_p(H);
 }
 
@@ -186,7 +186,7 @@ bdc_status bdc_get_p(bdc_handle_t H, double* p, int64_t R) {
     const double* src = nullptr;
     bdc_status rc = engine_current_p(H, &src);
     if (rc != BDC_OK) return rc;
-    BDC_CUDA_TRY(host_copy(H, p, src, sizeof(double) * R, cudaMemcpyDeviceToHost));
+    BDC_CUDA_TRY(copy_to_host(H, p, src, sizeof(double) * R));
     return BDC_OK;
 }
 
@@ -299,7 +299,7 @@ bdc_status bdc_mi_backward(bdc_handle_t H, double* grad, int64_t R) {
     }
     if (rc != BDC_OK) return rc;
     BDC_CUDA_TRY(launch_mi_grad(H->n, H->d_reps, H->R, H->d_d, H->d_logw, H->stream));
-    BDC_CUDA_TRY(host_copy(H, grad, H->d_logw, sizeof(double) * R, cudaMemcpyDeviceToHost));
+    BDC_CUDA_TRY(copy_to_host(H, grad, H->d_logw, sizeof(double) * R));
     return BDC_OK;
 }
 
@@ -370,7 +370,7 @@ static bdc_status divergence_common(bdc_handle_t H, const double* lnq, int64_t R
         BDC_CUDA_TRY(launch_logw(H->n, H->d_reps, H->R, p, H->d_d, H->d_logw, H->stream));
         src = H->d_logw;
     }
-    BDC_CUDA_TRY(host_copy(H, out, src, sizeof(double) * R, cudaMemcpyDeviceToHost));
+    BDC_CUDA_TRY(copy_to_host(H, out, src, sizeof(double) * R));
     return BDC_OK;
 }
 

@@ -58,7 +58,7 @@ struct bdc_handle {
     bool p_set = false;
     bool strict_load = false;  // the last load kept exact zeros at ln p = -inf (engine_after_set_p)
     int64_t nonzero_pairs = 0;  // sum over reps of distinct length-k subsequences
-    void* staging = nullptr;  // pinned buffers of large pageable copies (bdc_hostcopy.cu), on first use
+    void* staging = nullptr;  // pinned buffers of large copies into fresh pages (bdc_hostcopy.cu), on first use
     // factored engine
     FactoredState* fac = nullptr;
     // scratch blocks of the certified solver, reused across its calls (bdc_solve.cu)
@@ -78,11 +78,10 @@ inline cudaError_t upload(void* dst, const void* src, size_t bytes) {
     return e != cudaSuccess ? e : cudaStreamSynchronize(cudaStreamLegacy);
 }
 
-// `bytes` between host memory and the device, ordered with the work queued on
-// H->stream; a copy to the host is complete on return.  Large copies from or
-// to pageable memory go through pinned buffers of the handle, several at a
-// time.
-cudaError_t host_copy(bdc_handle* H, void* dst, const void* src, size_t bytes, cudaMemcpyKind kind);
+// `bytes` from the device to host memory after the work queued on H->stream,
+// complete on return.  Large copies into fresh pageable memory go through
+// pinned buffers of the handle, several at a time.
+cudaError_t copy_to_host(bdc_handle* H, void* dst, const void* src, size_t bytes);
 void host_copy_free(bdc_handle* H);
 
 int select_engine(int requested, int n, int k);

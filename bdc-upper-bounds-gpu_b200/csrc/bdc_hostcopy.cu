@@ -1,28 +1,40 @@
-// bdc_hostcopy.cu -- vectors of representatives between pageable host memory
-// and the device.
+// bdc_hostcopy.cu -- vectors of representatives from the device into pageable
+// host memory.
 //
-// The driver copies pageable memory through one pinned buffer on the calling
-// thread: 33.6 MB (24/12) took 1.8 ms in and 6.8 ms out, the latter mostly the
-// first touch of the caller's fresh pages.  Here a few threads each take every
-// kThreads-th piece of 128 KB through two pinned buffers of their own, one being
-// filled by the DMA engine while the other is copied, so that the copies and
-// the page faults run in parallel.  Small and pinned copies go as before.
+// The driver copies into pageable memory through one pinned buffer on the
+// calling thread.  Where the caller's pages are resident that is the fastest
+// way; a large result buffer fresh from the allocator is not, and then the
+// copy is mostly its page faults.  For those a few threads each take every
+// n-th piece of 128 KB through two pinned buffers of their own, one being
+// filled by the DMA engine while the other is copied, so that the page faults
+// run in parallel.  Everything else goes the driver's way.
 #include <algorithm>
 #include <cstring>
 #include <exception>
 #include <new>
 #include <thread>
 
+#include <sched.h>
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include "bdc_engine.cuh"
 
 namespace bdc {
 
-// A host-vector iteration at 24/12 (two copies of 33.6 MB), a handle's first,
-// which pins the buffers, and later ones: 10.7-11.1 ms through the driver; pieces
-// of 1 MB 10-17 and 3.1, 512 KB 8-14 and 3.8, 256 KB 8.4-11.4 and 4.6, 128 KB 6-9 and 5.5.
-// (the largest that leaves the first call no slower than the driver's copies)
-constexpr size_t kPiece = 128 << 10;
-constexpr size_t kStagedFrom = 4 << 20;  // below this the threads cost what they give (0.46 against 0.41 ms a step at 2.1 MB)
+// Milliseconds of a copy to the host, the driver's way / by the threads (16
+// cores; 4.2, 8.4, 16.8, 33.6 and 67 MB):
+//   resident pages   0.27/0.34  0.47/0.64  0.88/1.3  1.7/2.5  3.4/4.9
+//   fresh pages       1.9/-      3.7/-      7.3/1.7  14.6/3.3  29/6.1
+//   from numpy.empty    -          -          -       7.4/2.8  13.7/5.5
+// A handle's first copy by the threads takes 1.2 to 2.2 ms longer (it pins the
+// buffers): fresh pages 3.8/2.5 at 16.8 MB, at 8.4 MB no gain, so the line lies
+// between.  With 4 of the cores 14.8/4.9 at 33.6 MB; with one the first copy
+// lost (6.7/7.5).  Copies to the device go the driver's way: 33.6 MB took the
+// threads 2.4, the driver 1.8 from a source in the CPU's caches and 3.2 else.
+constexpr size_t kStagedFrom = 16 << 20;
+constexpr int kMinCpus = 4;
+constexpr size_t kPiece = 128 << 10;  // larger pieces pin more: the first copy was slower than the driver's from 512 KB on
 constexpr int kThreads = 6;
 
 // one thread's buffers and stream
@@ -72,50 +84,58 @@ static Staging* staging(bdc_handle* H) {
     return S->ok ? S : nullptr;
 }
 
+// most of the pages of [p, p + bytes) have no memory behind them yet, by a
+// sample of them (16 us for 64 pages)
+static bool fresh_pages(const void* p, size_t bytes) {
+    constexpr int kSample = 64;
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    int fresh = 0;
+    for (int i = 0; i < kSample; ++i) {
+        unsigned char in = 1;
+        const uintptr_t at = ((uintptr_t)p + bytes / kSample * i) / page * page;
+        if (mincore((void*)at, page, &in) != 0) return false;
+        fresh += !(in & 1);
+    }
+    return fresh > kSample / 2;
+}
+
+static bool enough_cpus() {
+    cpu_set_t set;
+    CPU_ZERO(&set);
+    return sched_getaffinity(0, sizeof(set), &set) == 0 && CPU_COUNT(&set) >= kMinCpus;
+}
+
 // every kThreads-th piece from piece t on; returns with its copies complete
-static cudaError_t run_lane(int device, Lane& l, int t, char* dst, const char* src, size_t bytes, bool to_host) {
+static cudaError_t run_lane(int device, Lane& l, int t, char* dst, const char* src, size_t bytes) {
     cudaError_t e = cudaSetDevice(device);
     const size_t stride = kPiece * kThreads;
-    auto size = [&](size_t at) { return std::min(kPiece, bytes - at); };
+    auto queue = [&](int i, size_t at) {
+        const cudaError_t c =
+            cudaMemcpyAsync(l.buf[i], src + at, std::min(kPiece, bytes - at), cudaMemcpyDeviceToHost, l.stream);
+        return c != cudaSuccess ? c : cudaEventRecord(l.landed[i], l.stream);
+    };
     int i = 0;
-    bool ahead = false;  // (to the host) the current piece's copy is already queued
-    for (size_t at = kPiece * (size_t)t; at < bytes && e == cudaSuccess; at += stride, i ^= 1) {
-        if (to_host) {
-            if (!ahead) {
-                e = cudaMemcpyAsync(l.buf[i], src + at, size(at), cudaMemcpyDeviceToHost, l.stream);
-                if (e == cudaSuccess) e = cudaEventRecord(l.landed[i], l.stream);
-            }
-            const size_t next = at + stride;
-            ahead = next < bytes;
-            if (e == cudaSuccess && ahead) {
-                e = cudaMemcpyAsync(l.buf[i ^ 1], src + next, size(next), cudaMemcpyDeviceToHost, l.stream);
-                if (e == cudaSuccess) e = cudaEventRecord(l.landed[i ^ 1], l.stream);
-            }
-            if (e == cudaSuccess) e = cudaEventSynchronize(l.landed[i]);
-            if (e == cudaSuccess) memcpy(dst + at, l.buf[i], size(at));
-        } else {
-            e = cudaEventSynchronize(l.landed[i]);  // the buffer's last copy is done
-            if (e != cudaSuccess) break;
-            memcpy(l.buf[i], src + at, size(at));
-            e = cudaMemcpyAsync(dst + at, l.buf[i], size(at), cudaMemcpyHostToDevice, l.stream);
-            if (e == cudaSuccess) e = cudaEventRecord(l.landed[i], l.stream);
-        }
+    size_t at = kPiece * (size_t)t;
+    if (e == cudaSuccess && at < bytes) e = queue(i, at);
+    for (; at < bytes && e == cudaSuccess; at += stride, i ^= 1) {
+        if (at + stride < bytes) e = queue(i ^ 1, at + stride);
+        if (e == cudaSuccess) e = cudaEventSynchronize(l.landed[i]);
+        if (e == cudaSuccess) memcpy(dst + at, l.buf[i], std::min(kPiece, bytes - at));
     }
     const cudaError_t e2 = cudaStreamSynchronize(l.stream);
     return e != cudaSuccess ? e : e2;
 }
 
-cudaError_t host_copy(bdc_handle* H, void* dst, const void* src, size_t bytes, cudaMemcpyKind kind) {
-    const bool to_host = kind == cudaMemcpyDeviceToHost;
+cudaError_t copy_to_host(bdc_handle* H, void* dst, const void* src, size_t bytes) {
     Staging* S = nullptr;
     if (bytes >= kStagedFrom) {
         cudaPointerAttributes at{};
-        if (cudaPointerGetAttributes(&at, to_host ? dst : src) != cudaSuccess) (void)cudaGetLastError();
-        if (at.type == cudaMemoryTypeUnregistered) S = staging(H);
+        if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) (void)cudaGetLastError();
+        if (at.type == cudaMemoryTypeUnregistered && enough_cpus() && fresh_pages(dst, bytes)) S = staging(H);
     }
     if (!S) {
-        const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, H->stream);
-        return e != cudaSuccess || !to_host ? e : cudaStreamSynchronize(H->stream);
+        const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, H->stream);
+        return e != cudaSuccess ? e : cudaStreamSynchronize(H->stream);
     }
     // the lanes' streams do not follow H->stream: it must be idle
     cudaError_t e = cudaStreamSynchronize(H->stream);
@@ -127,14 +147,14 @@ cudaError_t host_copy(bdc_handle* H, void* dst, const void* src, size_t bytes, c
         for (; started + 1 < kThreads; ++started) {
             const int t = started + 1;
             threads[t] = std::thread([=, &got] {
-                got[t] = run_lane(H->device, S->lanes[t], t, (char*)dst, (const char*)src, bytes, to_host);
+                got[t] = run_lane(H->device, S->lanes[t], t, (char*)dst, (const char*)src, bytes);
             });
         }
     } catch (const std::exception&) {  // no more threads: this one takes the rest
     }
-    got[0] = run_lane(H->device, S->lanes[0], 0, (char*)dst, (const char*)src, bytes, to_host);
+    got[0] = run_lane(H->device, S->lanes[0], 0, (char*)dst, (const char*)src, bytes);
     for (int t = started + 1; t < kThreads; ++t)
-        got[t] = run_lane(H->device, S->lanes[t], t, (char*)dst, (const char*)src, bytes, to_host);
+        got[t] = run_lane(H->device, S->lanes[t], t, (char*)dst, (const char*)src, bytes);
     for (int t = 1; t <= started; ++t) threads[t].join();
     for (cudaError_t g : got)
         if (g != cudaSuccess) return g;

@@ -102,3 +102,33 @@ def test_every_pass_of_a_momentum_step_runs_over_the_grid(fake):
         assert fake.fake_grid(b"k_acc_extrap") > 100
         assert fake.fake_grid(b"k_acc_setz") == fake.fake_grid(b"k_acc_extrap")
     """)
+
+
+@pytest.mark.parametrize("cpus", [1, 4])
+def test_host_vectors_in_pieces_only_into_fresh_pages(fake, cpus):
+    """A vector goes in one copy in either direction, but for a large result
+    whose pages are not there yet, where several cores can share the faults."""
+    if len(os.sched_getaffinity(0)) < cpus:
+        pytest.skip("fewer cores here")
+    fake(f"""
+        import mmap
+        os.sched_setaffinity(0, sorted(os.sched_getaffinity(0))[:{cpus}])
+        f64p = ctypes.POINTER(ctypes.c_double)
+        L = bdc.library()
+        for n in (22, 24):
+            E = bdc.Engine(n, 3)
+            p = np.random.default_rng(n).random(E.R + 1)[1:]
+            fake.fake_clear()
+            E.set_p(p)
+            assert fake.fake_copies(1, 100000) == 1
+            maps = [mmap.mmap(-1, 8 * E.R + 4096, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS) for _ in range(2)]
+            used, fresh = [np.frombuffer(m, dtype=np.float64)[3:3 + E.R] for m in maps]
+            used[:] = 0.0
+            many = -(-8 * E.R // 131072) if n == 24 and {cpus} == 4 else 1
+            for out, pieces in ((used, 1), (fresh, many), (fresh, 1)):
+                fake.fake_clear()
+                assert L.bdc_get_p(E._h, out.ctypes.data_as(f64p), E.R) == 0
+                assert fake.fake_copies(2, 1000) == pieces
+                assert np.array_equal(out, p)
+            E.close()
+    """)

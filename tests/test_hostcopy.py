@@ -47,3 +47,24 @@ def test_handles_in_two_threads(bdc):
     for t in ts:
         t.join()
     assert res == {1: [True] * 5, 2: [True] * 5}
+
+
+@pytest.mark.gpu
+def test_fresh_and_resident_results(bdc):
+    """A result of 33.6 MB into pages that are not there yet, at an odd offset,
+    and into the same pages again."""
+    import ctypes
+    import mmap
+
+    import torch
+    with bdc.Engine(24, 3) as E:
+        E.set_p(np.random.default_rng(4).exponential(size=E.R) / (4.0 * E.R))
+        d = torch.empty(E.R, dtype=torch.float64, device="cuda")
+        E.get_p_device(d.data_ptr())
+        want = d.cpu().numpy()
+        m = mmap.mmap(-1, 8 * E.R + 4096, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+        out = np.frombuffer(m, dtype=np.float64)[3:3 + E.R]
+        for _ in range(2):
+            assert bdc.library().bdc_get_p(E._h, out.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), E.R) == 0
+            np.testing.assert_array_equal(out, want)
+            out[:] = 0.0
