@@ -967,7 +967,12 @@ static bdc_status tune_product(bdc_handle* H, TuneFile& tf, const char* key, Lau
     float best = 1e30f;
     int best_cfg = cfgs[0], best_s = 1;
     bool pinned = tf.get(key, &best_cfg, &best_s);
-    if (pinned && std::find(cfgs.begin(), cfgs.end(), best_cfg) == cfgs.end()) pinned = false;
+    // (the slices' buffers hold max_split of them)
+    if (pinned && (std::find(cfgs.begin(), cfgs.end(), best_cfg) == cfgs.end() || best_s < 1 || best_s > max_split)) {
+        pinned = false;
+        best_cfg = cfgs[0];
+        best_s = 1;
+    }
     for (int cfg : cfgs) {
         if (pinned) break;
         for (int S = 1; S <= max_split; S *= 2) {
@@ -1586,7 +1591,11 @@ bdc_status factored_init(bdc_handle* H) {
         ep.eta = 1.0;
         ep.row0 = F->row0;
         int unused = 0;
-        const bool pinned = tf.get("g", &best_cfg, &unused);
+        bool pinned = tf.get("g", &best_cfg, &unused);
+        if (pinned && std::find(cfgs, cfgs + 3, best_cfg) == cfgs + 3) {
+            pinned = false;
+            best_cfg = CFG_128x64;
+        }
         for (int c : cfgs) {
             if (pinned) break;
             Launch T;

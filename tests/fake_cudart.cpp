@@ -4,7 +4,8 @@
 // representatives is written for them, and an iteration's last kernel counts).  What the runtime or the device would
 // only show now and then is checked on each call instead: copies out of an
 // allocation's range, a copy on the legacy stream over work that a
-// non-blocking stream still has queued, launches without blocks or with more
+// non-blocking stream still has queued, products outside their operands and
+// results, launches without blocks or with more
 // shared memory than the kernel's limit.  A test can let allocations fail and
 // let a kernel leave an error code in the device state.
 #include <cstdint>
@@ -19,7 +20,9 @@
 #include <cuda_runtime_api.h>
 
 #define __ldg(p) (*(p))
-#include "../bdc-upper-bounds-gpu_b200/csrc/bdc_common.cuh"
+#include <cmath>
+using std::isfinite;
+#include "../bdc-upper-bounds-gpu_b200/csrc/bdc_gemm.cuh"
 
 namespace {
 
@@ -118,6 +121,27 @@ void advance(int iterations) {
         }
 }
 
+// what the tiles of a grouped product read and write
+void check_products(const bdc::GemmDesc* d, const int* map, unsigned tiles) {
+    in_range(map, sizeof(int) * tiles, "tile map");
+    for (unsigned t = 0; t < tiles; ++t) {
+        if (t > 0 && map[t] == map[t - 1]) continue;
+        const bdc::GemmDesc& e = d[map[t]];
+        in_range(&e, sizeof(e), "product descriptor");
+        auto operand = [&](const bdc::Operand& o, int64_t rows, int64_t cols, const char* what) {
+            if (rows < 1 || cols < 1) return;
+            const int64_t end = (o.trans ? (cols - 1) * o.ld + rows : (rows - 1) * o.ld + cols);
+            if (find(o.ptr) == W().blocks.end()) fault("out of range:", what);
+            in_range(o.ptr, 8 * end, what);
+        };
+        operand(e.A, e.M, e.K, "product operand A");
+        operand(e.B, e.K, e.N, "product operand B");
+        const int64_t end = (e.M - 1) * e.ldc_m + (e.N - 1) * e.ldc_n + 1;
+        if (e.K < 0 || find(e.C) == W().blocks.end()) fault("out of range:", "product result");
+        in_range(e.C, 8 * end, "product result");
+    }
+}
+
 cudaError_t launch(const void* f, dim3 grid, void** args, size_t smem) {
     World& w = W();
     Lock l(w.mu);
@@ -129,6 +153,7 @@ cudaError_t launch(const void* f, dim3 grid, void** args, size_t smem) {
     }
     w.launches[name] += 1;
     w.grids[name] = grid.x;
+    if (named(name, "k_mma_store")) check_products(*(const bdc::GemmDesc**)args[0], *(const int**)args[1], grid.x);
     const bool last_of_iteration = named(name, "k_fac_finalize");
     if (w.capturing) {
         w.iterations += last_of_iteration;

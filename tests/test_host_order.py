@@ -132,3 +132,18 @@ def test_host_vectors_in_pieces_only_into_fresh_pages(fake, cpus):
                 assert np.array_equal(out, p)
             E.close()
     """)
+
+
+@pytest.mark.parametrize("line", ["u 3 64", "v 7 64", "u 3 0", "v 7 -3", "u 0 1", "v 99 2", "g 0 0", "g 99 0"])
+def test_tuning_choices_outside_the_candidates_are_measured_anew(fake, tmp_path, line):
+    """A tune file of another build, or edited by hand, can name a split or a
+    tile shape that the set-up has no room or no kernel for."""
+    tune = tmp_path / "tune.txt"
+    tune.write_text("20 12 u 3 2\n20 12 v 7 2\n20 12 g 3 0\n20 12 oz 0 0\n20 12 " + line + "\n")
+    fake("""
+        E = bdc.Engine(20, 12, engine="factored")
+        E.set_p(np.full(E.R, 0.5 ** 20))
+        E.iterate(1)
+        E.close()
+        assert faults() == "", faults()
+    """, BDC_TUNE_FILE=str(tune))
