@@ -35,6 +35,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <initializer_list>
 #include <map>
 #include <string>
 #include <type_traits>
@@ -939,6 +940,10 @@ struct TuneFile {
         *b = it->second.second;
         return true;
     }
+    // whether every one of these choices is made already
+    bool has(std::initializer_list<const char*> keys) const {
+        return std::all_of(keys.begin(), keys.end(), [&](const char* key) { return m.count(key) != 0; });
+    }
     void put(const char* key, int a, int b) {
         if (path.empty()) return;
         m[key] = {a, b};
@@ -1453,7 +1458,7 @@ bdc_status factored_init(bdc_handle* H) {
     // the candidates below are compared by their times: on an idle GPU the
     // first ones would run at a lower clock and from cold instruction caches
     // (the choices at 22/11 and 23/11 then differed by 15 to 30 us a run)
-    if (tf.m.empty()) {
+    if (!tf.has({"u", "v", "g", "oz"})) {
         cudaEvent_t e0, e1;
         BDC_CUDA_TRY(cudaEventCreate(&e0));
         BDC_CUDA_TRY(cudaEventCreate(&e1));

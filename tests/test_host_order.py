@@ -147,3 +147,21 @@ def test_tuning_choices_outside_the_candidates_are_measured_anew(fake, tmp_path,
         E.close()
         assert faults() == "", faults()
     """, BDC_TUNE_FILE=str(tune))
+
+
+def test_warm_up_runs_when_a_choice_is_measured(fake, tmp_path):
+    """The GPU is brought up before any candidate is timed, also with a tune
+    file that holds only other keys or some of the choices; with all of them
+    pinned there is nothing to warm up for."""
+    def transforms(lines):
+        tune = tmp_path / "tune.txt"
+        tune.write_text("".join(f"20 12 {ln}\n" for ln in lines))
+        return int(fake("""
+            E = bdc.Engine(20, 12, engine="factored")
+            print(fake.fake_launches(b"k_words_q"))
+        """, BDC_TUNE_FILE=str(tune)))
+
+    u, v, rest = "u 3 2", "v 7 2", ["g 3 0", "oz 0 0"]
+    assert transforms([u, v] + rest) == 0
+    assert transforms(["ul 3 8", "qf 1 0"]) == transforms([])
+    assert transforms([u, v, rest[0]]) > 0
