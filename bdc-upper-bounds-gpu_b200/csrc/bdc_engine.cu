@@ -426,7 +426,8 @@ bdc_status engine_log_q(bdc_handle* H) {
 }
 
 bdc_status engine_divergence(bdc_handle* H) {
-    if (factored_has_passes(H)) return factored_divergence(H);
+    // (the count pass needs no buffer beside the handle's own)
+    if (factored_has_passes(H) && factored_dense_d(H)) return factored_divergence(H);
     const CountLaunch L = count_launch(H);
     BDC_CUDA_TRY(launch_dpass(L, H->d_lnq, H->d_h, H->inv_c, H->log_c, H->d_d, H->d_st, 0));
     return BDC_OK;

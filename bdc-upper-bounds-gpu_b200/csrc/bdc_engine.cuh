@@ -145,6 +145,7 @@ bdc_status factored_map(bdc_handle* H, const double* p_in, double* p_out, double
 bool factored_has_passes(const bdc_handle* H);
 bdc_status factored_log_q(bdc_handle* H);
 bdc_status factored_divergence(bdc_handle* H);
+bool factored_dense_d(bdc_handle* H);  // whether there is room for it
 bdc_status factored_evaluate(bdc_handle* H, double* D_out, double* rate);
 // Device buffers for dgemm_nt: one product descriptor and a tile map (every
 // tile on descriptor 0) of up to `tiles` 64x64 tiles, allocated once by the

@@ -1928,15 +1928,26 @@ bdc_status factored_log_q(bdc_handle* H) {
     return BDC_OK;
 }
 
+// D in dense order, allocated on first use; false where there is no memory for
+// it (a gigabyte at n = 28)
+bool factored_dense_d(bdc_handle* H) {
+    FactoredState* F = H->fac;
+    if (F->Ddense) return true;
+    const size_t bytes = sizeof(double) * (size_t)F->H1h * F->H2;
+    if (cudaMalloc(&F->Ddense, bytes) != cudaSuccess) {
+        (void)cudaGetLastError();
+        F->Ddense = nullptr;
+        return false;
+    }
+    H->bytes += bytes;
+    return true;
+}
+
 // the D side from lnq_full: G with an epilogue that leaves the state alone;
 // D per representative into D_out, or nowhere (nullptr)
 static bdc_status eval_d(bdc_handle* H, double* D_out) {
     FactoredState* F = H->fac;
-    if (D_out && !F->Ddense) {
-        const size_t bytes = sizeof(double) * (size_t)F->H1h * F->H2;
-        BDC_CUDA_TRY(cudaMalloc(&F->Ddense, bytes));
-        H->bytes += bytes;
-    }
+    if (D_out && !factored_dense_d(H)) return fail(BDC_ERR_CUDA, "no device memory for D in dense order");
     BDC_CUDA_TRY(launch_words(false, F, H->stream, H->d_st));
     BaEpilogue ep = make_epilogue(H);
     ep.Lt = nullptr;

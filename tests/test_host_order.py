@@ -21,7 +21,6 @@ fake.fake_faults.restype = ctypes.c_char_p
 fake.fake_fail_malloc.argtypes = [ctypes.c_size_t]
 fake.fake_copies.argtypes = [ctypes.c_int, ctypes.c_size_t]
 fake.fake_copies.restype = fake.fake_launches.restype = fake.fake_grid.restype = ctypes.c_long
-NO_LIMIT = 2 ** 64 - 1
 faults = lambda: fake.fake_faults().decode()
 """
 
@@ -165,3 +164,22 @@ def test_warm_up_runs_when_a_choice_is_measured(fake, tmp_path):
     assert transforms([u, v] + rest) == 0
     assert transforms(["ul 3 8", "qf 1 0"]) == transforms([])
     assert transforms([u, v, rest[0]]) > 0
+
+
+def test_divergence_needs_no_memory_of_its_own(fake):
+    """Where D in dense order cannot be had, the passes that go by it take the
+    count path, which needs no buffer beside the handle's."""
+    fake("""
+        E = bdc.Engine(20, 12, engine="factored")
+        E.set_p(np.full(E.R, 0.5 ** 20))
+        lnq = np.zeros(bdc.num_q_slots(12))
+        fake.fake_fail_malloc(8 << 19)
+        for call in (E.divergence, lambda: E.divergence(lnq), E.log_w, E.rate):
+            fake.fake_clear()
+            call()
+            assert fake.fake_launches(b"k_dpass") == 1 and fake.fake_launches(b"k_mma_ba") == 0
+        fake.fake_fail_malloc(ctypes.c_size_t(-1).value)
+        fake.fake_clear()
+        E.rate()
+        assert fake.fake_launches(b"k_dpass") == 0 and fake.fake_launches(b"k_mma_ba") == 1
+    """)
