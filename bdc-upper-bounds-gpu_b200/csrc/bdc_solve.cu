@@ -1502,7 +1502,7 @@ static cudaError_t rs_enqueue_step(bdc_handle* H, Restricted& rs, RsAA& aa, doub
 }
 
 // The cluster loop's buffers for a restricted problem; ctas = 0 when the rows
-// do not fit 16 CTAs or the device cannot place the cluster
+// do not fit 16 CTAs, the device cannot place the cluster or has no memory left
 struct RcLoop {
     DevBuf rows, members, yreps;
     RcPlan plan{};
@@ -1560,9 +1560,14 @@ struct RcLoop {
             P.ctas = 0;
             return BDC_OK;
         }
-        BDC_CUDA_TRY(dalloc(rows, sizeof(float) * (size_t)P.S * P.NYp));
-        BDC_CUDA_TRY(dalloc(members, sizeof(double) * P.NYp));
-        BDC_CUDA_TRY(dalloc(yreps, sizeof(uint32_t) * P.NY));
+        e = dalloc(rows, sizeof(float) * (size_t)P.S * P.NYp);
+        if (e == cudaSuccess) e = dalloc(members, sizeof(double) * P.NYp);
+        if (e == cudaSuccess) e = dalloc(yreps, sizeof(uint32_t) * P.NY);
+        if (e != cudaSuccess) {  // the launches need none of these
+            (void)cudaGetLastError();
+            P.ctas = 0;
+            return BDC_OK;
+        }
         BDC_CUDA_TRY(cudaStreamSynchronize(H->stream));  // (a pool block may still be read by queued work)
         BDC_CUDA_TRY(upload(members.p, mem.data(), sizeof(double) * P.NYp));
         BDC_CUDA_TRY(upload(yreps.p, yr.data(), sizeof(uint32_t) * P.NY));
