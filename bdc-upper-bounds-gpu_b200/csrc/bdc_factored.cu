@@ -1280,12 +1280,12 @@ bdc_status factored_init(bdc_handle* H) {
         BDC_CUDA_TRY(upload(F->d_rowstart, rs.data(), sizeof(int64_t) * rs.size()));
         BDC_CUDA_TRY(cudaMalloc(&F->rpart, sizeof(double) * 2 * (size_t)F->H1h));
         F->rows_smem = rows_smem_bytes(s.n2);
-        if (F->rows_smem > 48 * 1024) {
-            BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_load_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, F->rows_smem));
-            BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_rows<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, F->rows_smem));
-            BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_rows<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, F->rows_smem));
-            BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_rows<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, F->rows_smem));
-        }
+        // (a limit belongs to the process: the largest, n = 28, for every handle)
+        constexpr int rows_max = rows_smem_bytes(14);
+        BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_load_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_max));
+        BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_rows<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_max));
+        BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_rows<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_max));
+        BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_rows<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_max));
     }
     // words of length a of the high half, b of the low half
     const int k = H->k, wa = k / 2, wb = k - 1 - wa;

@@ -768,8 +768,9 @@ bdc_status ozaki_init(bdc_handle* H, const OzakiInput& in, OzakiG** out, const c
         *why = "tensor map encoding failed";
         return BDC_OK;
     }
-    BDC_CUDA_TRY(cudaFuncSetAttribute(k_oz_ba<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, oz->smem));
-    BDC_CUDA_TRY(cudaFuncSetAttribute(k_oz_ba<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, oz->smem));
+    // (a limit belongs to the process: the most that any handle's choice above can take)
+    BDC_CUDA_TRY(cudaFuncSetAttribute(k_oz_ba<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_smem - 2048));
+    BDC_CUDA_TRY(cudaFuncSetAttribute(k_oz_ba<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_smem - 2048));
     *out = oz;
     return BDC_OK;
 }

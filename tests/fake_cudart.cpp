@@ -163,9 +163,13 @@ cudaError_t launch(const void* f, dim3 grid, void** args, size_t smem) {
     if (named(name, "k_rep_count")) {
         const int n = *(int*)args[0];
         w.reps.clear();
-        for (uint32_t x = 0; x < (1u << (n - 1)); ++x)  // a representative's top bit is 0
-            if (bdc::is_rep(x, n)) w.reps.push_back(x);
-        if (n == 1) w.reps.assign(1, 0);
+        for (uint32_t x = 0; x < (1u << (n - 1)); ++x) {  // a representative's top bit is 0
+            uint32_t r = __builtin_bswap32(x);
+            r = (r & 0x0F0F0F0Fu) << 4 | (r >> 4 & 0x0F0F0F0Fu);
+            r = (r & 0x33333333u) << 2 | (r >> 2 & 0x33333333u);
+            r = ((r & 0x55555555u) << 1 | (r >> 1 & 0x55555555u)) >> (32 - n);
+            if (x <= r && x <= (r ^ bdc::low_mask(n))) w.reps.push_back(x);
+        }
     } else if (named(name, "k_rep_scan")) {
         **(int64_t**)args[2] = (int64_t)w.reps.size();
     } else if (named(name, "k_rep_write")) {

@@ -183,3 +183,18 @@ def test_divergence_needs_no_memory_of_its_own(fake):
         E.rate()
         assert fake.fake_launches(b"k_dpass") == 0 and fake.fake_launches(b"k_mma_ba") == 1
     """)
+
+
+@pytest.mark.parametrize("first,second,env", [((28, 2), (26, 2), {}), ((18, 14), (20, 11), {"BDC_G_KERNEL": "ozaki"})])
+def test_a_later_handle_leaves_the_shared_memory_limits(fake, first, second, env):
+    """A kernel's limit belongs to the process: a handle that needs less must
+    not take it from one that needs more."""
+    fake(f"""
+        A = bdc.Engine{first}
+        B = bdc.Engine{second}
+        for E in (A, B):
+            E.set_uniform()
+            E.iterate(1)
+            E.divergence()
+        assert faults() == "", faults()
+    """, **env)
