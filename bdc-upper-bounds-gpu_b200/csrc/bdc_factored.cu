@@ -1222,7 +1222,6 @@ static bdc_status direct_init(bdc_handle* H) {
     BDC_CUDA_TRY(direct_kernel<false>(F->d_lpx, F->d_m, attr));
     BDC_CUDA_TRY(cudaStreamSynchronize(H->stream));
     cudaFree(d_y);
-    F->launches_per_iter = 1;
     if (H->verbose)
         printf("bdc: direct iteration: %d output representatives, %.1f MB, %d lanes a row, %d CTAs\n", P.NY,
                tb / 1048576.0, F->d_lpx, F->d_grid);
@@ -1775,8 +1774,6 @@ static cudaError_t enqueue_stage(bdc_handle* H, int stage, double a) {
     FactoredState* F = H->fac;
     cudaStream_t s = H->stream;
     cudaError_t e = cudaSuccess;
-    // (a direct iteration is timed as a whole)
-    if (F->direct) return stage == ST_G ? enqueue_direct(H, a, 1) : cudaSuccess;
     switch (stage) {
         case ST_QBIG: {
             // U and V are independent: V runs on a branch beside U
@@ -2611,9 +2608,45 @@ bdc_status factored_accelerate(bdc_handle* H, int64_t max_evals, double gap_bits
     return BDC_OK;
 }
 
+// a direct handle's iterations have no stages, and a chain of them reads the
+// folded matrix once each: the chain is timed as a whole
+static bdc_status direct_profile(bdc_handle* H, int iters, bdc_profile_t* out) {
+    FactoredState* F = H->fac;
+    cudaEvent_t ev[2];
+    for (auto& e : ev) BDC_CUDA_TRY(cudaEventCreate(&e));
+    const long long target = H->h_st->iter + iters;
+    double tot = 0.0;
+    while (H->h_st->iter < target) {
+        BDC_CUDA_TRY(cudaEventRecord(ev[0], H->stream));
+        BDC_CUDA_TRY(enqueue_iterations(H, -INFINITY, (int)(target - H->h_st->iter)));
+        BDC_CUDA_TRY(cudaEventRecord(ev[1], H->stream));
+        BDC_CUDA_TRY(cudaMemcpyAsync(H->h_st, H->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, H->stream));
+        BDC_CUDA_TRY(cudaStreamSynchronize(H->stream));
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, ev[0], ev[1]);
+        tot += ms;
+        if (!H->h_st->error) continue;
+        // an out-of-range shift interrupted the chain: finish that iteration
+        bdc_status rc = factored_recover(H, -INFINITY);
+        if (rc != BDC_OK) return rc;
+        BDC_CUDA_TRY(cudaMemcpyAsync(H->h_st, H->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, H->stream));
+        BDC_CUDA_TRY(cudaStreamSynchronize(H->stream));
+    }
+    for (auto& e : ev) cudaEventDestroy(e);
+    out->ms_q = out->ms_fold = out->ms_update = 0.0;
+    out->ms_iter = out->ms_d = out->ms_main = tot / iters;
+    out->work_main = 4.0 * (double)H->R * (double)F->dp.NY;
+    out->bytes_main = (double)H->R * (2.0 * (double)F->dp.NYp + 40.0);
+    out->launches = 1;
+    out->iters = iters;
+    out->main_kind = 3;
+    return BDC_OK;
+}
+
 bdc_status factored_profile(bdc_handle* H, int iters, bdc_profile_t* out) {
     FactoredState* F = H->fac;
     BDC_CUDA_TRY(cudaMemsetAsync(&H->d_st->done, 0, sizeof(int), H->stream));
+    if (F->direct) return direct_profile(H, iters, out);
     cudaEvent_t ev[ST_COUNT + 1];
     for (auto& e : ev) BDC_CUDA_TRY(cudaEventCreate(&e));
     double acc[ST_COUNT] = {0}, tot = 0;
@@ -2647,10 +2680,10 @@ bdc_status factored_profile(bdc_handle* H, int iters, bdc_profile_t* out) {
     out->ms_iter = tot / iters;
     out->ms_main = acc[ST_G] / iters;
     // algorithmic work of G: one K-long dot product per representative
-    out->work_main = 2.0 * (double)H->R * (double)(F->direct ? F->dp.NY : F->KL + F->KR);
+    out->work_main = 2.0 * (double)H->R * (double)(F->KL + F->KR);
     out->launches = F->launches_per_iter;
     out->iters = iters;
-    out->main_kind = F->direct ? 3 : F->use_oz ? 2 : 1;
+    out->main_kind = F->use_oz ? 2 : 1;
     out->bytes_main = 40.0 * (double)F->Rl;
     return BDC_OK;
 }

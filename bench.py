@@ -383,18 +383,27 @@ def ours_arm(args) -> None:
                     "work_per_launch": f"40 bytes per representative (read h, ln p, p; write ln p, p) x R = "
                                        f"{prof['bytes_main']:.4e} bytes",
                     "peak_source": f"MEASURED_PEAKS.json hbm_gbs ({peak_src})"}
+    elif prof["main_kind"] == 3:
+        # a whole iteration of a small problem: D, the update and the next q from
+        # one read of the folded count rows, on the FP64 units
+        achieved = prof["work_main"] / (prof["ms_main"] / 1e3)
+        roofline = {"bound": "fp64 multiply-add pipe",
+                    "kernel": "k_direct (D, the update and the next q from one read of the folded count rows)",
+                    "achieved": achieved / 1e12, "peak": 2 * dfma / 1e12, "unit": "TFLOP/s",
+                    "frac": achieved / (2 * dfma), "traffic": None,
+                    "work_per_launch": f"4*R*NY = {prof['work_main']:.4e} flops: two multiply-adds per "
+                                       f"representative and output orbit (R = {R})",
+                    "peak_source": "bdc_peak_probe FP64 fused multiply-add chains on all SMs, measured in this "
+                                   "run (2 flops per multiply-add)"}
     else:
         # the G stage: one k_mma_ba launch (FP64 mma.sync tiles, the BA update
         # fused in the epilogue); ms_main is its CUDA-event time per iteration
         achieved = prof["work_main"] / (prof["ms_main"] / 1e3)
         dmma = bdc_b200.peak_probe("dmma", local)
         roofline = {"bound": "tensor",
-                    "kernel": "k_direct (D, the update and the next q from one read of the folded count rows)"
-                              if prof["main_kind"] == 3 else
-                              "k_mma_ba (G = [A_L | N_R] [M_L ; B_R^T] on FP64 mma.sync, BA update in the epilogue)",
+                    "kernel": "k_mma_ba (G = [A_L | N_R] [M_L ; B_R^T] on FP64 mma.sync, BA update in the epilogue)",
                     "achieved": achieved / 1e12, "peak": 2 * dmma / 1e12, "unit": "TFLOP/s",
-                    "frac": achieved / (2 * dmma), "traffic": profile_traffic("k_direct" if prof["main_kind"] == 3 else "k_mma_ba",
-                                                                        args.n, args.k),
+                    "frac": achieved / (2 * dmma), "traffic": profile_traffic("k_mma_ba", args.n, args.k),
                     "work_per_launch": f"2*R*K = {prof['work_main']:.4e} flops: one K-long dot product per "
                                        f"representative (R = {R}, K = the words of one length per half); the "
                                        f"launch executes the tiles that hold representatives, 1.07x that",

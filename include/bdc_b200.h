@@ -281,12 +281,14 @@ typedef struct {
                            over the nonzero pairs (count) or FP64 flops (factored) */
     int launches;       /* kernel launches per iteration */
     int iters;          /* iterations averaged */
-    int main_kind;      /* the dominant kernel: 3 the direct iteration of a small problem (one
-                           launch, timed whole), 0 the count D pass, 1 G on the FP64
-                           tensor path (mma.sync), 2 G on the int8 tensor cores */
+    int main_kind;      /* the dominant kernel: 3 the direct iteration of a small problem (a
+                           chain of `iters`, timed whole: ms_iter = ms_d = ms_main), 0 the
+                           count D pass, 1 G on the FP64 tensor path (mma.sync), 2 G on the
+                           int8 tensor cores */
     double bytes_main;  /* its algorithmic device-memory bytes per launch: the
                            update's 40 bytes per representative (read h, ln p, p;
-                           write ln p, p) for G, 0 for the count D pass */
+                           write ln p, p) for G, those and the folded matrix's row of
+                           16-bit counts for the direct iteration, 0 for the count D pass */
 } bdc_profile_t;
 
 /* Runs `iters` iterations (a = -inf, so none stops early) with CUDA events

@@ -154,12 +154,14 @@ cudaError_t launch(const void* f, dim3 grid, void** args, size_t smem) {
     w.launches[name] += 1;
     w.grids[name] = grid.x;
     if (named(name, "k_mma_store")) check_products(*(const bdc::GemmDesc**)args[0], *(const int**)args[1], grid.x);
-    const bool last_of_iteration = named(name, "k_fac_finalize");
+    // the iterations that this launch ends: k_direct does what & 2 of one, or `iters` alone
+    int done = named(name, "k_fac_finalize");
+    if (named(name, "k_direct") && (*(int*)args[1] & 2)) done = name.find("Lb1E") != name.npos ? *(int*)args[3] : 1;
     if (w.capturing) {
-        w.iterations += last_of_iteration;
+        w.iterations += done;
         return cudaSuccess;
     }
-    if (last_of_iteration) advance(1);
+    if (done) advance(done);
     if (named(name, "k_rep_count")) {
         const int n = *(int*)args[0];
         w.reps.clear();

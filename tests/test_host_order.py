@@ -198,3 +198,22 @@ def test_a_later_handle_leaves_the_shared_memory_limits(fake, first, second, env
             E.divergence()
         assert faults() == "", faults()
     """, **env)
+
+
+@pytest.mark.parametrize("n,k,launches", [(10, 5, 1), (17, 9, 21)])
+def test_profile_of_a_direct_handle_times_a_chain(fake, n, k, launches):
+    """Twenty iterations of a small problem are one launch of one CTA, or one
+    each after a first one for q; the profile times those and counts both
+    passes over the folded matrix."""
+    fake(f"""
+        E = bdc.Engine({n}, {k}, engine="factored")
+        E.set_uniform()
+        fake.fake_clear()
+        d = E.profile(20)
+        assert fake.fake_launches(b"8k_direct") == {launches}
+        orbits = len(bdc.canonical_reps({k}))
+        assert d["work_main"] == 4.0 * E.R * orbits
+        assert d["bytes_main"] == E.R * (2.0 * (-(-orbits // 8) * 8) + 40.0)
+        assert d["main_kind"] == 3 and d["launches"] == 1 and d["iters"] == 20
+        assert d["ms_iter"] == d["ms_main"] == d["ms_d"] == 5.0 / 20
+    """)
