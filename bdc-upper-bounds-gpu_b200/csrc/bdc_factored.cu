@@ -1016,7 +1016,7 @@ static int block_slices(int S, int kb, int kfull) {
     return std::max(1, (int)(((int64_t)S * kb + kfull - 1) / kfull));
 }
 
-// the word transforms of both sides; a round has at most 2^{r-3} items, one per thread
+// the word transforms of both sides
 static cudaError_t launch_words(bool q_side, const FactoredState* F, cudaStream_t s, const DevState* st) {
     const int g = F->plan.ctas, sm = F->words_smem;
     if (F->words_threads == 256) {
@@ -1436,7 +1436,7 @@ bdc_status factored_init(bdc_handle* H) {
         }
         P.ctas = cta;
         P.parts_l = P.side[1].cta0;
-        F->words_threads = std::max(P.side[0].r, P.side[1].r) <= 11 ? 256 : 512;
+        F->words_threads = word_threads(std::max(P.side[0].r, P.side[1].r));
         BDC_CUDA_TRY(set_words_attrs());
         BDC_CUDA_TRY(cudaMalloc(&F->d_plan, sizeof(WordPlan)));
         BDC_CUDA_TRY(upload(F->d_plan, &P, sizeof(WordPlan)));

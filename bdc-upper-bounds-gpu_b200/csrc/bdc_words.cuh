@@ -56,7 +56,7 @@ struct WordTerm {
 struct WordSide {
     int words_log;      // a (or b): 2^words_log words
     int last0;          // 1: the strings carry a fixed last character 0 beside the leaf bits
-    int r, t;           // leaf bits: r in the tree, t leading ones fixed per CTA
+    int r, t;           // leaf bits: r >= 1 in the tree, t leading ones fixed per CTA
     int leaf0, leaves;  // leaves [leaf0, leaf0 + leaves) are held
     int cta0;           // first CTA of this side
     // N(w, v) / C(half length - |v|, words_log - |v|) for the words |v| <= words_log:
@@ -162,11 +162,31 @@ __host__ __device__ constexpr int word_buf(int k, int r) { return (1 << k) > (2 
 __host__ __device__ constexpr int word_smem(int k, int r) { return (int)sizeof(double) * (word_buf(k, r) + (2 << r)); }
 
 // characters per tree round, from the root: 4, 4, ..., then the rest
-__device__ __forceinline__ int word_round(int rem) { return rem < 4 ? rem : 4; }
+__host__ __device__ constexpr int word_round(int rem) { return rem < 4 ? rem : 4; }
+
+// threads of a transform CTA whose slices have r characters, and the most items
+// (nodes times tails) of a round: k_words_q takes one a thread.  From r = 9 on
+// that is 2^{r-3} or the 256 nodes after eight characters, whichever is more.
+__host__ __device__ constexpr int word_threads(int r) { return r <= 11 ? 256 : 512; }
+__host__ __device__ constexpr int word_items(int k, int r) {
+    int most = 0;
+    for (int i = 0; i < r; i += word_round(r - i)) {
+        const int rem = r - i, left = rem - word_round(rem), tails = (2 << (left < k ? left : k)) - 1;
+        most = (tails << i) > most ? (tails << i) : most;
+    }
+    return most;
+}
+constexpr bool word_items_fit() {
+    for (int k = 1; k <= 2 * kWordMaxHalf; ++k)
+        for (int r = 1; r <= 12; ++r)
+            if (word_items(k, r) > word_threads(r)) return false;
+    return true;
+}
+static_assert(word_items_fit(), "a round of the q side has more items than its CTA threads");
 
 // one round of the D side for one item: node u after i characters, tail at
-// heap index h; Lp, Lc: longest word of a parent / child node.  LN: the root
-// round, whose words of length k are ln q itself.
+// heap index h; Lp, Lc: longest word of a parent / child node.  In the root's
+// round the words of length k are ln q itself (times s0).
 template <int Q>
 __device__ __forceinline__ void word_expand_item(double* wsm, int src, int dst, int u, int h, int i, int Lp, int Lc, int k, const double* __restrict__ lnq,
                                                  double s0, bool root, bool leaf, double* __restrict__ out,
@@ -293,11 +313,6 @@ __global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan
     }
     // the tree over the r free characters
     double* out = S.out + (int64_t)w * S.word_stride;
-    if (r == 0) {
-        if (tid == 0 && first >= S.leaf0 && first < S.leaf0 + S.leaves)
-            out[(int64_t)(first - S.leaf0) * S.leaf_stride] = wsm[src + 1];
-        return;
-    }
     for (int i = 0; i < r;) {
         const int rem = r - i, q = word_round(rem);
         const int Lp = min(k, rem), Lc = min(k, rem - q);
@@ -364,8 +379,8 @@ __device__ __forceinline__ void word_contract_add(const double (&X)[32], double*
 
 // q side: the products' columns U_w (summed over their split slices) -> this
 // word's and slice's share of acc[y] = sum_x |O| e(x) N(x, y), one vector of
-// 2^k per CTA (the second side's with y reversed).  The items of a round
-// number at most T.
+// 2^k per CTA (the second side's with y reversed).  One item of a round a thread
+// (word_items).
 template <int T>
 __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan, double* __restrict__ parts,
                                                const DevState* st) {
@@ -442,10 +457,6 @@ __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan
     // the root is in the second buffer
     const double* root = wsm + second;
     double* c = wsm;
-    if (r == 0) {  // no round: the leaf is the root (src is the second buffer)
-        if (tid == 0) wsm[second + 1] = wsm[second];
-        __syncthreads();
-    }
     // the root's words up to length min(k, r).  The fixed last characters
     // p: a word z u takes N(p, u) t[z], up to `fixed` characters u
     const int fixed = S.last0 + t, tailc = (int)reverse_bits((uint32_t)beta, t) << S.last0;
