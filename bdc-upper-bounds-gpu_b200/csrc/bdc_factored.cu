@@ -56,11 +56,11 @@ constexpr int kErrShift = 1;  // DevState::error: exp shift out of range, re-sca
 
 // tile configurations of the FP64 tensor-core products (BM x BN, warps WM x WN)
 enum MmaConfig {
-    CFG_128x128 = 0, CFG_128x64, CFG_64x128, CFG_64x64, CFG_128x16, CFG_16x128, CFG_128x32, CFG_64x32, CFG_32x128,
-    CFG_32x64, CFG_COUNT
+    CFG_128x64 = 1, CFG_64x128, CFG_64x64, CFG_128x16, CFG_16x128, CFG_128x32, CFG_64x32, CFG_32x128,
+    CFG_32x64, CFG_COUNT  // (the numbers stand in tune files)
 };
-static const int kCfgBM[CFG_COUNT] = {128, 128, 64, 64, 128, 16, 128, 64, 32, 32};
-static const int kCfgBN[CFG_COUNT] = {128, 64, 128, 64, 16, 128, 32, 32, 128, 64};
+static const int kCfgBM[CFG_COUNT] = {0, 128, 64, 64, 128, 16, 128, 64, 32, 32};
+static const int kCfgBN[CFG_COUNT] = {0, 64, 128, 64, 16, 128, 32, 32, 128, 64};
 
 struct Launch {
     GemmDesc* d = nullptr;   // device descriptors
@@ -339,7 +339,6 @@ __global__ void __launch_bounds__(256, (BM * BN <= 4096) ? 4 : 2) k_mma_ba(const
     }
 }
 
-#define BDC_CFG_ARGS_128x128 128, 128, 2, 4
 #define BDC_CFG_ARGS_128x64 128, 64, 4, 2
 #define BDC_CFG_ARGS_64x128 64, 128, 2, 4
 #define BDC_CFG_ARGS_64x64 64, 64, 2, 4
@@ -361,7 +360,6 @@ static int cfg_smem(int cfg, int layout = -1) {
             default: return mma_smem_bytes<ARGS>();                                             \
         }
     switch (cfg) {
-        CASE_(CFG_128x128, BDC_CFG_ARGS_128x128)
         CASE_(CFG_128x64, BDC_CFG_ARGS_128x64)
         CASE_(CFG_64x128, BDC_CFG_ARGS_64x128)
         CASE_(CFG_64x64, BDC_CFG_ARGS_64x64)
@@ -398,7 +396,6 @@ static cudaError_t set_smem_attrs() {
     SET_K((k_mma_ba<ARGS, false>), (mma_cp_smem_bytes<ARGS, false, true, g_stages(ARGS)>()))                  \
     SET_K((k_mma_ba<ARGS, true>), (mma_cp_smem_bytes<ARGS, false, true, g_stages(ARGS)>()))
     SET_STORE(BDC_CFG_ARGS_64x64)
-    SET_STORE_CP(BDC_CFG_ARGS_128x128)
     SET_STORE_CP(BDC_CFG_ARGS_128x64)
     SET_STORE_CP(BDC_CFG_ARGS_64x128)
     SET_STORE_CP(BDC_CFG_ARGS_64x64)
@@ -434,7 +431,6 @@ static cudaError_t launch_store(const Launch& L, cudaStream_t s, const DevState*
         return cudaGetLastError();
     }
     switch (L.cfg) {
-        GO_(128x128)
         GO_(128x64)
         GO_(64x128)
         GO_(64x64)
