@@ -98,7 +98,7 @@ struct FactoredState {
     bdc::WordPlan* d_plan = nullptr;
     int words_smem = 0, words_threads = 256;
     void* d_wtab[2] = {};     // each side's weights, terms and their ranges
-    double* qparts = nullptr; // [plan.ctas][2^k]  shares of acc[y] per transform CTA
+    double* qparts = nullptr; // [plan.parts][2^k]  shares of acc[y] of the transforms' CTAs
     double* qacc = nullptr;   // [2^k]     a shard's sums
     int* d_mids = nullptr;    // the fold's middles, one per CTA
     int n_mids = 0;
@@ -1027,7 +1027,7 @@ static cudaError_t launch_words(bool q_side, const FactoredState* F, cudaStream_
 
 // the largest transform's shared memory (k = 14), for every handle
 static cudaError_t set_words_attrs() {
-    const int smem = word_smem(14, 12);
+    const int smem = word_smem(13, 12);
     cudaError_t e = cudaFuncSetAttribute(k_words_q<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_words_d<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_words_q<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -1428,15 +1428,17 @@ bdc_status factored_init(bdc_handle* H) {
             BDC_CUDA_TRY(upload(F->d_ns[d], none.data(), none.size()));
             S.ns = F->d_ns[d];
             cta += 1 << (S.words_log + S.t);
-            F->words_smem = std::max(F->words_smem, word_smem(k, S.r));
+            S.part0 = P.parts;
+            P.parts += word_parts(S, k);
+            if (d == 0) P.parts_l = P.parts;
+            F->words_smem = std::max(F->words_smem, word_smem(word_cap(S, k), S.r));
         }
         P.ctas = cta;
-        P.parts_l = P.side[1].cta0;
         F->words_threads = word_threads(std::max(P.side[0].r, P.side[1].r));
         BDC_CUDA_TRY(set_words_attrs());
         BDC_CUDA_TRY(cudaMalloc(&F->d_plan, sizeof(WordPlan)));
         BDC_CUDA_TRY(upload(F->d_plan, &P, sizeof(WordPlan)));
-        BDC_CUDA_TRY(al(&F->qparts, (size_t)cta << k));
+        BDC_CUDA_TRY(al(&F->qparts, (size_t)P.parts << k));
         BDC_CUDA_TRY(al(&F->qacc, (size_t)ny));
         const int mb = k - 2 * fold_edge(k);
         std::vector<int> mids;
@@ -1781,7 +1783,7 @@ static cudaError_t enqueue_stage(bdc_handle* H, int stage, double a) {
             return cudaStreamWaitEvent(s, F->ev_join, 0);
         }
         case ST_QSMALL: return launch_words(true, F, s, H->d_st);
-        case ST_FOLD: return launch_fold(H, F->qparts, F->plan.ctas, s);
+        case ST_FOLD: return launch_fold(H, F->qparts, F->plan.parts, s);
         case ST_DSMALL:
             if ((e = launch_words(false, F, s, H->d_st)) != cudaSuccess) return e;
             if (F->use_oz) return ozaki_prepare(F->oz, H->d_st, s);
@@ -1996,7 +1998,7 @@ bdc_status factored_shard_q(bdc_handle* H, double* acc) {
     BDC_CUDA_TRY(enqueue_stage(H, ST_QBIG, -INFINITY));
     BDC_CUDA_TRY(enqueue_stage(H, ST_QSMALL, -INFINITY));
     const int ny = 1 << H->k;
-    k_words_acc<<<(ny + 255) / 256, 256, 0, s>>>(F->qparts, F->plan.parts_l, F->plan.ctas, H->k, F->qacc);
+    k_words_acc<<<(ny + 255) / 256, 256, 0, s>>>(F->qparts, F->plan.parts_l, F->plan.parts, H->k, F->qacc);
     BDC_CUDA_TRY(cudaGetLastError());
     BDC_CUDA_TRY(cudaMemcpyAsync(acc, F->qacc, sizeof(double) * ny, cudaMemcpyDeviceToHost, s));
     BDC_CUDA_TRY(cudaStreamSynchronize(s));

@@ -59,6 +59,7 @@ struct WordSide {
     int r, t;           // leaf bits: r >= 1 in the tree, t leading ones fixed per CTA
     int leaf0, leaves;  // leaves [leaf0, leaf0 + leaves) are held
     int cta0;           // first CTA of this side
+    int part0;          // its first partial q vector (word_parts of them)
     // N(w, v) / C(half length - |v|, words_log - |v|) for the words |v| <= words_log:
     // dense by heap index, and the nonzero ones by length (terms of w: [first[w][j], first[w][j + 1]))
     const double* weight;        // [2^words_log][2^{words_log + 1}]
@@ -77,9 +78,33 @@ struct WordSide {
 struct WordPlan {
     WordSide side[2];
     int k;
-    int ctas;      // CTAs of both sides
-    int parts_l;   // partial q vectors of the first side (= side[1].cta0)
+    int ctas;           // CTAs of both sides
+    int parts_l, parts; // partial q vectors of the first side and of both
 };
+
+// An output word y = v z takes |v| <= words_log characters from this half and z
+// from the other, which has `reach` of them.  So v has at least word_least
+// characters, and the other half's words at most word_cap; for k above n / 2
+// that leaves few of the splits.
+__host__ __device__ __forceinline__ int word_reach(const WordSide& S) { return S.r + S.t + S.last0; }
+__host__ __device__ __forceinline__ int word_least(const WordSide& S, int k) {
+    return k > word_reach(S) ? k - word_reach(S) : 0;
+}
+__host__ __device__ __forceinline__ int word_cap(const WordSide& S, int k) {
+    return k - 1 < word_reach(S) ? k - 1 : word_reach(S);
+}
+// k = n - 1: v is all of w and z all of the other half, so a transform is a
+// permutation of ln q and its transpose one of U, and the side's shares of acc
+// are one vector.  The general steps, on 2^k coefficients a word, took 15/14 from
+// the 44 us an iteration of the products per word length to 90; 34 so (12/11: 34,
+// 37, 24; with least and cap alone 15/14 46).  Those two are what short halves
+// need elsewhere: 16/14 92 -> 59, 17/14 98 -> 62 (92 and 91 per word length).
+__host__ __device__ __forceinline__ bool word_whole(const WordSide& S, int k) {
+    return k - S.words_log == word_reach(S);
+}
+__host__ __device__ __forceinline__ int word_parts(const WordSide& S, int k) {
+    return word_whole(S, k) ? 1 : 1 << (S.t + S.words_log);
+}
 
 __device__ __forceinline__ int word_len(int h) { return 31 - __clz(h); }
 
@@ -156,10 +181,12 @@ struct WordContract<0> {
     static __device__ __forceinline__ void run(double (&X)[2], const double* in, int) { X[1] = in[0]; }
 };
 
-// shared memory of a transform CTA, in doubles: a buffer for the words shorter
-// than k or the 2^{r+1} coefficients of a tree level, and one for a level
-__host__ __device__ constexpr int word_buf(int k, int r) { return (1 << k) > (2 << r) ? (1 << k) : (2 << r); }
-__host__ __device__ constexpr int word_smem(int k, int r) { return (int)sizeof(double) * (word_buf(k, r) + (2 << r)); }
+// shared memory of a transform CTA, in doubles: a buffer for the words of up to
+// cap characters or the 2^{r+1} coefficients of a tree level, and one for a level
+__host__ __device__ constexpr int word_buf(int cap, int r) { return 2 << (cap > r ? cap : r); }
+__host__ __device__ constexpr int word_smem(int cap, int r) {
+    return (int)sizeof(double) * (word_buf(cap, r) + (2 << r));
+}
 
 // characters per tree round, from the root: 4, 4, ..., then the rest
 __host__ __device__ constexpr int word_round(int rem) { return rem < 4 ? rem : 4; }
@@ -222,19 +249,30 @@ __global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan
                                                const DevState* st) {
     if (st && (st->done || st->error)) return;
     extern __shared__ __align__(16) double wsm[];
-    const WordSide S = plan->side[(int)blockIdx.x >= plan->parts_l ? 1 : 0];
+    const int side = (int)blockIdx.x >= plan->side[1].cta0 ? 1 : 0;
+    const WordSide S = plan->side[side];
     const int k = plan->k, a = S.words_log, r = S.r, t = S.t, tid = threadIdx.x;
     const int id = (int)blockIdx.x - S.cta0;
     const int w = id >> t, beta = id & ((1 << t) - 1);
     const int first = beta << r;
     if (first + (1 << r) <= S.leaf0 || first >= S.leaf0 + S.leaves) return;  // no held leaf in this slice
+    double* out = S.out + (int64_t)w * S.word_stride;
+    if (word_whole(S, k)) {
+        const double* q = lnq + ((side ? (int)reverse_bits((uint32_t)w, a) : w) << (k - a));
+        for (int i = tid; i < (1 << r); i += T) {
+            const int at = first + i - S.leaf0;
+            if (at >= 0 && at < S.leaves)
+                out[(int64_t)at * S.leaf_stride] = __ldg(q + reverse_bits((uint32_t)(first + i), k - a));
+        }
+        return;
+    }
+    const int cap = word_cap(S, k);  // longest word that can still occur
     double* c = wsm;
-    double* other = wsm + word_buf(k, r);
+    double* other = wsm + word_buf(cap, r);
     const int nk = 1 << k;  // heap indices of the words shorter than k: [1, nk)
     // the last characters that are fixed in this CTA (the first of them highest)
     const int fixed = S.last0 + t;
     const int tailc = (int)reverse_bits((uint32_t)beta, t) << S.last0;
-    const int cap = min(k - 1, r + fixed);  // longest word that can still occur
     __shared__ WordAux aux;
     for (int e = tid; e < kWordTerms; e += T) aux.terms[e] = S.terms[w * kWordTerms + e];
     if (tid < kWordMaxHalf + 2) aux.first[tid] = S.first[w * (kWordMaxHalf + 2) + tid];
@@ -258,9 +296,8 @@ __global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan
     __syncthreads();
     const double s0 = aux.terms[0].weight;  // |v| = 0
     // ... else the terms of w, four tails z a thread at a time
-    for (int j = 1; j <= a; ++j) {
+    for (int j = max(1, k - cap); j <= a; ++j) {
         const int d = k - j, n = 1 << d;
-        if (d > cap) continue;
         const int e0 = aux.first[j], e1 = aux.first[j + 1];
         for (int z = tid; z < n; z += 4 * T) {
             double x[4] = {0.0, 0.0, 0.0, 0.0};
@@ -285,7 +322,7 @@ __global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan
     }
     __syncthreads();
     // (buffers as offsets: pointers that change roles would be generic ones)
-    const int second = word_buf(k, r);
+    const int second = word_buf(cap, r);
     int src = 0, dst = second;
     if (fixed > 0) {
         // consume the fixed last characters: c[z] <- sum_u N(p, u) c[z u] over
@@ -312,7 +349,6 @@ __global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan
         dst = 0;
     }
     // the tree over the r free characters
-    double* out = S.out + (int64_t)w * S.word_stride;
     for (int i = 0; i < r;) {
         const int rem = r - i, q = word_round(rem);
         const int Lp = min(k, rem), Lc = min(k, rem - q);
@@ -378,29 +414,45 @@ __device__ __forceinline__ void word_contract_add(const double (&X)[32], double*
 }
 
 // q side: the products' columns U_w (summed over their split slices) -> this
-// word's and slice's share of acc[y] = sum_x |O| e(x) N(x, y), one vector of
-// 2^k per CTA (the second side's with y reversed).  One item of a round a thread
+// word's and slice's share of acc[y] = sum_x |O| e(x) N(x, y), a vector of 2^k
+// (the second side's with y reversed).  One item of a round a thread
 // (word_items).
 template <int T>
 __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan, double* __restrict__ parts,
                                                const DevState* st) {
     if (st && (st->done || st->error)) return;
     extern __shared__ __align__(16) double wsm[];
-    const WordSide S = plan->side[(int)blockIdx.x >= plan->parts_l ? 1 : 0];
+    const int side = (int)blockIdx.x >= plan->side[1].cta0 ? 1 : 0;
+    const WordSide S = plan->side[side];
     const int k = plan->k, a = S.words_log, r = S.r, t = S.t, tid = threadIdx.x;
     const int id = (int)blockIdx.x - S.cta0;
     const int w = id >> t, beta = id & ((1 << t) - 1);
     const int first = beta << r;
-    double* part = parts + ((int64_t)blockIdx.x << k);
-    if (first + (1 << r) <= S.leaf0 || first >= S.leaf0 + S.leaves) {
-        for (int y = tid; y < (1 << k); y += T) part[y] = 0.0;
+    const int nk = 1 << k;
+    if (word_whole(S, k)) {
+        double* q = parts + ((int64_t)S.part0 << k) + ((side ? (int)reverse_bits((uint32_t)w, a) : w) << (k - a));
+        for (int i = tid; i < (1 << r); i += T) {
+            const int at = first + i - S.leaf0, n = at >= 0 && at < S.leaves ? (int)S.ns[at >> 4] : 0;
+            const double* p = S.in + (int64_t)w * S.leaves + at;
+            double x = 0.0;
+#pragma unroll 4
+            for (int s = 0; s < n; ++s) x += __ldg(p + s * S.slice_stride);
+            const int z = (int)reverse_bits((uint32_t)(first + i), k - a);
+            q[z] = x;
+            if (S.last0) q[z + 1] = 0.0;  // (the strings end in 0)
+        }
         return;
     }
-    const int nk = 1 << k;
+    double* part = parts + ((int64_t)(S.part0 + id) << k);
+    if (first + (1 << r) <= S.leaf0 || first >= S.leaf0 + S.leaves) {
+        for (int y = tid; y < nk; y += T) part[y] = 0.0;
+        return;
+    }
+    const int least = word_least(S, k), cap = word_cap(S, k);
     // the tree, deepest characters first; the rounds alternate between the
     // buffers so that the root ends in the second
     const int rounds = (r + 3) / 4;
-    const int second = word_buf(k, r);
+    const int second = word_buf(cap, r);
     int dst = (rounds & 1) ? second : 0, src = (rounds & 1) ? 0 : second;
     // the leaves first: the split slices added up, 4 leaves x 4 slices of a
     // thread in flight (a slice at a time, each added slice waited for L2)
@@ -482,16 +534,20 @@ __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan
         return x;
     };
     // (k - a >= 1, so the shortest words read begin at an even index)
-    for (int h = (1 << (k - a)) + 2 * tid; h < nk; h += 2 * T) *reinterpret_cast<double2*>(c + h) = after(h);
+    for (int h = (1 << (k - a)) + 2 * tid; h < (2 << cap); h += 2 * T) *reinterpret_cast<double2*>(c + h) = after(h);
     __syncthreads();
     // acc[v z] = sum over the splits of y into |v| <= a characters and the
     // rest; two adjacent y share v and their z are adjacent
     for (int y = 2 * tid; y < nk; y += 2 * T) {
-        const double2 z0 = after(nk + y);
-        double2 x = make_double2(wt[1] * z0.x, wt[1] * z0.y);
+        double2 x = make_double2(0.0, 0.0);
+        if (least == 0) {
+            const double2 z0 = after(nk + y);
+            x = make_double2(wt[1] * z0.x, wt[1] * z0.y);
+        }
 #pragma unroll
         for (int j = 1; j <= kWordMaxHalf; ++j) {
             if (j > a) break;
+            if (j < least) continue;
             const int d = k - j;
             const double w = wt[(1 << j) + (y >> d)];
             const double2 z = *reinterpret_cast<const double2*>(c + (1 << d) + (y & ((1 << d) - 1)));
