@@ -1035,13 +1035,16 @@ static cudaError_t set_words_attrs() {
     return e;
 }
 
-// N(x, y) for short words on the host
-static int word_occurrences(int x, int nx, int y, int ny) {
-    int d[kWordMaxHalf + 1] = {1};
-    for (int i = 0; i < nx; ++i)
-        for (int j = ny; j > 0; --j)
-            if (((y >> (ny - j)) & 1) == ((x >> (nx - 1 - i)) & 1)) d[j] += d[j - 1];
-    return d[ny];
+// N(w, v) of every word v in the `len` characters of w, by heap index
+static std::vector<int> word_occurrences(int w, int len) {
+    std::vector<int> occ((size_t)2 << len, 0);
+    occ[1] = 1;
+    for (int i = len - 1; i >= 0; --i) {  // the next character ends v or is skipped
+        const int b = (w >> i) & 1;
+        for (int j = len - i; j > 0; --j)
+            for (int v = b; v < (1 << j); v += 2) occ[(1 << j) + v] += occ[(1 << (j - 1)) + (v >> 1)];
+    }
+    return occ;
 }
 
 cudaError_t dgemm_scratch_alloc(DgemmScratch& sc, int max_tiles, cudaStream_t s) {
@@ -1393,11 +1396,12 @@ bdc_status factored_init(bdc_handle* H) {
             for (int w = 0; w < (1 << W); ++w) {
                 // (the second side's words are consumed from their last character)
                 const int path = d == 0 ? w : (int)reverse_bits((uint32_t)w, W);
+                const std::vector<int> in_path = word_occurrences(path, W);
                 int cnt = 0;
                 for (int j = 0; j <= W; ++j) {
                     first[(size_t)w * (kWordMaxHalf + 2) + j] = cnt;
                     for (int v = 0; v < (1 << j); ++v) {
-                        const int occ = word_occurrences(path, W, v, j);
+                        const int occ = in_path[(1 << j) + v];
                         if (!occ) continue;
                         const double c = (double)occ / (double)binom(half[d] - j, W - j);
                         wt[((size_t)w << (W + 1)) + (1 << j) + v] = c;
@@ -1454,8 +1458,10 @@ bdc_status factored_init(bdc_handle* H) {
 
     // the candidates below are compared by their times: on an idle GPU the
     // first ones would run at a lower clock and from cold instruction caches
-    // (the choices at 22/11 and 23/11 then differed by 15 to 30 us a run)
-    if (!tf.has({"u", "v", "g", "oz"})) {
+    // (the choices at 22/11 and 23/11 then differed by 15 to 30 us a run; up to
+    // n = 16 the products take 6 to 10 us by any of them, and 4 ms is a third of
+    // the set-up)
+    if (H->n > 16 && !tf.has({"u", "v", "g", "oz"})) {
         cudaEvent_t e0, e1;
         BDC_CUDA_TRY(cudaEventCreate(&e0));
         BDC_CUDA_TRY(cudaEventCreate(&e1));
