@@ -425,9 +425,13 @@ bdc_status engine_log_q(bdc_handle* H) {
     return BDC_OK;
 }
 
+constexpr int64_t kCountPairs = 20 << 20;
 bdc_status engine_divergence(bdc_handle* H) {
-    // (the count pass needs no buffer beside the handle's own)
-    if (factored_has_passes(H) && factored_dense_d(H)) return factored_divergence(H);
+    // the factored products where the pairs (x, y) are many (24/12: 36 ms on the
+    // count path, 0.2 here) and there is room for D in dense order.  Below about
+    // 2^24 pairs the count pass is faster, or as fast: 13/12 43 us against 52 for
+    // the call, 14/12 55 and 63, 22/1 484 and 557; 14/13 (2^25) 78 and 56.
+    if (factored_has_passes(H) && H->R << H->k > kCountPairs && factored_dense_d(H)) return factored_divergence(H);
     const CountLaunch L = count_launch(H);
     BDC_CUDA_TRY(launch_dpass(L, H->d_lnq, H->d_h, H->inv_c, H->log_c, H->d_d, H->d_st, 0));
     return BDC_OK;

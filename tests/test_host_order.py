@@ -217,3 +217,18 @@ def test_profile_of_a_direct_handle_times_a_chain(fake, n, k, launches):
         assert d["main_kind"] == 3 and d["launches"] == 1 and d["iters"] == 20
         assert d["ms_iter"] == d["ms_main"] == d["ms_d"] == 5.0 / 20
     """)
+
+
+@pytest.mark.parametrize("n,k,products", [(13, 12, 0), (14, 12, 0), (22, 1, 0), (14, 13, 1), (19, 9, 1)])
+def test_divergence_counts_few_pairs(fake, n, k, products):
+    """D of a small problem by the count pass, which is the faster one there,
+    also on handles with products."""
+    fake(f"""
+        E = bdc.Engine({n}, {k}, engine="factored")
+        E.set_uniform()
+        for call in (E.divergence, E.log_w, E.rate):
+            fake.fake_clear()
+            call()
+            assert fake.fake_launches(b"8k_mma_ba") == {products}
+            assert fake.fake_launches(b"7k_dpass") == {1 - products}
+    """)
