@@ -2211,10 +2211,11 @@ bdc_status factored_iterate(bdc_handle* H, int64_t max_iters, double a, bdc_stat
     BDC_CUDA_TRY(cudaMemsetAsync(&H->d_st->done, 0, sizeof(int), H->stream));
     const long long it0 = H->h_st->iter;
     long long target = it0 + max_iters;
-    // the host reads the state after a chunk: chunks grow from 8 (iterations
-    // past convergence cost their launches only), or start at the largest
-    // when no threshold can end the loop
-    int64_t chunk = a == -INFINITY ? 256 : 8;
+    // the host reads the state after a chunk.  With a threshold the chunks grow
+    // from 1, since iterations past the stop still cost their launches (4 us each:
+    // 22/1, which stops after one, 120 us from chunks of 8 on, 91 from 1); a direct
+    // handle's launches past it cost 1 us.  Without one nothing ends the loop early.
+    int64_t chunk = a == -INFINITY ? 256 : F->direct ? 8 : 1;
     for (int guard = 0; guard < 1000000; ++guard) {
         const long long done_iters = H->h_st->iter;
         const int64_t remaining = target - done_iters;

@@ -59,6 +59,7 @@ struct World {
     size_t fail_from = SIZE_MAX;
     std::string fault_kernel;
     int fault_code = 0;
+    long long stop_after = INT64_MAX;  // the iteration that meets the threshold
     std::vector<uint32_t> reps;
     cudaError_t last = cudaSuccess;
 };
@@ -116,7 +117,8 @@ bool named(const std::string& mangled, const char* name) {
 void advance(int iterations) {
     for (auto& b : W().blocks)
         if (b.second.device && b.second.bytes == sizeof(bdc::DevState)) {
-            ((bdc::DevState*)b.first)->iter += iterations;
+            auto* st = (bdc::DevState*)b.first;
+            for (int i = 0; i < iterations && !st->done; ++i) st->done = ++st->iter >= W().stop_after;
             b.second.written = true;
         }
 }
@@ -213,6 +215,7 @@ void fake_fault_in(const char* kernel, int code) {
     W().fault_kernel = kernel;
     W().fault_code = code;
 }
+void fake_stop_after(int iterations) { W().stop_after = iterations; }
 long fake_launches(const char* part) {
     Lock l(W().mu);
     long t = 0;

@@ -232,3 +232,16 @@ def test_divergence_counts_few_pairs(fake, n, k, products):
             assert fake.fake_launches(b"8k_mma_ba") == {products}
             assert fake.fake_launches(b"7k_dpass") == {1 - products}
     """)
+
+
+@pytest.mark.parametrize("stop,queued", [(1, 1), (2, 3), (3, 3), (5, 7)])
+def test_few_iterations_are_queued_past_a_threshold(fake, stop, queued):
+    fake(f"""
+        E = bdc.Engine(20, 12, engine="factored")
+        E.set_uniform()
+        fake.fake_clear()
+        fake.fake_stop_after({stop})
+        st = E.iterate(64, 1e-13)
+        assert st["iters"] == {stop} and st["converged"]
+        assert fake.fake_launches(b"14k_fac_finalize") == {queued}
+    """)
