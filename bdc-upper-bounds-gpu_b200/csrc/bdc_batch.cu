@@ -58,7 +58,9 @@ static bdc_status batch_capture(bdc_batch* B, double a) {
         e = cudaStreamWaitEvent(B->lanes[i], B->fork, 0);
         cudaStream_t keep = H->stream;
         H->stream = B->lanes[i];
+        factored_beside(H, (int)B->hs.size());
         if (e == cudaSuccess) e = engine_enqueue_iterations(H, a, kBatchIters);
+        factored_beside(H, 1);
         H->stream = keep;
         if (e == cudaSuccess) e = cudaEventRecord(B->joins[i], B->lanes[i]);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(B->origin, B->joins[i], 0);
@@ -94,7 +96,9 @@ static bdc_status batch_capture_acc(bdc_batch* B, double eta) {
         e = cudaStreamWaitEvent(B->lanes[i], B->fork, 0);
         cudaStream_t keep = H->stream;
         H->stream = B->lanes[i];
+        factored_beside(H, (int)B->hs.size());
         if (e == cudaSuccess) e = factored_enqueue_acc_steps(H, kAccBatchSteps, eta);
+        factored_beside(H, 1);
         H->stream = keep;
         if (e == cudaSuccess) e = cudaEventRecord(B->joins[i], B->lanes[i]);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(B->origin, B->joins[i], 0);

@@ -161,8 +161,14 @@ k_direct(DirectPlan P, int what, int slot, int iters, double a, double eta, doub
     const int64_t step = (int64_t)gridDim.x * kDirectWarps * XPW * U;
     const int64_t i0 = (((int64_t)blockIdx.x * kDirectWarps + warp) * XPW + grp) * U;
     // sums of q over shares [y] in v (this thread's y = tid) -> slnq
+    // (entries 2e, 2e + 1 of the pieces that the lanes of a group read together
+    // lie side by side: at their place in the row, 64 bytes apart, a read took 4
+    // or 8 passes)
     auto to_lnq = [&](double sum) {
-        if (tid < P.NYp) slnq[tid] = direct_lnq(sum, P.members[tid], P.inv_c, exp(-S.log_z));
+        const int m = (tid >> 3) / LPX, lane8 = (tid >> 3) % LPX, e = tid & 7;
+        if (tid < P.NYp)
+            slnq[((m * 4 + (e >> 1)) * LPX + lane8) * 2 + (e & 1)] =
+                direct_lnq(sum, P.members[tid], P.inv_c, exp(-S.log_z));
     };
     if (SOLO) {
         if (S.done || S.error) return;
@@ -227,6 +233,18 @@ k_direct(DirectPlan P, int what, int slot, int iters, double a, double eta, doub
                                      : make_uint4(0u, 0u, 0u, 0u);
                 }
         };
+        // the longest rows of the next step on their way to L1 (k = 9, 10; shorter
+        // ones lose more to the instructions than they gain)
+        auto touch_rows = [&](int64_t ib) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    const int pc = m * LPX + sub;
+                    if (ib + u < P.R && pc < pieces)
+                        asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const uint4*>(P.T + (ib + u) * P.NYp) + pc));
+                }
+        };
         auto fetch_rep = [&](int64_t ib) { nx = ib + ul < P.R ? __ldg(P.reps + ib + ul) : 0u; };
         auto fetch_state = [&](int64_t ib) {
             nxd = (nx & ~low_mask(P.n2)) | reverse_bits(nx & low_mask(P.n2), P.n2);
@@ -252,6 +270,7 @@ k_direct(DirectPlan P, int what, int slot, int iters, double a, double eta, doub
             const bool live = ib + ul < P.R;
             const double pw = live ? npw : 0.0, lt = nlt, hx = nhx;
             if (M == 1) fetch_rows(ib + step);
+            else if (LPX >= 8) touch_rows(ib + step);
             fetch_rep(ib + step);
             double wq = pw;
             if (do_d) {
@@ -262,7 +281,7 @@ k_direct(DirectPlan P, int what, int slot, int iters, double a, double eta, doub
                 for (int m = 0; m < M; ++m)
 #pragma unroll
                     for (int e2 = 0; e2 < 4; ++e2) {
-                        const double2 l = *reinterpret_cast<const double2*>(slnq + (m * LPX + sub) * 8 + 2 * e2);
+                        const double2 l = *reinterpret_cast<const double2*>(slnq + ((m * 4 + e2) * LPX + sub) * 2);
 #pragma unroll
                         for (int u = 0; u < U; ++u) {
                             const uint32_t p = e2 == 0 ? row[u][m].x : e2 == 1 ? row[u][m].y : e2 == 2 ? row[u][m].z : row[u][m].w;

@@ -136,6 +136,8 @@ double factored_acc_eta();
 bdc_status factored_acc_start(bdc_handle* H, double gap_bits);
 bdc_status factored_acc_buffers(bdc_handle* H);  // the loop's snapshot vectors (before any capture)
 cudaError_t factored_enqueue_acc_steps(bdc_handle* H, int steps, double eta);
+// what is queued next runs beside as many instances in all (1: alone)
+void factored_beside(bdc_handle* H, int instances);
 cudaError_t factored_enqueue_iterations(bdc_handle* H, double a, int iters);
 // finishes an iteration that stopped on an exp-shift overflow (on H->stream);
 // any other device error is returned as BDC_ERR_NUMERIC

@@ -105,8 +105,10 @@ struct FactoredState {
     double* lnq_full = nullptr;  // [2^k]
     // small problems: the iteration straight from the folded matrix (bdc_direct.cuh)
     bool direct = false;
+    bool products = false;    // the products are set up (beside the direct form: see kBesideBytes)
     bdc::DirectPlan dp{};
-    int d_lpx = 0, d_m = 1, d_grid = 0;
+    int d_lpx = 0, d_m = 1, d_grid = 0;  // d_grid: the most CTAs, which the slots have room for
+    int beside = 1;                      // instances that run at the same time (a batch)
     double* d_members = nullptr;
     double* epart = nullptr;  // [ctas][8]
     double* spart = nullptr;  // [kStatRows][8]
@@ -1139,13 +1141,44 @@ static cudaError_t direct_kernel(int lpx, int m, F&& f) {
     }
 }
 
-static cudaError_t launch_direct(bdc_handle* H, int what, int slot, int iters, double a) {
+// In a batch the direct iteration of a large problem loses to the products: its
+// time grows with the rows of all instances, which no longer fit beside one
+// another, that of the products hardly.  Handles above one of these sizes hold
+// both forms and a batch of more than kBesideDirect instances takes the
+// products.  Measured, ms of 48 accelerated steps, products per word length /
+// direct / products: 18/10 x 16 12.4 / 21.1 / 9.4, x 3 5.2 / 5.5 / 3.4, 21/5 x 4 6.3 /
+// 7.3 / 5.2, 20/3 x 16 12.3 / 14.2 / 9.5, 18/9 x 8 6.8 / 7.3 / 5.3; below them
+// 17/9 x 16 8.4 / 8.3 / 9.1, 16/8 x 16 8.2 / 4.8 / 7.0, 19/7 x 8 6.9 / 6.5 / 5.1.
+constexpr int64_t kBesideBytes = 12ll << 20, kBesideReps = 200000;
+constexpr int kBesideDirect = 2;
+
+static bool direct_holds_products(const bdc_handle* H) {
+    return H->R > kBesideReps || H->R * ((orbit_count(H->k) + 7) / 8 * 8) * 2 > kBesideBytes;
+}
+
+static bool runs_direct(const FactoredState* F) {
+    return F->direct && !(F->products && F->beside > kBesideDirect);
+}
+
+// The CTAs of a launch: alone as many as have a pass over rows to do, one an SM;
+// in a batch the instances share the SMs.  Instances that each take all of them
+// run one after the other, every one with the latency of a launch and all its
+// CTAs adding all shares: 64 iterations of 17/9 x 16 17.7 ms so, 9.0 shared.
+static int direct_grid(const bdc_handle* H) {
+    return std::max(1, std::min(H->fac->d_grid, H->num_sms / H->fac->beside));
+}
+
+void factored_beside(bdc_handle* H, int instances) {
+    if (H->fac) H->fac->beside = std::max(1, instances);
+}
+
+static cudaError_t launch_direct(bdc_handle* H, int grid, int what, int slot, int iters, double a) {
     FactoredState* F = H->fac;
     auto go = [&](auto* k, int smem) {
-        k<<<F->d_grid, kDirectThreads, smem, H->stream>>>(F->dp, what, slot, iters, a, F->eta, F->dout, H->d_st);
+        k<<<grid, kDirectThreads, smem, H->stream>>>(F->dp, what, slot, iters, a, F->eta, F->dout, H->d_st);
         return cudaGetLastError();
     };
-    return F->d_grid == 1 ? direct_kernel<true>(F->d_lpx, F->d_m, go) : direct_kernel<false>(F->d_lpx, F->d_m, go);
+    return grid == 1 ? direct_kernel<true>(F->d_lpx, F->d_m, go) : direct_kernel<false>(F->d_lpx, F->d_m, go);
 }
 
 // `iters` iterations from the current state: one launch with one CTA; else
@@ -1153,13 +1186,14 @@ static cudaError_t launch_direct(bdc_handle* H, int what, int slot, int iters, d
 static cudaError_t enqueue_direct(bdc_handle* H, double a, int iters) {
     FactoredState* F = H->fac;
     if (iters < 1) return cudaSuccess;
-    if (F->d_grid == 1) return launch_direct(H, kDirectQ | kDirectD, 0, iters, a);
-    cudaError_t e = launch_direct(H, kDirectQ, 0, 0, a);
+    const int grid = direct_grid(H);
+    if (grid == 1) return launch_direct(H, grid, kDirectQ | kDirectD, 0, iters, a);
+    cudaError_t e = launch_direct(H, grid, kDirectQ, 0, 0, a);
     // (iters > 0 in the kernel: the slot holds an update's statistics)
     for (int i = 0; i < iters && e == cudaSuccess; ++i)
-        e = launch_direct(H, i + 1 < iters ? kDirectQ | kDirectD : kDirectD, i & 1, i, a);
+        e = launch_direct(H, grid, i + 1 < iters ? kDirectQ | kDirectD : kDirectD, i & 1, i, a);
     if (e != cudaSuccess) return e;
-    k_direct_finish<<<1, 160, 0, H->stream>>>(F->dp.slot[iters & 1], F->d_grid, a, F->eta, H->d_st);
+    k_direct_finish<<<1, 160, 0, H->stream>>>(F->dp.slot[iters & 1], grid, a, F->eta, H->d_st);
     return cudaGetLastError();
 }
 
@@ -1221,6 +1255,7 @@ static bdc_status direct_init(bdc_handle* H) {
     BDC_CUDA_TRY(direct_kernel<false>(F->d_lpx, F->d_m, attr));
     BDC_CUDA_TRY(cudaStreamSynchronize(H->stream));
     cudaFree(d_y);
+    F->direct = true;
     if (H->verbose)
         printf("bdc: direct iteration: %d output representatives, %.1f MB, %d lanes a row, %d CTAs\n", P.NY,
                tb / 1048576.0, F->d_lpx, F->d_grid);
@@ -1303,8 +1338,8 @@ bdc_status factored_init(bdc_handle* H) {
     BDC_CUDA_TRY(al(&F->Pw, NX));
     BDC_CUDA_TRY(al(&F->Lt, NX));
     BDC_CUDA_TRY(al(&F->hx, NX));
-    if (direct_supports(H)) {
-        F->direct = true;
+    const bool direct = direct_supports(H);
+    if (direct && !direct_holds_products(H)) {
         BDC_CUDA_TRY(cudaMemsetAsync(F->hx, 0, sizeof(double) * NX, H->stream));
         BDC_CUDA_TRY(cudaMemsetAsync(F->Pw, 0, sizeof(double) * NX, H->stream));
         BDC_CUDA_TRY(cudaMemsetAsync(F->Lt, 0, sizeof(double) * NX, H->stream));
@@ -1709,7 +1744,8 @@ bdc_status factored_init(bdc_handle* H) {
     // slicing kernel on the int8 path); finalize
     F->launches_per_iter = (F->ul.n > 0) + (F->vr.n > 0) + 3 + 1 + 1 + (F->use_oz ? 1 : F->ctas_g > kStatMany ? 1 : 0);
     BDC_CUDA_TRY(cudaStreamSynchronize(H->stream));
-    return BDC_OK;
+    F->products = true;
+    return direct ? direct_init(H) : BDC_OK;
 }
 
 void factored_free(bdc_handle* H) {
@@ -1813,7 +1849,7 @@ static cudaError_t enqueue_stage(bdc_handle* H, int stage, double a) {
 }
 
 static cudaError_t enqueue_iterations(bdc_handle* H, double a, int iters) {
-    if (H->fac->direct) return enqueue_direct(H, a, iters);
+    if (runs_direct(H->fac)) return enqueue_direct(H, a, iters);
     for (int i = 0; i < iters; ++i) {
         for (int st = 0; st < ST_COUNT; ++st) {
             cudaError_t e = enqueue_stage(H, st, a);
