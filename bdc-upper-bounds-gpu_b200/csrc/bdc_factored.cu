@@ -96,7 +96,7 @@ struct FactoredState {
     // the word transforms (bdc_words.cuh)
     bdc::WordPlan plan;
     bdc::WordPlan* d_plan = nullptr;
-    int words_smem = 0, words_threads = 256;
+    int words_smem = 0, words_r = 0;  // words_r: characters of the longest slice
     void* d_wtab[2] = {};     // each side's weights, terms and their ranges
     double* qparts = nullptr; // [plan.parts][2^k]  shares of acc[y] of the transforms' CTAs
     double* qacc = nullptr;   // [2^k]     a shard's sums
@@ -1014,27 +1014,30 @@ static int block_slices(int S, int kb, int kfull) {
     return std::max(1, (int)(((int64_t)S * kb + kfull - 1) / kfull));
 }
 
+// f with the transforms' kernels for slices of up to r characters
+template <typename F>
+static cudaError_t words_kernels(int r, F&& f) {
+    if (word_threads(r) == 512) return f(k_words_q<512, 1>, k_words_d<512, 1>);
+    return word_ctas(r) == 3 ? f(k_words_q<256, 3>, k_words_d<256, 3>) : f(k_words_q<256, 1>, k_words_d<256, 1>);
+}
+
 // the word transforms of both sides
 static cudaError_t launch_words(bool q_side, const FactoredState* F, cudaStream_t s, const DevState* st) {
-    const int g = F->plan.ctas, sm = F->words_smem;
-    if (F->words_threads == 256) {
-        if (q_side) k_words_q<256><<<g, 256, sm, s>>>(F->d_plan, F->qparts, st);
-        else k_words_d<256><<<g, 256, sm, s>>>(F->d_plan, F->lnq_full, st);
-    } else {
-        if (q_side) k_words_q<512><<<g, 512, sm, s>>>(F->d_plan, F->qparts, st);
-        else k_words_d<512><<<g, 512, sm, s>>>(F->d_plan, F->lnq_full, st);
-    }
-    return cudaGetLastError();
+    const int g = F->plan.ctas, sm = F->words_smem, t = word_threads(F->words_r);
+    return words_kernels(F->words_r, [&](auto* q, auto* d) {
+        if (q_side) q<<<g, t, sm, s>>>(F->d_plan, F->qparts, st);
+        else d<<<g, t, sm, s>>>(F->d_plan, F->lnq_full, st);
+        return cudaGetLastError();
+    });
 }
 
 // the largest transform's shared memory (k = 14), for every handle
-static cudaError_t set_words_attrs() {
+static cudaError_t set_words_attrs(int r) {
     const int smem = word_smem(13, 12);
-    cudaError_t e = cudaFuncSetAttribute(k_words_q<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_words_d<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_words_q<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_words_d<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    return e;
+    return words_kernels(r, [&](auto* q, auto* d) {
+        const cudaError_t e = cudaFuncSetAttribute(q, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(d, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    });
 }
 
 // N(w, v) of every word v in the `len` characters of w, by heap index
@@ -1473,11 +1476,13 @@ bdc_status factored_init(bdc_handle* H) {
             F->words_smem = std::max(F->words_smem, word_smem(word_cap(S, k), S.r));
         }
         P.ctas = cta;
-        F->words_threads = word_threads(std::max(P.side[0].r, P.side[1].r));
-        BDC_CUDA_TRY(set_words_attrs());
+        F->words_r = std::max(P.side[0].r, P.side[1].r);
+        BDC_CUDA_TRY(set_words_attrs(F->words_r));
         BDC_CUDA_TRY(cudaMalloc(&F->d_plan, sizeof(WordPlan)));
         BDC_CUDA_TRY(upload(F->d_plan, &P, sizeof(WordPlan)));
         BDC_CUDA_TRY(al(&F->qparts, (size_t)P.parts << k));
+        // (what a CTA can have no share of stays 0: it is never written)
+        BDC_CUDA_TRY(cudaMemsetAsync(F->qparts, 0, sizeof(double) * ((size_t)P.parts << k), H->stream));
         BDC_CUDA_TRY(al(&F->qacc, (size_t)ny));
         const int mb = k - 2 * fold_edge(k);
         std::vector<int> mids;

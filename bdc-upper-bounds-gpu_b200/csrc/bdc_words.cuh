@@ -195,6 +195,11 @@ __host__ __device__ constexpr int word_round(int rem) { return rem < 4 ? rem : 4
 // (nodes times tails) of a round: k_words_q takes one a thread.  From r = 9 on
 // that is 2^{r-3} or the 256 nodes after eight characters, whichever is more.
 __host__ __device__ constexpr int word_threads(int r) { return r <= 11 ? 256 : 512; }
+// CTAs an SM that the registers are kept to: three for short slices, which leave
+// room for them and meet in batches (48 accelerated steps of 13/11 x 64 23.9 ms with
+// two, 21.0 with three, 14/12 x 64 26.4 and 23.3); longer ones lose more to the
+// spilled registers (22/11 62.0 us an iteration with one, 64.7 with three)
+__host__ __device__ constexpr int word_ctas(int r) { return r <= 8 ? 3 : 1; }
 __host__ __device__ constexpr int word_items(int k, int r) {
     int most = 0;
     for (int i = 0; i < r; i += word_round(r - i)) {
@@ -244,8 +249,8 @@ __device__ __forceinline__ void word_expand_item(double* wsm, int src, int dst, 
 }
 
 // D side: ln q -> F_w over the strings of the other half
-template <int T>
-__global__ void __launch_bounds__(T) k_words_d(const WordPlan* __restrict__ plan, const double* __restrict__ lnq,
+template <int T, int CTAS>
+__global__ void __launch_bounds__(T, CTAS) k_words_d(const WordPlan* __restrict__ plan, const double* __restrict__ lnq,
                                                const DevState* st) {
     if (st && (st->done || st->error)) return;
     extern __shared__ __align__(16) double wsm[];
@@ -417,8 +422,8 @@ __device__ __forceinline__ void word_contract_add(const double (&X)[32], double*
 // word's and slice's share of acc[y] = sum_x |O| e(x) N(x, y), a vector of 2^k
 // (the second side's with y reversed).  One item of a round a thread
 // (word_items).
-template <int T>
-__global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan, double* __restrict__ parts,
+template <int T, int CTAS>
+__global__ void __launch_bounds__(T, CTAS) k_words_q(const WordPlan* __restrict__ plan, double* __restrict__ parts,
                                                const DevState* st) {
     if (st && (st->done || st->error)) return;
     extern __shared__ __align__(16) double wsm[];
@@ -444,10 +449,7 @@ __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan
         return;
     }
     double* part = parts + ((int64_t)(S.part0 + id) << k);
-    if (first + (1 << r) <= S.leaf0 || first >= S.leaf0 + S.leaves) {
-        for (int y = tid; y < nk; y += T) part[y] = 0.0;
-        return;
-    }
+    if (first + (1 << r) <= S.leaf0 || first >= S.leaf0 + S.leaves) return;
     const int least = word_least(S, k), cap = word_cap(S, k);
     // the tree, deepest characters first; the rounds alternate between the
     // buffers so that the root ends in the second
@@ -539,6 +541,8 @@ __global__ void __launch_bounds__(T) k_words_q(const WordPlan* __restrict__ plan
     // acc[v z] = sum over the splits of y into |v| <= a characters and the
     // rest; two adjacent y share v and their z are adjacent
     for (int y = 2 * tid; y < nk; y += 2 * T) {
+        // (y begins with the `least` characters that come from w at least)
+        if (least > 0 && wt[(1 << least) + (y >> (k - least))] == 0.0) continue;
         double2 x = make_double2(0.0, 0.0);
         if (least == 0) {
             const double2 z0 = after(nk + y);
