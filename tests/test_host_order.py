@@ -245,3 +245,22 @@ def test_few_iterations_are_queued_past_a_threshold(fake, stop, queued):
         assert st["iters"] == {stop} and st["converged"]
         assert fake.fake_launches(b"14k_fac_finalize") == {queued}
     """)
+
+
+@pytest.mark.parametrize("n,k,count,products,grid", [(14, 7, 4, 0, 9), (17, 9, 64, 0, 2), (18, 9, 2, 0, 74),
+                                                     (18, 9, 3, 1, 0), (21, 2, 4, 1, 0), (20, 10, 2, 1, 0)])
+def test_forms_in_a_batch(fake, n, k, count, products, grid):
+    """Direct instances of a batch take their share of 148 SMs; the larger ones
+    go by the products where more than two run together."""
+    fake(f"""
+        E = [bdc.Engine({n}, {k}, engine="factored") for _ in range({count})]
+        for e in E:
+            e.set_uniform()
+        B = bdc.Batch(E)
+        fake.fake_clear()
+        B.iterate(4000)  # (the fake device counts an iteration of one handle for all)
+        assert (fake.fake_launches(b"8k_mma_ba") >= 8 * {count}) == bool({products})
+        if not {products}:
+            assert fake.fake_launches(b"8k_mma_ba") == 0 and fake.fake_grid(b"k_direct") == {grid}
+        assert faults() == "", faults()
+    """)
