@@ -1110,9 +1110,9 @@ static BaEpilogue make_epilogue(bdc_handle* H);
 // ------------------------------------------------------- small problems
 // The direct iteration (bdc_direct.cuh) where the folded matrix has 16-bit
 // entries, at most 512 output representatives and kDirectBytes in all.  Its
-// time grows with the matrix, that of the products hardly: 18/10 (37 MB) 30 us
-// an iteration against 52, 22/5 (1,049,600 representatives) 76 against 61.5;
-// 21/5 (526,848) takes 23, 16/8 13, 17/9 17.
+// time grows with the matrix, that of the products hardly: 18/10 (37 MB) 28 us
+// an iteration against 45, 22/5 (1,049,600 representatives) 76 against 61.5;
+// 21/5 (526,848) takes 24 (42), 16/8 13, 17/9 16 (41).
 constexpr int64_t kDirectBytes = 40ll << 20;
 constexpr int64_t kDirectReps = 600000;
 // one CTA runs a problem of up to this many passes over its rows, many

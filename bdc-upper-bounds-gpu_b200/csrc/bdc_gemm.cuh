@@ -37,7 +37,7 @@ struct BaEpilogue {
     double* Lt;                  // log of the unnormalised iterate (in place)
     double* Pw;                  // |O(x)| * exp(Lt - shift) (in place)
     double inv_c;
-    double* part;                // per-CTA partials [ctas][4]
+    double* part;                // per-CTA partials [ctas][8]: max D, sum |O| e, max logW, sum |O| p D, zero flag
     const DevState* st;
     double* Dout;                // optional: D(x) at every representative (dense layout)
     double eta;                  // step of the exponentiated-gradient update: ln p' = ln p + eta D - ln Z
