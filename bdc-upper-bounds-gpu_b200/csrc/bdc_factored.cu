@@ -1152,6 +1152,8 @@ static cudaError_t direct_kernel(int lpx, int m, F&& f) {
 // direct / products: 18/10 x 16 12.4 / 21.1 / 9.4, x 3 5.2 / 5.5 / 3.4, 21/5 x 4 6.3 /
 // 7.3 / 5.2, 20/3 x 16 12.3 / 14.2 / 9.5, 18/9 x 8 6.8 / 7.3 / 5.3; below them
 // 17/9 x 16 8.4 / 8.3 / 9.1, 16/8 x 16 8.2 / 4.8 / 7.0, 19/7 x 8 6.9 / 6.5 / 5.1.
+// The second form costs 9 ms of set-up (18/10 7 and 16 ms; 38 with the products
+// per word length alone) and less memory than the folded matrix.
 constexpr int64_t kBesideBytes = 12ll << 20, kBesideReps = 200000;
 constexpr int kBesideDirect = 2;
 
@@ -1316,12 +1318,14 @@ bdc_status factored_init(bdc_handle* H) {
         BDC_CUDA_TRY(upload(F->d_rowstart, rs.data(), sizeof(int64_t) * rs.size()));
         BDC_CUDA_TRY(cudaMalloc(&F->rpart, sizeof(double) * 2 * (size_t)F->H1h));
         F->rows_smem = rows_smem_bytes(s.n2);
-        // (a limit belongs to the process: the largest, n = 28, for every handle)
-        constexpr int rows_max = rows_smem_bytes(14);
-        BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_load_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_max));
-        BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_rows<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_max));
-        BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_rows<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_max));
-        BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_rows<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_max));
+        // (a limit belongs to the process: the largest, n = 28, by every handle that needs one)
+        if (F->rows_smem > 48 * 1024) {
+            constexpr int rows_max = rows_smem_bytes(14);
+            BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_load_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_max));
+            BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_rows<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_max));
+            BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_rows<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_max));
+            BDC_CUDA_TRY(cudaFuncSetAttribute(k_fac_rows<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_max));
+        }
     }
     // words of length a of the high half, b of the low half
     const int k = H->k, wa = k / 2, wb = k - 1 - wa;
@@ -1500,8 +1504,8 @@ bdc_status factored_init(bdc_handle* H) {
     // first ones would run at a lower clock and from cold instruction caches
     // (the choices at 22/11 and 23/11 then differed by 15 to 30 us a run; up to
     // n = 16 the products take 6 to 10 us by any of them, and 4 ms is a third of
-    // the set-up)
-    if (H->n > 16 && !tf.has({"u", "v", "g", "oz"})) {
+    // the set-up, as where only a batch takes them)
+    if (H->n > 16 && !direct && !tf.has({"u", "v", "g", "oz"})) {
         cudaEvent_t e0, e1;
         BDC_CUDA_TRY(cudaEventCreate(&e0));
         BDC_CUDA_TRY(cudaEventCreate(&e1));
