@@ -962,11 +962,13 @@ struct TuneFile {
 // chooses tile shape (from cfgs) and split of U or V by timing run(candidate),
 // the product together with the transform that reads its slices; gen(cfg, S)
 // lists the descriptors of a candidate (S: the split of the longest
-// contraction, kfull its length), post(cfg, S) tells the transform its slices
+// contraction, kfull its length), post(cfg, S) tells the transform its slices.
+// preset: no timing; the first shape and the largest split, which the timing
+// finds for nearly every direct problem's products (G 64x64 for all of them)
 template <typename Gen, typename Post, typename Run>
 static bdc_status tune_product(bdc_handle* H, TuneFile& tf, const char* key, Launch& L, Gen&& gen, Post&& post, Run&& run,
                                const std::vector<int>& cfgs, int kfull, int max_split, int kmin, const char* what,
-                               int* split_out) {
+                               int* split_out, bool preset) {
     float best = 1e30f;
     int best_cfg = cfgs[0], best_s = 1;
     bool pinned = tf.get(key, &best_cfg, &best_s);
@@ -976,8 +978,10 @@ static bdc_status tune_product(bdc_handle* H, TuneFile& tf, const char* key, Lau
         best_cfg = cfgs[0];
         best_s = 1;
     }
+    if (preset && !pinned)
+        while (2 * best_s <= max_split && kfull / (2 * best_s) >= kmin) best_s *= 2;
     for (int cfg : cfgs) {
-        if (pinned) break;
+        if (pinned || preset) break;
         for (int S = 1; S <= max_split; S *= 2) {
             if (S > 1 && kfull / S < kmin) break;
             std::vector<GemmDesc> v = gen(cfg, S);
@@ -999,7 +1003,7 @@ static bdc_status tune_product(bdc_handle* H, TuneFile& tf, const char* key, Lau
             }
         }
     }
-    if (!pinned) tf.put(key, best_cfg, best_s);
+    if (!pinned && !preset) tf.put(key, best_cfg, best_s);
     BDC_CUDA_TRY(make_launch(L, gen(best_cfg, best_s), best_cfg));
     BDC_CUDA_TRY(post(best_cfg, best_s));
     *split_out = best_s;
@@ -1152,8 +1156,8 @@ static cudaError_t direct_kernel(int lpx, int m, F&& f) {
 // direct / products: 18/10 x 16 12.4 / 21.1 / 9.4, x 3 5.2 / 5.5 / 3.4, 21/5 x 4 6.3 /
 // 7.3 / 5.2, 20/3 x 16 12.3 / 14.2 / 9.5, 18/9 x 8 6.8 / 7.3 / 5.3; below them
 // 17/9 x 16 8.4 / 8.3 / 9.1, 16/8 x 16 8.2 / 4.8 / 7.0, 19/7 x 8 6.9 / 6.5 / 5.1.
-// The second form costs 9 ms of set-up (18/10 7 and 16 ms; 38 with the products
-// per word length alone) and less memory than the folded matrix.
+// The second form is set up without timing its choices (18/10 7 -> 9 ms; 38 with the
+// products per word length alone) and takes less memory than the folded matrix.
 constexpr int64_t kBesideBytes = 12ll << 20, kBesideReps = 200000;
 constexpr int kBesideDirect = 2;
 
@@ -1563,7 +1567,7 @@ bdc_status factored_init(bdc_handle* H) {
         bdc_status rc = tune_product(H, tf, "u", F->ul, gen, post, [&](const Launch& T) {
             const cudaError_t e = launch_store(T, H->stream, nullptr);
             return e != cudaSuccess ? e : launch_words(true, F, H->stream, nullptr);
-        }, cfgs, H1, max_split, 16, "U = AL^T Pw", &F->S1);
+        }, cfgs, H1, max_split, 16, "U = AL^T Pw", &F->S1, direct);
         if (rc != BDC_OK) return rc;
     }
     {
@@ -1615,7 +1619,7 @@ bdc_status factored_init(bdc_handle* H) {
             cudaError_t e = enqueue_stage(H, ST_QBIG, -INFINITY);
             F->vr = keep;
             return e != cudaSuccess ? e : launch_words(true, F, H->stream, nullptr);
-        }, cfgs, H2, max_split, 16, "V = Pw BR", &F->S2);
+        }, cfgs, H2, max_split, 16, "V = Pw BR", &F->S2, direct);
         if (rc != BDC_OK) return rc;
     }
 
@@ -1648,8 +1652,10 @@ bdc_status factored_init(bdc_handle* H) {
             pinned = false;
             best_cfg = CFG_128x64;
         }
+        const bool preset = direct && !pinned;
+        if (preset) best_cfg = CFG_64x64;
         for (int c : cfgs) {
-            if (pinned) break;
+            if (pinned || preset) break;
             Launch T;
             BDC_CUDA_TRY(make_tile_launch(T, d, c, F->colmax));
             cudaError_t e = cudaSuccess;
@@ -1661,7 +1667,7 @@ bdc_status factored_init(bdc_handle* H) {
             }
             free_launch(T);
         }
-        if (!pinned) tf.put("g", best_cfg, 0);
+        if (!pinned && !preset) tf.put("g", best_cfg, 0);
         tf.save();
         BDC_CUDA_TRY(make_tile_launch(F->g, d, best_cfg, F->colmax));
         F->ctas_g = F->g.tiles;
@@ -1669,7 +1675,7 @@ bdc_status factored_init(bdc_handle* H) {
             printf("bdc: tuned G: tile %dx%d, %d of %d tiles hold representatives, %d CTAs, %.1f us%s\n",
                    kCfgBM[best_cfg], kCfgBN[best_cfg], F->g.tiles,
                    ((H1 + kCfgBM[best_cfg] - 1) / kCfgBM[best_cfg]) * ((H2 + kCfgBN[best_cfg] - 1) / kCfgBN[best_cfg]),
-                   F->ctas_g, pinned ? 0.f : best * 1e3f, pinned ? " (pinned)" : "");
+                   F->ctas_g, pinned || preset ? 0.f : best * 1e3f, pinned ? " (pinned)" : preset ? " (preset)" : "");
         BDC_CUDA_TRY(cudaMemsetAsync(F->Pw, 0, sizeof(double) * NX, H->stream));
         BDC_CUDA_TRY(cudaMemsetAsync(F->Lt, 0, sizeof(double) * NX, H->stream));
         BDC_CUDA_TRY(cudaMemsetAsync(H->d_st, 0, sizeof(DevState), H->stream));
@@ -1686,7 +1692,7 @@ bdc_status factored_init(bdc_handle* H) {
         // warps); a forced int8 G ignores a pinned FP64 one
         const bool has_pick = tf.get("oz", &pick, &unused);
         const bool pinned = has_pick && !(force_oz && pick == 0);
-        if (!force_fp && !(pinned && pick == 0)) {
+        if (!force_fp && !(pinned && pick == 0) && (!direct || force_oz)) {
             // an entry of ML is ln q against nonnegative weights that add up to
             // sum_j C(a, j) C(n2, k - j) / C(n1 - j, a - j); NR the same from
             // the other side
